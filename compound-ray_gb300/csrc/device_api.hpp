@@ -75,6 +75,11 @@ struct DevEye {
   float4* cuts = nullptr;
   float cutRadius = 0.f;
   float maxRel = 0.f;
+  // cones: null, or P x N x kConeStride words receiving the cone lists of the
+  //       launch (render.cu, coneList): what the samples of an ommatidium can
+  //       hit first at a pose, found once for all of them.  Replaces the
+  //       cuts.  Results do not depend on it.
+  uint2* cones = nullptr;
   // netDraws: sample s of ommatidium o at pose p of the launch takes point s
   //       of a digitally shifted two-dimensional Sobol' net, the shift drawn
   //       from (drawSeed, (frame0 + p) * N + o) (render.cu, netDraw): no
@@ -89,6 +94,10 @@ struct DevEye {
 constexpr int kWideStackEntries = 128;
 constexpr int kCutEntries = 8;
 constexpr int kCutStride = 1 + 2 * kCutEntries;
+// A cone list: its count, then up to kConeEntries entries, 8 bytes each.
+constexpr int kConeEntries = 11;
+constexpr int kConeStride = 1 + kConeEntries;
+constexpr uint32_t kConeMinSamples = 32;
 
 // One pose = 4 x float4: position, local x axis, local y axis, local z axis
 // (w components unused).
@@ -156,9 +165,14 @@ size_t renderDrawBytes(uint32_t N, uint32_t spp, uint32_t P);
 // Floats of scratch needed by launchRender for P poses of the scene (0 when
 // spp <= 32 or when the chunk partials are summed inside the blocks), for a
 // recording (rec) or counting (stats) launch or neither; forceScratch: the
-// scratch plan (chunk partials in global memory, summed by a second kernel).
+// scratch plan (chunk partials in global memory, summed by a second kernel);
+// cones: the launch has cone lists (DevEye::cones).
 size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false,
-                           bool stats = false, bool forceScratch = false);
+                           bool stats = false, bool forceScratch = false, bool cones = false);
+
+// Cone lists (DevEye::cones, kConeStride words each) worth providing for a
+// P-pose launch: P x N, or 0 when the launch does not use them.
+size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false);
 
 cudaError_t launchRngInit(const DevEye& eye, uint32_t* errFlag, cudaStream_t stream);
 

@@ -53,6 +53,10 @@ size_t& devCap() {
   return cap;
 }
 
+// Gives back the buffers that only make renders faster (Renderer::cones);
+// true when there was one.  An allocation that fails tries again after it.
+bool releaseOptional();
+
 template <typename T>
 struct DevBuf {
   T* ptr = nullptr;
@@ -65,15 +69,36 @@ struct DevBuf {
     ptr = nullptr;
     count = 0;
   }
+  // ensure() for a buffer that only makes a render faster: false, and nothing
+  // held, when the memory is not to be had.
+  bool tryEnsure(size_t n) {
+    if (n <= count && ptr) return true;
+    release();
+    const size_t bytes = n * sizeof(T);
+    if (n == 0 || (devCap() && devHeld() + bytes > devCap())) return false;
+    if (cudaMalloc(reinterpret_cast<void**>(&ptr), bytes) != cudaSuccess) {
+      cudaGetLastError();
+      ptr = nullptr;
+      return false;
+    }
+    devHeld() += bytes;
+    count = n;
+    return true;
+  }
   void ensure(size_t n) {
     if (n <= count && ptr) return;
     release();
     if (n == 0) return;
     const size_t bytes = n * sizeof(T);
-    if (devCap() && devHeld() + bytes > devCap())
+    if (devCap() && devHeld() + bytes > devCap() && !(releaseOptional() && devHeld() + bytes <= devCap()))
       throw std::runtime_error("device memory cap reached: " + std::to_string(devHeld()) + " bytes held, " +
                                std::to_string(bytes) + " more requested, cap " + std::to_string(devCap()));
-    check(cudaMalloc(reinterpret_cast<void**>(&ptr), bytes), "cudaMalloc");
+    cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), bytes);
+    if (e != cudaSuccess && releaseOptional()) {
+      cudaGetLastError();
+      e = cudaMalloc(reinterpret_cast<void**>(&ptr), bytes);
+    }
+    check(e, "cudaMalloc");
     devHeld() += bytes;
     count = n;
   }
@@ -167,6 +192,7 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
 }
 
 constexpr uint32_t kMaxPosesPerLaunch = 256;
+constexpr size_t kConeListBytes = size_t(512) << 20;  // cone lists of one launch at most
 constexpr size_t kTuneSlots = 20;
 
 // Order in which warp segments take an eye's ommatidia: by the 30-bit Morton
@@ -245,6 +271,8 @@ struct Renderer {
   DevBuf<float> scratch;
   DevBuf<float2> draws;  // pre-drawn random numbers of small-eye launches
   DevBuf<float4> cuts;   // per-pose near-field cuts
+  DevBuf<uint2> cones;   // cone lists of a launch
+  bool conesOff = false; // crAutotune times the cut radii without cone lists
   float cutFactor = 0.f; // cut radius as a fraction of the scene extent (0: off)
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
   // samples per warp 8/16/32, cut radius 0, 1/256 .. 1/16 of the extent.
@@ -282,6 +310,7 @@ struct Renderer {
     poses.release();
     scratch.release();
     draws.release();
+    cones.release();
     batchOut.release();
     err.release();
     hostFrame.clear();
@@ -568,15 +597,14 @@ struct Renderer {
   void renderDevicePoses(EyeDev& e, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                          unsigned long long* stats = nullptr) {
     ensureRng(e);
-    for (size_t first = 0; first < count; first += kMaxPosesPerLaunch) {
-      const uint32_t P = static_cast<uint32_t>(std::min<size_t>(kMaxPosesPerLaunch, count - first));
-      const size_t need = renderScratchFloats(dev, e.N, e.spp, P, rec != nullptr, stats != nullptr);
-      if (need) scratch.ensure(need);
+    const size_t perLaunch = posesPerLaunch(e.N);
+    for (size_t first = 0; first < count; first += perLaunch) {
+      const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
       DevEye de = devEye(e);
       withDraws(de, P, !rec && !stats);
       withCuts(de, P, e.maxRel);
-      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * e.N, need ? scratch.ptr : nullptr,
-                         errWord(), rec, stream(), stats),
+      float* s = withCones(de, P, scratch, rec != nullptr, stats != nullptr);
+      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * e.N, s, errWord(), rec, stream(), stats),
             "render launch");
     }
   }
@@ -591,6 +619,33 @@ struct Renderer {
     de.cuts = cuts.ptr;
     de.cutRadius = cutFactor * dev.extent;
     de.maxRel = maxRel;
+  }
+
+  // Poses of one launch: at most kMaxPosesPerLaunch, and fewer for large eyes
+  // so that a launch's cone lists stay within kConeListBytes.
+  static size_t posesPerLaunch(uint32_t N) {
+    const size_t fit = kConeListBytes / (sizeof(uint2) * kConeStride * std::max<size_t>(1, N));
+    return std::min<size_t>(kMaxPosesPerLaunch, std::max<size_t>(1, fit));
+  }
+
+  // Cone lists for a P-pose launch that uses them, when the memory for them
+  // is to be had, and the launch's scratch (returned; null when it needs
+  // none).  No lists while the stream is being captured: the buffer may be
+  // given back before the captured graph runs.
+  float* withCones(DevEye& de, uint32_t P, DevBuf<float>& scr, bool rec, bool stats) {
+    de.cones = nullptr;
+    const size_t lists = conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec);
+    if (lists && lists * kConeStride * sizeof(uint2) <= kConeListBytes) {
+      cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+      check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
+      if (st == cudaStreamCaptureStatusNone && cones.tryEnsure(lists * kConeStride)) de.cones = cones.ptr;
+    }
+    for (;;) {
+      const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, de.cones != nullptr);
+      if (need) scr.ensure(need);
+      if (!de.cones || cones.ptr) return need ? scr.ptr : nullptr;
+      de.cones = nullptr;  // the scratch took their memory
+    }
   }
 
   // Gives a P-pose launch of a small eye a buffer for its pre-drawn random
@@ -649,6 +704,12 @@ struct Renderer {
 Renderer& R() {
   static Renderer r;
   return r;
+}
+
+bool releaseOptional() {
+  const bool had = R().cones.ptr != nullptr;
+  R().cones.release();
+  return had;
 }
 
 // A batch of eyes recorded as one CUDA graph (see crBatchCreate).
@@ -1651,7 +1712,10 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
           }
         }
         setRenderLayout(bestBlock, bestSeg);
-        // Near-field cut radius (fraction of the scene extent), with the best variant and layout.
+        // Near-field cut radius (fraction of the scene extent), with the best
+        // variant and layout, without cone lists: renders that use those
+        // ignore the radius, the others take the one timed here.
+        r.conesOff = true;
         const float factors[] = {0.f, 1.f / 256, 1.f / 128, 1.f / 64, 1.f / 32, 1.f / 16};
         float bestCut = 0.f, bestCutMs = INFINITY;
         for (int k = 0; k < 6; ++k) {
@@ -1682,7 +1746,9 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
           bestCut = refined;
           r.cutFactor = bestCut;
         }
-        // BVH width: the two-wide BVH with its best cut against the wide ones.
+        r.conesOff = false;
+        // BVH width: the two-wide BVH with its best cut (or the cone lists)
+        // against the wide ones.
         const int prevWidth = r.bvhWidth;
         int bestWidth = 2;
         float bestWidthMs = INFINITY;
@@ -2024,14 +2090,14 @@ int crDenoiserAddTrainingPoses(const float* poses12, size_t count, int featureSp
         EyeDev& e = denoiseEye(r, d);
         uploadPoses12(d.poses, poses12, count, r.stream());
         denoiseFeatures(r, d, e, d.poses.ptr, count, static_cast<uint32_t>(featureSpp));
-        const DevEye te = streamsFor(r, e, d.targetRng, d.targetSpp, d.targetReady, static_cast<uint32_t>(targetSpp));
+        DevEye te = streamsFor(r, e, d.targetRng, d.targetSpp, d.targetReady, static_cast<uint32_t>(targetSpp));
         d.out.ensure(std::max<size_t>(1, count * e.N * 3));
-        for (size_t first = 0; first < count; first += kMaxPosesPerLaunch) {
-          const uint32_t P = static_cast<uint32_t>(std::min<size_t>(kMaxPosesPerLaunch, count - first));
-          const size_t need = renderScratchFloats(r.dev, e.N, te.spp, P);
-          if (need) d.scratch.ensure(need);
-          check(launchRender(r.dev, te, d.poses.ptr + 4 * first, P, d.out.ptr + 3 * first * e.N,
-                             need ? d.scratch.ptr : nullptr, r.errWord(), nullptr, r.stream()),
+        const size_t perLaunch = Renderer::posesPerLaunch(e.N);
+        for (size_t first = 0; first < count; first += perLaunch) {
+          const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
+          float* scr = r.withCones(te, P, d.scratch, false, false);
+          check(launchRender(r.dev, te, d.poses.ptr + 4 * first, P, d.out.ptr + 3 * first * e.N, scr, r.errWord(),
+                             nullptr, r.stream()),
                 "target render");
         }
         d.net.addRows(d.X.ptr, d.base.ptr, d.out.ptr, count * e.N, r.stream());

@@ -126,8 +126,8 @@ __device__ __forceinline__ float rcpApprox(float d) {
   return r;
 }
 
-__device__ __forceinline__ Ray setupRay(v3 o, v3 d, float extent) {
-  Ray r;
+// Slab-test half of the ray set-up (see Ray).
+__device__ __forceinline__ void setupSlabs(Ray& r, v3 o, v3 d, float extent) {
   r.idx = rcpApprox(d.x);
   r.idy = rcpApprox(d.y);
   r.idz = rcpApprox(d.z);
@@ -137,6 +137,10 @@ __device__ __forceinline__ Ray setupRay(v3 o, v3 d, float extent) {
   r.slx = (extent + fabsf(o.x)) * fabsf(r.idx) * 4.76837158e-07f;
   r.sly = (extent + fabsf(o.y)) * fabsf(r.idy) * 4.76837158e-07f;
   r.slz = (extent + fabsf(o.z)) * fabsf(r.idz) * 4.76837158e-07f;
+}
+
+// Triangle-test half: the shear of the watertight test.
+__device__ __forceinline__ void setupShear(Ray& r, v3 o, v3 d) {
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0;
   float m = ax;
@@ -162,6 +166,12 @@ __device__ __forceinline__ Ray setupRay(v3 o, v3 d, float extent) {
   r.okx = sel3(o.x, o.y, o.z, kx);
   r.oky = sel3(o.x, o.y, o.z, ky);
   r.okz = sel3(o.x, o.y, o.z, kz);
+}
+
+__device__ __forceinline__ Ray setupRay(v3 o, v3 d, float extent) {
+  Ray r;
+  setupSlabs(r, o, d, extent);
+  setupShear(r, o, d);
   return r;
 }
 
@@ -766,6 +776,257 @@ __device__ __forceinline__ void buildCut(const DevScene& sc, const float4* __res
   }
 }
 
+// ---------------------------------------------------------------------------
+// Cone lists.  All samples of one ommatidium at one pose share their origin
+// and leave within a few standard deviations of its axis, so what they can
+// hit first is found once for all of them: coneList walks the BVH2 with the
+// cone of kConeSigmas standard deviations and lists, nearest first, the
+// subtrees and leaf triangles that the cone meets (at most kConeEntries,
+// which together cover everything in the cone).  A ray then tests the list
+// instead of descending from the root; a ray outside the cone (one sample in
+// 5,700) searches from the root.  Either way the result is the closest hit.
+// A triangle that covers the whole cone ends the list: nothing that begins
+// beyond it can be hit.
+//
+// Everything errs on the side of keeping an entry.  theta is widened by 1% +
+// 1e-4 rad, which covers the rounding of the samples' rotations and a pose
+// frame or axis that is orthonormal to 1e-3 (others get no list:
+// kConeFromRoot); boxes and edge planes are widened by a few float ulps of
+// (extent + |origin|); distances of entries are stored shortened by 0.5%,
+// which covers |direction| != 1.
+// ---------------------------------------------------------------------------
+constexpr float kConeSigmas = 3.75f;
+constexpr float kConeMaxAngle = 0.5f;  // wider cones are searched from the root
+constexpr int kConeSteps = 64;         // node visits of one list at most
+constexpr uint32_t kConeFromRoot = 0xffffffffu;
+constexpr int kConeThreads = 128;
+
+// A cone and, per axis, the factors of the interval slab test: with the
+// direction component in [lo, hi], a slab [b0, b1] (relative to the apex) is
+// entered no earlier than max(b0 * en0, b1 * en1) and left no later than
+// min(b1 * ex1 + of1, b0 * ex0 + of0).
+struct Cone {
+  v3 o, a;
+  float sinT, cosT;
+  float en0[3], en1[3], ex0[3], ex1[3], of0[3], of1[3];
+  float slack;
+};
+
+__device__ __forceinline__ void coneAxis(Cone& c, int k, float a) {
+  const float big = 1e30f;
+  const float s = sqrtf(fmaxf(0.0f, 1.0f - a * a)) * c.sinT;
+  const float hi = (a >= c.cosT ? 1.0f : a * c.cosT + s) + 2e-6f;
+  const float lo = (a <= -c.cosT ? -1.0f : a * c.cosT - s) - 2e-6f;
+  c.en0[k] = hi > 0.0f ? 1.0f / hi : big;
+  c.en1[k] = lo < 0.0f ? 1.0f / lo : -big;
+  c.ex1[k] = lo > 0.0f ? 1.0f / lo : 0.0f;
+  c.of1[k] = lo > 0.0f ? 0.0f : big;
+  c.ex0[k] = hi < 0.0f ? 1.0f / hi : 0.0f;
+  c.of0[k] = hi < 0.0f ? 0.0f : big;
+}
+
+// Entry distance of the cone into a box; true when some ray of the cone may
+// meet the box within tmax.
+__device__ __forceinline__ bool coneSpan(const Cone& c, float cx, float cy, float cz, float ex, float ey, float ez,
+                                         float tmax, float& tn) {
+  const float m[3] = {cx - c.o.x, cy - c.o.y, cz - c.o.z};
+  const float e[3] = {ex + c.slack, ey + c.slack, ez + c.slack};
+  float tf = tmax;
+  tn = 0.0f;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const float b0 = m[k] - e[k], b1 = m[k] + e[k];
+    tn = max3(tn, b0 * c.en0[k], b1 * c.en1[k]);
+    tf = min3(tf, fmaf(b1, c.ex1[k], c.of1[k]), fmaf(b0, c.ex0[k], c.of0[k]));
+  }
+  return !(tn > tf);
+}
+
+// Whether some ray of the cone may meet the triangle; covers: every ray of
+// the cone hits it, no nearer than tmin, and no farther than tCover (updated).
+__device__ __forceinline__ bool coneTriangle(const Cone& c, float4 v0, float4 v1, float4 v2, float tmin,
+                                             float& tCover) {
+  const v3 A = mk(v0.x, v0.y, v0.z) - c.o, B = mk(v1.x, v1.y, v1.z) - c.o, C = mk(v2.x, v2.y, v2.z) - c.o;
+  const v3 n0 = cross(A, B), n1 = cross(B, C), n2 = cross(C, A);
+  const float vol = dot(n0, C);
+  const float L = fabsf(A.x) + fabsf(A.y) + fabsf(A.z) + fabsf(B.x) + fabsf(B.y) + fabsf(B.z) + fabsf(C.x) +
+                  fabsf(C.y) + fabsf(C.z);
+  const float err = 4.0f * (c.slack + 1e-6f * L) * L;
+  if (!(fabsf(vol) > err * L)) return true;  // edge-on or degenerate: keep it
+  const float s = vol > 0.0f ? 1.0f : -1.0f;
+  const float q0 = s * dot(n0, c.a), w0 = sqrtf(dot(n0, n0)) * c.sinT + err;
+  const float q1 = s * dot(n1, c.a), w1 = sqrtf(dot(n1, n1)) * c.sinT + err;
+  const float q2 = s * dot(n2, c.a), w2 = sqrtf(dot(n2, n2)) * c.sinT + err;
+  if (q0 < -w0 || q1 < -w1 || q2 < -w2) return false;
+  if (q0 > w0 && q1 > w1 && q2 > w2) {
+    const v3 n = cross(B - A, C - A);
+    const float nl = sqrtf(dot(n, n));
+    const float cosP = fminf(fabsf(dot(n, c.a)) / nl, 1.0f);
+    const float worst = cosP * c.cosT - sqrtf(fmaxf(0.0f, 1.0f - cosP * cosP)) * c.sinT;
+    const float dist = fabsf(dot(n, A)) / nl;
+    if (worst > 0.05f && dist * 0.99f - 20.0f * c.slack > tmin)
+      tCover = fminf(tCover, (dist * 1.01f + 20.0f * c.slack) / worst);
+  }
+  return true;
+}
+
+// The list of ommatidium o at `pose`, written to out (kConeStride words: the
+// entry count, or kConeFromRoot, then (ref, entry distance) pairs; ref as in
+// the BVH, leaves possibly narrowed to some of their triangles).  work: the
+// thread's column of a [kConeEntries][kConeThreads] array, holding the
+// entries found (from the front) and the traversal stack (from the back).
+//
+// One thread per list: a list is ~30 dependent node visits, so the lists of
+// 32 neighbouring ommatidia share a warp, whose lanes walk nearly the same
+// nodes, instead of the lanes of a warp sharing a list.
+__device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, uint32_t o,
+                                         const float4* __restrict__ pose, uint2* __restrict__ work,
+                                         uint2* __restrict__ out) {
+  const float4 P0 = __ldg(pose), X = __ldg(pose + 1), Y = __ldg(pose + 2), Z = __ldg(pose + 3);
+  const float4 r0 = __ldg(eye.omm + 2 * o), r1 = __ldg(eye.omm + 2 * o + 1);
+  const v3 ax = mk(r0.w, r1.x, r1.y), x = mk(X.x, X.y, X.z), y = mk(Y.x, Y.y, Y.z), z = mk(Z.x, Z.y, Z.z);
+  const float fpo = r1.w;
+  const v3 rel = mk(r0.x, r0.y, r0.z) - normalize(ax) * fpo;
+  Cone c;
+  c.o = mk(P0.x, P0.y, P0.z) + x * rel.x + y * rel.y + z * rel.z;
+  const float theta = kConeSigmas * fabsf(r1.z / 2.35482004503094938202313865291f) * 1.01f + 1e-4f;
+  const float tol = 1e-3f;
+  const bool ok = fabsf(dot(ax, ax) - 1.0f) <= tol && fabsf(dot(x, x) - 1.0f) <= tol &&
+                  fabsf(dot(y, y) - 1.0f) <= tol && fabsf(dot(z, z) - 1.0f) <= tol && fabsf(dot(x, y)) <= tol &&
+                  fabsf(dot(x, z)) <= tol && fabsf(dot(y, z)) <= tol && theta <= kConeMaxAngle &&
+                  fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z) < 1e15f && fabsf(fpo) < 1e15f;
+  if (!ok) {  // also for NaNs
+    out[0] = make_uint2(kConeFromRoot, 0u);
+    return;
+  }
+  c.a = normalize(x * ax.x + y * ax.y + z * ax.z);
+  c.sinT = sinf(theta);
+  c.cosT = cosf(theta);
+  c.slack = (sc.extent + fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z)) * 1e-6f;
+  coneAxis(c, 0, c.a.x);
+  coneAxis(c, 1, c.a.y);
+  coneAxis(c, 2, c.a.z);
+
+  int nOut = 0, sp = 0, steps = 0, node = 0;
+  float tNode = 0.0f, tCover = 1e30f;
+  auto stackAt = [&](int k) -> uint2& { return work[(kConeEntries - 1 - k) * kConeThreads]; };
+  // nOut + sp + 1 (the current node) <= kConeEntries throughout.
+  for (;;) {
+    if (node >= 0 && nOut + sp + 2 <= kConeEntries && steps < kConeSteps) {
+      ++steps;
+      const float4* n = sc.nodes + 4 * static_cast<size_t>(node);
+      const float4 n0 = __ldg(n), n1 = __ldg(n + 1), n2 = __ldg(n + 2);
+      const int4 n3 = __ldg(reinterpret_cast<const int4*>(n + 3));
+      float t0, t1;
+      const bool hit0 = coneSpan(c, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, tCover, t0);
+      const bool hit1 = coneSpan(c, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, tCover, t1);
+      if (hit0 || hit1) {
+        const bool second = hit1 && (!hit0 || t1 < t0);
+        node = second ? n3.y : n3.x;
+        tNode = second ? t1 : t0;
+        if (hit0 && hit1) {
+          stackAt(sp) = make_uint2(static_cast<uint32_t>(second ? n3.x : n3.y), __float_as_uint(second ? t0 : t1));
+          ++sp;
+        }
+        continue;
+      }
+    } else {
+      int ref = node;
+      bool keep = true;
+      if (node < 0) {  // a leaf: the range of its triangles that the cone meets
+        const uint32_t code = ~static_cast<uint32_t>(node);
+        const uint32_t first = code >> 3, count = (code & 7u) + 1u;
+        uint32_t lo = count, hi = 0;
+        for (uint32_t k = 0; k < count; ++k) {
+          const float4* t = sc.tris + 3 * static_cast<size_t>(first + k);
+          if (coneTriangle(c, __ldg(t), __ldg(t + 1), __ldg(t + 2), fpo, tCover)) {
+            lo = min(lo, k);
+            hi = k;
+          }
+        }
+        keep = lo < count;
+        ref = static_cast<int>(~(((first + lo) << 3) | (hi - lo)));
+      }
+      if (keep) {
+        work[nOut * kConeThreads] = make_uint2(static_cast<uint32_t>(ref), __float_as_uint(tNode));
+        ++nOut;
+      }
+    }
+    do {  // next deferred entry that does not begin beyond a covering triangle
+      if (--sp < 0) break;
+      const uint2 e = stackAt(sp);
+      node = static_cast<int>(e.x);
+      tNode = __uint_as_float(e.y);
+    } while (tNode > tCover);
+    if (sp < 0) break;
+  }
+  // tCover bounds distances, t <= tCover * 1.005 (|direction| != 1).
+  uint32_t count = 0;
+  for (int k = 0; k < nOut; ++k) {
+    const uint2 e = work[k * kConeThreads];
+    const float te = __uint_as_float(e.y);
+    if (te > tCover) continue;
+    ++count;
+    out[count] = make_uint2(e.x, __float_as_uint(te * 0.995f));
+  }
+  out[0] = make_uint2(count, 0u);
+}
+
+// Cone lists of P poses of an eye, list (p, o) at cones + (p * N + o) *
+// kConeStride; threads in the eye's direction order.
+__global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses,
+                                                           uint32_t P) {
+  __shared__ uint2 work[kConeEntries * kConeThreads];
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
+  if (i >= static_cast<uint64_t>(P) * eye.N) return;
+  const uint32_t p = static_cast<uint32_t>(i / eye.N), slot = static_cast<uint32_t>(i - static_cast<uint64_t>(p) * eye.N);
+  const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
+  coneList(sc, eye, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+           eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
+}
+
+// Closest hit of a ray of the cone-list path: nd is its normal draw (the
+// angle to the axis in standard deviations).  All lanes of an ommatidium take
+// the list's entries in step, so a triangle's nine coordinates are one
+// broadcast load for the warp and no lane waits for another's traversal.
+// The slab half of the ray set-up is made only for the entries that are
+// subtrees, the shear only when there is something to test.
+template <bool kCount>
+__device__ __forceinline__ void traceCone(const DevScene& sc, v3 org, v3 dir, float tmin, float nd,
+                                          const uint2* __restrict__ list, Hit& h, uint32_t* errFlag,
+                                          uint32_t& nodeVisits, uint32_t& triTests) {
+  h.t = 1e16f;
+  h.id = 0xffffffffu;
+  h.pos = 0;
+  const uint32_t listed = __ldg(list).x;
+  const bool root = listed == kConeFromRoot || !(fabsf(nd) <= kConeSigmas);
+  const uint32_t count = root ? 1u : listed;
+  if (count == 0) return;
+  Ray ray;
+  setupShear(ray, org, dir);
+  for (uint32_t k = 0; k < count; ++k) {
+    int node = 0;
+    if (!root) {
+      const uint2 e = __ldg(list + 1 + k);
+      if (!(__uint_as_float(e.y) <= h.t)) continue;
+      node = static_cast<int>(e.x);
+    }
+    if (node < 0) {
+      const uint32_t code = ~static_cast<uint32_t>(node);
+      const uint32_t first = code >> 3, n = (code & 7u) + 1u;
+      if (kCount) triTests += n;
+      for (uint32_t j = 0; j < n; ++j) {
+        const float4* t = sc.tris + 3 * (first + j);
+        testTriangle(ray, __ldg(t), __ldg(t + 1), __ldg(t + 2), first + j, tmin, h);
+      }
+    } else {
+      int stack[kStackSize];
+      setupSlabs(ray, org, dir, sc.extent);
+      traverseFrom<kCount>(sc, ray, tmin, h, stack, 0, node, errFlag, nodeVisits, triTests);
+    }
+  }
+}
+
 __global__ void cutKernel(DevScene sc, const float4* __restrict__ poses, uint32_t P, float R, float maxRel,
                           float4* __restrict__ cuts) {
   const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1102,7 +1363,8 @@ __device__ __forceinline__ void flushChunkSums(const float* __restrict__ part, c
 // calls this function with the same poses (flushChunkSums has barriers).
 // kWidth: 2 searches the BVH2 (with the near-field cut when eye.cuts is
 // set), 4 or 8 the wide BVH of that width (no cut).
-template <int kMode, int kWidth = 2>
+// kCone: closest hits through the cone lists at eye.cones (kWidth 2).
+template <int kMode, int kWidth = 2, bool kCone = false>
 __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye, const float4* __restrict__ poses,
                                            uint32_t P, const WarpPlan& plan, uint64_t task, float* __restrict__ out,
                                            float* __restrict__ scratch, uint32_t* errFlag,
@@ -1194,9 +1456,12 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       const v3 org = mk(P0.x, P0.y, P0.z) + mk(X.x, X.y, X.z) * relPos.x + mk(Y.x, Y.y, Y.z) * relPos.y +
                      mk(Z.x, Z.y, Z.z) * relPos.z;
       const v3 dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
-      const Ray ray = setupRay(org, dir, sc.extent);
       Hit h;
-      if (kWidth != 2) {
+      if (kCone) {
+        traceCone<kCount>(sc, org, dir, fpo, nd, eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride, h,
+                          errFlag, nodeVisits, triTests);
+      } else if (kWidth != 2) {
+        const Ray ray = setupRay(org, dir, sc.extent);
         h.t = 1e16f;
         h.id = 0xffffffffu;
         h.pos = 0;
@@ -1206,11 +1471,13 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
           traverseWide<kWidth == 8 ? 8 : 4>(sc, ray, fpo, h, wstack, wsp, wnode, errFlag, nodeVisits, triTests, kCount,
                                              0x7fffffff);
         }
-      } else if (eye.cuts) {
-        traceClosest<kCount>(sc, ray, fpo, 1e16f, h, errFlag, nodeVisits, triTests,
-                             eye.cuts + static_cast<size_t>(p) * kCutStride, sqrtf(dot(dir, dir)));
       } else {
-        traceClosest<kCount>(sc, ray, fpo, 1e16f, h, errFlag, nodeVisits, triTests);
+        const Ray ray = setupRay(org, dir, sc.extent);
+        if (eye.cuts)
+          traceClosest<kCount>(sc, ray, fpo, 1e16f, h, errFlag, nodeVisits, triTests,
+                               eye.cuts + static_cast<size_t>(p) * kCutStride, sqrtf(dot(dir, dir)));
+        else
+          traceClosest<kCount>(sc, ray, fpo, 1e16f, h, errFlag, nodeVisits, triTests);
       }
       v3 c;
       float b1 = 0.f, b2 = 0.f;
@@ -1320,7 +1587,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
 // per-pose chunk partial in shared memory, and after every kInBlockPoses
 // poses the block sums each (ommatidium, pose) of the group over its chunks
 // in chunk order (flushChunkSums), so the buffer holds 16 poses at a time.
-template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false>
+template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false, bool kCone = false>
 __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses, uint32_t P,
                                                 WarpPlan plan, float* __restrict__ out, float* __restrict__ scratch,
                                                 uint32_t* errFlag, RayRecord* __restrict__ rec,
@@ -1331,8 +1598,8 @@ __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const f
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t task = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (task >= plan.tasks) return;  // whole warps exit together (never with inBlock: whole blocks)
-  renderTask<kMode, kWidth>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits, triTests,
-                            kInBlock ? chunkPart : nullptr);
+  renderTask<kMode, kWidth, kCone>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits, triTests,
+                                   kInBlock ? chunkPart : nullptr);
   if (kCount) {
     unsigned long long nv = nodeVisits, tt = triTests;
     for (int m = 16; m >= 1; m >>= 1) {
@@ -1812,15 +2079,21 @@ WarpPlan planBatch(uint32_t N, uint32_t spp) {
 
 uint32_t batchBlockThreads() { return g_blockThreads ? g_blockThreads : 128u; }
 
-// In-block chunk sums are built for the plain and recording renders on the
-// two-wide BVH only.
-static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats) {
-  return !stats && !scene.lighting && (scene.width == 2 || rec);
+// In-block chunk sums are built for the plain and recording renders through
+// cone lists only.
+static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool cones) {
+  return !stats && !scene.lighting && cones;
+}
+
+size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec) {
+  if (scene.triCount == 0 || spp < kConeMinSamples) return 0;
+  if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
+  return static_cast<size_t>(P) * N;
 }
 
 size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec, bool stats,
-                           bool forceScratch) {
-  const WarpPlan p = planRender(N, spp, P, forceScratch, inBlockAllowed(scene, rec, stats));
+                           bool forceScratch, bool cones) {
+  const WarpPlan p = planRender(N, spp, P, forceScratch, inBlockAllowed(scene, rec, stats, cones));
   if (p.chunks == 1 || p.inBlock) return 0;
   return static_cast<size_t>(P) * N * p.chunks * 3;
 }
@@ -1842,10 +2115,9 @@ cudaError_t launchRngInit(const DevEye& eye, uint32_t* errFlag, cudaStream_t str
 }
 
 namespace {
-// One launch of renderKernel<kMode, kRegs> with the plan's block size and,
-// for in-block chunk sums, the shared memory of the partials.
-// Launch of the kernel instance with (kInBlock) or without in-block chunk sums.
-template <int kMode, int kRegs, int kWidth, bool kInBlock>
+// One launch of a render kernel instance with the plan's block size and, for
+// in-block chunk sums, the shared memory of the partials.
+template <int kMode, int kRegs, int kWidth, bool kInBlock, bool kCone>
 cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                             const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                             unsigned long long* stats, cudaStream_t stream) {
@@ -1856,31 +2128,36 @@ cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const floa
   if (kInBlock) {
     smem = static_cast<size_t>(plan.groupsPerBlock) * plan.ommPerWarp * kInBlockPoses * plan.chunks * 3 * sizeof(float);
     if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock>,
+      const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock, kCone>,
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(kChunkSmemMax));
       if (e != cudaSuccess) return e;
     }
   }
-  renderKernel<kMode, kRegs, kWidth, kInBlock><<<static_cast<unsigned>(blocks), block, smem, stream>>>(
+  renderKernel<kMode, kRegs, kWidth, kInBlock, kCone><<<static_cast<unsigned>(blocks), block, smem, stream>>>(
       scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats);
   return cudaGetLastError();
 }
 
-// In-block chunk sums exist for the plain and recording renders on the
-// two-wide BVH (planRender offers them only there, see inBlockAllowed).
-template <int kMode, int kRegs, int kWidth = 2>
+// The instance for the two-wide BVH: through the cone lists when the eye has
+// them (with in-block chunk sums where the plan says so; planRender offers
+// those only to plain and recording renders), else without.
+template <int kMode, int kRegs>
 cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                       const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                       unsigned long long* stats, cudaStream_t stream) {
-  constexpr bool kHasInBlock = (kMode == 0 || kMode == 1) && kWidth == 2;
+  constexpr bool kHasInBlock = kMode == 0 || kMode == 1;
+  constexpr bool kHasCone = kMode != 3;
   if (plan.inBlock) {
-    if (!kHasInBlock) return cudaErrorInvalidValue;
-    return runRenderKernel<kMode, kRegs, kWidth, kHasInBlock>(scene, eye, poses, P, plan, out, scratch, errFlag,
-                                                              rec, stats, stream);
+    if (!kHasInBlock || !eye.cones) return cudaErrorInvalidValue;
+    return runRenderKernel<kMode, kRegs, 2, kHasInBlock, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag,
+                                                                   rec, stats, stream);
   }
-  return runRenderKernel<kMode, kRegs, kWidth, false>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
-                                                      stats, stream);
+  if (kHasCone && eye.cones)
+    return runRenderKernel<kMode, kRegs, 2, false, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
+                                                             stats, stream);
+  return runRenderKernel<kMode, kRegs, 2, false, false>(scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats,
+                                                        stream);
 }
 
 // The plain render (mode 0) or the counting render (mode 2) of the scene's
@@ -1889,13 +2166,16 @@ template <int kMode, int kRegs>
 cudaError_t runRenderWidth(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                            const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag,
                            unsigned long long* stats, cudaStream_t stream) {
+  if (scene.width != 2 && (plan.inBlock || eye.cones)) return cudaErrorInvalidValue;
   switch (scene.width) {
     case 4:
-      return runRender<kMode, kRegs, 4>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr, stats, stream);
+      return runRenderKernel<kMode, kRegs, 4, false, false>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr,
+                                                            stats, stream);
     case 8:
-      return runRender<kMode, kRegs, 8>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr, stats, stream);
+      return runRenderKernel<kMode, kRegs, 8, false, false>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr,
+                                                            stats, stream);
     default:
-      return runRender<kMode, kRegs, 2>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr, stats, stream);
+      return runRender<kMode, kRegs>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr, stats, stream);
   }
 }
 }  // namespace
@@ -1904,7 +2184,9 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
                          float* scratch, uint32_t* errFlag, RayRecord* rec, cudaStream_t stream,
                          unsigned long long* stats, bool forceScratch) {
   if (P == 0 || eye.N == 0) return cudaSuccess;
-  WarpPlan plan = planRender(eye.N, eye.spp, P, forceScratch, inBlockAllowed(scene, rec != nullptr, stats != nullptr));
+  if (eye.cones && renderConeLists(scene, eye.N, eye.spp, P, rec != nullptr) == 0) return cudaErrorInvalidValue;
+  WarpPlan plan = planRender(eye.N, eye.spp, P, forceScratch,
+                             inBlockAllowed(scene, rec != nullptr, stats != nullptr, eye.cones != nullptr));
   if (plan.chunks > 1 && !plan.inBlock && scratch == nullptr) return cudaErrorInvalidValue;
   if (eye.draws) {
     if (plan.inBlock) return cudaErrorInvalidValue;  // planRender keeps splittable launches out of shared memory
@@ -1914,7 +2196,13 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     if (e != cudaSuccess) return e;
     plan = splitPoses(plan, P);
   }
-  if (eye.cuts && (scene.width == 2 || rec || scene.lighting)) {  // the wide BVH searches without a cut
+  if (eye.cones) {
+    const uint64_t lists = static_cast<uint64_t>(P) * eye.N, blocks = (lists + kConeThreads - 1) / kConeThreads;
+    if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
+    coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  } else if (eye.cuts && (scene.width == 2 || rec || scene.lighting)) {  // the wide BVH searches without a cut
     if (!(eye.cutRadius > 0.f)) return cudaErrorInvalidValue;
     cutKernel<<<(P + 63) / 64, 64, 0, stream>>>(scene, poses, P, eye.cutRadius, eye.maxRel, eye.cuts);
     const cudaError_t e = cudaGetLastError();
