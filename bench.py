@@ -60,6 +60,7 @@ def parse_args():
                     help="scene of the --profile-adaptive case")
     ap.add_argument("--profile-train", type=int, default=0, metavar="STEPS",
                     help="profiling case: STEPS denoiser training steps of 8192 rows on the terrain eye")
+    ap.add_argument("--no-lists", action="store_true", help="--profile without cone lists")
     ap.add_argument("--denoiser-kernel", type=int, default=1, help="denoiser inference kernel for --profile-learned: "
                     "0 mma.sync, 1 tcgen05")
     return ap.parse_args()
@@ -68,7 +69,7 @@ def parse_args():
 def render_kernels_per_launch(spp, layout, cut_fraction):
     """The library's kernels in one render launch under the autotuned layout
     (the rule of render.cu planRender): the near-field cut when a radius is
-    set, the render kernel, and the chunk sums when an ommatidium's samples
+    set (or, in its place, the cone lists), the render kernel, and the chunk sums when an ommatidium's samples
     span several warp segments and a block cannot hold all of them."""
     block, spw = layout
     spw = 32 if spw in (0, 32) else spw
@@ -108,10 +109,18 @@ def source_sha16(path=RENDER_SRC):
         return hashlib.sha256(f.read()).hexdigest()[:16]
 
 
+def list_counters(layout, path=COUNTERS_MD):
+    """launch_counters for the render through cone lists, which the register
+    variant and the cut radius do not enter: the entry with "cone_lists" true
+    and this layout."""
+    return launch_counters(None, None, layout, path)
+
+
 def launch_counters(variant, cut_fraction, layout, path=COUNTERS_MD):
     """ncu counters of one full 256-pose launch of this workload, read from
     the committed profile summary's JSON block: entries keyed by render
-    variant and near-field cut fraction, each with the warp instructions
+    variant and near-field cut fraction (renders without cone lists; both None
+    for the render with them), each with the warp instructions
     (smsp__inst_executed.sum) and DRAM bytes (read + write) of the render
     kernel per launch, and the sha256 prefix of render.cu they were taken
     with.  Returns (entry, reason): entry None when no entry matches the
@@ -125,11 +134,15 @@ def launch_counters(variant, cut_fraction, layout, path=COUNTERS_MD):
         return None, "no counters (%s)" % type(e).__name__
     sha = source_sha16()
     for e in entries:
-        if e["variant"] == variant and abs(e["cut_fraction"] - cut_fraction) < 1e-9 and \
+        lists = bool(e.get("cone_lists"))
+        if (lists if variant is None else not lists and e["variant"] == variant
+                and abs(e["cut_fraction"] - cut_fraction) < 1e-9) and \
                 [e["block_threads"], e["samples_per_warp"]] == list(layout):
             if e["render_cu_sha16"] != sha:
                 return None, "counters taken with another render.cu (%s, now %s)" % (e["render_cu_sha16"], sha)
             return e, "matched"
+    if variant is None:
+        return None, "no counters for cone lists, layout %s" % list(layout)
     return None, "no counters for variant %d, cut %g, layout %s" % (variant, cut_fraction, list(layout))
 
 
@@ -513,8 +526,9 @@ def run_ours(args):
     launch_s = statistics.mean(full) / 1000.0
     hbm_peak, src = peaks()
     l2_peak = l2_copy_gbs(dev)
-    counters, why = launch_counters(best.value, cut_fraction, layout) if launch_n == POSES_PER_LAUNCH \
-        else (None, "partial launch")
+    # 393 M rays a launch: through cone lists on the two-wide BVH.
+    counters, why = (None, "partial launch") if launch_n != POSES_PER_LAUNCH else (
+        list_counters(layout) if bvh_width == 2 else launch_counters(best.value, cut_fraction, layout))
     issue_peak = 4.0 * SM_COUNT * sm_max_mhz() * 1e6 / 1e12  # T warp instructions/s
     if counters:
         instr_per_ray = counters["warp_instructions"] / counters["rays"]
@@ -543,10 +557,11 @@ def run_ours(args):
                                      "bvh_width_2_4_8": [round(float(x), 3) for x in tune_all[15:18]],
                                      "cut_refined_div_mul_sqrt2": [round(float(x), 3) for x in tune_all[18:20]]},
                      "bvh_width": bvh_width},
-        # per 256-pose launch: the poses' near-field cuts (when a radius is
-        # set), the render kernel and, when the layout keeps chunk partials in
-        # scratch, their sums
-        "gpu_launches": args.steps * len(chunks) * render_kernels_per_launch(spp, layout, cut_fraction),
+        # per 256-pose launch: the cone lists (on the two-wide BVH), the render
+        # kernel and, when the layout keeps chunk partials in scratch, their
+        # sums
+        "gpu_launches": args.steps * len(chunks) * render_kernels_per_launch(
+            spp, layout, 1.0 if bvh_width == 2 else cut_fraction),
         "roofline": {"bound": "issue", "achieved": issue_achieved, "peak": issue_peak,
                      "unit": "T warp instructions/s", "frac": (issue_achieved / issue_peak) if counters else None,
                      "traffic": traffic,
@@ -1393,6 +1408,11 @@ def run_profile(args):
         raise RuntimeError(eh.lastError(lib))
     P = min(args.poses, POSES_PER_LAUNCH)
     poses = info["poses"][:P]
+    if args.no_lists:  # a memory cap with no room for the lists: the render searches the BVH
+        eh.renderPoses(lib, poses[:1])
+        n, k = info["n_omm"], -(-info["spp"] // 32)
+        if lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + P * n * 12 * (k + 1) + (64 << 20)) != 0:
+            raise RuntimeError(eh.lastError(lib))
     for _ in range(2):
         out = eh.renderPoses(lib, poses)
     print(json.dumps({"profile_case": "first %d poses of the terrain trajectory" % P, "checksum": float(out.sum()),

@@ -75,11 +75,11 @@ struct DevEye {
   float4* cuts = nullptr;
   float cutRadius = 0.f;
   float maxRel = 0.f;
-  // cones: null, or P x N x kConeStride words receiving the cone lists of the
+  // cones: null, or P x N x kConeStride float4 receiving the cone lists of the
   //       launch (render.cu, coneList): what the samples of an ommatidium can
   //       hit first at a pose, found once for all of them.  Replaces the
   //       cuts.  Results do not depend on it.
-  uint2* cones = nullptr;
+  float4* cones = nullptr;
   // netDraws: sample s of ommatidium o at pose p of the launch takes point s
   //       of a digitally shifted two-dimensional Sobol' net, the shift drawn
   //       from (drawSeed, (frame0 + p) * N + o) (render.cu, netDraw): no
@@ -94,10 +94,11 @@ struct DevEye {
 constexpr int kWideStackEntries = 128;
 constexpr int kCutEntries = 8;
 constexpr int kCutStride = 1 + 2 * kCutEntries;
-// A cone list: its count, then up to kConeEntries entries, 8 bytes each.
-constexpr int kConeEntries = 11;
-constexpr int kConeStride = 1 + kConeEntries;
-constexpr uint32_t kConeMinSamples = 32;
+// A cone list (render.cu, coneList): head, up to kConeEntries 8-byte entries,
+// three rows of relative vertex coordinates per single-triangle entry.
+constexpr int kConeEntries = 8;
+constexpr int kConeRow0 = 1 + (kConeEntries + 1) / 2;
+constexpr int kConeStride = kConeRow0 + 3 * kConeEntries;
 
 // One pose = 4 x float4: position, local x axis, local y axis, local z axis
 // (w components unused).
@@ -143,8 +144,8 @@ struct WarpPlan {
 // The default plan: 32-sample segments (whole ommatidia when spp < 32).
 WarpPlan planWarps(uint32_t N, uint32_t spp);
 // Layout of the plain render kernel, process-wide (the autotuner sets it):
-// block size in threads (0 = the smallest of 128, 256, 512 that holds all
-// chunk warps of an ommatidium, else 128) and samples per warp segment
+// block size in threads (0 = 128, or for few poses the smallest of 128, 256,
+// 512 that holds all chunk warps of an ommatidium) and samples per warp segment
 // (0 = 32, or 8 / 16: segments of 8 or 16 samples, several ommatidia per
 // warp; a smaller segment changes the order in which samples are summed,
 // so results change within float rounding).  Results never depend on the
@@ -170,7 +171,7 @@ size_t renderDrawBytes(uint32_t N, uint32_t spp, uint32_t P);
 size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false,
                            bool stats = false, bool forceScratch = false, bool cones = false);
 
-// Cone lists (DevEye::cones, kConeStride words each) worth providing for a
+// Cone lists (DevEye::cones, kConeStride float4 each) worth providing for a
 // P-pose launch: P x N, or 0 when the launch does not use them.
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false);
 

@@ -192,7 +192,7 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
 }
 
 constexpr uint32_t kMaxPosesPerLaunch = 256;
-constexpr size_t kConeListBytes = size_t(512) << 20;  // cone lists of one launch at most
+constexpr size_t kConeListBytes = size_t(1) << 30;  // cone lists of one launch at most
 constexpr size_t kTuneSlots = 20;
 
 // Order in which warp segments take an eye's ommatidia: by the 30-bit Morton
@@ -271,8 +271,8 @@ struct Renderer {
   DevBuf<float> scratch;
   DevBuf<float2> draws;  // pre-drawn random numbers of small-eye launches
   DevBuf<float4> cuts;   // per-pose near-field cuts
-  DevBuf<uint2> cones;   // cone lists of a launch
-  bool conesOff = false; // crAutotune times the cut radii without cone lists
+  DevBuf<float4> cones;   // cone lists of a launch
+  bool conesOff = false; // crAutotune times variants and cut radii without cone lists
   float cutFactor = 0.f; // cut radius as a fraction of the scene extent (0: off)
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
   // samples per warp 8/16/32, cut radius 0, 1/256 .. 1/16 of the extent.
@@ -624,7 +624,7 @@ struct Renderer {
   // Poses of one launch: at most kMaxPosesPerLaunch, and fewer for large eyes
   // so that a launch's cone lists stay within kConeListBytes.
   static size_t posesPerLaunch(uint32_t N) {
-    const size_t fit = kConeListBytes / (sizeof(uint2) * kConeStride * std::max<size_t>(1, N));
+    const size_t fit = kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N));
     return std::min<size_t>(kMaxPosesPerLaunch, std::max<size_t>(1, fit));
   }
 
@@ -635,7 +635,7 @@ struct Renderer {
   float* withCones(DevEye& de, uint32_t P, DevBuf<float>& scr, bool rec, bool stats) {
     de.cones = nullptr;
     const size_t lists = conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec);
-    if (lists && lists * kConeStride * sizeof(uint2) <= kConeListBytes) {
+    if (lists && lists * kConeStride * sizeof(float4) <= kConeListBytes) {
       cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
       check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
       if (st == cudaStreamCaptureStatusNone && cones.tryEnsure(lists * kConeStride)) de.cones = cones.ptr;
@@ -1647,11 +1647,17 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
         cudaEvent_t a, b;
         check(cudaEventCreate(&a), "cudaEventCreate");
         check(cudaEventCreate(&b), "cudaEventCreate");
+        struct Restore {  // whatever ends the tuning
+          ~Restore() { R().conesOff = false; }
+        } restore;
         const int prev = renderVariant();
         int best = 0;
         float bestMs = INFINITY;
         float variantMs[3] = {0.f, 0.f, 0.f};
         setRenderLayout(0, 0);  // variants timed with the automatic layout
+        // Renders through cone lists have one variant and no cut radius: both
+        // are chosen for the renders without (few samples, feature renders).
+        r.conesOff = true;
         for (int v = 0; v < renderVariantCount(); ++v) {
           setRenderVariant(v);
           float ms = INFINITY;
@@ -1684,6 +1690,7 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
           }
           return ms;
         };
+        r.conesOff = false;
         setRenderVariant(best);
         r.tuneTimes.assign(kTuneSlots, 0.f);
         for (int v = 0; v < 3; ++v) r.tuneTimes[v] = variantMs[v];
@@ -1713,8 +1720,7 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
         }
         setRenderLayout(bestBlock, bestSeg);
         // Near-field cut radius (fraction of the scene extent), with the best
-        // variant and layout, without cone lists: renders that use those
-        // ignore the radius, the others take the one timed here.
+        // variant and layout, again without cone lists.
         r.conesOff = true;
         const float factors[] = {0.f, 1.f / 256, 1.f / 128, 1.f / 64, 1.f / 32, 1.f / 16};
         float bestCut = 0.f, bestCutMs = INFINITY;

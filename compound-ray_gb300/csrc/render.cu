@@ -6,8 +6,9 @@
 //   1. draws one normal and one uniform number per sample (cuRAND, as
 //      libEyeRenderer3/shaders.cu:680-695),
 //   2. builds the splayed ray (shaders.cu:648-709),
-//   3. finds the closest triangle in the BVH2 (replaces optixTrace,
-//      shaders.cu:110-137),
+//   3. finds the closest triangle (replaces optixTrace, shaders.cu:110-137):
+//      long launches through a list of what the ommatidium's cone can meet,
+//      built once per (pose, ommatidium), others in the BVH2,
 //   4. shades it with the lighting-off whitted closest-hit program or the
 //      miss program (shaders.cu:740-811, cuda/LocalGeometry.h:55-156),
 //   5. scales by 1/spp (shaders.cu:730) and reduces the warp's samples with
@@ -89,7 +90,21 @@ __device__ __forceinline__ float xsqrt(float a) {
   asm("sqrt.rn.f32 %0, %1;" : "=f"(r) : "f"(a));
   return r;
 }
-__device__ __forceinline__ float xneg(float a) { return __int_as_float(__float_as_int(a) ^ 0x80000000); }
+__device__ __forceinline__ float xneg(float a) {
+  float r;
+  asm("neg.f32 %0, %1;" : "=f"(r) : "f"(a));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float min3(float a, float b, float c) {
+  float r;
+  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
 
 __device__ __forceinline__ float sel3(float x, float y, float z, int k) { return k == 0 ? x : (k == 1 ? y : z); }
 
@@ -139,8 +154,9 @@ __device__ __forceinline__ void setupSlabs(Ray& r, v3 o, v3 d, float extent) {
   r.slz = (extent + fabsf(o.z)) * fabsf(r.idz) * 4.76837158e-07f;
 }
 
-// Triangle-test half: the shear of the watertight test.
-__device__ __forceinline__ void setupShear(Ray& r, v3 o, v3 d) {
+// Triangle-test half: the shear of the watertight test, and the origin in its
+// axis order.
+__device__ __forceinline__ void setupShear(Ray& r, v3 d) {
   const float ax = fabsf(d.x), ay = fabsf(d.y), az = fabsf(d.z);
   int kz = 0;
   float m = ax;
@@ -163,15 +179,18 @@ __device__ __forceinline__ void setupShear(Ray& r, v3 o, v3 d) {
   r.Sz = xdiv(1.0f, dkz);
   r.nSx = xneg(xmul(sel3(d.x, d.y, d.z, kx), r.Sz));
   r.nSy = xneg(xmul(sel3(d.x, d.y, d.z, ky), r.Sz));
-  r.okx = sel3(o.x, o.y, o.z, kx);
-  r.oky = sel3(o.x, o.y, o.z, ky);
-  r.okz = sel3(o.x, o.y, o.z, kz);
+}
+__device__ __forceinline__ void setupOrigin(Ray& r, v3 o) {
+  r.okx = sel3(o.x, o.y, o.z, r.kx);
+  r.oky = sel3(o.x, o.y, o.z, r.ky);
+  r.okz = sel3(o.x, o.y, o.z, r.kz);
 }
 
 __device__ __forceinline__ Ray setupRay(v3 o, v3 d, float extent) {
   Ray r;
   setupSlabs(r, o, d, extent);
-  setupShear(r, o, d);
+  setupShear(r, d);
+  setupOrigin(r, o);
   return r;
 }
 
@@ -182,19 +201,12 @@ struct Hit {
   float U, V, W, det;
 };
 
-// Watertight test of one triangle; updates `h` when the hit is closer in the
+// Watertight test of one triangle given by its vertices relative to the ray
+// origin, in the ray's axis order; updates `h` when the hit is closer in the
 // (t, id) order and lies in [tmin, h.t].
-__device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1, float4 v2, uint32_t pos, float tmin,
-                                             Hit& h) {
-  const float Akx = xsub(sel3(v0.x, v0.y, v0.z, r.kx), r.okx);
-  const float Aky = xsub(sel3(v0.x, v0.y, v0.z, r.ky), r.oky);
-  const float Akz = xsub(sel3(v0.x, v0.y, v0.z, r.kz), r.okz);
-  const float Bkx = xsub(sel3(v1.x, v1.y, v1.z, r.kx), r.okx);
-  const float Bky = xsub(sel3(v1.x, v1.y, v1.z, r.ky), r.oky);
-  const float Bkz = xsub(sel3(v1.x, v1.y, v1.z, r.kz), r.okz);
-  const float Ckx = xsub(sel3(v2.x, v2.y, v2.z, r.kx), r.okx);
-  const float Cky = xsub(sel3(v2.x, v2.y, v2.z, r.ky), r.oky);
-  const float Ckz = xsub(sel3(v2.x, v2.y, v2.z, r.kz), r.okz);
+__device__ __forceinline__ void testRelative(const Ray& r, float Akx, float Aky, float Akz, float Bkx, float Bky,
+                                             float Bkz, float Ckx, float Cky, float Ckz, uint32_t id, uint32_t pos,
+                                             float tmin, Hit& h) {
   const float Ax = xfma(r.nSx, Akz, Akx);
   const float Ay = xfma(r.nSy, Akz, Aky);
   const float Bx = xfma(r.nSx, Bkz, Bkx);
@@ -204,7 +216,7 @@ __device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1,
   float U = xfma(Cx, By, xneg(xmul(Cy, Bx)));
   float V = xfma(Ax, Cy, xneg(xmul(Ay, Cx)));
   float W = xfma(Bx, Ay, xneg(xmul(By, Ax)));
-  if (U == 0.0f || V == 0.0f || W == 0.0f) {
+  if (min3(fabsf(U), fabsf(V), fabsf(W)) == 0.0f) {
     const double CxBy = (double)Cx * (double)By, CyBx = (double)Cy * (double)Bx;
     const double AxCy = (double)Ax * (double)Cy, AyCx = (double)Ay * (double)Cx;
     const double BxAy = (double)Bx * (double)Ay, ByAx = (double)By * (double)Ax;
@@ -212,7 +224,8 @@ __device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1,
     V = __double2float_rn(__dsub_rn(AxCy, AyCx));
     W = __double2float_rn(__dsub_rn(BxAy, ByAx));
   }
-  if ((U < 0.0f || V < 0.0f || W < 0.0f) && (U > 0.0f || V > 0.0f || W > 0.0f)) return;
+  // some sign negative and some positive: outside (a NaN has neither)
+  if (min3(U, V, W) < 0.0f && max3(U, V, W) > 0.0f) return;
   const float det = xadd(xadd(U, V), W);
   if (det == 0.0f) return;
   const float Az = xmul(r.Sz, Akz);
@@ -221,7 +234,6 @@ __device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1,
   const float T = xfma(U, Az, xfma(V, Bz, xmul(W, Cz)));
   const float t = xdiv(T, det);
   if (!(t >= tmin && t <= h.t)) return;
-  const uint32_t id = __float_as_uint(v0.w);
   if (t == h.t && id >= h.id) return;
   h.t = t;
   h.id = id;
@@ -232,18 +244,16 @@ __device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1,
   h.det = det;
 }
 
-constexpr int kStackSize = 64;
+__device__ __forceinline__ void testTriangle(const Ray& r, float4 v0, float4 v1, float4 v2, uint32_t pos, float tmin,
+                                             Hit& h) {
+  testRelative(r, xsub(sel3(v0.x, v0.y, v0.z, r.kx), r.okx), xsub(sel3(v0.x, v0.y, v0.z, r.ky), r.oky),
+               xsub(sel3(v0.x, v0.y, v0.z, r.kz), r.okz), xsub(sel3(v1.x, v1.y, v1.z, r.kx), r.okx),
+               xsub(sel3(v1.x, v1.y, v1.z, r.ky), r.oky), xsub(sel3(v1.x, v1.y, v1.z, r.kz), r.okz),
+               xsub(sel3(v2.x, v2.y, v2.z, r.kx), r.okx), xsub(sel3(v2.x, v2.y, v2.z, r.ky), r.oky),
+               xsub(sel3(v2.x, v2.y, v2.z, r.kz), r.okz), __float_as_uint(v0.w), pos, tmin, h);
+}
 
-__device__ __forceinline__ float max3(float a, float b, float c) {
-  float r;
-  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
-__device__ __forceinline__ float min3(float a, float b, float c) {
-  float r;
-  asm("min.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
-  return r;
-}
+constexpr int kStackSize = 64;
 
 // Entry/exit distances of one child box given as centre and half-extent.
 __device__ __forceinline__ void childSpan(const Ray& r, float cx, float cy, float cz, float ex, float ey, float ez,
@@ -776,6 +786,14 @@ __device__ __forceinline__ void buildCut(const DevScene& sc, const float4* __res
   }
 }
 
+// Ray origin of an ommatidium in the eye's frame (its position moved back by
+// the focal offset), and in the world.  The cone lists and the renders both
+// form it with these, so it is the same float everywhere.
+__device__ __forceinline__ v3 relativeOrigin(v3 pos, v3 axis, float fpo) { return pos - normalize(axis) * fpo; }
+__device__ __forceinline__ v3 rayOrigin(v3 p, v3 x, v3 y, v3 z, v3 rel) {
+  return p + x * rel.x + y * rel.y + z * rel.z;
+}
+
 // ---------------------------------------------------------------------------
 // Cone lists.  All samples of one ommatidium at one pose share their origin
 // and leave within a few standard deviations of its axis, so what they can
@@ -870,25 +888,29 @@ __device__ __forceinline__ bool coneTriangle(const Cone& c, float4 v0, float4 v1
   return true;
 }
 
-// The list of ommatidium o at `pose`, written to out (kConeStride words: the
-// entry count, or kConeFromRoot, then (ref, entry distance) pairs; ref as in
-// the BVH, leaves possibly narrowed to some of their triangles).  work: the
-// thread's column of a [kConeEntries][kConeThreads] array, holding the
-// entries found (from the front) and the traversal stack (from the back).
+// The list of ommatidium o at `pose`, written to out (kConeStride float4):
+//   [0] (entry count, or kConeFromRoot; origin xyz),
+//   [1 ..] (entry distance, ref) pairs, two to a float4; ref as in the BVH, a
+//       leaf as one entry for each of its triangles that the cone meets while
+//       there is room,
+//   [kConeRow0 + 3 k ..] for a single-triangle entry k its vertices relative
+//       to the origin (the subtraction each ray would make), one row per
+//       axis: (A, B, C, triangle id).
+// work: the thread's column of a [kConeEntries][kConeThreads] array, holding
+// the entries found (from the front) and the traversal stack (from the back).
 //
 // One thread per list: a list is ~30 dependent node visits, so the lists of
 // 32 neighbouring ommatidia share a warp, whose lanes walk nearly the same
 // nodes, instead of the lanes of a warp sharing a list.
 __device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, uint32_t o,
                                          const float4* __restrict__ pose, uint2* __restrict__ work,
-                                         uint2* __restrict__ out) {
+                                         float4* __restrict__ out) {
   const float4 P0 = __ldg(pose), X = __ldg(pose + 1), Y = __ldg(pose + 2), Z = __ldg(pose + 3);
   const float4 r0 = __ldg(eye.omm + 2 * o), r1 = __ldg(eye.omm + 2 * o + 1);
   const v3 ax = mk(r0.w, r1.x, r1.y), x = mk(X.x, X.y, X.z), y = mk(Y.x, Y.y, Y.z), z = mk(Z.x, Z.y, Z.z);
   const float fpo = r1.w;
-  const v3 rel = mk(r0.x, r0.y, r0.z) - normalize(ax) * fpo;
   Cone c;
-  c.o = mk(P0.x, P0.y, P0.z) + x * rel.x + y * rel.y + z * rel.z;
+  c.o = rayOrigin(mk(P0.x, P0.y, P0.z), x, y, z, relativeOrigin(mk(r0.x, r0.y, r0.z), ax, fpo));
   const float theta = kConeSigmas * fabsf(r1.z / 2.35482004503094938202313865291f) * 1.01f + 1e-4f;
   const float tol = 1e-3f;
   const bool ok = fabsf(dot(ax, ax) - 1.0f) <= tol && fabsf(dot(x, x) - 1.0f) <= tol &&
@@ -896,7 +918,7 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, 
                   fabsf(dot(x, z)) <= tol && fabsf(dot(y, z)) <= tol && theta <= kConeMaxAngle &&
                   fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z) < 1e15f && fabsf(fpo) < 1e15f;
   if (!ok) {  // also for NaNs
-    out[0] = make_uint2(kConeFromRoot, 0u);
+    out[0] = make_float4(__uint_as_float(kConeFromRoot), c.o.x, c.o.y, c.o.z);
     return;
   }
   c.a = normalize(x * ax.x + y * ax.y + z * ax.z);
@@ -910,9 +932,21 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, 
   int nOut = 0, sp = 0, steps = 0, node = 0;
   float tNode = 0.0f, tCover = 1e30f;
   auto stackAt = [&](int k) -> uint2& { return work[(kConeEntries - 1 - k) * kConeThreads]; };
-  // nOut + sp + 1 (the current node) <= kConeEntries throughout.
-  for (;;) {
-    if (node >= 0 && nOut + sp + 2 <= kConeEntries && steps < kConeSteps) {
+  // Next deferred entry that does not begin beyond a covering triangle.
+  auto pop = [&]() {
+    while (sp > 0) {
+      const uint2 e = stackAt(--sp);
+      node = static_cast<int>(e.x);
+      tNode = __uint_as_float(e.y);
+      if (!(tNode > tCover)) return true;
+    }
+    return false;
+  };
+  // nOut + sp + 1 (the current node) <= kConeEntries throughout.  The lanes of
+  // a warp first all descend to a leaf, then test triangles together.
+  bool more = true;
+  while (more) {
+    while (more && node >= 0 && nOut + sp + 2 <= kConeEntries && steps < kConeSteps) {
       ++steps;
       const float4* n = sc.nodes + 4 * static_cast<size_t>(node);
       const float4 n0 = __ldg(n), n1 = __ldg(n + 1), n2 = __ldg(n + 2);
@@ -928,48 +962,52 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, 
           stackAt(sp) = make_uint2(static_cast<uint32_t>(second ? n3.x : n3.y), __float_as_uint(second ? t0 : t1));
           ++sp;
         }
-        continue;
-      }
-    } else {
-      int ref = node;
-      bool keep = true;
-      if (node < 0) {  // a leaf: the range of its triangles that the cone meets
-        const uint32_t code = ~static_cast<uint32_t>(node);
-        const uint32_t first = code >> 3, count = (code & 7u) + 1u;
-        uint32_t lo = count, hi = 0;
-        for (uint32_t k = 0; k < count; ++k) {
-          const float4* t = sc.tris + 3 * static_cast<size_t>(first + k);
-          if (coneTriangle(c, __ldg(t), __ldg(t + 1), __ldg(t + 2), fpo, tCover)) {
-            lo = min(lo, k);
-            hi = k;
-          }
-        }
-        keep = lo < count;
-        ref = static_cast<int>(~(((first + lo) << 3) | (hi - lo)));
-      }
-      if (keep) {
-        work[nOut * kConeThreads] = make_uint2(static_cast<uint32_t>(ref), __float_as_uint(tNode));
-        ++nOut;
+      } else {
+        more = pop();
       }
     }
-    do {  // next deferred entry that does not begin beyond a covering triangle
-      if (--sp < 0) break;
-      const uint2 e = stackAt(sp);
-      node = static_cast<int>(e.x);
-      tNode = __uint_as_float(e.y);
-    } while (tNode > tCover);
-    if (sp < 0) break;
+    if (!more) break;
+    auto emit = [&](int ref) {
+      work[nOut * kConeThreads] = make_uint2(static_cast<uint32_t>(ref), __float_as_uint(tNode));
+      ++nOut;
+    };
+    if (node < 0) {  // a leaf: those of its triangles that the cone meets
+      const uint32_t code = ~static_cast<uint32_t>(node);
+      const uint32_t first = code >> 3, n = (code & 7u) + 1u;
+      uint32_t met = 0;
+      for (uint32_t k = 0; k < n; ++k) {
+        const float4* t = sc.tris + 3 * static_cast<size_t>(first + k);
+        if (coneTriangle(c, __ldg(t), __ldg(t + 1), __ldg(t + 2), fpo, tCover)) met |= 1u << k;
+      }
+      if (nOut + sp + __popc(met) <= kConeEntries) {
+        for (; met; met &= met - 1) emit(~static_cast<int>((first + __ffs(met) - 1) << 3));
+      } else {
+        emit(node);
+      }
+    } else {
+      emit(node);
+    }
+    more = pop();
   }
   // tCover bounds distances, t <= tCover * 1.005 (|direction| != 1).
   uint32_t count = 0;
+  float2* pair = reinterpret_cast<float2*>(out + 1);
   for (int k = 0; k < nOut; ++k) {
     const uint2 e = work[k * kConeThreads];
     const float te = __uint_as_float(e.y);
     if (te > tCover) continue;
+    pair[count] = make_float2(te * 0.995f, __uint_as_float(e.x));
+    if (static_cast<int>(e.x) < 0 && (~e.x & 7u) == 0u) {
+      const float4* t = sc.tris + 3 * static_cast<size_t>(~e.x >> 3);
+      const float4 v0 = __ldg(t), v1 = __ldg(t + 1), v2 = __ldg(t + 2);
+      float4* row = out + kConeRow0 + 3 * count;
+      row[0] = make_float4(xsub(v0.x, c.o.x), xsub(v1.x, c.o.x), xsub(v2.x, c.o.x), v0.w);
+      row[1] = make_float4(xsub(v0.y, c.o.y), xsub(v1.y, c.o.y), xsub(v2.y, c.o.y), v0.w);
+      row[2] = make_float4(xsub(v0.z, c.o.z), xsub(v1.z, c.o.z), xsub(v2.z, c.o.z), v0.w);
+    }
     ++count;
-    out[count] = make_uint2(e.x, __float_as_uint(te * 0.995f));
   }
-  out[0] = make_uint2(count, 0u);
+  out[0] = make_float4(__uint_as_float(count), c.o.x, c.o.y, c.o.z);
 }
 
 // Cone lists of P poses of an eye, list (p, o) at cones + (p * N + o) *
@@ -985,45 +1023,75 @@ __global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye e
            eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
-// Closest hit of a ray of the cone-list path: nd is its normal draw (the
-// angle to the axis in standard deviations).  All lanes of an ommatidium take
-// the list's entries in step, so a triangle's nine coordinates are one
-// broadcast load for the warp and no lane waits for another's traversal.
-// The slab half of the ray set-up is made only for the entries that are
-// subtrees, the shear only when there is something to test.
+// Copies a warp's list into shared memory asynchronously, one float4 a lane:
+// the list of pose p + 1 arrives while pose p is traced.
+static_assert(kConeStride <= 32, "one float4 of a list for each lane");
+__device__ __forceinline__ void fetchCone(const float4* __restrict__ list, float4* __restrict__ dst, uint32_t lane) {
+  if (lane < static_cast<uint32_t>(kConeStride))
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
+                     static_cast<uint32_t>(__cvta_generic_to_shared(dst + lane))),
+                 "l"(list + lane)
+                 : "memory");
+}
+__device__ __forceinline__ void fetchDraw(const float2* __restrict__ src, float2* __restrict__ dst) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void commitCone() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void awaitOlderCone() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+
+// Closest hit of a ray of the cone-list path: list is its ommatidium's list
+// (in shared memory), nd its normal draw (the angle to the axis in standard
+// deviations); org receives the origin.  The lanes of the warp test the
+// list's triangles in step: a test reads three rows in the ray's axis order,
+// without selects or subtractions, and no lane waits for another's
+// traversal.  Entries that are subtrees come last, when most of them begin
+// beyond the hit.
 template <bool kCount>
-__device__ __forceinline__ void traceCone(const DevScene& sc, v3 org, v3 dir, float tmin, float nd,
-                                          const uint2* __restrict__ list, Hit& h, uint32_t* errFlag,
-                                          uint32_t& nodeVisits, uint32_t& triTests) {
+__device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __restrict__ list, v3& org, v3 dir,
+                                          float tmin, float nd, Hit& h, uint32_t* errFlag, uint32_t& nodeVisits,
+                                          uint32_t& triTests) {
   h.t = 1e16f;
   h.id = 0xffffffffu;
   h.pos = 0;
-  const uint32_t listed = __ldg(list).x;
-  const bool root = listed == kConeFromRoot || !(fabsf(nd) <= kConeSigmas);
-  const uint32_t count = root ? 1u : listed;
-  if (count == 0) return;
-  Ray ray;
-  setupShear(ray, org, dir);
-  for (uint32_t k = 0; k < count; ++k) {
-    int node = 0;
-    if (!root) {
-      const uint2 e = __ldg(list + 1 + k);
-      if (!(__uint_as_float(e.y) <= h.t)) continue;
-      node = static_cast<int>(e.x);
-    }
-    if (node < 0) {
-      const uint32_t code = ~static_cast<uint32_t>(node);
-      const uint32_t first = code >> 3, n = (code & 7u) + 1u;
-      if (kCount) triTests += n;
-      for (uint32_t j = 0; j < n; ++j) {
-        const float4* t = sc.tris + 3 * (first + j);
-        testTriangle(ray, __ldg(t), __ldg(t + 1), __ldg(t + 2), first + j, tmin, h);
+  const float4 head = list[0];
+  org = mk(head.y, head.z, head.w);
+  const uint32_t listed = __float_as_uint(head.x);
+  const float2* pair = reinterpret_cast<const float2*>(list + 1);
+  uint32_t later = 0;  // entries (or, bit 31, the root) to search as trees
+  if (listed == kConeFromRoot || !(fabsf(nd) <= kConeSigmas)) {
+    later = 0x80000000u;
+  } else {
+    Ray ray;
+    setupShear(ray, dir);
+    const float4* rows = list + kConeRow0;
+    for (uint32_t k = 0; k < listed; ++k, rows += 3) {
+      const float2 e = pair[k];
+      const int node = __float_as_int(e.y);
+      if (node < 0 && (~node & 7) == 0) {
+        if (!(e.x <= h.t)) continue;
+        if (kCount) ++triTests;
+        const float4 x = rows[ray.kx], y = rows[ray.ky], z = rows[ray.kz];
+        testRelative(ray, x.x, y.x, z.x, x.y, y.y, z.y, x.z, y.z, z.z, __float_as_uint(x.w),
+                     ~static_cast<uint32_t>(node) >> 3, tmin, h);
+      } else {
+        later |= 1u << k;
       }
-    } else {
-      int stack[kStackSize];
-      setupSlabs(ray, org, dir, sc.extent);
-      traverseFrom<kCount>(sc, ray, tmin, h, stack, 0, node, errFlag, nodeVisits, triTests);
     }
+  }
+  while (later) {
+    const int k = __ffs(later) - 1;
+    later &= later - 1;
+    int node = 0;
+    if (k != 31) {
+      const float2 e = pair[k];
+      if (!(e.x <= h.t)) continue;
+      node = __float_as_int(e.y);
+    }
+    const Ray ray = setupRay(org, dir, sc.extent);
+    int stack[kStackSize];
+    traverseFrom<kCount>(sc, ray, tmin, h, stack, 0, node, errFlag, nodeVisits, triTests);
   }
 }
 
@@ -1273,11 +1341,31 @@ __global__ void drawsKernel(DevEye eye, uint32_t P) {
   if (idx >= total) return;
   curandState st;
   loadState(eye.rng, total, idx, st);
-  for (uint32_t p = 0; p < P; ++p) {
+  float2* out = eye.draws + idx;
+  auto one = [&] {
     const float nd = curand_normal(&st);
     const float ud = curand_uniform(&st);
-    eye.draws[static_cast<size_t>(p) * total + idx] = make_float2(nd, ud);
+    *out = make_float2(nd, ud);
+    out += total;
+  };
+  // Pairs of frames: one Box-Muller transform gives both normals, and drawing
+  // the pair without the branch on the cached one lets its arithmetic overlap
+  // the generator's serial chain, which is what bounds this kernel (a thread
+  // per stream).
+  uint32_t p = 0;
+  if (P > 0 && st.boxmuller_flag != 0) {
+    one();
+    p = 1;
   }
+  for (; p + 1 < P; p += 2) {
+    const float2 n = curand_normal2(&st);
+    const float u0 = curand_uniform(&st), u1 = curand_uniform(&st);
+    st.boxmuller_extra = n.y;
+    out[0] = make_float2(n.x, u0);
+    out[total] = make_float2(n.y, u1);
+    out += 2 * total;
+  }
+  if (p < P) one();
   storeState(eye.rng, total, idx, st);
 }
 
@@ -1351,6 +1439,73 @@ __device__ __forceinline__ void flushChunkSums(const float* __restrict__ part, c
   __syncthreads();
 }
 
+// Shared memory of a warp of the cone-list path, in float4: two list buffers,
+// the ommatidium's constants and the lanes' PairStreams (32 x (16 + 8 + 8) B).
+constexpr uint32_t kConeWarpFloat4 = 2 * kConeStride + 3 + 64;
+
+// A lane's random numbers, the same as one curand_normal and one
+// curand_uniform per frame: the stream of a pair of frames is drawn at once
+// (one Box-Muller transform gives both normals) without the per-frame branch
+// on the cached normal, and the generator waits in shared memory instead of
+// eight registers.
+struct PairStream {
+  uint4* a;      // d, v0, v1, v2
+  uint2* b;      // v3, v4
+  float2* ahead;  // the second frame's numbers; .x keeps the last cached normal
+  bool ready;     // ahead holds the next frame
+  int flag;       // cached-normal flag of the state to store
+
+  // With pre-drawn numbers: where those of pose p wait.
+  __device__ __forceinline__ float2* drawSlot(uint32_t p) const {
+    return p & 1u ? ahead : reinterpret_cast<float2*>(b);
+  }
+  __device__ __forceinline__ void load(curandState& st) const {
+    const uint4 x = *a;
+    const uint2 y = *b;
+    st.d = x.x;
+    st.v[0] = x.y;
+    st.v[1] = x.z;
+    st.v[2] = x.w;
+    st.v[3] = y.x;
+    st.v[4] = y.y;
+  }
+  __device__ __forceinline__ void save(const curandState& st) const {
+    *a = make_uint4(st.d, st.v[0], st.v[1], st.v[2]);
+    *b = make_uint2(st.v[3], st.v[4]);
+  }
+  __device__ __forceinline__ void begin(curandState& st) {
+    ready = st.boxmuller_flag != 0;  // an odd number of frames so far: its normal is cached
+    flag = 0;
+    float u = 0.f;
+    if (ready) u = curand_uniform(&st);
+    *ahead = make_float2(st.boxmuller_extra, u);
+    save(st);
+  }
+  // The next frame's numbers; more: another frame follows.
+  __device__ __forceinline__ float2 next(bool more) {
+    if (ready) {
+      ready = false;
+      return *ahead;
+    }
+    curandState st;
+    load(st);
+    const float2 n = curand_normal2(&st);
+    const float u = curand_uniform(&st);
+    float u2 = 0.f;
+    if (more) u2 = curand_uniform(&st);
+    ready = more;
+    flag = more ? 0 : 1;
+    *ahead = make_float2(n.y, u2);
+    save(st);
+    return make_float2(n.x, u);
+  }
+  __device__ __forceinline__ void end(curandState& st) const {
+    load(st);
+    st.boxmuller_flag = flag;
+    st.boxmuller_extra = ahead->x;
+  }
+};
+
 // kMode: 0 = render, 1 = render and record every ray, 2 = render and count
 // node visits / triangle tests into stats[0..1].  kMinBlocks: resident
 // 128-thread blocks per SM the register allocation is sized for (the
@@ -1369,11 +1524,13 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
                                            uint32_t P, const WarpPlan& plan, uint64_t task, float* __restrict__ out,
                                            float* __restrict__ scratch, uint32_t* errFlag,
                                            RayRecord* __restrict__ rec, uint32_t& nodeVisits, uint32_t& triTests,
-                                           float* __restrict__ part = nullptr) {
+                                           float* __restrict__ part = nullptr, float4* __restrict__ coneSmem = nullptr) {
   constexpr bool kRecord = (kMode & 3) == 1;
   constexpr bool kFeat = (kMode & 3) == 3;
   constexpr bool kCount = (kMode & 3) == 2 || kFeat;  // feature mode: the per-entry traversal cost
   constexpr bool kLit = (kMode & 4) != 0;  // lighting-on shading (modes 4 render, 5 record)
+  // Cone lists are for whole-warp segments (renderConeLists).
+  const uint32_t segWidth = kCone ? 32u : plan.segWidth, ommPerWarp = kCone ? 1u : plan.ommPerWarp;
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t p0 = 0, p1 = P;
   if (plan.poseSplits > 1) {
@@ -1385,9 +1542,10 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
   }
   const uint32_t group = static_cast<uint32_t>(task / plan.chunks);
   const uint32_t chunk = static_cast<uint32_t>(task % plan.chunks);
-  const uint32_t slot = group * plan.ommPerWarp + lane / plan.segWidth;
+  const uint32_t segLane = lane & (segWidth - 1u);  // segments are powers of two
+  const uint32_t slot = group * ommPerWarp + lane / segWidth;
   const uint32_t o = (eye.order && slot < eye.N) ? __ldg(eye.order + slot) : slot;
-  const uint32_t s = chunk * plan.segWidth + lane % plan.segWidth;
+  const uint32_t s = chunk * segWidth + segLane;
   const bool valid = slot < eye.N && s < eye.spp;
   const size_t plane = static_cast<size_t>(eye.N) * eye.spp;
   const size_t sidx = static_cast<size_t>(o) * eye.spp + s;
@@ -1400,7 +1558,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     dst0 = out + static_cast<size_t>(o) * 3;
     dstStride = static_cast<size_t>(eye.N) * 3;
   } else if (part) {  // pose p's partial at (p - p0) % kInBlockPoses of the group
-    const uint32_t gs = (group % plan.groupsPerBlock) * plan.ommPerWarp + lane / plan.segWidth;
+    const uint32_t gs = (group % plan.groupsPerBlock) * ommPerWarp + lane / segWidth;
     dst0 = part + (static_cast<size_t>(gs) * kInBlockPoses * plan.chunks + chunk) * 3;
     dstStride = static_cast<size_t>(plan.chunks) * 3;
   } else {
@@ -1423,11 +1581,51 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     // its test on the component sum.
     perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
     perp = (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
-    relPos = pos - normalize(axis) * fpo;
+    relPos = relativeOrigin(pos, axis, fpo);
   }
   const float invSpp = 1.0f / static_cast<float>(eye.spp);
+  // The cone-list path keeps what is the same for a whole pose loop in shared
+  // memory, so that the loop's registers hold the ray.
+  float4* fixed = kCone ? coneSmem + (threadIdx.x >> 5) * kConeWarpFloat4 + 2 * kConeStride : nullptr;
+  PairStream pair{reinterpret_cast<uint4*>(fixed + 3) + lane, reinterpret_cast<uint2*>(fixed + 3 + 32) + lane,
+                  reinterpret_cast<float2*>(fixed + 3 + 48) + lane, false, 0};
+  if (kCone) {
+    if (valid && !eye.draws) pair.begin(st);
+    if (lane == 0) {
+      const v3 c = cross(perp, axis);
+      fixed[0] = make_float4(axis.x, axis.y, axis.z, sd);
+      fixed[1] = make_float4(perp.x, perp.y, perp.z, dot(perp, axis));
+      fixed[2] = make_float4(c.x, c.y, c.z, fpo);
+    }
+  }
+  // Cone lists: the warp's two buffers in shared memory, and the list to
+  // fetch next; pre-drawn numbers come the same way, into the slots that a
+  // PairStream would use.
+  float4* coneBuf = nullptr;
+  const float4* coneNext = nullptr;
+  const float2* drawNext = nullptr;
+  if (kCone) {
+    coneBuf = coneSmem + (threadIdx.x >> 5) * kConeWarpFloat4;
+    coneNext = eye.cones + (static_cast<size_t>(p0) * eye.N + o) * kConeStride;
+    if (slot < eye.N) fetchCone(coneNext, coneBuf + (p0 & 1u) * kConeStride, lane);
+    if (eye.draws) drawNext = eye.draws + (static_cast<size_t>(p0) * eye.N + o) * eye.spp + s;
+    if (eye.draws && valid) fetchDraw(drawNext, pair.drawSlot(p0));
+    commitCone();
+  }
 
   for (uint32_t p = p0; p < p1; ++p) {
+    if (kCone) {
+      __syncwarp();  // every lane has read the buffer that is filled next
+      coneNext += static_cast<size_t>(eye.N) * kConeStride;
+      if (slot < eye.N && p + 1 < p1) fetchCone(coneNext, coneBuf + ((p + 1) & 1u) * kConeStride, lane);
+      if (eye.draws) {
+        drawNext += plane;
+        if (valid && p + 1 < p1) fetchDraw(drawNext, pair.drawSlot(p + 1));
+      }
+      commitCone();
+      awaitOlderCone();
+      __syncwarp();
+    }
     v3 col = mk(0.f, 0.f, 0.f);
     // Feature mode: per-sample squared colour, hit flag, hit distance and the
     // hit triangle's normal in the eye's frame (facing the ray), all / spp.
@@ -1441,25 +1639,48 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         const float2 dr = netDraw(eye.drawSeed, (eye.frame0 + p) * eye.N + o, s);
         nd = dr.x;
         ud = dr.y;
+      } else if (eye.draws && kCone) {
+        const float2 dr = *pair.drawSlot(p);
+        nd = dr.x;
+        ud = dr.y;
       } else if (eye.draws) {
         const float2 dr = eye.draws[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s];
+        nd = dr.x;
+        ud = dr.y;
+      } else if (kCone) {
+        const float2 dr = pair.next(p + 1 < p1);
         nd = dr.x;
         ud = dr.y;
       } else {
         nd = curand_normal(&st);
         ud = curand_uniform(&st);
       }
+      if (kCone) {
+        const float4 f0 = fixed[0], f2 = fixed[2];
+        axis = mk(f0.x, f0.y, f0.z);
+        sd = f0.w;
+        fpo = f2.w;
+      }
       const float splayAngle = nd * sd;
       const float axisAngle = ud * CR_PI_F;
-      const v3 splayed = rotatePoint(axis, splayAngle, perp);
+      v3 splayed;
+      if (kCone) {  // rotatePoint(axis, splayAngle, perp)
+        const float4 f1 = fixed[1], f2 = fixed[2];
+        splayed = cosf(splayAngle) * axis + sinf(splayAngle) * mk(f2.x, f2.y, f2.z) +
+                  (1 - cosf(splayAngle)) * f1.w * mk(f1.x, f1.y, f1.z);
+      } else {
+        splayed = rotatePoint(axis, splayAngle, perp);
+      }
       const v3 rel = rotatePoint(splayed, axisAngle, axis);
-      const v3 org = mk(P0.x, P0.y, P0.z) + mk(X.x, X.y, X.z) * relPos.x + mk(Y.x, Y.y, Y.z) * relPos.y +
-                     mk(Z.x, Z.y, Z.z) * relPos.z;
       const v3 dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
       Hit h;
+      v3 org;
+      if (kCone) {  // the list holds the origin
+        traceCone<kCount>(sc, coneBuf + (p & 1u) * kConeStride, org, dir, fpo, nd, h, errFlag, nodeVisits, triTests);
+      } else {
+        org = rayOrigin(mk(P0.x, P0.y, P0.z), mk(X.x, X.y, X.z), mk(Y.x, Y.y, Y.z), mk(Z.x, Z.y, Z.z), relPos);
+      }
       if (kCone) {
-        traceCone<kCount>(sc, org, dir, fpo, nd, eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride, h,
-                          errFlag, nodeVisits, triTests);
       } else if (kWidth != 2) {
         const Ray ray = setupRay(org, dir, sc.extent);
         h.t = 1e16f;
@@ -1528,7 +1749,27 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       }
     }
     // Segmented butterfly reduction over the samples of each ommatidium.
-    for (uint32_t m = plan.segWidth >> 1; m >= 1u; m >>= 1) {
+    if constexpr (kCone) {
+      // Whole-warp segments: the same pairwise sums with 6 exchanges in place
+      // of 15.  After the first step the halves of the warp hold the sums of
+      // x and y, after the second the quarters x, z, y, z.
+      const float give = lane & 16u ? col.x : col.y;
+      const float zz = col.z + __shfl_xor_sync(0xffffffffu, col.z, 16);
+      const float xy = (lane & 16u ? col.y : col.x) + __shfl_xor_sync(0xffffffffu, give, 16);
+      const float give8 = lane & 8u ? xy : zz;
+      float v = (lane & 8u ? zz : xy) + __shfl_xor_sync(0xffffffffu, give8, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 4);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      // lane 0 holds x, lane 16 y, lane 8 z
+      float* dst = dst0 + (part ? (p - p0) % kInBlockPoses : p) * dstStride;
+      if ((lane & 7u) == 0u && lane != 24u && o < eye.N) dst[lane == 0u ? 0 : (lane == 16u ? 1 : 2)] = v;
+      if (part && ((p - p0 + 1) % kInBlockPoses == 0 || p + 1 == p1)) {
+        const uint32_t pg0 = p0 + (p - p0) / kInBlockPoses * kInBlockPoses;
+        flushChunkSums(part, plan, eye, out, pg0, p + 1 - pg0);
+      }
+    } else {
+    for (uint32_t m = segWidth >> 1; m >= 1u; m >>= 1) {
       col.x += __shfl_xor_sync(0xffffffffu, col.x, static_cast<int>(m));
       col.y += __shfl_xor_sync(0xffffffffu, col.y, static_cast<int>(m));
       col.z += __shfl_xor_sync(0xffffffffu, col.z, static_cast<int>(m));
@@ -1545,7 +1786,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       }
     }
     if (kFeat) {
-      if ((lane % plan.segWidth) == 0u && o < eye.N) {
+      if (segLane == 0u && o < eye.N) {
         float* dst = out + (static_cast<size_t>(p) * eye.N + o) * kFeatureStats;
         dst[0] = col.x;
         dst[1] = col.y;
@@ -1562,7 +1803,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       }
       continue;
     }
-    if ((lane % plan.segWidth) == 0u && o < eye.N) {
+    if (segLane == 0u && o < eye.N) {
       float* dst = dst0 + (part ? (p - p0) % kInBlockPoses : p) * dstStride;
       dst[0] = col.x;
       dst[1] = col.y;
@@ -1575,8 +1816,12 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       const uint32_t pg0 = p0 + (p - p0) / kInBlockPoses * kInBlockPoses;
       flushChunkSums(part, plan, eye, out, pg0, p + 1 - pg0);
     }
+    }
   }
-  if (!kFeat && valid && !eye.draws) storeState(eye.rng, plane, sidx, st);
+  if (!kFeat && valid && !eye.draws) {
+    if (kCone) pair.end(st);
+    storeState(eye.rng, plane, sidx, st);
+  }
 }
 
 // kRegs: registers per thread the kernel is compiled for (the autotuner's
@@ -1592,14 +1837,18 @@ __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const f
                                                 WarpPlan plan, float* __restrict__ out, float* __restrict__ scratch,
                                                 uint32_t* errFlag, RayRecord* __restrict__ rec,
                                                 unsigned long long* stats) {
-  extern __shared__ float chunkPart[];
+  // kCone: the warps' cone lists; kInBlock: then the block's chunk partials.
+  extern __shared__ float4 renderSmem[];
   constexpr bool kCount = kMode == 2;
   uint32_t nodeVisits = 0, triTests = 0;
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t task = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (task >= plan.tasks) return;  // whole warps exit together (never with inBlock: whole blocks)
   renderTask<kMode, kWidth, kCone>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits, triTests,
-                                   kInBlock ? chunkPart : nullptr);
+                                   kInBlock ? reinterpret_cast<float*>(
+                                                  renderSmem + (kCone ? (blockDim.x >> 5) * kConeWarpFloat4 : 0))
+                                            : nullptr,
+                                   renderSmem);
   if (kCount) {
     unsigned long long nv = nodeVisits, tt = triTests;
     for (int m = 16; m >= 1; m >>= 1) {
@@ -2025,8 +2274,12 @@ WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, boo
   }
   uint32_t bw = g_blockThreads / 32;
   if (bw == 0) {
+    // The automatic layout sums chunks in the block only where that saves the
+    // second launch (few poses): on long launches the block's barriers cost
+    // more than the partials' round trip (256 terrain poses: 7.3 ms with
+    // 256-thread blocks and sums in the block, 6.9 ms with 128 and scratch).
     bw = 4;
-    if (p.chunks > 1 && !forceScratch && inBlockAllowed)
+    if (p.chunks > 1 && P <= kInBlockPoses && !forceScratch && inBlockAllowed)
       for (uint32_t c : {4u, 8u, 16u})
         if (p.chunks <= c && c % p.chunks == 0) {
           bw = c;
@@ -2085,8 +2338,21 @@ static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool con
   return !stats && !scene.lighting && cones;
 }
 
+// When a launch uses cone lists: whole-warp segments (more than 16 samples in
+// the default layout; a warp then holds one list), and enough rays to hide
+// the ~20-35 us that the first list takes to build.  The line lies at 2^19
+// rays on deep trees and at 2^21 on shallow ones, whose traversals are
+// shorter.  Speed-up with lists over without (64 registers), terrain / box
+// scene, by rays: 0.3 M 0.95 / 0.82, 0.5 M 1.2 / 0.9, 1 M 1.3 / 0.93, 2 M
+// 1.5 / 1.1, 6 M 2.7 / 1.5, 82 M 3.6 / 2.0; at acceptance angles of 6 degrees
+// 82 M 3.0 / 1.6.
+constexpr uint32_t kConeDeepTris = 16384;
+constexpr uint64_t kConeRaysDeep = 1ull << 19, kConeRaysShallow = 1ull << 21;
+
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec) {
-  if (scene.triCount == 0 || spp < kConeMinSamples) return 0;
+  const uint64_t rays = static_cast<uint64_t>(N) * spp * P;
+  if (scene.triCount == 0 || rays < (scene.triCount >= kConeDeepTris ? kConeRaysDeep : kConeRaysShallow)) return 0;
+  if (planRender(N, spp, P, true).segWidth != 32) return 0;
   if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
   return static_cast<size_t>(P) * N;
 }
@@ -2124,20 +2390,25 @@ cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const floa
   const unsigned block = 32u * plan.blockWarps;
   const uint64_t blocks = (plan.tasks + plan.blockWarps - 1) / plan.blockWarps;
   if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
-  size_t smem = 0;
-  if (kInBlock) {
-    smem = static_cast<size_t>(plan.groupsPerBlock) * plan.ommPerWarp * kInBlockPoses * plan.chunks * 3 * sizeof(float);
-    if (smem > 48 * 1024) {
-      const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock, kCone>,
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(kChunkSmemMax));
-      if (e != cudaSuccess) return e;
-    }
+  size_t smem = kCone ? plan.blockWarps * kConeWarpFloat4 * sizeof(float4) : 0;
+  if (kInBlock)
+    smem += static_cast<size_t>(plan.groupsPerBlock) * plan.ommPerWarp * kInBlockPoses * plan.chunks * 3 * sizeof(float);
+  if (smem > 48 * 1024) {
+    const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock, kCone>,
+                                               cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    if (e != cudaSuccess) return e;
   }
   renderKernel<kMode, kRegs, kWidth, kInBlock, kCone><<<static_cast<unsigned>(blocks), block, smem, stream>>>(
       scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats);
   return cudaGetLastError();
 }
+
+// Register budget of the plain render through cone lists.  Its loop needs
+// fewer than the tree search does: on 256 terrain poses x 6000 ommatidia x
+// 256 samples 48, 56, 64, 72, 80 and 96 registers take 7.6, 7.0, 6.9, 6.9,
+// 7.8 and 9.7 ms, and 64 is also the fastest on the box scene (1000 x 32), so
+// the variants (renderVariant) are for renders without lists.
+constexpr int kConeRegs = 64;
 
 // The instance for the two-wide BVH: through the cone lists when the eye has
 // them (with in-block chunk sums where the plan says so; planRender offers
@@ -2146,8 +2417,8 @@ template <int kMode, int kRegs>
 cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                       const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                       unsigned long long* stats, cudaStream_t stream) {
-  constexpr bool kHasInBlock = kMode == 0 || kMode == 1;
-  constexpr bool kHasCone = kMode != 3;
+  constexpr bool kHasCone = kMode == 0 ? kRegs == kConeRegs : kMode != 3;
+  constexpr bool kHasInBlock = kHasCone && (kMode == 0 || kMode == 1);
   if (plan.inBlock) {
     if (!kHasInBlock || !eye.cones) return cudaErrorInvalidValue;
     return runRenderKernel<kMode, kRegs, 2, kHasInBlock, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag,
@@ -2167,6 +2438,8 @@ cudaError_t runRenderWidth(const DevScene& scene, const DevEye& eye, const float
                            const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag,
                            unsigned long long* stats, cudaStream_t stream) {
   if (scene.width != 2 && (plan.inBlock || eye.cones)) return cudaErrorInvalidValue;
+  if (kMode == 0 && eye.cones)  // one register budget: see kConeRegs
+    return runRender<kMode, kConeRegs>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr, stats, stream);
   switch (scene.width) {
     case 4:
       return runRenderKernel<kMode, kRegs, 4, false, false>(scene, eye, poses, P, plan, out, scratch, errFlag, nullptr,
@@ -2194,7 +2467,10 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     drawsKernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(eye, P);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    plan = splitPoses(plan, P);
+    // With cone lists a task is short: twice the tasks, for a smaller last wave
+    // (1000 poses x 1000 ommatidia x 32 samples of the box scene: 1.28 ms
+    // against 1.37 at the same number, and 1.32 at four times).
+    plan = splitPoses(plan, P, eye.cones ? 2 * kFillWarps : kFillWarps);
   }
   if (eye.cones) {
     const uint64_t lists = static_cast<uint64_t>(P) * eye.N, blocks = (lists + kConeThreads - 1) / kConeThreads;

@@ -169,7 +169,11 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
  * (8, 16, 32), then the near-field cut radius, keeping the fastest of each;
  * a non-zero best radius is refined by trying it divided and multiplied by
  * sqrt(2).  Last it times the BVH widths 4 and 8 (crSetBvhWidth) against the
- * two-wide BVH with its best cut, and keeps the fastest tree.
+ * two-wide BVH with its best cut, and keeps the fastest tree.  Long renders
+ * of more than 16 samples go through cone lists (what an ommatidium's samples
+ * can hit first at a pose, found once for all of them) and depend on neither
+ * the variant nor the radius: those two are timed, and kept, for the renders
+ * without lists.
  * crGetAutotuneTimes copies its timings (ms): variants 0-2, blocks 128 / 256
  * / 512, samples per warp 8 / 16 / 32, cut radius 0, 1/256, 1/128, 1/64,
  * 1/32, 1/16 of the scene extent, BVH width 2 / 4 / 8, and the refinement's
@@ -177,9 +181,9 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
  * radius was 0). */
 int crGetAutotuneTimes(float* ms, size_t n);
 /* No counterpart in the reference.  Layout of the render kernel: block size
- * in threads (0 = the smallest of 128 / 256 / 512 holding all 32-sample
- * chunk warps of an ommatidium, whose chunk sums then stay in shared memory;
- * else 128) and samples per warp segment (8, 16 or 32; below 32 a warp
+ * in threads (0 = 128, or, for up to 16 poses through cone lists, the smallest
+ * of 128 / 256 / 512 holding all 32-sample chunk warps of an ommatidium, whose
+ * chunk sums then stay in shared memory) and samples per warp segment (8, 16 or 32; below 32 a warp
  * holds several ommatidia, and the samples are summed in another order:
  * results change within float rounding).  The block size changes no result.
  * Also used by batches created afterwards.  0 on success. */
@@ -190,6 +194,7 @@ int crGetRenderLayout(int* blockThreads, int* samplesPerWarp);
  * ray searches first (0 = off, the default).  A hit found there within the
  * ball is final; other rays continue from the root, so results never depend
  * on it.  crAutotune also picks this radius among 0 and 1/256 .. 1/16.
+ * Renders through cone lists do not use it.
  * No counterpart in the reference. */
 int crSetCutRadius(float fractionOfExtent);
 /* Lighting-on shading (shaders.cu:812-880): 1 = the GGX/Smith path with four

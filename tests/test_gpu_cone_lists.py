@@ -1,0 +1,151 @@
+"""Renders through cone lists against renders that search the BVH from its root.
+
+crRenderPosesDevice builds, for launches with many rays, a list per (pose,
+ommatidium) of what that ommatidium's samples can hit first;
+crRenderPosesDeviceNoAlloc never does.  Both find the same closest hits and
+sum them in the same order, so their results are equal bit for bit, for any
+eye and pose.
+"""
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+import eyeRendererHelperFunctions as eh
+import scenes
+
+pytestmark = pytest.mark.gpu
+
+# spp: the smallest that fills a warp segment, tails of one sample, one
+# chunk, several chunks in a block, chunks that no block holds.
+SPP = [17, 31, 32, 33, 64, 96, 256, 300, 513]
+
+
+def _eye(n, kind):
+    rng = np.random.default_rng(n)
+    d = scenes.fibonacci_sphere(n)
+    omm = np.zeros((n, 8), np.float32)
+    omm[:, 0:3], omm[:, 3:6] = d * 0.001, d
+    omm[:, 6] = np.radians(rng.uniform(0.5, 6.0, n))
+    if kind == "odd":  # axes on the coordinate planes, wide, narrow, negative and zero cones, offsets, long axes
+        s = math.sqrt(0.5)
+        omm[:6, 3:6] = [[0, 1, 0], [0, -1, 0], [s, 0, s], [1, 0, 0], [0, 0, -1], [-s, 0, -s]]
+        omm[6:12, 6] = np.radians([60.0, 25.0, 0.0, -3.0, 1e-4, 179.0])
+        omm[12:40, 7] = np.linspace(-0.01, 0.02, 28)
+        omm[40:50, 3:6] *= np.linspace(0.5, 2.0, 10)[:, None].astype(np.float32)
+        omm[50:60, 3:6] *= np.float32(1.0004)
+        omm[60, 3:6] = 0.0
+        omm[61, 6] = np.nan
+    return omm
+
+
+def _poses(boxes, count, seed):
+    p = scenes.open_poses(boxes, count, np.random.default_rng(seed))
+    p16 = np.zeros((count, 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = p[:, 3 * k:3 * k + 3]
+    p16[0, 1] = 0.0  # on the ground plane
+    p16[1, 0:3] = boxes[0].mean(axis=0)  # inside a box
+    p16[2, 0:3] = boxes[1][1]  # on a box's corner
+    p16[3, 4:7] *= 1.0004  # a frame within the lists' tolerance, and three outside it
+    p16[4, 4:16] *= 2.0
+    p16[5, 4:7] = p16[5, 8:11]
+    p16[6, 8:11] = 0.0
+    p16[7, 0:3] = [500.0, 300.0, -900.0]  # far outside
+    p16[8, 0] = np.nan
+    return p16
+
+
+def _render(lib, fn, d_poses, P, n):
+    import torch
+
+    out = torch.full((P, n, 3), -1.0, device="cuda")
+    torch.cuda.synchronize()
+    assert fn(d_poses.data_ptr(), P, out.data_ptr()) == 0, eh.lastError(lib)
+    assert lib.crSynchronize() == 0, eh.lastError(lib)
+    return out.cpu().numpy()
+
+
+def _both(lib, omm, spp, p16):
+    """Frames of both entry points from the same random streams, after one
+    frame through each path's set-up, and the streams they leave."""
+    import torch
+
+    n, P = len(omm), len(p16)
+    d_poses = torch.from_numpy(p16).cuda()
+    res = []
+    for fn in (lib.crRenderPosesDevice, lib.crRenderPosesDeviceNoAlloc):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        _render(lib, lib.crRenderPosesDevice, d_poses, 1, n)  # one frame: odd, so a normal is cached
+        held = lib.crGetDeviceMemoryHeld()
+        a = _render(lib, fn, d_poses, P, n)
+        b = _render(lib, fn, d_poses, 1, n)
+        states = np.zeros(8 * n * spp, np.uint32)
+        assert lib.crGetRandomStates(states) == 0
+        res.append((a, b, states, lib.crGetDeviceMemoryHeld() - held))
+    return res
+
+
+@pytest.mark.parametrize("kind", ["plain", "odd"])
+@pytest.mark.parametrize("spp", SPP)
+def test_lists_change_no_bit(lib, small, kind, spp):
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(small["gltf"].encode())
+    eh.gotoFirstCompoundEye(lib)
+    n = 701
+    P = 2 + 2 ** 21 // (n * spp)  # just past the fewest rays that use lists
+    if P < 9:
+        n, P = 2 ** 21 // (9 * spp) + 1, 9
+    with_lists, without = _both(lib, _eye(n, kind), spp, _poses(small["boxes"], P, spp))
+    assert with_lists[3] >= 400 * n * P and without[3] == 0  # the first did build lists
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
+
+
+def test_lists_of_a_single_leaf_scene(lib, tmp_path):
+    """A scene that is one BVH leaf (the root's second child is a dummy)."""
+    g = scenes.GltfBuilder()
+    v, f = scenes.box_mesh([-1.0, 0.0, -1.0], [1.0, 1.0, 1.0])
+    g.mesh("ground", v, f[:7], colours=np.random.default_rng(1).uniform(0, 1, (8, 4)))
+    d = scenes.fibonacci_sphere(10)
+    scenes.write_eye(str(tmp_path / "e.eye"), d * 0.001, d, 0.05, 0.0)
+    g.compound_camera("eye", "e.eye")
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(g.write(str(tmp_path / "one.gltf")).encode())
+    assert eh.lastError(lib) == ""
+    eh.gotoFirstCompoundEye(lib)
+    p = np.zeros((64, 16), np.float32)
+    rng = np.random.default_rng(2)
+    p[:, 0:3] = rng.uniform(-2.0, 2.0, (64, 3))
+    p[:, 4] = p[:, 9] = p[:, 14] = 1.0
+    with_lists, without = _both(lib, _eye(1100, "plain"), 32, p)
+    assert with_lists[3] > 0
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y)
+
+
+def test_lists_give_way_under_a_memory_cap(lib, small):
+    """Lists are dropped, not the render, when their memory is not to be had."""
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(small["gltf"].encode())
+    eh.gotoFirstCompoundEye(lib)
+    omm, p16 = _eye(800, "plain"), _poses(small["boxes"], 90, 3)
+    want = _both(lib, omm, 64, p16)[0][0]
+    lib.loadGlTFscene(small["gltf"].encode())  # gives back every buffer
+    eh.gotoFirstCompoundEye(lib)
+    lib.setOmmatidia(omm.ctypes.data, len(omm))
+    lib.setCurrentEyeSamplesPerOmmatidium(64)
+    import torch
+
+    d_poses = torch.from_numpy(p16).cuda()
+    _render(lib, lib.crRenderPosesDevice, d_poses, 1, len(omm))
+    # room for the partials and pre-drawn numbers of the launch, not for the lists
+    need = 4 * 90 * 800 * 2 * 3 + 8 * 90 * 800 * 64
+    assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + need + (1 << 20)) == 0
+    try:
+        got = _render(lib, lib.crRenderPosesDevice, d_poses, 90, len(omm))
+    finally:
+        lib.crSetDeviceMemoryCap(0)
+    assert np.array_equal(got, want, equal_nan=True)
