@@ -174,6 +174,9 @@ size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint
 // Cone lists (DevEye::cones, kConeStride float4 each) worth providing for a
 // P-pose launch: P x N, or 0 when the launch does not use them.
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false);
+// The same for an eye of a batch with that plan; batchRays: the rays of the
+// whole batch.
+size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, uint32_t P, uint64_t batchRays);
 
 cudaError_t launchRngInit(const DevEye& eye, uint32_t* errFlag, cudaStream_t stream);
 
@@ -322,19 +325,35 @@ struct BatchEye {
   uint32_t P;
 };
 
-// Resident blocks per SM of the batch kernel for a render variant.
-int batchBlocksPerSM(int variant);
+// Resident blocks per SM of the batch kernel for a render variant and BVH
+// width; cones: some eye has cone lists.
+int batchBlocksPerSM(int variant, int width, bool cones);
 
-// Persistent launch over all eyes' warp tasks (taskBase: nEyes ascending
-// task offsets) followed by the chunk sums of the eyes with chunks > 1
-// (cellBase: nEyes ascending offsets into their P*N cells).  ctrl must hold
-// 2 + nEyes words, set to {0, ~0, 0...} before the launch.  cutPoses > 0:
-// first build the near-field cuts of the eyes whose DevEye::cuts is set
-// (cutPoses poses per eye, each eye's cuts laid out like a plain launch's).
-cudaError_t launchBatch(const DevScene& scene, const BatchEye* eyes, const unsigned long long* taskBase,
-                        const unsigned long long* cellBase, uint32_t nEyes, unsigned long long totalTasks,
-                        unsigned long long totalCells, unsigned long long* ctrl, uint32_t* errFlag, int variant,
-                        int gridBlocks, uint32_t cutPoses, cudaStream_t stream);
+// Device tables of a batch: its eyes, and per eye ascending offsets into
+//  taskBaseLists / taskBaseOther  the warp tasks of the eyes with / without
+//                                 cone lists (the other kind's eyes have none),
+//  cellBase                       the P*N cells of the eyes with chunks > 1,
+//  coneBase                       the P*N lists of the eyes with cone lists,
+// with the totals.
+struct BatchTables {
+  const BatchEye* eyes = nullptr;
+  const unsigned long long* taskBaseLists = nullptr;
+  const unsigned long long* taskBaseOther = nullptr;
+  const unsigned long long* cellBase = nullptr;
+  const unsigned long long* coneBase = nullptr;
+  unsigned long long tasksLists = 0, tasksOther = 0, cells = 0, lists = 0;
+  uint32_t nEyes = 0;
+};
+// The cone lists, the persistent launch over the warp tasks of the eyes that
+// have them, the one over the other eyes' (each with the given number of
+// blocks), and the chunk sums; parts without work are left out.  ctrl must
+// hold 3 + nEyes words, set to {0, ~0, 0...} before the launch: two task
+// counters (first and last), the start and the eyes' completion times.
+// cutPoses > 0: first build the near-field cuts of the eyes whose
+// DevEye::cuts is set (cutPoses poses per eye, each eye's cuts laid out like a
+// plain launch's).
+cudaError_t launchBatch(const DevScene& scene, const BatchTables& b, unsigned long long* ctrl, uint32_t* errFlag,
+                        int variant, int blocksLists, int blocksOther, uint32_t cutPoses, cudaStream_t stream);
 
 // Adaptive sampling (render.cu).  An entry e = pose * N + ommatidium is
 // rendered at its bucket's sample count; buckets hold counts 4 << index.

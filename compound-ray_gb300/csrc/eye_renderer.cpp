@@ -193,6 +193,7 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
 
 constexpr uint32_t kMaxPosesPerLaunch = 256;
 constexpr size_t kConeListBytes = size_t(1) << 30;  // cone lists of one launch at most
+constexpr size_t kBatchConeBytes = size_t(4) << 30;  // cone lists of one batch at most
 constexpr size_t kTuneSlots = 20;
 
 // Order in which warp segments take an eye's ommatidia: by the 30-bit Morton
@@ -718,14 +719,16 @@ struct Batch {
   size_t P = 0;
   std::vector<size_t> outOffset;  // floats, per camera
   DevBuf<BatchEye> table;
-  DevBuf<unsigned long long> taskBase, cellBase, ctrl;
+  DevBuf<unsigned long long> bases;  // BatchTables' four offset tables, nEyes each
+  DevBuf<unsigned long long> ctrl;
   DevBuf<float> scratch;
   DevBuf<float4> cuts;  // per eye P x kCutStride, when the near-field cut is on
+  DevBuf<float4> cones;  // cone lists of the eyes that use them
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
-  unsigned long long totalTasks = 0, totalCells = 0;
+  BatchTables tables;
   uint32_t cutPoses = 0;
-  int variant = 0, grid = 0;
+  int variant = 0;
   uint64_t generation = 0;
   void release() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -733,11 +736,11 @@ struct Batch {
     exec = nullptr;
     graph = nullptr;
     table.release();
-    taskBase.release();
-    cellBase.release();
+    bases.release();
     ctrl.release();
     scratch.release();
     cuts.release();
+    cones.release();
   }
 };
 
@@ -1421,7 +1424,7 @@ int crBatchCreate(const int* cams, size_t nCams, size_t posesPerCam, const float
         b.cams.assign(cams, cams + nCams);
         b.P = posesPerCam;
         std::vector<BatchEye> table(nCams);
-        std::vector<unsigned long long> tb(nCams), cb(nCams);
+        std::vector<unsigned long long> bases(4 * nCams);  // lists' tasks, other tasks, cells, lists
         size_t outOff = 0, scratchFloats = 0;
         // The near-field cut radius in force now is recorded into the graph.
         r.ensureUploaded();
@@ -1452,15 +1455,9 @@ int crBatchCreate(const int* cams, size_t nCams, size_t posesPerCam, const float
             be.eye.cutRadius = r.cutFactor * r.dev.extent;
             be.eye.maxRel = e.maxRel;
           }
-          tb[i] = b.totalTasks;
-          cb[i] = b.totalCells;
           b.outOffset.push_back(outOff);
           outOff += 3 * posesPerCam * e.N;
-          b.totalTasks += e.N ? be.plan.tasks * 1ull : 0ull;
-          if (be.plan.chunks > 1 && e.N) {
-            scratchFloats += posesPerCam * e.N * be.plan.chunks * 3;
-            b.totalCells += static_cast<unsigned long long>(posesPerCam) * e.N;
-          }
+          if (be.plan.chunks > 1 && e.N) scratchFloats += posesPerCam * e.N * be.plan.chunks * 3;
         }
         if (scratchFloats) b.scratch.ensure(scratchFloats);
         size_t so = 0;
@@ -1470,29 +1467,57 @@ int crBatchCreate(const int* cams, size_t nCams, size_t posesPerCam, const float
             so += posesPerCam * table[i].eye.N * table[i].plan.chunks * 3;
           }
         b.table.ensure(nCams);
-        b.taskBase.ensure(nCams);
-        b.cellBase.ensure(nCams);
-        b.ctrl.ensure(2 + nCams);
+        b.bases.ensure(4 * nCams);
+        b.ctrl.ensure(3 + nCams);
+        // Cone lists of the eyes that use them, as far as kBatchConeBytes goes
+        // and when that memory is to be had.
+        BatchTables& bt = b.tables;
+        uint64_t batchRays = 0;
+        for (const BatchEye& be : table) batchRays += static_cast<uint64_t>(be.eye.N) * be.eye.spp * be.P;
+        std::vector<size_t> lists(nCams, 0);
+        for (size_t i = 0; i < nCams; ++i) {
+          const size_t n = batchConeLists(r.dev, table[i].plan, table[i].eye.N, table[i].P, batchRays);
+          bases[3 * nCams + i] = bt.lists;
+          if ((bt.lists + n) * kConeStride * sizeof(float4) > kBatchConeBytes) continue;
+          lists[i] = n;
+          bt.lists += n;
+        }
+        if (bt.lists && !b.cones.tryEnsure(bt.lists * kConeStride)) bt.lists = 0;
+        for (size_t i = 0; i < nCams; ++i) {
+          BatchEye& be = table[i];
+          if (bt.lists && lists[i]) be.eye.cones = b.cones.ptr + bases[3 * nCams + i] * kConeStride;
+          bases[i] = bt.tasksLists;
+          bases[nCams + i] = bt.tasksOther;
+          bases[2 * nCams + i] = bt.cells;
+          if (!be.eye.N) continue;
+          (be.eye.cones ? bt.tasksLists : bt.tasksOther) += be.plan.tasks;
+          if (be.plan.chunks > 1) bt.cells += static_cast<unsigned long long>(posesPerCam) * be.eye.N;
+        }
         cudaStream_t st = r.stream();
         check(cudaMemcpyAsync(b.table.ptr, table.data(), nCams * sizeof(BatchEye), cudaMemcpyHostToDevice, st), "cudaMemcpy");
-        check(cudaMemcpyAsync(b.taskBase.ptr, tb.data(), nCams * sizeof(unsigned long long), cudaMemcpyHostToDevice, st),
+        check(cudaMemcpyAsync(b.bases.ptr, bases.data(), bases.size() * sizeof(unsigned long long),
+                              cudaMemcpyHostToDevice, st),
               "cudaMemcpy");
-        check(cudaMemcpyAsync(b.cellBase.ptr, cb.data(), nCams * sizeof(unsigned long long), cudaMemcpyHostToDevice, st),
-              "cudaMemcpy");
+        bt.eyes = b.table.ptr;
+        bt.taskBaseLists = b.bases.ptr;
+        bt.taskBaseOther = b.bases.ptr + nCams;
+        bt.cellBase = b.bases.ptr + 2 * nCams;
+        bt.coneBase = b.bases.ptr + 3 * nCams;
+        bt.nEyes = static_cast<uint32_t>(nCams);
         uint32_t* err = r.errWord();
         check(cudaStreamSynchronize(st), "batch set-up");
         int dev = 0, sms = 0;
         check(cudaGetDevice(&dev), "cudaGetDevice");
         check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
         b.variant = renderVariant();
-        b.grid = sms * std::max(1, batchBlocksPerSM(b.variant));
-        // Record: reset the counters, the persistent launch, the chunk sums.
+        const int blocksLists = bt.tasksLists ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, true)) : 0;
+        const int blocksOther = bt.tasksOther ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, false)) : 0;
+        // Record: reset the counters, the persistent launches, the chunk sums.
         check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-        cudaError_t ce = cudaMemsetAsync(b.ctrl.ptr, 0, (2 + nCams) * sizeof(unsigned long long), st);
+        cudaError_t ce = cudaMemsetAsync(b.ctrl.ptr, 0, (3 + nCams) * sizeof(unsigned long long), st);
         if (ce == cudaSuccess) ce = cudaMemsetAsync(b.ctrl.ptr + 1, 0xff, sizeof(unsigned long long), st);
         if (ce == cudaSuccess)
-          ce = launchBatch(r.dev, b.table.ptr, b.taskBase.ptr, b.cellBase.ptr, static_cast<uint32_t>(nCams),
-                           b.totalTasks, b.totalCells, b.ctrl.ptr, err, b.variant, b.grid, b.cutPoses, st);
+          ce = launchBatch(r.dev, bt, b.ctrl.ptr, err, b.variant, blocksLists, blocksOther, b.cutPoses, st);
         cudaGraph_t g = nullptr;
         const cudaError_t ee = cudaStreamEndCapture(st, &g);
         check(ce, "batch capture");

@@ -1590,6 +1590,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
   PairStream pair{reinterpret_cast<uint4*>(fixed + 3) + lane, reinterpret_cast<uint2*>(fixed + 3 + 32) + lane,
                   reinterpret_cast<float2*>(fixed + 3 + 48) + lane, false, 0};
   if (kCone) {
+    __syncwarp();  // the warp's previous task has read its shared memory
     if (valid && !eye.draws) pair.begin(st);
     if (lane == 0) {
       const v3 c = cross(perp, axis);
@@ -2098,27 +2099,31 @@ __device__ __forceinline__ uint32_t lastAtMost(const T* base, uint32_t n, uint64
 // Persistent kernel over the warp tasks of every eye of a batch: each warp
 // takes the next task from a global counter until none are left.  Task t
 // belongs to the last eye whose taskBase <= t; the eyes' tasks are laid out
-// one eye after another.  ctrl[0] = task counter, ctrl[1] = earliest start
+// one eye after another.  ctrl[1] = earliest start
 // (ns), ctrl[2 + e] = completion time of eye e's last task (ns).
-template <int kRegs, int kWidth = 2>
+// kCone: the kernel of the eyes that have cone lists (taskBase then counts
+// theirs alone, and the other kernel's the others').
+template <int kRegs, int kWidth = 2, bool kCone = false>
 __global__ void __maxnreg__(kRegs) batchKernel(DevScene sc, const BatchEye* __restrict__ eyes,
                                                                const unsigned long long* __restrict__ taskBase,
                                                                uint32_t nEyes, unsigned long long totalTasks,
-                                                               unsigned long long* ctrl, uint32_t* errFlag) {
+                                                               unsigned long long* counter, unsigned long long* ctrl,
+                                                               uint32_t* errFlag) {
+  extern __shared__ float4 renderSmem[];  // kCone: kConeWarpFloat4 per warp
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t nv = 0, tt = 0;
   bool first = true;
   for (;;) {
     unsigned long long task = 0;
-    if (lane == 0) task = atomicAdd(&ctrl[0], 1ull);
+    if (lane == 0) task = atomicAdd(counter, 1ull);
     task = __shfl_sync(0xffffffffu, task, 0);
     if (task >= totalTasks) break;
     if (first && lane == 0) atomicMin(&ctrl[1], globalTimerNs());
     first = false;
     const uint32_t e = lastAtMost(taskBase, nEyes, task);
     const BatchEye be = eyes[e];
-    renderTask<0, kWidth>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag, nullptr, nv,
-                  tt);
+    renderTask<0, kWidth, kCone>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag,
+                                 nullptr, nv, tt, nullptr, renderSmem);
     if (lane == 0) atomicMax(&ctrl[2 + e], globalTimerNs());
   }
 }
@@ -2132,6 +2137,24 @@ __global__ void batchCutKernel(DevScene sc, const BatchEye* __restrict__ eyes, u
   const DevEye& de = eyes[e].eye;
   if (!de.cuts || p >= eyes[e].P) return;
   buildCut(sc, eyes[e].poses + 4 * p, de.cutRadius, de.maxRel, de.cuts + static_cast<size_t>(p) * kCutStride);
+}
+
+// Cone lists of every eye of a batch that has them: list i - coneBase[e] of
+// the last eye e whose coneBase <= i, pose by pose in the eye's direction
+// order.
+__global__ void __launch_bounds__(kConeThreads)
+    batchConeKernel(DevScene sc, const BatchEye* __restrict__ eyes, const unsigned long long* __restrict__ coneBase,
+                    uint32_t nEyes, unsigned long long totalLists) {
+  __shared__ uint2 work[kConeEntries * kConeThreads];
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
+  if (i >= totalLists) return;
+  const uint32_t e = lastAtMost(coneBase, nEyes, i);
+  const DevEye& eye = eyes[e].eye;
+  const uint64_t local = i - coneBase[e];
+  const uint32_t p = static_cast<uint32_t>(local / eye.N), slot = static_cast<uint32_t>(local % eye.N);
+  const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
+  coneList(sc, eye, o, eyes[e].poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+           eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
 // Chunk sums of every eye with more than 32 samples: cell c belongs to the
@@ -2349,9 +2372,17 @@ static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool con
 constexpr uint32_t kConeDeepTris = 16384;
 constexpr uint64_t kConeRaysDeep = 1ull << 19, kConeRaysShallow = 1ull << 21;
 
+static bool coneWorth(const DevScene& scene, uint64_t rays) {
+  return scene.triCount > 0 && rays >= (scene.triCount >= kConeDeepTris ? kConeRaysDeep : kConeRaysShallow);
+}
+
+size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, uint32_t P, uint64_t batchRays) {
+  if (scene.width != 2 || plan.segWidth != 32 || !coneWorth(scene, batchRays)) return 0;
+  return static_cast<size_t>(P) * N;
+}
+
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec) {
-  const uint64_t rays = static_cast<uint64_t>(N) * spp * P;
-  if (scene.triCount == 0 || rays < (scene.triCount >= kConeDeepTris ? kConeRaysDeep : kConeRaysShallow)) return 0;
+  if (!coneWorth(scene, static_cast<uint64_t>(N) * spp * P)) return 0;
   if (planRender(N, spp, P, true).segWidth != 32) return 0;
   if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
   return static_cast<size_t>(P) * N;
@@ -2534,47 +2565,73 @@ cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float
   }
 }
 
-int batchBlocksPerSM(int variant) {
-  int blocks = 0;
-  cudaError_t e;
-  const int bt = static_cast<int>(batchBlockThreads());
-  switch (variant) {
-    case 1: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, batchKernel<80>, bt, 0); break;
-    case 2: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, batchKernel<64>, bt, 0); break;
-    default: e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, batchKernel<96>, bt, 0); break;
+namespace {
+// f(kernel, dynamic shared memory) of the batch kernel for a register variant
+// (the cone-list kernel has one budget, kConeRegs), BVH width and block size.
+template <typename F>
+cudaError_t withBatchKernel(int variant, int width, bool cones, F&& f) {
+  if (cones) {
+    const size_t smem = batchBlockThreads() / 32 * kConeWarpFloat4 * sizeof(float4);
+    return width == 2 ? f(batchKernel<kConeRegs, 2, true>, smem) : cudaErrorInvalidValue;
   }
-  return e == cudaSuccess ? blocks : 0;
-}
-
-cudaError_t launchBatch(const DevScene& scene, const BatchEye* eyes, const unsigned long long* taskBase,
-                        const unsigned long long* cellBase, uint32_t nEyes, unsigned long long totalTasks,
-                        unsigned long long totalCells, unsigned long long* ctrl, uint32_t* errFlag, int variant,
-                        int gridBlocks, uint32_t cutPoses, cudaStream_t stream) {
-  if (nEyes == 0 || gridBlocks <= 0) return cudaSuccess;
-  if (cutPoses) {
-    const uint64_t n = static_cast<uint64_t>(nEyes) * cutPoses;
-    batchCutKernel<<<static_cast<unsigned>((n + 63) / 64), 64, 0, stream>>>(scene, eyes, nEyes, cutPoses);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-  }
-  const unsigned bt = batchBlockThreads();
   auto run = [&](auto regsTag) {
     constexpr int R = decltype(regsTag)::value;
-    switch (scene.width) {
-      case 4: batchKernel<R, 4><<<gridBlocks, bt, 0, stream>>>(scene, eyes, taskBase, nEyes, totalTasks, ctrl, errFlag); break;
-      case 8: batchKernel<R, 8><<<gridBlocks, bt, 0, stream>>>(scene, eyes, taskBase, nEyes, totalTasks, ctrl, errFlag); break;
-      default: batchKernel<R, 2><<<gridBlocks, bt, 0, stream>>>(scene, eyes, taskBase, nEyes, totalTasks, ctrl, errFlag); break;
+    switch (width) {
+      case 4: return f(batchKernel<R, 4>, size_t(0));
+      case 8: return f(batchKernel<R, 8>, size_t(0));
+      default: return f(batchKernel<R, 2>, size_t(0));
     }
   };
   switch (variant) {
-    case 1: run(std::integral_constant<int, 80>{}); break;
-    case 2: run(std::integral_constant<int, 64>{}); break;
-    default: run(std::integral_constant<int, 96>{}); break;
+    case 1: return run(std::integral_constant<int, 80>{});
+    case 2: return run(std::integral_constant<int, 64>{});
+    default: return run(std::integral_constant<int, 96>{});
   }
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess || totalCells == 0) return e;
-  batchCombineKernel<<<static_cast<unsigned>((totalCells + 255) / 256), 256, 0, stream>>>(eyes, cellBase, nEyes,
-                                                                                            totalCells);
+}
+}  // namespace
+
+int batchBlocksPerSM(int variant, int width, bool cones) {
+  int blocks = 0;
+  const cudaError_t e = withBatchKernel(variant, width, cones, [&](auto kernel, size_t smem) {
+    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, kernel, static_cast<int>(batchBlockThreads()), smem);
+  });
+  return e == cudaSuccess ? blocks : 0;
+}
+
+cudaError_t launchBatch(const DevScene& scene, const BatchTables& b, unsigned long long* ctrl, uint32_t* errFlag,
+                        int variant, int blocksLists, int blocksOther, uint32_t cutPoses, cudaStream_t stream) {
+  const uint32_t nEyes = b.nEyes;
+  if (nEyes == 0) return cudaSuccess;
+  if (b.lists) {
+    const uint64_t blocks = (b.lists + kConeThreads - 1) / kConeThreads;
+    if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
+    batchConeKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, b.eyes, b.coneBase, nEyes,
+                                                                                b.lists);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  if (cutPoses && b.tasksOther) {
+    const uint64_t n = static_cast<uint64_t>(nEyes) * cutPoses;
+    batchCutKernel<<<static_cast<unsigned>((n + 63) / 64), 64, 0, stream>>>(scene, b.eyes, nEyes, cutPoses);
+    const cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+  }
+  cudaError_t e = cudaSuccess;
+  if (b.tasksLists)
+    e = withBatchKernel(variant, scene.width, true, [&](auto kernel, size_t smem) {
+      kernel<<<blocksLists, batchBlockThreads(), smem, stream>>>(scene, b.eyes, b.taskBaseLists, nEyes, b.tasksLists,
+                                                                 ctrl, ctrl, errFlag);
+      return cudaGetLastError();
+    });
+  if (e == cudaSuccess && b.tasksOther)
+    e = withBatchKernel(variant, scene.width, false, [&](auto kernel, size_t smem) {
+      kernel<<<blocksOther, batchBlockThreads(), smem, stream>>>(scene, b.eyes, b.taskBaseOther, nEyes, b.tasksOther,
+                                                                 ctrl + 2 + nEyes, ctrl, errFlag);
+      return cudaGetLastError();
+    });
+  if (e != cudaSuccess || b.cells == 0) return e;
+  batchCombineKernel<<<static_cast<unsigned>((b.cells + 255) / 256), 256, 0, stream>>>(b.eyes, b.cellBase, nEyes,
+                                                                                       b.cells);
   return cudaGetLastError();
 }
 

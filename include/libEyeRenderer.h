@@ -129,8 +129,9 @@ int crRenderPosesDevice(const float* d_poses, size_t count, float* d_out);
  * Results are bit-identical to crRenderPosesDevice's.  0 on success. */
 int crRenderPosesDeviceNoAlloc(const float* d_poses, size_t count, float* d_out);
 
-/* Batched rendering of several compound cameras of the scene in ONE
- * persistent launch (work-queue kernel over every eye's warp tasks),
+/* Batched rendering of several compound cameras of the scene in one
+ * persistent launch (work-queue kernel over every eye's warp tasks; a second
+ * one for the eyes without cone lists, if any),
  * recorded once into a CUDA graph and replayed by crBatchLaunch.
  *  cams: nCams camera indices (each a compound eye, each at most once);
  *  d_poses: device, nCams x posesPerCam poses of 16 floats, camera-major;

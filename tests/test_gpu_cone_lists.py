@@ -149,3 +149,46 @@ def test_lists_give_way_under_a_memory_cap(lib, small):
     finally:
         lib.crSetDeviceMemoryCap(0)
     assert np.array_equal(got, want, equal_nan=True)
+
+
+def test_batch_with_and_without_lists(lib, tmp_path):
+    """A batch whose eyes partly go through lists (16 samples fill no warp
+    segment) equals each eye's render without lists, frame by frame."""
+    import torch
+
+    P, spp = 5, [16, 48, 256, 1, 100]
+    info = scenes.batch_scene(str(tmp_path), n_eyes=len(spp), poses_per_eye=P, n_min=600, n_max=3000)
+    lib.loadGlTFscene(info["gltf"].encode())
+    cams = np.arange(info["first_batch_camera"], info["first_batch_camera"] + len(spp), dtype=np.int32)
+    p12 = info["poses"].reshape(-1, 12)
+    p16 = np.zeros((len(p12), 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = p12[:, 3 * k:3 * k + 3]
+    assert sum(n * s for n, s in zip(info["n"], spp)) * P >= 2 ** 21
+    d_poses = torch.from_numpy(p16).cuda()
+    want = []
+    for i, c in enumerate(cams):
+        lib.gotoCamera(int(c))
+        lib.setCurrentEyeSamplesPerOmmatidium(spp[i])
+        _render(lib, lib.crRenderPosesDevice, d_poses[i * P:], 1, info["n"][i])
+        lib.crSynchronize()
+        want.append(_render(lib, lib.crRenderPosesDeviceNoAlloc, d_poses[i * P:], P, info["n"][i]))
+    for i, c in enumerate(cams):  # the same streams again, one frame in
+        lib.gotoCamera(int(c))
+        lib.setCurrentEyeSamplesPerOmmatidium(spp[i])
+        _render(lib, lib.crRenderPosesDevice, d_poses[i * P:], 1, info["n"][i])
+    out = torch.full((3 * P * sum(info["n"]),), -1.0, device="cuda")
+    torch.cuda.synchronize()
+    held = lib.crGetDeviceMemoryHeld()
+    h = lib.crBatchCreate(cams, len(cams), P, d_poses.data_ptr(), out.data_ptr())
+    assert h > 0, eh.lastError(lib)
+    assert lib.crGetDeviceMemoryHeld() - held >= 400 * P * sum(n for n, s in zip(info["n"], spp) if s > 16)
+    assert lib.crBatchLaunch(h) == 0 and lib.crSynchronize() == 0, eh.lastError(lib)
+    got = out.cpu().numpy()
+    lat, total = np.zeros(len(cams), np.float32), ctypes.c_float(0.0)
+    assert lib.crBatchLatencies(h, lat, ctypes.byref(total)) == 0
+    assert (lat > 0).all() and total.value == lat.max()
+    for i in range(len(cams)):
+        o = lib.crBatchOutputOffset(h, i)
+        assert np.array_equal(got[o:o + want[i].size].reshape(want[i].shape), want[i]), spp[i]
+    lib.crBatchDestroy(h)
