@@ -94,11 +94,10 @@ struct DevEye {
 constexpr int kWideStackEntries = 128;
 constexpr int kCutEntries = 8;
 constexpr int kCutStride = 1 + 2 * kCutEntries;
-// A cone list (render.cu, coneList): head, up to kConeEntries 8-byte entries,
-// three rows of relative vertex coordinates per single-triangle entry.
-constexpr int kConeEntries = 8;
-constexpr int kConeRow0 = 1 + (kConeEntries + 1) / 2;
-constexpr int kConeStride = kConeRow0 + 3 * kConeEntries;
+// A cone list (render.cu, coneList): a head and three rows per entry.  Ten
+// entries are what one float4 a lane can fetch.
+constexpr int kConeEntries = 10;
+constexpr int kConeStride = 1 + 3 * kConeEntries;
 
 // One pose = 4 x float4: position, local x axis, local y axis, local z axis
 // (w components unused).
@@ -380,6 +379,7 @@ struct AdaptiveBucket {
   uint64_t taskBase = 0;      // first warp task of the bucket
   uint64_t tasks = 0;         // warp tasks of the bucket
   uint64_t poolBase = 0;      // first warp pool of the bucket (a pool: up to 8 rounds of 32 samples)
+  const float4* cones = nullptr;  // null, or the entries' cone lists (launchEntryCones)
 };
 struct AdaptiveLaunch {
   AdaptiveBucket b[kAdaptiveBuckets];
@@ -393,11 +393,22 @@ struct AdaptiveLaunch {
   // Resident 128-thread blocks per SM the kernel's register budget is sized
   // for on the two-wide BVH: 5 (96 registers), 6 (80) or 8 (64).
   int blocksPerSM = 5;
+  // Rounds of 32 samples per pool, and (list kernel) those its shared memory
+  // holds: a pool has at least one task.
+  uint32_t poolRounds = 8, slotRounds = 8;
 };
 // Table of the non-empty buckets among nBuckets (entries, counts, spp and
 // partial buffers per bucket) with their warp-task offsets.
+// cones: null, or every bucket's cone lists: the launch then goes through
+// them.
 AdaptiveLaunch planAdaptive(const uint32_t* const* entries, const uint64_t* counts, const uint32_t* spp,
-                            float* const* partials, uint32_t nBuckets);
+                            float* const* partials, uint32_t nBuckets, const float4* const* cones = nullptr);
+// Whether a bucket of `spp` samples goes through cone lists in an adaptive
+// render with launchRays rays in such buckets.
+bool adaptiveLists(const DevScene& scene, uint32_t spp, uint64_t launchRays);
+// The lists of `count` entries (kConeStride float4 each).
+cudaError_t launchEntryCones(const DevScene& scene, const float4* omm, uint32_t N, const float4* poses,
+                             const uint32_t* entries, uint64_t count, float4* cones, cudaStream_t stream);
 // The process-wide ray-refill schedule of the adaptive kernel (planAdaptive
 // copies it into every launch): refill at >= refillIdle idle lanes (1..32),
 // check every `steps` BVH steps (1..4096).  Results do not depend on it.

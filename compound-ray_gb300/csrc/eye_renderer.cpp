@@ -649,6 +649,18 @@ struct Renderer {
     }
   }
 
+  // Cone lists of `count` entries for adaptive launches of `rays` rays at `spp`
+  // (or more) samples each; null when those do not use them or the memory is
+  // not to be had.
+  const float4* entryCones(const EyeDev& e, const float4* dposes, const uint32_t* entries, uint64_t count, uint32_t spp,
+                           uint64_t rays) {
+    if (!count || !adaptiveLists(dev, spp, rays) || count * kConeStride * sizeof(float4) > kConeListBytes ||
+        !cones.tryEnsure(count * kConeStride))
+      return nullptr;
+    check(launchEntryCones(dev, e.omm.ptr, e.N, dposes, entries, count, cones.ptr, stream()), "cone lists");
+    return cones.ptr;
+  }
+
   // Gives a P-pose launch of a small eye a buffer for its pre-drawn random
   // numbers, so that its poses spread over more warps (renderDrawBytes).
   void withDraws(DevEye& de, uint32_t P, bool allowed) {
@@ -2400,10 +2412,12 @@ int crAllocatorAddTrainingPoses(const float* poses12, size_t count, int featureS
         check(cudaMemsetAsync(d.labels.ptr, 0, rows * 2, st), "cudaMemset");
         d.labelOuts.ensure(static_cast<size_t>(seeds) * rows * 3);
         d.partials.ensure(std::max<size_t>(1, adaptivePartialFloats(rows, 1024)));
+        const float4* cones = nullptr;  // the same entries in every launch: their lists are built once
         for (uint32_t c = 4; c <= 1024; c *= 2) {
           const uint32_t* ent = d.entries.ptr;
           float* part = d.partials.ptr;
-          const AdaptiveLaunch L = planAdaptive(&ent, &rows, &c, &part, 1);
+          if (!cones) cones = r.entryCones(e, d.poses.ptr, ent, rows, c, rows * c);
+          const AdaptiveLaunch L = planAdaptive(&ent, &rows, &c, &part, 1, cones ? &cones : nullptr);
           DevEye ce;
           r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
           if (ce.cuts)
@@ -2582,21 +2596,45 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
             uint64_t n[kAdaptiveBuckets];
             uint32_t spp[kAdaptiveBuckets];
             float* part[kAdaptiveBuckets];
+            const float4* cone[kAdaptiveBuckets];
             uint64_t pf = 0;
+            // The buckets from firstList on (at least 16 samples) go through
+            // cone lists when those are worth it, the others search the BVH.
+            uint32_t firstList = kAdaptiveBuckets;
+            uint64_t listRays = 0;
+            for (uint32_t k = kAdaptiveBuckets; k-- > 0 && adaptiveLists(r.dev, 4u << k, ~0ull);) {
+              firstList = k;
+              listRays += cnt[k] * (4ull << k);
+            }
+            const float4* cones = nullptr;
+            if (firstList < kAdaptiveBuckets)
+              cones = r.entryCones(e, poses + 4 * first, d.entries.ptr + off[firstList], total - off[firstList],
+                                   4u << firstList, listRays);
+            if (!cones) firstList = kAdaptiveBuckets;
             for (uint32_t k = 0; k < kAdaptiveBuckets; ++k) {
               ent[k] = d.entries.ptr + off[k];
               n[k] = cnt[k];
               spp[k] = 4u << k;
               part[k] = d.partials.ptr + pf;
               pf += adaptivePartialFloats(cnt[k], spp[k]);
+              cone[k] = k >= firstList ? cones + (off[k] - off[firstList]) * kConeStride : nullptr;
             }
-            const AdaptiveLaunch L = planAdaptive(ent, n, spp, part, kAdaptiveBuckets);
+            const AdaptiveLaunch L = planAdaptive(ent, n, spp, part, firstList);
             DevEye ce;
-            r.withCuts(ce, P, e.maxRel);
-            if (ce.cuts) check(launchCuts(r.dev, poses + 4 * first, P, ce.cutRadius, ce.maxRel, ce.cuts, st), "cuts");
+            if (L.totalPools) {
+              r.withCuts(ce, P, e.maxRel);
+              if (ce.cuts) check(launchCuts(r.dev, poses + 4 * first, P, ce.cutRadius, ce.maxRel, ce.cuts, st), "cuts");
+            }
             check(launchAdaptive(r.dev, e.omm.ptr, e.N, poses + 4 * first, L, 0xada90000ull + d.adaptiveFrame,
                                  d.sums.ptr, r.errWord(), nullptr, st, ce.cuts),
                   "adaptive render");
+            if (cones) {
+              const uint32_t f = firstList;
+              const AdaptiveLaunch LL = planAdaptive(ent + f, n + f, spp + f, part + f, kAdaptiveBuckets - f, cone + f);
+              check(launchAdaptive(r.dev, e.omm.ptr, e.N, poses + 4 * first, LL, 0xada90000ull + d.adaptiveFrame,
+                                   d.sums.ptr, r.errWord(), nullptr, st),
+                    "adaptive render");
+            }
           }
           check(launchAdaptiveFinish(d.level.ptr, rows, fs, d.stats.ptr, learned, d.sums.ptr, d_out + 3 * first * e.N,
                                      st),
@@ -2706,7 +2744,8 @@ int crAdaptiveRecord(const float* poses12, size_t count, int spp, unsigned long 
         const uint32_t* ep = ent.ptr;
         float* pp = part.ptr;
         const uint32_t c = static_cast<uint32_t>(spp);
-        const AdaptiveLaunch L = planAdaptive(&ep, &rows, &c, &pp, 1);
+        const float4* cones = r.entryCones(e, d.poses.ptr, ep, rows, c, rows * c);
+        const AdaptiveLaunch L = planAdaptive(&ep, &rows, &c, &pp, 1, cones ? &cones : nullptr);
         DevEye ce;
         r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
         if (ce.cuts)

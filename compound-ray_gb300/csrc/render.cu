@@ -23,6 +23,7 @@
 #include <cuda_runtime.h>
 #include <curand_kernel.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -890,23 +891,22 @@ __device__ __forceinline__ bool coneTriangle(const Cone& c, float4 v0, float4 v1
 
 // The list of ommatidium o at `pose`, written to out (kConeStride float4):
 //   [0] (entry count, or kConeFromRoot; origin xyz),
-//   [1 ..] (entry distance, ref) pairs, two to a float4; ref as in the BVH, a
-//       leaf as one entry for each of its triangles that the cone meets while
-//       there is room,
-//   [kConeRow0 + 3 k ..] for a single-triangle entry k its vertices relative
-//       to the origin (the subtraction each ray would make), one row per
-//       axis: (A, B, C, triangle id).
+//   [1 + 3 k ..] entry k: three rows, one per axis.  x to z: for an entry
+//       that is a single triangle its vertices A, B, C relative to the origin
+//       (the subtraction each ray would make).  w: the entry distance, the
+//       ref (as in the BVH, a leaf as one entry for each of its triangles that
+//       the cone meets while there is room), the triangle's id.
 // work: the thread's column of a [kConeEntries][kConeThreads] array, holding
 // the entries found (from the front) and the traversal stack (from the back).
 //
 // One thread per list: a list is ~30 dependent node visits, so the lists of
 // 32 neighbouring ommatidia share a warp, whose lanes walk nearly the same
 // nodes, instead of the lanes of a warp sharing a list.
-__device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, uint32_t o,
+__device__ __forceinline__ void coneList(const DevScene& sc, const float4* __restrict__ omm, uint32_t o,
                                          const float4* __restrict__ pose, uint2* __restrict__ work,
                                          float4* __restrict__ out) {
   const float4 P0 = __ldg(pose), X = __ldg(pose + 1), Y = __ldg(pose + 2), Z = __ldg(pose + 3);
-  const float4 r0 = __ldg(eye.omm + 2 * o), r1 = __ldg(eye.omm + 2 * o + 1);
+  const float4 r0 = __ldg(omm + 2 * o), r1 = __ldg(omm + 2 * o + 1);
   const v3 ax = mk(r0.w, r1.x, r1.y), x = mk(X.x, X.y, X.z), y = mk(Y.x, Y.y, Y.z), z = mk(Z.x, Z.y, Z.z);
   const float fpo = r1.w;
   Cone c;
@@ -991,20 +991,21 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const DevEye& eye, 
   }
   // tCover bounds distances, t <= tCover * 1.005 (|direction| != 1).
   uint32_t count = 0;
-  float2* pair = reinterpret_cast<float2*>(out + 1);
   for (int k = 0; k < nOut; ++k) {
     const uint2 e = work[k * kConeThreads];
     const float te = __uint_as_float(e.y);
     if (te > tCover) continue;
-    pair[count] = make_float2(te * 0.995f, __uint_as_float(e.x));
+    float4 v0 = make_float4(0.f, 0.f, 0.f, 0.f), v1 = v0, v2 = v0;
     if (static_cast<int>(e.x) < 0 && (~e.x & 7u) == 0u) {
       const float4* t = sc.tris + 3 * static_cast<size_t>(~e.x >> 3);
-      const float4 v0 = __ldg(t), v1 = __ldg(t + 1), v2 = __ldg(t + 2);
-      float4* row = out + kConeRow0 + 3 * count;
-      row[0] = make_float4(xsub(v0.x, c.o.x), xsub(v1.x, c.o.x), xsub(v2.x, c.o.x), v0.w);
-      row[1] = make_float4(xsub(v0.y, c.o.y), xsub(v1.y, c.o.y), xsub(v2.y, c.o.y), v0.w);
-      row[2] = make_float4(xsub(v0.z, c.o.z), xsub(v1.z, c.o.z), xsub(v2.z, c.o.z), v0.w);
+      v0 = __ldg(t);
+      v1 = __ldg(t + 1);
+      v2 = __ldg(t + 2);
     }
+    float4* row = out + 1 + 3 * count;
+    row[0] = make_float4(xsub(v0.x, c.o.x), xsub(v1.x, c.o.x), xsub(v2.x, c.o.x), te * 0.995f);
+    row[1] = make_float4(xsub(v0.y, c.o.y), xsub(v1.y, c.o.y), xsub(v2.y, c.o.y), __uint_as_float(e.x));
+    row[2] = make_float4(xsub(v0.z, c.o.z), xsub(v1.z, c.o.z), xsub(v2.z, c.o.z), v0.w);
     ++count;
   }
   out[0] = make_float4(__uint_as_float(count), c.o.x, c.o.y, c.o.z);
@@ -1019,19 +1020,20 @@ __global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye e
   if (i >= static_cast<uint64_t>(P) * eye.N) return;
   const uint32_t p = static_cast<uint32_t>(i / eye.N), slot = static_cast<uint32_t>(i - static_cast<uint64_t>(p) * eye.N);
   const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
-  coneList(sc, eye, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+  coneList(sc, eye.omm, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
            eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
 // Copies a warp's list into shared memory asynchronously, one float4 a lane:
 // the list of pose p + 1 arrives while pose p is traced.
 static_assert(kConeStride <= 32, "one float4 of a list for each lane");
+__device__ __forceinline__ void fetchFloat4(const float4* __restrict__ src, float4* __restrict__ dst) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src)
+               : "memory");
+}
 __device__ __forceinline__ void fetchCone(const float4* __restrict__ list, float4* __restrict__ dst, uint32_t lane) {
-  if (lane < static_cast<uint32_t>(kConeStride))
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(
-                     static_cast<uint32_t>(__cvta_generic_to_shared(dst + lane))),
-                 "l"(list + lane)
-                 : "memory");
+  if (lane < static_cast<uint32_t>(kConeStride)) fetchFloat4(list + lane, dst + lane);
 }
 __device__ __forceinline__ void fetchDraw(const float2* __restrict__ src, float2* __restrict__ dst) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
@@ -1041,58 +1043,121 @@ __device__ __forceinline__ void fetchDraw(const float2* __restrict__ src, float2
 __device__ __forceinline__ void commitCone() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void awaitOlderCone() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
+// Entry distance and ref of a list's entry k.
+__device__ __forceinline__ float coneDistance(const float4* list, uint32_t k) { return list[1 + 3 * k].w; }
+__device__ __forceinline__ int coneRef(const float4* list, uint32_t k) { return __float_as_int(list[2 + 3 * k].w); }
+
+// Searches the subtrees of a list that a ray has left: the entries whose bit
+// is set in `later` (nearest first; bit 31: the root).  They wait on the
+// traversal stack as entry numbers, so that one loop serves them all (a lane
+// that is through with one does not wait for the others' before the next) and
+// an entry that begins beyond the hit is dropped when its turn comes.  All
+// lanes descend to leaves, then test leaves together, as in traverseBurst
+// (24 uneven eyes 5.0 ms, the adaptive terrain render 2.19 ms; with one loop
+// whose step is a node or a leaf 5.16 and 2.42 ms, with the lanes held
+// together by votes 5.3 and 2.38 ms).
+constexpr int kStackEntry = 0x40000000;  // stack values from here on are kStackEntry + entry
+
+template <bool kCount>
+__device__ __forceinline__ void searchEntries(const DevScene& sc, v3 org, v3 dir, float tmin,
+                                              const float4* __restrict__ list, uint32_t later, Hit& h,
+                                              uint32_t* errFlag, uint32_t& nodeVisits, uint32_t& triTests) {
+  const Ray r = setupRay(org, dir, sc.extent);
+  int stack[kStackSize];
+  int sp = 0, node = 0;
+  bool more = true;
+  auto pop = [&]() {
+    while (sp > 0) {
+      node = stack[--sp];
+      if (node < kStackEntry) return true;
+      const uint32_t k = static_cast<uint32_t>(node - kStackEntry);
+      node = coneRef(list, k);
+      if (coneDistance(list, k) <= h.t) return true;
+    }
+    return false;
+  };
+  if (later != 0x80000000u) {
+    for (; later; later &= ~(0x80000000u >> __clz(later))) stack[sp++] = kStackEntry + 31 - __clz(later);
+    more = pop();
+  }
+  while (more) {
+    while (more && node >= 0) {
+      if (kCount) ++nodeVisits;
+      const float4* n = sc.nodes + 4 * node;
+      const float4 n0 = __ldg(n + 0);
+      const float4 n1 = __ldg(n + 1);
+      const float4 n2 = __ldg(n + 2);
+      const int4 n3 = __ldg(reinterpret_cast<const int4*>(n + 3));
+      float tn0, tf0, tn1, tf1;
+      childSpan(r, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y, tmin, h.t, tn0, tf0);
+      childSpan(r, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w, tmin, h.t, tn1, tf1);
+      const bool hit0 = tn0 <= tf0, hit1 = tn1 <= tf1;
+      if (hit0 || hit1) {
+        const bool second = hit1 && (!hit0 || tn1 < tn0);
+        node = second ? n3.y : n3.x;
+        if (hit0 && hit1) {
+          if (sp >= kStackSize) {
+            atomicOr(errFlag, kErrStackOverflow);
+            return;
+          }
+          stack[sp++] = second ? n3.x : n3.y;
+        }
+      } else {
+        more = pop();
+      }
+    }
+    if (!more) break;
+    const uint32_t code = ~static_cast<uint32_t>(node);
+    const uint32_t first = code >> 3, count = (code & 7u) + 1u;
+    if (kCount) triTests += count;
+    for (uint32_t k = 0; k < count; ++k) {
+      const float4* t = sc.tris + 3 * (first + k);
+      testTriangle(r, __ldg(t), __ldg(t + 1), __ldg(t + 2), first + k, tmin, h);
+    }
+    more = pop();
+  }
+}
+
 // Closest hit of a ray of the cone-list path: list is its ommatidium's list
 // (in shared memory), nd its normal draw (the angle to the axis in standard
-// deviations); org receives the origin.  The lanes of the warp test the
-// list's triangles in step: a test reads three rows in the ray's axis order,
-// without selects or subtractions, and no lane waits for another's
-// traversal.  Entries that are subtrees come last, when most of them begin
-// beyond the hit.
+// deviations); org receives the origin.  Called by whole warps: the lanes
+// test `entries` entries (the longest list of the warp) in step, and meet
+// after each, so a triangle's test runs once for all 32 (left to itself the
+// compiler lets lanes that are through with a triangle run ahead: 20 of 32
+// lanes at a time, 10.9 ms instead of 6.5 for 256 terrain poses).  A test
+// reads three rows in the ray's axis order, without selects or subtractions.
+// Entries that are subtrees come last, when most of them begin beyond the hit.
 template <bool kCount>
-__device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __restrict__ list, v3& org, v3 dir,
-                                          float tmin, float nd, Hit& h, uint32_t* errFlag, uint32_t& nodeVisits,
-                                          uint32_t& triTests) {
+__device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __restrict__ list, uint32_t listed,
+                                          uint32_t entries, v3 org, v3 dir, float tmin, float nd, Hit& h,
+                                          uint32_t* errFlag, uint32_t& nodeVisits, uint32_t& triTests) {
   h.t = 1e16f;
   h.id = 0xffffffffu;
   h.pos = 0;
-  const float4 head = list[0];
-  org = mk(head.y, head.z, head.w);
-  const uint32_t listed = __float_as_uint(head.x);
-  const float2* pair = reinterpret_cast<const float2*>(list + 1);
-  uint32_t later = 0;  // entries (or, bit 31, the root) to search as trees
-  if (listed == kConeFromRoot || !(fabsf(nd) <= kConeSigmas)) {
-    later = 0x80000000u;
-  } else {
-    Ray ray;
-    setupShear(ray, dir);
-    const float4* rows = list + kConeRow0;
-    for (uint32_t k = 0; k < listed; ++k, rows += 3) {
-      const float2 e = pair[k];
-      const int node = __float_as_int(e.y);
+  const bool root = listed == kConeFromRoot || !(fabsf(nd) <= kConeSigmas);
+  const uint32_t mine = root ? 0u : listed;
+  uint32_t later = root ? 0x80000000u : 0u;  // entries (or, bit 31, the root) to search as trees
+  Ray ray;
+  setupShear(ray, dir);
+  const float4* rows = list + 1;
+  for (uint32_t k = 0; k < entries; ++k, rows += 3) {
+    if (k < mine) {
+      const int node = __float_as_int(rows[1].w);
       if (node < 0 && (~node & 7) == 0) {
-        if (!(e.x <= h.t)) continue;
-        if (kCount) ++triTests;
-        const float4 x = rows[ray.kx], y = rows[ray.ky], z = rows[ray.kz];
-        testRelative(ray, x.x, y.x, z.x, x.y, y.y, z.y, x.z, y.z, z.z, __float_as_uint(x.w),
-                     ~static_cast<uint32_t>(node) >> 3, tmin, h);
+        if (rows[0].w <= h.t) {
+          if (kCount) ++triTests;
+          const float4 x = rows[ray.kx], y = rows[ray.ky], z = rows[ray.kz];
+          testRelative(ray, x.x, y.x, z.x, x.y, y.y, z.y, x.z, y.z, z.z, __float_as_uint(rows[2].w),
+                       ~static_cast<uint32_t>(node) >> 3, tmin, h);
+        }
       } else {
         later |= 1u << k;
       }
     }
+    __syncwarp();
   }
-  while (later) {
-    const int k = __ffs(later) - 1;
-    later &= later - 1;
-    int node = 0;
-    if (k != 31) {
-      const float2 e = pair[k];
-      if (!(e.x <= h.t)) continue;
-      node = __float_as_int(e.y);
-    }
-    const Ray ray = setupRay(org, dir, sc.extent);
-    int stack[kStackSize];
-    traverseFrom<kCount>(sc, ray, tmin, h, stack, 0, node, errFlag, nodeVisits, triTests);
-  }
+  if (later) searchEntries<kCount>(sc, org, dir, tmin, list, later, h, errFlag, nodeVisits, triTests);
+  __syncwarp();
 }
 
 __global__ void cutKernel(DevScene sc, const float4* __restrict__ poses, uint32_t P, float R, float maxRel,
@@ -1506,6 +1571,13 @@ struct PairStream {
   }
 };
 
+// Register budget of the plain render through cone lists.  Its loop needs
+// fewer than the tree search does: on 256 terrain poses x 6000 ommatidia x
+// 256 samples 48, 56, 64, 72, 80 and 96 registers take 7.6, 7.0, 6.9, 6.9,
+// 7.8 and 9.7 ms, and 64 is also the fastest on the box scene (1000 x 32), so
+// the variants (renderVariant) are for renders without lists.
+constexpr int kConeRegs = 64;
+
 // kMode: 0 = render, 1 = render and record every ray, 2 = render and count
 // node visits / triangle tests into stats[0..1].  kMinBlocks: resident
 // 128-thread blocks per SM the register allocation is sized for (the
@@ -1519,7 +1591,8 @@ struct PairStream {
 // kWidth: 2 searches the BVH2 (with the near-field cut when eye.cuts is
 // set), 4 or 8 the wide BVH of that width (no cut).
 // kCone: closest hits through the cone lists at eye.cones (kWidth 2).
-template <int kMode, int kWidth = 2, bool kCone = false>
+// kDraws: the launch may have pre-drawn numbers (eye.draws).
+template <int kMode, int kWidth = 2, bool kCone = false, bool kDraws = true>
 __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye, const float4* __restrict__ poses,
                                            uint32_t P, const WarpPlan& plan, uint64_t task, float* __restrict__ out,
                                            float* __restrict__ scratch, uint32_t* errFlag,
@@ -1530,6 +1603,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
   constexpr bool kCount = (kMode & 3) == 2 || kFeat;  // feature mode: the per-entry traversal cost
   constexpr bool kLit = (kMode & 4) != 0;  // lighting-on shading (modes 4 render, 5 record)
   // Cone lists are for whole-warp segments (renderConeLists).
+  const float2* draws = kDraws ? eye.draws : nullptr;
   const uint32_t segWidth = kCone ? 32u : plan.segWidth, ommPerWarp = kCone ? 1u : plan.ommPerWarp;
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t p0 = 0, p1 = P;
@@ -1570,7 +1644,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
   v3 axis = mk(0.f, 1.f, 0.f), relPos = mk(0.f, 0.f, 0.f), perp = mk(0.f, 0.f, 1.f);
   float sd = 0.f, fpo = 0.f;
   if (valid) {
-    if (!kFeat && !eye.draws) loadState(eye.rng, plane, sidx, st);
+    if (!kFeat && !draws) loadState(eye.rng, plane, sidx, st);
     const float4 a = __ldg(eye.omm + 2 * o);
     const float4 b = __ldg(eye.omm + 2 * o + 1);
     axis = mk(a.w, b.x, b.y);
@@ -1591,7 +1665,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
                   reinterpret_cast<float2*>(fixed + 3 + 48) + lane, false, 0};
   if (kCone) {
     __syncwarp();  // the warp's previous task has read its shared memory
-    if (valid && !eye.draws) pair.begin(st);
+    if (valid && !draws) pair.begin(st);
     if (lane == 0) {
       const v3 c = cross(perp, axis);
       fixed[0] = make_float4(axis.x, axis.y, axis.z, sd);
@@ -1609,8 +1683,8 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     coneBuf = coneSmem + (threadIdx.x >> 5) * kConeWarpFloat4;
     coneNext = eye.cones + (static_cast<size_t>(p0) * eye.N + o) * kConeStride;
     if (slot < eye.N) fetchCone(coneNext, coneBuf + (p0 & 1u) * kConeStride, lane);
-    if (eye.draws) drawNext = eye.draws + (static_cast<size_t>(p0) * eye.N + o) * eye.spp + s;
-    if (eye.draws && valid) fetchDraw(drawNext, pair.drawSlot(p0));
+    if (draws) drawNext = draws + (static_cast<size_t>(p0) * eye.N + o) * eye.spp + s;
+    if (draws && valid) fetchDraw(drawNext, pair.drawSlot(p0));
     commitCone();
   }
 
@@ -1619,7 +1693,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       __syncwarp();  // every lane has read the buffer that is filled next
       coneNext += static_cast<size_t>(eye.N) * kConeStride;
       if (slot < eye.N && p + 1 < p1) fetchCone(coneNext, coneBuf + ((p + 1) & 1u) * kConeStride, lane);
-      if (eye.draws) {
+      if (draws) {
         drawNext += plane;
         if (valid && p + 1 < p1) fetchDraw(drawNext, pair.drawSlot(p + 1));
       }
@@ -1632,20 +1706,23 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     // hit triangle's normal in the eye's frame (facing the ray), all / spp.
     float f2x = 0.f, f2y = 0.f, f2z = 0.f, fHit = 0.f, fT = 0.f, fnx = 0.f, fny = 0.f, fnz = 0.f, fCost = 0.f;
     const uint32_t steps0 = nodeVisits + triTests;
-    if (valid) {
+    // With cone lists all lanes of a warp with an ommatidium go on together;
+    // those past its last sample trace the axis and count for nothing.
+    if (kCone ? slot < eye.N : valid) {
       const float4* pp = poses + 4 * p;
       const float4 P0 = __ldg(pp), X = __ldg(pp + 1), Y = __ldg(pp + 2), Z = __ldg(pp + 3);
-      float nd, ud;
-      if (kFeat) {  // feature renders: each ommatidium's samples a net (launchFeatures requires eye.netDraws)
+      float nd = 0.f, ud = 0.f;
+      if (kCone && !valid) {
+      } else if (kFeat) {  // feature renders: each ommatidium's samples a net (launchFeatures requires eye.netDraws)
         const float2 dr = netDraw(eye.drawSeed, (eye.frame0 + p) * eye.N + o, s);
         nd = dr.x;
         ud = dr.y;
-      } else if (eye.draws && kCone) {
+      } else if (draws && kCone) {
         const float2 dr = *pair.drawSlot(p);
         nd = dr.x;
         ud = dr.y;
-      } else if (eye.draws) {
-        const float2 dr = eye.draws[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s];
+      } else if (draws) {
+        const float2 dr = draws[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s];
         nd = dr.x;
         ud = dr.y;
       } else if (kCone) {
@@ -1677,7 +1754,12 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       Hit h;
       v3 org;
       if (kCone) {  // the list holds the origin
-        traceCone<kCount>(sc, coneBuf + (p & 1u) * kConeStride, org, dir, fpo, nd, h, errFlag, nodeVisits, triTests);
+        const float4* list = coneBuf + (p & 1u) * kConeStride;
+        const float4 head = list[0];
+        org = mk(head.y, head.z, head.w);
+        const uint32_t listed = __float_as_uint(head.x);
+        traceCone<kCount>(sc, list, listed, listed == kConeFromRoot ? 0u : listed, org, dir, fpo, nd, h,
+                                     errFlag, nodeVisits, triTests);
       } else {
         org = rayOrigin(mk(P0.x, P0.y, P0.z), mk(X.x, X.y, X.z), mk(Y.x, Y.y, Y.z), mk(Z.x, Z.y, Z.z), relPos);
       }
@@ -1711,7 +1793,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       } else {
         c = shadeMiss(sc.miss, dir);
       }
-      if (kRecord) {
+      if (kRecord && valid) {
         RayRecord& R = rec[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s];
         R.normalDraw = nd;
         R.uniformDraw = ud;
@@ -1730,7 +1812,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         R.b = c.z;
         R.pad = 0.f;
       }
-      col = c * invSpp;
+      if (!kCone || valid) col = c * invSpp;
       if (kFeat) {
         fCost = static_cast<float>(nodeVisits + triTests - steps0) * invSpp;
         f2x = c.x * c.x * invSpp;
@@ -1819,7 +1901,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     }
     }
   }
-  if (!kFeat && valid && !eye.draws) {
+  if (!kFeat && valid && !draws) {
     if (kCone) pair.end(st);
     storeState(eye.rng, plane, sidx, st);
   }
@@ -1833,7 +1915,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
 // per-pose chunk partial in shared memory, and after every kInBlockPoses
 // poses the block sums each (ommatidium, pose) of the group over its chunks
 // in chunk order (flushChunkSums), so the buffer holds 16 poses at a time.
-template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false, bool kCone = false>
+template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false, bool kCone = false, bool kDraws = !kCone>
 __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses, uint32_t P,
                                                 WarpPlan plan, float* __restrict__ out, float* __restrict__ scratch,
                                                 uint32_t* errFlag, RayRecord* __restrict__ rec,
@@ -1845,7 +1927,8 @@ __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const f
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t task = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (task >= plan.tasks) return;  // whole warps exit together (never with inBlock: whole blocks)
-  renderTask<kMode, kWidth, kCone>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits, triTests,
+  renderTask<kMode, kWidth, kCone, kDraws>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits,
+                                           triTests,
                                    kInBlock ? reinterpret_cast<float*>(
                                                   renderSmem + (kCone ? (blockDim.x >> 5) * kConeWarpFloat4 : 0))
                                             : nullptr,
@@ -2121,8 +2204,8 @@ __global__ void __maxnreg__(kRegs) batchKernel(DevScene sc, const BatchEye* __re
     if (first && lane == 0) atomicMin(&ctrl[1], globalTimerNs());
     first = false;
     const uint32_t e = lastAtMost(taskBase, nEyes, task);
-    const BatchEye be = eyes[e];
-    renderTask<0, kWidth, kCone>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag,
+    const BatchEye& be = eyes[e];
+    renderTask<0, kWidth, kCone, !kCone>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag,
                                  nullptr, nv, tt, nullptr, renderSmem);
     if (lane == 0) atomicMax(&ctrl[2 + e], globalTimerNs());
   }
@@ -2153,7 +2236,7 @@ __global__ void __launch_bounds__(kConeThreads)
   const uint64_t local = i - coneBase[e];
   const uint32_t p = static_cast<uint32_t>(local / eye.N), slot = static_cast<uint32_t>(local % eye.N);
   const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
-  coneList(sc, eye, o, eyes[e].poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+  coneList(sc, eye.omm, o, eyes[e].poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
            eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
@@ -2414,7 +2497,7 @@ cudaError_t launchRngInit(const DevEye& eye, uint32_t* errFlag, cudaStream_t str
 namespace {
 // One launch of a render kernel instance with the plan's block size and, for
 // in-block chunk sums, the shared memory of the partials.
-template <int kMode, int kRegs, int kWidth, bool kInBlock, bool kCone>
+template <int kMode, int kRegs, int kWidth, bool kInBlock, bool kCone, bool kDraws = !kCone>
 cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                             const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                             unsigned long long* stats, cudaStream_t stream) {
@@ -2425,21 +2508,14 @@ cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const floa
   if (kInBlock)
     smem += static_cast<size_t>(plan.groupsPerBlock) * plan.ommPerWarp * kInBlockPoses * plan.chunks * 3 * sizeof(float);
   if (smem > 48 * 1024) {
-    const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock, kCone>,
+    const cudaError_t e = cudaFuncSetAttribute(renderKernel<kMode, kRegs, kWidth, kInBlock, kCone, kDraws>,
                                                cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
     if (e != cudaSuccess) return e;
   }
-  renderKernel<kMode, kRegs, kWidth, kInBlock, kCone><<<static_cast<unsigned>(blocks), block, smem, stream>>>(
+  renderKernel<kMode, kRegs, kWidth, kInBlock, kCone, kDraws><<<static_cast<unsigned>(blocks), block, smem, stream>>>(
       scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats);
   return cudaGetLastError();
 }
-
-// Register budget of the plain render through cone lists.  Its loop needs
-// fewer than the tree search does: on 256 terrain poses x 6000 ommatidia x
-// 256 samples 48, 56, 64, 72, 80 and 96 registers take 7.6, 7.0, 6.9, 6.9,
-// 7.8 and 9.7 ms, and 64 is also the fastest on the box scene (1000 x 32), so
-// the variants (renderVariant) are for renders without lists.
-constexpr int kConeRegs = 64;
 
 // The instance for the two-wide BVH: through the cone lists when the eye has
 // them (with in-block chunk sums where the plan says so; planRender offers
@@ -2455,6 +2531,11 @@ cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* po
     return runRenderKernel<kMode, kRegs, 2, kHasInBlock, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag,
                                                                    rec, stats, stream);
   }
+  constexpr bool kMayDraw = kHasCone && (kMode == 0 || kMode == 4);  // only plain renders pre-draw
+  if (eye.cones && eye.draws)
+    return kMayDraw ? runRenderKernel<kMode, kRegs, 2, false, kHasCone, kMayDraw || !kHasCone>(
+                          scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats, stream)
+                    : cudaErrorInvalidValue;
   if (kHasCone && eye.cones)
     return runRenderKernel<kMode, kRegs, 2, false, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
                                                              stats, stream);
@@ -2718,6 +2799,9 @@ __device__ __forceinline__ uint32_t coneKey(float nd, float ud) {
 constexpr uint32_t kAdaptiveSortMinTris = 16384;
 
 constexpr uint32_t kPoolRounds = 8;
+// Tasks of a pool of `rounds` rounds when a task has spl.
+CR_HOST_DEVICE inline uint32_t poolTasks(uint32_t rounds, uint32_t spl) { return rounds > spl ? rounds / spl : 1u; }
+constexpr uint32_t kListEntries = 2;  // entries per warp of the list kernel at most (16 samples each)
 constexpr uint32_t kPoolSlots = 32 * kPoolRounds;
 constexpr uint32_t kAdaptiveWarps = 4;  // warps per 128-thread block
 
@@ -2748,7 +2832,7 @@ __global__ void __launch_bounds__(128, kMinBlocks)
   // segWidth, spl and chunks are powers of two (spp is): their logarithms
   // turn the slot arithmetic below into shifts and masks.
   const uint32_t lsw = __ffs(segWidth) - 1, lspl = __ffs(spl) - 1, lch = __ffs(chunks) - 1;
-  const uint32_t tpp = kPoolRounds / spl;  // tasks per pool
+  const uint32_t tpp = poolTasks(kPoolRounds, spl);  // tasks per pool
   const uint64_t task0 = static_cast<uint64_t>(pool - B.poolBase) * tpp;
   const uint64_t left = B.tasks - task0;
   const uint32_t nTasks = left < tpp ? static_cast<uint32_t>(left) : tpp;
@@ -2951,6 +3035,188 @@ __global__ void __launch_bounds__(128, kMinBlocks)
       const uint32_t chunk = static_cast<uint32_t>(t) & (chunks - 1u);
       float* dst = chunks == 1 ? sums + 3 * static_cast<size_t>(B.entries[i])
                                : B.partials + (static_cast<size_t>(i) * chunks + chunk) * 3;
+      dst[0] = col.x;
+      dst[1] = col.y;
+      dst[2] = col.z;
+    }
+  }
+}
+
+// Cone lists of a bucket's entries, list i at B.cones + i * kConeStride.
+__global__ void __launch_bounds__(kConeThreads)
+    entryConeKernel(DevScene sc, const float4* __restrict__ omm, uint32_t N, const float4* __restrict__ poses,
+                    const uint32_t* __restrict__ entries, uint64_t count, float4* __restrict__ cones) {
+  __shared__ uint2 work[kConeEntries * kConeThreads];
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
+  if (i >= count) return;
+  const uint32_t e = entries[i], p = e / N;
+  coneList(sc, omm, e - p * N, poses + 4 * static_cast<size_t>(p), work + threadIdx.x, cones + i * kConeStride);
+}
+
+// The adaptive render through cone lists (entries of at least 16 samples, see
+// adaptiveLists).  A warp is a block of its own and works through the tasks of
+// one pool, round by round: 32 rays of one entry (two entries of 16) test
+// their list's triangles in step, the list of the next task arriving in
+// shared memory meanwhile.  Draws, their order (sorted by coneKey on deep
+// scenes with several rounds a task) and the order of the sums are
+// adaptiveKernel's, so the results are the same bits.  There is no refill:
+// with the lists few rays are long, and whole rounds were the fastest
+// schedule before too.  Pools start with the largest sample counts, whose
+// rays are the longest, so that the launch does not end on them.
+template <bool kRec>
+__global__ void __maxnreg__(kConeRegs)
+    adaptiveListKernel(DevScene sc, const float4* __restrict__ omm, uint32_t N, const float4* __restrict__ poses,
+                       AdaptiveLaunch L, unsigned long long seed, float* __restrict__ sums, uint32_t* errFlag,
+                       RayRecord* __restrict__ rec) {
+  extern __shared__ float4 renderSmem[];
+  const uint32_t lane = threadIdx.x;
+  const uint32_t pool = static_cast<uint32_t>(L.totalPools) - 1u - blockIdx.x;
+  uint32_t bi = 0;
+  while (bi + 1 < L.nBuckets && pool >= L.b[bi + 1].poolBase) ++bi;
+  const AdaptiveBucket& B = L.b[bi];
+  const uint32_t spp = B.spp;
+  const uint32_t segWidth = spp < 32u ? spp : 32u;
+  const uint32_t spl = adaptiveSamplesPerLane(spp);  // rounds per task
+  const uint32_t chunks = adaptiveChunks(spp);
+  const uint32_t lsw = __ffs(segWidth) - 1, lspl = __ffs(spl) - 1, lch = __ffs(chunks) - 1;
+  const uint32_t tpp = poolTasks(L.poolRounds, spl);
+  const uint64_t task0 = static_cast<uint64_t>(pool - B.poolBase) * tpp;
+  const uint64_t left = B.tasks - task0;
+  const uint32_t nTasks = left < tpp ? static_cast<uint32_t>(left) : tpp;
+  const bool sorted = spl > 1 && sc.triCount >= kAdaptiveSortMinTris;
+  const float invSpp = 1.0f / static_cast<float>(spp);
+  const uint32_t segLane = lane & (segWidth - 1u), segIdx = lane >> lsw;
+  float4* lists = renderSmem + segIdx * (2 * kConeStride);
+  float2* draw = reinterpret_cast<float2*>(renderSmem + kListEntries * 2 * kConeStride);
+  uint32_t* key = reinterpret_cast<uint32_t*>(draw + 32 * L.slotRounds);
+  uint32_t* idx = key + 32 * L.slotRounds;
+
+  // Entry (index within the bucket) of the lane's segment in task q.
+  auto entryOf = [&](uint32_t q) -> uint64_t { return (((task0 + q) >> lch) << (5 - lsw)) + segIdx; };
+  auto fetch = [&](uint32_t q) {
+    const uint64_t i = entryOf(q);
+    if (q < nTasks && i < B.count) {
+      const float4* src = B.cones + i * kConeStride;
+      float4* dst = lists + (q & 1u) * kConeStride;
+      for (uint32_t j = segLane; j < static_cast<uint32_t>(kConeStride); j += segWidth) fetchFloat4(src + j, dst + j);
+    }
+    commitCone();
+  };
+  fetch(0);
+
+  if (sorted) {  // as adaptiveKernel: draws and keys of every slot, then a bitonic sort of each task's
+    const uint32_t nSlots = nTasks * spl * 32u;
+    for (uint32_t j = lane; j < nSlots; j += 32u) {
+      const uint32_t q = (j >> 5) >> lspl, k = j & ((32u << lspl) - 1u);
+      const uint64_t t = task0 + q;
+      const uint64_t i = t >> lch;
+      const uint32_t chunk = static_cast<uint32_t>(t) & (chunks - 1u);
+      float2 d = make_float2(0.f, 0.f);
+      if (i < B.count) d = netDraw(seed, B.entries[i], (chunk << (5 + lspl)) + k);
+      draw[j] = d;
+      key[j] = coneKey(d.x, d.y);
+      idx[j] = k;
+    }
+    __syncwarp();
+    const uint32_t n = 32u * spl, lhalf = 4 + lspl;
+    for (uint32_t size = 2; size <= n; size <<= 1)
+      for (uint32_t ls = __ffs(size) - 2, stride = size >> 1; stride > 0; stride >>= 1, --ls) {
+        for (uint32_t m = lane; m < nSlots / 2; m += 32u) {
+          const uint32_t seg = (m >> lhalf) << (lhalf + 1), mm = m & ((1u << lhalf) - 1u);
+          const uint32_t lo = seg + (((mm >> ls) << ls) << 1) + (mm & (stride - 1u)), hi = lo + stride;
+          const bool up = ((lo - seg) & size) == 0u;
+          const uint32_t ka = key[lo], kb = key[hi];
+          if ((ka > kb) == up) {
+            key[lo] = kb;
+            key[hi] = ka;
+            const uint32_t t2 = idx[lo];
+            idx[lo] = idx[hi];
+            idx[hi] = t2;
+          }
+        }
+        __syncwarp();
+      }
+  }
+
+  for (uint32_t q = 0; q < nTasks; ++q) {
+    __syncwarp();  // every lane has read the buffer that is filled next
+    fetch(q + 1);
+    awaitOlderCone();
+    __syncwarp();
+    const uint64_t i = entryOf(q);
+    const uint32_t chunk = static_cast<uint32_t>(task0 + q) & (chunks - 1u);
+    const bool valid = i < B.count;
+    v3 col = mk(0.f, 0.f, 0.f);
+    const uint32_t e = valid ? B.entries[i] : 0u;
+    // Lanes past the bucket's last entry go along with entry 0 of the eye and
+    // count for nothing.
+    const float4* list = lists + (q & 1u) * kConeStride;
+    const float4 head = valid ? list[0] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const v3 org = mk(head.y, head.z, head.w);
+    const uint32_t listed = __float_as_uint(head.x);
+    const uint32_t entries = __reduce_max_sync(0xffffffffu, listed == kConeFromRoot ? 0u : listed);
+    {
+      const uint32_t p = e / N, o = e - p * N;
+      const float4 a = __ldg(omm + 2 * o), b = __ldg(omm + 2 * o + 1);
+      const v3 axis = mk(a.w, b.x, b.y);
+      const float fpo = b.w, sd = b.z / FWHM_SD_RATIO;
+      v3 perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
+      perp = (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
+      const float4* pp = poses + 4 * static_cast<size_t>(p);
+      for (uint32_t r = 0; r < spl; ++r) {
+        const uint32_t seg = q << (5 + lspl), j = seg + (r << 5) + lane;
+        const uint32_t k = sorted ? idx[j] : (spl > 1 ? (r << 5) + lane : segLane);
+        const uint32_t sample = (chunk << (5 + lspl)) + k;
+        const float2 d = sorted ? draw[seg + k] : netDraw(seed, e, sample);
+        const float4 X = __ldg(pp + 1), Y = __ldg(pp + 2), Z = __ldg(pp + 3);
+        const v3 splayed = rotatePoint(axis, d.x * sd, perp);
+        const v3 rel = rotatePoint(splayed, d.y * CR_PI_F, axis);
+        const v3 dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
+        Hit h;
+        uint32_t nv = 0, tt = 0;
+        traceCone<false>(sc, list, listed, entries, org, dir, fpo, valid ? d.x : 0.0f, h, errFlag, nv, tt);
+        v3 c;
+        float b1 = 0.f, b2 = 0.f;
+        if (h.id != 0xffffffffu) {
+          b1 = xdiv(h.V, h.det);
+          b2 = xdiv(h.W, h.det);
+          c = shadeHit(sc, h.pos, b1, b2);
+        } else {
+          c = shadeMiss(sc.miss, dir);
+        }
+        if (kRec && valid) {
+          RayRecord& R = rec[static_cast<size_t>(i) * spp + sample];
+          R.normalDraw = d.x;
+          R.uniformDraw = d.y;
+          R.ox = org.x;
+          R.oy = org.y;
+          R.oz = org.z;
+          R.dx = dir.x;
+          R.dy = dir.y;
+          R.dz = dir.z;
+          R.t = h.id != 0xffffffffu ? h.t : -1.0f;
+          R.b1 = b1;
+          R.b2 = b2;
+          R.hitId = h.id != 0xffffffffu ? static_cast<int32_t>(h.id) : -1;
+          R.r = c.x;
+          R.g = c.y;
+          R.b = c.z;
+          R.pad = 0.f;
+        }
+        if (valid) {
+          col.x = fmaf(c.x, invSpp, col.x);
+          col.y = fmaf(c.y, invSpp, col.y);
+          col.z = fmaf(c.z, invSpp, col.z);
+        }
+      }
+    }
+    for (uint32_t m = segWidth >> 1; m >= 1u; m >>= 1) {
+      col.x += __shfl_xor_sync(0xffffffffu, col.x, static_cast<int>(m));
+      col.y += __shfl_xor_sync(0xffffffffu, col.y, static_cast<int>(m));
+      col.z += __shfl_xor_sync(0xffffffffu, col.z, static_cast<int>(m));
+    }
+    if (segLane == 0u && valid) {
+      float* dst = chunks == 1 ? sums + 3 * static_cast<size_t>(e) : B.partials + (i * chunks + chunk) * 3;
       dst[0] = col.x;
       dst[1] = col.y;
       dst[2] = col.z;
@@ -3165,8 +3431,15 @@ void setAdaptiveBlocksPerSM(int blocks) { g_adaptiveBlocks = (blocks == 6 || blo
 int adaptiveBlocksPerSM() { return g_adaptiveBlocks; }
 
 AdaptiveLaunch planAdaptive(const uint32_t* const* entries, const uint64_t* counts, const uint32_t* spp,
-                            float* const* partials, uint32_t nBuckets) {
+                            float* const* partials, uint32_t nBuckets, const float4* const* cones) {
   AdaptiveLaunch L{};
+  if (cones) {
+    // Rounds per pool of the list kernel: fewer when the launch has fewer than
+    // eight pools of 8 for each of the GPU's warps (152 SMs x 32).
+    uint64_t rounds = 0;
+    for (uint32_t k = 0; k < nBuckets; ++k) rounds += (counts[k] * spp[k] + 31) / 32;
+    while (L.poolRounds > 1 && rounds / L.poolRounds < 8ull * 152 * 32) L.poolRounds /= 2;
+  }
   uint64_t tasks = 0, pools = 0;
   for (uint32_t k = 0; k < nBuckets && L.nBuckets < kAdaptiveBuckets; ++k) {
     if (counts[k] == 0) continue;
@@ -3175,12 +3448,13 @@ AdaptiveLaunch planAdaptive(const uint32_t* const* entries, const uint64_t* coun
     B.count = counts[k];
     B.spp = spp[k];
     B.partials = partials[k];
+    B.cones = cones ? cones[k] : nullptr;
     B.taskBase = tasks;
     B.poolBase = pools;
     const uint64_t segWidth = spp[k] < 32 ? spp[k] : 32;
     const uint64_t perWarp = 32 / segWidth, chunks = adaptiveChunks(spp[k]);
     B.tasks = (counts[k] + perWarp - 1) / perWarp * chunks;
-    const uint64_t tpp = kPoolRounds / adaptiveSamplesPerLane(spp[k]);
+    const uint64_t tpp = poolTasks(L.poolRounds, adaptiveSamplesPerLane(spp[k]));
     tasks += B.tasks;
     pools += (B.tasks + tpp - 1) / tpp;
   }
@@ -3314,7 +3588,29 @@ cudaError_t launchAdaptive(const DevScene& scene, const float4* omm, uint32_t N,
   if (L.totalPools >= (1ull << 26)) return cudaErrorInvalidConfiguration;  // 32-bit thread ids
   if (L.refillIdle < 1 || L.refillIdle > 32 || L.steps < 1) return cudaErrorInvalidValue;
   const uint64_t blocks = (L.totalPools * 32 + 127) / 128;
-  switch (scene.width) {
+  const bool lists = L.b[0].cones != nullptr;
+  for (uint32_t k = 0; k < L.nBuckets; ++k)
+    if ((L.b[k].cones != nullptr) != lists || (lists && (L.b[k].spp < 32u / kListEntries || scene.width != 2)))
+      return cudaErrorInvalidValue;
+  if (lists) {
+    // Slots of a pool: its rounds, or one task's when that has more.
+    uint32_t rounds = L.poolRounds;
+    bool sorted = false;
+    for (uint32_t k = 0; k < L.nBuckets; ++k) {
+      rounds = std::max(rounds, adaptiveSamplesPerLane(L.b[k].spp));
+      sorted = sorted || adaptiveSamplesPerLane(L.b[k].spp) > 1;
+    }
+    AdaptiveLaunch M = L;
+    M.slotRounds = rounds;
+    sorted = sorted && scene.triCount >= kAdaptiveSortMinTris;
+    const size_t smem = kListEntries * 2 * kConeStride * sizeof(float4) + (sorted ? 32ull * rounds * 16 : 0);
+    if (rec)
+      adaptiveListKernel<true><<<static_cast<unsigned>(L.totalPools), 32, smem, stream>>>(scene, omm, N, poses, M, seed,
+                                                                                          sums, errFlag, rec);
+    else
+      adaptiveListKernel<false><<<static_cast<unsigned>(L.totalPools), 32, smem, stream>>>(scene, omm, N, poses, M,
+                                                                                           seed, sums, errFlag, rec);
+  } else switch (scene.width) {
     case 4:
       adaptiveKernel<4><<<static_cast<unsigned>(blocks), 128, 0, stream>>>(scene, omm, N, poses, L, seed, sums, errFlag,
                                                                            rec, nullptr);
@@ -3342,6 +3638,20 @@ cudaError_t launchAdaptive(const DevScene& scene, const float4* omm, uint32_t N,
     e = cudaGetLastError();
   }
   return e;
+}
+
+bool adaptiveLists(const DevScene& scene, uint32_t spp, uint64_t launchRays) {
+  return scene.width == 2 && spp >= 32u / kListEntries && coneWorth(scene, launchRays);
+}
+
+cudaError_t launchEntryCones(const DevScene& scene, const float4* omm, uint32_t N, const float4* poses,
+                             const uint32_t* entries, uint64_t count, float4* cones, cudaStream_t stream) {
+  if (count == 0) return cudaSuccess;
+  const uint64_t blocks = (count + kConeThreads - 1) / kConeThreads;
+  if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
+  entryConeKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, omm, N, poses, entries, count,
+                                                                             cones);
+  return cudaGetLastError();
 }
 
 cudaError_t launchLabels(const float* outs, int k, uint64_t rows, uint32_t spp, float thr, uint16_t* label,

@@ -192,3 +192,96 @@ def test_batch_with_and_without_lists(lib, tmp_path):
         o = lib.crBatchOutputOffset(h, i)
         assert np.array_equal(got[o:o + want[i].size].reshape(want[i].shape), want[i]), spp[i]
     lib.crBatchDestroy(h)
+
+
+def _deep_scene(lib, tmp_path):
+    """A terrain deep enough for sorted rounds (at least 16384 triangles)."""
+    info = scenes.terrain_scene(str(tmp_path), cells=96, extent=60.0, cones=40, n_omm=500, poses=1)
+    lib.loadGlTFscene(info["gltf"].encode())
+    assert eh.lastError(lib) == "" and lib.crGetTriangleCount() >= 16384
+    eh.gotoFirstCompoundEye(lib)
+    return info
+
+
+@pytest.mark.parametrize("deep", [False, True])
+@pytest.mark.parametrize("spp", [16, 32, 64, 256, 512])
+def test_adaptive_records_with_and_without_lists(lib, small, tmp_path, deep, spp):
+    """crAdaptiveRecord through lists and (under a memory cap) without: the
+    same rays, hits, colours and sums.  Two entries a warp, one round, several,
+    a pool's worth, two chunks; an odd number of entries."""
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    if deep:
+        info = _deep_scene(lib, tmp_path)
+        p12 = scenes.random_poses(info["height_fn"], 3, np.random.default_rng(5), 20.0)
+    else:
+        lib.loadGlTFscene(small["gltf"].encode())
+        eh.gotoFirstCompoundEye(lib)
+        p12 = scenes.open_poses(small["boxes"], 3, np.random.default_rng(6))
+    n = (2 ** (19 if deep else 21) // (3 * spp) + 2) | 1
+    omm = _eye(n, "odd")
+    lib.setOmmatidia(omm.ctypes.data, n)
+    lib.setCurrentEyeSamplesPerOmmatidium(1)
+    p12 = np.ascontiguousarray(p12, np.float32)
+    rows = 3 * n
+    got = []
+    for lists in (True, False):
+        rec = np.zeros((rows, spp), eh.RAY_RECORD_DTYPE)
+        sums = np.zeros((rows, 3), np.float32)
+        if lists:
+            assert lib.crAdaptiveRecord(p12[:1], 1, 1, 9, np.zeros((n, 1), eh.RAY_RECORD_DTYPE).ctypes.data,
+                                        np.zeros((n, 3), np.float32)) == 0, eh.lastError(lib)
+        else:
+            lib.loadGlTFscene(info["gltf"].encode() if deep else small["gltf"].encode())  # gives the lists back
+            eh.gotoFirstCompoundEye(lib)
+            lib.setOmmatidia(omm.ctypes.data, n)
+            lib.setCurrentEyeSamplesPerOmmatidium(1)
+            assert lib.crAdaptiveRecord(p12[:1], 1, 1, 9, np.zeros((n, 1), eh.RAY_RECORD_DTYPE).ctypes.data,
+                                        np.zeros((n, 3), np.float32)) == 0, eh.lastError(lib)
+            need = rows * (4 + 12 + 12 * max(1, spp // 256) + 64 * spp) + rows * 100
+            assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + need) == 0
+        held = lib.crGetDeviceMemoryHeld()
+        try:
+            assert lib.crAdaptiveRecord(p12, 3, spp, 9, rec.ctypes.data, sums) == 0, eh.lastError(lib)
+        finally:
+            lib.crSetDeviceMemoryCap(0)
+        assert (lib.crGetDeviceMemoryHeld() - held >= rows * (64 * spp + 400)) == lists
+        got.append((rec, sums))
+    assert got[0][0].tobytes() == got[1][0].tobytes()
+    assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
+
+
+def test_adaptive_render_with_and_without_lists(lib, tmp_path):
+    """The whole adaptive render with entries in several buckets."""
+    import torch
+
+    info = _deep_scene(lib, tmp_path)
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    omm, P = _eye(2501, "plain"), 20
+    p12 = scenes.random_poses(info["height_fn"], P, np.random.default_rng(8), 20.0)
+    p16 = np.zeros((P, 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = p12[:, 3 * k:3 * k + 3]
+    d_poses = torch.from_numpy(p16).cuda()
+    res = []
+    lib.crDenoiserRelease()
+    assert lib.crAllocatorInit(3) == 0 and lib.crSetAllocatorHalvings(-4.0) == 0
+    try:
+        for lists in (True, False):
+            lib.loadGlTFscene(info["gltf"].encode())
+            eh.gotoFirstCompoundEye(lib)
+            lib.setOmmatidia(omm.ctypes.data, len(omm))
+            lib.setCurrentEyeSamplesPerOmmatidium(1)
+            out = torch.full((P, len(omm), 3), -1.0, device="cuda")
+            lev = torch.zeros((P, len(omm)), dtype=torch.uint8, device="cuda")
+            torch.cuda.synchronize()
+            if not lists:  # buffers of the first render are still there; no room for lists
+                assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + (12 << 20)) == 0
+            assert lib.crAdaptiveRenderPosesDevice(d_poses.data_ptr(), P, 8, out.data_ptr(),
+                                                   lev.data_ptr(), None) == 0, eh.lastError(lib)
+            assert lib.crSynchronize() == 0, eh.lastError(lib)
+            res.append((out.cpu().numpy(), lev.cpu().numpy()))
+    finally:
+        lib.crSetDeviceMemoryCap(0)
+        lib.crSetAllocatorHalvings(0.0)
+    assert len(np.unique(res[0][1])) >= 2 and (res[0][1] != 255).mean() > 0.5
+    assert np.array_equal(res[0][1], res[1][1]) and np.array_equal(res[0][0], res[1][0])
