@@ -172,7 +172,8 @@ size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint
 
 // Cone lists (DevEye::cones, kConeStride float4 each) worth providing for a
 // P-pose launch: P x N, or 0 when the launch does not use them.
-size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false);
+size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec = false,
+                       bool stats = false);
 // The same for an eye of a batch with that plan; batchRays: the rays of the
 // whole batch.
 size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, uint32_t P, uint64_t batchRays);
@@ -195,7 +196,10 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
 // triangle tests; the allocator's cost term).  stats: P x N x kFeatureStats
 // floats.
 // cutsReady: eye.cuts already holds these poses' near-field cuts (else they
-// are built first when eye.cuts is set).
+// are built first when eye.cuts is set).  Through cone lists (eye.cones, for
+// featureConeLists() lists) the traversal cost is 0: for callers that do not
+// read it.
+size_t featureConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P);
 constexpr int kFeatureStats = 12;
 constexpr int kCostStat = 11;  // index of the traversal cost in a stats row
 cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P, float* stats,

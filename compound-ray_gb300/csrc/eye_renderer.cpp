@@ -624,23 +624,27 @@ struct Renderer {
 
   // Poses of one launch: at most kMaxPosesPerLaunch, and fewer for large eyes
   // so that a launch's cone lists stay within kConeListBytes.
-  static size_t posesPerLaunch(uint32_t N) {
-    const size_t fit = kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N));
-    return std::min<size_t>(kMaxPosesPerLaunch, std::max<size_t>(1, fit));
+  static size_t conePoses(uint32_t N) {
+    return std::max<size_t>(1, kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N)));
+  }
+  static size_t posesPerLaunch(uint32_t N) { return std::min<size_t>(kMaxPosesPerLaunch, conePoses(N)); }
+
+  // Sets de.cones to a buffer of `lists` cone lists when there are any to
+  // build and the memory is to be had; not while the stream is being captured
+  // (the buffer may be given back before the captured graph runs).
+  void takeCones(DevEye& de, size_t lists) {
+    de.cones = nullptr;
+    if (!lists || lists * kConeStride * sizeof(float4) > kConeListBytes) return;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
+    if (st == cudaStreamCaptureStatusNone && cones.tryEnsure(lists * kConeStride)) de.cones = cones.ptr;
   }
 
   // Cone lists for a P-pose launch that uses them, when the memory for them
   // is to be had, and the launch's scratch (returned; null when it needs
-  // none).  No lists while the stream is being captured: the buffer may be
-  // given back before the captured graph runs.
+  // none).
   float* withCones(DevEye& de, uint32_t P, DevBuf<float>& scr, bool rec, bool stats) {
-    de.cones = nullptr;
-    const size_t lists = conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec);
-    if (lists && lists * kConeStride * sizeof(float4) <= kConeListBytes) {
-      cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-      check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
-      if (st == cudaStreamCaptureStatusNone && cones.tryEnsure(lists * kConeStride)) de.cones = cones.ptr;
-    }
+    takeCones(de, conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec, stats));
     for (;;) {
       const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, de.cones != nullptr);
       if (need) scr.ensure(need);
@@ -2052,8 +2056,10 @@ DevEye streamsFor(Renderer& r, EyeDev& e, DevBuf<uint32_t>& rng, uint32_t& haveS
 // layer-by-layer path use.
 constexpr unsigned long long kFeatureSeed = 0xfea70000ull;  // draw seed of the feature renders
 
+// cost: the caller reads the statistics' traversal cost (the adaptive render);
+// without it the render may go through cone lists.
 void denoiseFeatures(Renderer& r, DenoiseState& d, EyeDev& e, const float4* dposes, size_t count, uint32_t featSpp,
-                     bool rows = true) {
+                     bool rows = true, bool cost = false) {
   if (featSpp < 1 || featSpp > 32) throw std::runtime_error("feature renders use 1 to 32 samples per ommatidium");
   if (count > 0xffffffffull) throw std::runtime_error("too many poses in one feature render");
   // Stratified draws keyed by frame (featFrame + p) of the eye and the
@@ -2071,8 +2077,18 @@ void denoiseFeatures(Renderer& r, DenoiseState& d, EyeDev& e, const float4* dpos
   d.lastPassRows = 0;  // the statistics of the last adaptive pass are overwritten
   d.stats.ensure(std::max<size_t>(1, count * e.N * kFeatureStats));
   r.withCuts(fe, static_cast<uint32_t>(count), e.maxRel);
-  check(launchFeatures(r.dev, fe, dposes, static_cast<uint32_t>(count), d.stats.ptr, r.errWord(), r.stream(), false),
-        "feature render");
+  // One launch for all poses, or, with cone lists, one for each kConeListBytes
+  // of them.
+  const size_t perLaunch =
+      !cost && featureConeLists(r.dev, e.N, featSpp, static_cast<uint32_t>(count)) ? r.conePoses(e.N) : count;
+  for (size_t first = 0; first < count; first += perLaunch) {
+    const uint32_t P = static_cast<uint32_t>(std::min(perLaunch, count - first));
+    r.takeCones(fe, cost ? 0 : featureConeLists(r.dev, e.N, featSpp, P));
+    check(launchFeatures(r.dev, fe, dposes + 4 * first, P, d.stats.ptr + first * e.N * kFeatureStats, r.errWord(),
+                         r.stream(), false),
+          "feature render");
+    fe.frame0 += P;
+  }
   if (!rows) return;
   d.X.ensure(std::max<size_t>(1, count * e.N * kFeatureWidth));
   d.base.ensure(std::max<size_t>(1, count * e.N * 3));
@@ -2544,7 +2560,7 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
         for (size_t first = 0; first < count; first += perPass) {
           const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perPass, count - first));
           const uint64_t rows = static_cast<uint64_t>(P) * e.N;
-          denoiseFeatures(r, d, e, poses + 4 * first, P, fs, false);
+          denoiseFeatures(r, d, e, poses + 4 * first, P, fs, false, true);
           rays += static_cast<double>(rows) * fs;
           d.pred.ensure(rows * 3);
           if (d.inferKernel == 1) {

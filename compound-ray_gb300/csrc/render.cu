@@ -1504,9 +1504,11 @@ __device__ __forceinline__ void flushChunkSums(const float* __restrict__ part, c
   __syncthreads();
 }
 
-// Shared memory of a warp of the cone-list path, in float4: two list buffers,
-// the ommatidium's constants and the lanes' PairStreams (32 x (16 + 8 + 8) B).
-constexpr uint32_t kConeWarpFloat4 = 2 * kConeStride + 3 + 64;
+// Shared memory of the cone-list path, in float4: per segment two list buffers
+// and the ommatidium's constants, per warp those of its segments and the
+// lanes' PairStreams (32 x (16 + 8 + 8) B).
+constexpr uint32_t kConeSegFloat4 = 2 * kConeStride + 3;
+__host__ __device__ constexpr uint32_t coneWarpFloat4(uint32_t ommPerWarp) { return ommPerWarp * kConeSegFloat4 + 64; }
 
 // A lane's random numbers, the same as one curand_normal and one
 // curand_uniform per frame: the stream of a pair of frames is drawn at once
@@ -1590,9 +1592,10 @@ constexpr int kConeRegs = 64;
 // calls this function with the same poses (flushChunkSums has barriers).
 // kWidth: 2 searches the BVH2 (with the near-field cut when eye.cuts is
 // set), 4 or 8 the wide BVH of that width (no cut).
-// kCone: closest hits through the cone lists at eye.cones (kWidth 2).
+// kCone: closest hits through the cone lists at eye.cones (kWidth 2), for
+// whole-warp segments (1) or several ommatidia and lists per warp (2).
 // kDraws: the launch may have pre-drawn numbers (eye.draws).
-template <int kMode, int kWidth = 2, bool kCone = false, bool kDraws = true>
+template <int kMode, int kWidth = 2, int kCone = 0, bool kDraws = true>
 __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye, const float4* __restrict__ poses,
                                            uint32_t P, const WarpPlan& plan, uint64_t task, float* __restrict__ out,
                                            float* __restrict__ scratch, uint32_t* errFlag,
@@ -1600,11 +1603,10 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
                                            float* __restrict__ part = nullptr, float4* __restrict__ coneSmem = nullptr) {
   constexpr bool kRecord = (kMode & 3) == 1;
   constexpr bool kFeat = (kMode & 3) == 3;
-  constexpr bool kCount = (kMode & 3) == 2 || kFeat;  // feature mode: the per-entry traversal cost
+  constexpr bool kCount = (kMode & 3) == 2 || (kFeat && !kCone);  // feature mode without lists: the traversal cost
   constexpr bool kLit = (kMode & 4) != 0;  // lighting-on shading (modes 4 render, 5 record)
-  // Cone lists are for whole-warp segments (renderConeLists).
   const float2* draws = kDraws ? eye.draws : nullptr;
-  const uint32_t segWidth = kCone ? 32u : plan.segWidth, ommPerWarp = kCone ? 1u : plan.ommPerWarp;
+  const uint32_t segWidth = kCone == 1 ? 32u : plan.segWidth, ommPerWarp = kCone == 1 ? 1u : plan.ommPerWarp;
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t p0 = 0, p1 = P;
   if (plan.poseSplits > 1) {
@@ -1659,30 +1661,38 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
   }
   const float invSpp = 1.0f / static_cast<float>(eye.spp);
   // The cone-list path keeps what is the same for a whole pose loop in shared
-  // memory, so that the loop's registers hold the ray.
-  float4* fixed = kCone ? coneSmem + (threadIdx.x >> 5) * kConeWarpFloat4 + 2 * kConeStride : nullptr;
-  PairStream pair{reinterpret_cast<uint4*>(fixed + 3) + lane, reinterpret_cast<uint2*>(fixed + 3 + 32) + lane,
-                  reinterpret_cast<float2*>(fixed + 3 + 48) + lane, false, 0};
+  // memory, so that the loop's registers hold the ray: per segment two list
+  // buffers and its ommatidium's constants, then the lanes' PairStreams.
+  float4* coneBuf = nullptr;
+  const float4* coneNext = nullptr;  // the list to fetch next; pre-drawn numbers come the same way
+  const float2* drawNext = nullptr;
+  float4* fixed = nullptr;
+  PairStream pair{};
+  auto fetchList = [&](uint32_t p) {
+    float4* dst = coneBuf + (p & 1u) * kConeStride;
+    if (kCone == 1) fetchCone(coneNext, dst, lane);
+    else
+      for (uint32_t j = segLane; j < static_cast<uint32_t>(kConeStride); j += segWidth)
+        fetchFloat4(coneNext + j, dst + j);
+  };
   if (kCone) {
+    float4* warpSmem = coneSmem + (threadIdx.x >> 5) * coneWarpFloat4(ommPerWarp);
+    coneBuf = warpSmem + (lane / segWidth) * kConeSegFloat4;
+    fixed = coneBuf + 2 * kConeStride;
+    float4* streams = warpSmem + ommPerWarp * kConeSegFloat4;
+    pair.a = reinterpret_cast<uint4*>(streams) + lane;
+    pair.b = reinterpret_cast<uint2*>(streams + 32) + lane;
+    pair.ahead = reinterpret_cast<float2*>(streams + 48) + lane;
     __syncwarp();  // the warp's previous task has read its shared memory
-    if (valid && !draws) pair.begin(st);
-    if (lane == 0) {
+    if (!kFeat && valid && !draws) pair.begin(st);
+    if (segLane == 0) {  // valid wherever there is an ommatidium
       const v3 c = cross(perp, axis);
       fixed[0] = make_float4(axis.x, axis.y, axis.z, sd);
       fixed[1] = make_float4(perp.x, perp.y, perp.z, dot(perp, axis));
       fixed[2] = make_float4(c.x, c.y, c.z, fpo);
     }
-  }
-  // Cone lists: the warp's two buffers in shared memory, and the list to
-  // fetch next; pre-drawn numbers come the same way, into the slots that a
-  // PairStream would use.
-  float4* coneBuf = nullptr;
-  const float4* coneNext = nullptr;
-  const float2* drawNext = nullptr;
-  if (kCone) {
-    coneBuf = coneSmem + (threadIdx.x >> 5) * kConeWarpFloat4;
     coneNext = eye.cones + (static_cast<size_t>(p0) * eye.N + o) * kConeStride;
-    if (slot < eye.N) fetchCone(coneNext, coneBuf + (p0 & 1u) * kConeStride, lane);
+    if (slot < eye.N) fetchList(p0);
     if (draws) drawNext = draws + (static_cast<size_t>(p0) * eye.N + o) * eye.spp + s;
     if (draws && valid) fetchDraw(drawNext, pair.drawSlot(p0));
     commitCone();
@@ -1692,7 +1702,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     if (kCone) {
       __syncwarp();  // every lane has read the buffer that is filled next
       coneNext += static_cast<size_t>(eye.N) * kConeStride;
-      if (slot < eye.N && p + 1 < p1) fetchCone(coneNext, coneBuf + ((p + 1) & 1u) * kConeStride, lane);
+      if (slot < eye.N && p + 1 < p1) fetchList(p + 1);
       if (draws) {
         drawNext += plane;
         if (valid && p + 1 < p1) fetchDraw(drawNext, pair.drawSlot(p + 1));
@@ -1706,9 +1716,10 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     // hit triangle's normal in the eye's frame (facing the ray), all / spp.
     float f2x = 0.f, f2y = 0.f, f2z = 0.f, fHit = 0.f, fT = 0.f, fnx = 0.f, fny = 0.f, fnz = 0.f, fCost = 0.f;
     const uint32_t steps0 = nodeVisits + triTests;
-    // With cone lists all lanes of a warp with an ommatidium go on together;
-    // those past its last sample trace the axis and count for nothing.
-    if (kCone ? slot < eye.N : valid) {
+    // With cone lists all lanes of a warp go on together; those past an
+    // ommatidium's last sample (or past the last ommatidium, with an empty
+    // list) trace the axis and count for nothing.
+    if (kCone == 2 || (kCone == 1 ? slot < eye.N : valid)) {
       const float4* pp = poses + 4 * p;
       const float4 P0 = __ldg(pp), X = __ldg(pp + 1), Y = __ldg(pp + 2), Z = __ldg(pp + 3);
       float nd = 0.f, ud = 0.f;
@@ -1757,9 +1768,10 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         const float4* list = coneBuf + (p & 1u) * kConeStride;
         const float4 head = list[0];
         org = mk(head.y, head.z, head.w);
-        const uint32_t listed = __float_as_uint(head.x);
-        traceCone<kCount>(sc, list, listed, listed == kConeFromRoot ? 0u : listed, org, dir, fpo, nd, h,
-                                     errFlag, nodeVisits, triTests);
+        const uint32_t listed = kCone == 1 || slot < eye.N ? __float_as_uint(head.x) : 0u;
+        uint32_t entries = listed == kConeFromRoot ? 0u : listed;
+        if (kCone == 2) entries = __reduce_max_sync(0xffffffffu, entries);
+        traceCone<kCount>(sc, list, listed, entries, org, dir, fpo, nd, h, errFlag, nodeVisits, triTests);
       } else {
         org = rayOrigin(mk(P0.x, P0.y, P0.z), mk(X.x, X.y, X.z), mk(Y.x, Y.y, Y.z), mk(Z.x, Z.y, Z.z), relPos);
       }
@@ -1813,7 +1825,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         R.pad = 0.f;
       }
       if (!kCone || valid) col = c * invSpp;
-      if (kFeat) {
+      if (kFeat && (!kCone || valid)) {
         fCost = static_cast<float>(nodeVisits + triTests - steps0) * invSpp;
         f2x = c.x * c.x * invSpp;
         f2y = c.y * c.y * invSpp;
@@ -1832,7 +1844,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       }
     }
     // Segmented butterfly reduction over the samples of each ommatidium.
-    if constexpr (kCone) {
+    if constexpr (kCone == 1 && !kFeat) {
       // Whole-warp segments: the same pairwise sums with 6 exchanges in place
       // of 15.  After the first step the halves of the warp hold the sums of
       // x and y, after the second the quarters x, z, y, z.
@@ -1915,12 +1927,12 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
 // per-pose chunk partial in shared memory, and after every kInBlockPoses
 // poses the block sums each (ommatidium, pose) of the group over its chunks
 // in chunk order (flushChunkSums), so the buffer holds 16 poses at a time.
-template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false, bool kCone = false, bool kDraws = !kCone>
+template <int kMode, int kRegs, int kWidth = 2, bool kInBlock = false, int kCone = 0, bool kDraws = kCone == 0>
 __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses, uint32_t P,
                                                 WarpPlan plan, float* __restrict__ out, float* __restrict__ scratch,
                                                 uint32_t* errFlag, RayRecord* __restrict__ rec,
                                                 unsigned long long* stats) {
-  // kCone: the warps' cone lists; kInBlock: then the block's chunk partials.
+  // kCone: the warps' cone lists (kInBlock: of one segment each), then the block's chunk partials.
   extern __shared__ float4 renderSmem[];
   constexpr bool kCount = kMode == 2;
   uint32_t nodeVisits = 0, triTests = 0;
@@ -1930,7 +1942,7 @@ __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const f
   renderTask<kMode, kWidth, kCone, kDraws>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits,
                                            triTests,
                                    kInBlock ? reinterpret_cast<float*>(
-                                                  renderSmem + (kCone ? (blockDim.x >> 5) * kConeWarpFloat4 : 0))
+                                                  renderSmem + (kCone ? (blockDim.x >> 5) * coneWarpFloat4(1) : 0))
                                             : nullptr,
                                    renderSmem);
   if (kCount) {
@@ -2186,13 +2198,13 @@ __device__ __forceinline__ uint32_t lastAtMost(const T* base, uint32_t n, uint64
 // (ns), ctrl[2 + e] = completion time of eye e's last task (ns).
 // kCone: the kernel of the eyes that have cone lists (taskBase then counts
 // theirs alone, and the other kernel's the others').
-template <int kRegs, int kWidth = 2, bool kCone = false>
+template <int kRegs, int kWidth = 2, int kCone = 0>
 __global__ void __maxnreg__(kRegs) batchKernel(DevScene sc, const BatchEye* __restrict__ eyes,
                                                                const unsigned long long* __restrict__ taskBase,
                                                                uint32_t nEyes, unsigned long long totalTasks,
                                                                unsigned long long* counter, unsigned long long* ctrl,
                                                                uint32_t* errFlag) {
-  extern __shared__ float4 renderSmem[];  // kCone: kConeWarpFloat4 per warp
+  extern __shared__ float4 renderSmem[];  // kCone: coneWarpFloat4(1) per warp
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t nv = 0, tt = 0;
   bool first = true;
@@ -2205,7 +2217,7 @@ __global__ void __maxnreg__(kRegs) batchKernel(DevScene sc, const BatchEye* __re
     first = false;
     const uint32_t e = lastAtMost(taskBase, nEyes, task);
     const BatchEye& be = eyes[e];
-    renderTask<0, kWidth, kCone, !kCone>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag,
+    renderTask<0, kWidth, kCone, kCone == 0>(sc, be.eye, be.poses, be.P, be.plan, task - taskBase[e], be.out, be.scratch, errFlag,
                                  nullptr, nv, tt, nullptr, renderSmem);
     if (lane == 0) atomicMax(&ctrl[2 + e], globalTimerNs());
   }
@@ -2396,7 +2408,7 @@ WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, boo
   // A small eye's launch may spread its poses over more warps (pre-drawn
   // random numbers, splitPoses): that plan keeps the chunk partials in scratch.
   const bool maySplit = P >= 2 && p.tasks < kFillWarps / 2;
-  if (p.chunks > 1 && !forceScratch && inBlockAllowed && !maySplit && bw % p.chunks == 0) {
+  if (p.chunks > 1 && p.segWidth == 32 && !forceScratch && inBlockAllowed && !maySplit && bw % p.chunks == 0) {
     const uint32_t G = bw / p.chunks;
     const size_t bytes = static_cast<size_t>(G) * p.ommPerWarp * kInBlockPoses * p.chunks * 3 * sizeof(float);
     if (bytes <= kChunkSmemMax) {
@@ -2453,6 +2465,7 @@ static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool con
 // 1.5 / 1.1, 6 M 2.7 / 1.5, 82 M 3.6 / 2.0; at acceptance angles of 6 degrees
 // 82 M 3.0 / 1.6.
 constexpr uint32_t kConeDeepTris = 16384;
+constexpr uint32_t kConeMinSegment = 8;
 constexpr uint64_t kConeRaysDeep = 1ull << 19, kConeRaysShallow = 1ull << 21;
 
 static bool coneWorth(const DevScene& scene, uint64_t rays) {
@@ -2464,9 +2477,10 @@ size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, u
   return static_cast<size_t>(P) * N;
 }
 
-size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec) {
+size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec, bool stats) {
   if (!coneWorth(scene, static_cast<uint64_t>(N) * spp * P)) return 0;
-  if (planRender(N, spp, P, true).segWidth != 32) return 0;
+  const uint32_t seg = planRender(N, spp, P, true).segWidth;
+  if (seg < kConeMinSegment || (seg != 32 && (rec || stats || scene.lighting))) return 0;
   if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
   return static_cast<size_t>(P) * N;
 }
@@ -2497,14 +2511,14 @@ cudaError_t launchRngInit(const DevEye& eye, uint32_t* errFlag, cudaStream_t str
 namespace {
 // One launch of a render kernel instance with the plan's block size and, for
 // in-block chunk sums, the shared memory of the partials.
-template <int kMode, int kRegs, int kWidth, bool kInBlock, bool kCone, bool kDraws = !kCone>
+template <int kMode, int kRegs, int kWidth, bool kInBlock, int kCone, bool kDraws = kCone == 0>
 cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                             const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                             unsigned long long* stats, cudaStream_t stream) {
   const unsigned block = 32u * plan.blockWarps;
   const uint64_t blocks = (plan.tasks + plan.blockWarps - 1) / plan.blockWarps;
   if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
-  size_t smem = kCone ? plan.blockWarps * kConeWarpFloat4 * sizeof(float4) : 0;
+  size_t smem = kCone ? plan.blockWarps * coneWarpFloat4(plan.ommPerWarp) * sizeof(float4) : 0;
   if (kInBlock)
     smem += static_cast<size_t>(plan.groupsPerBlock) * plan.ommPerWarp * kInBlockPoses * plan.chunks * 3 * sizeof(float);
   if (smem > 48 * 1024) {
@@ -2524,23 +2538,38 @@ template <int kMode, int kRegs>
 cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                       const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                       unsigned long long* stats, cudaStream_t stream) {
-  constexpr bool kHasCone = kMode == 0 ? kRegs == kConeRegs : kMode != 3;
+  constexpr bool kHasCone = kMode == 0 || kMode == 3 ? kRegs == kConeRegs : true;
   constexpr bool kHasInBlock = kHasCone && (kMode == 0 || kMode == 1);
-  if (plan.inBlock) {
-    if (!kHasInBlock || !eye.cones) return cudaErrorInvalidValue;
-    return runRenderKernel<kMode, kRegs, 2, kHasInBlock, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag,
-                                                                   rec, stats, stream);
-  }
   constexpr bool kMayDraw = kHasCone && (kMode == 0 || kMode == 4);  // only plain renders pre-draw
-  if (eye.cones && eye.draws)
-    return kMayDraw ? runRenderKernel<kMode, kRegs, 2, false, kHasCone, kMayDraw || !kHasCone>(
-                          scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats, stream)
-                    : cudaErrorInvalidValue;
-  if (kHasCone && eye.cones)
-    return runRenderKernel<kMode, kRegs, 2, false, kHasCone>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
-                                                             stats, stream);
-  return runRenderKernel<kMode, kRegs, 2, false, false>(scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats,
-                                                        stream);
+  constexpr bool kSegments = kHasCone && (kMode == 0 || kMode == 3);  // several lists a warp
+  if (plan.inBlock && (!kHasInBlock || !eye.cones || plan.segWidth != 32)) return cudaErrorInvalidValue;
+  if (!eye.cones)
+    return runRenderKernel<kMode, kRegs, 2, false, 0>(scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats,
+                                                      stream);
+  if constexpr (kHasCone) {
+    if (plan.inBlock)
+      return runRenderKernel<kMode, kRegs, 2, kHasInBlock, 1>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
+                                                              stats, stream);
+    if (plan.segWidth != 32) {
+      if constexpr (kSegments) {
+        if (eye.draws)
+          return runRenderKernel<kMode, kRegs, 2, false, 2, kMode == 0>(scene, eye, poses, P, plan, out, scratch,
+                                                                        errFlag, rec, stats, stream);
+        return runRenderKernel<kMode, kRegs, 2, false, 2>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
+                                                          stats, stream);
+      }
+      return cudaErrorInvalidValue;
+    }
+    if (eye.draws) {
+      if constexpr (kMayDraw)
+        return runRenderKernel<kMode, kRegs, 2, false, 1, true>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
+                                                                stats, stream);
+      return cudaErrorInvalidValue;
+    }
+    return runRenderKernel<kMode, kRegs, 2, false, 1>(scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats,
+                                                      stream);
+  }
+  return cudaErrorInvalidValue;
 }
 
 // The plain render (mode 0) or the counting render (mode 2) of the scene's
@@ -2565,11 +2594,20 @@ cudaError_t runRenderWidth(const DevScene& scene, const DevEye& eye, const float
 }
 }  // namespace
 
+static cudaError_t launchCones(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
+                               cudaStream_t stream) {
+  const uint64_t lists = static_cast<uint64_t>(P) * eye.N, blocks = (lists + kConeThreads - 1) / kConeThreads;
+  if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
+  coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P);
+  return cudaGetLastError();
+}
+
 cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P, float* out,
                          float* scratch, uint32_t* errFlag, RayRecord* rec, cudaStream_t stream,
                          unsigned long long* stats, bool forceScratch) {
   if (P == 0 || eye.N == 0) return cudaSuccess;
-  if (eye.cones && renderConeLists(scene, eye.N, eye.spp, P, rec != nullptr) == 0) return cudaErrorInvalidValue;
+  if (eye.cones && renderConeLists(scene, eye.N, eye.spp, P, rec != nullptr, stats != nullptr) == 0)
+    return cudaErrorInvalidValue;
   WarpPlan plan = planRender(eye.N, eye.spp, P, forceScratch,
                              inBlockAllowed(scene, rec != nullptr, stats != nullptr, eye.cones != nullptr));
   if (plan.chunks > 1 && !plan.inBlock && scratch == nullptr) return cudaErrorInvalidValue;
@@ -2585,10 +2623,7 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     plan = splitPoses(plan, P, eye.cones ? 2 * kFillWarps : kFillWarps);
   }
   if (eye.cones) {
-    const uint64_t lists = static_cast<uint64_t>(P) * eye.N, blocks = (lists + kConeThreads - 1) / kConeThreads;
-    if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
-    coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P);
-    const cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launchCones(scene, eye, poses, P, stream);
     if (e != cudaSuccess) return e;
   } else if (eye.cuts && (scene.width == 2 || rec || scene.lighting)) {  // the wide BVH searches without a cut
     if (!(eye.cutRadius > 0.f)) return cudaErrorInvalidValue;
@@ -2624,6 +2659,11 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
   return cudaGetLastError();
 }
 
+size_t featureConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P) {
+  if (!coneWorth(scene, static_cast<uint64_t>(N) * spp * P) || planWarps(N, spp).segWidth < kConeMinSegment) return 0;
+  return static_cast<size_t>(P) * N;
+}
+
 cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P, float* stats,
                            uint32_t* errFlag, cudaStream_t stream, bool cutsReady) {
   if (P == 0 || eye.N == 0) return cudaSuccess;
@@ -2633,6 +2673,12 @@ cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float
   // Counter-based draws: spread the poses over enough warps for about a
   // dozen waves, so that the last one costs little.
   plan = splitPoses(plan, P, 4 * kFillWarps);
+  if (eye.cones) {
+    if (featureConeLists(scene, eye.N, eye.spp, P) == 0) return cudaErrorInvalidValue;
+    const cudaError_t e = launchCones(scene, eye, poses, P, stream);
+    if (e != cudaSuccess) return e;
+    return runRender<3, kConeRegs>(scene, eye, poses, P, plan, stats, nullptr, errFlag, nullptr, nullptr, stream);
+  }
   if (eye.cuts && !cutsReady) {
     if (!(eye.cutRadius > 0.f)) return cudaErrorInvalidValue;
     cutKernel<<<(P + 63) / 64, 64, 0, stream>>>(scene, poses, P, eye.cutRadius, eye.maxRel, eye.cuts);
@@ -2652,8 +2698,8 @@ namespace {
 template <typename F>
 cudaError_t withBatchKernel(int variant, int width, bool cones, F&& f) {
   if (cones) {
-    const size_t smem = batchBlockThreads() / 32 * kConeWarpFloat4 * sizeof(float4);
-    return width == 2 ? f(batchKernel<kConeRegs, 2, true>, smem) : cudaErrorInvalidValue;
+    const size_t smem = batchBlockThreads() / 32 * coneWarpFloat4(1) * sizeof(float4);
+    return width == 2 ? f(batchKernel<kConeRegs, 2, 1>, smem) : cudaErrorInvalidValue;
   }
   auto run = [&](auto regsTag) {
     constexpr int R = decltype(regsTag)::value;

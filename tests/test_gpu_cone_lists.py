@@ -17,9 +17,10 @@ import scenes
 
 pytestmark = pytest.mark.gpu
 
-# spp: the smallest that fills a warp segment, tails of one sample, one
-# chunk, several chunks in a block, chunks that no block holds.
-SPP = [17, 31, 32, 33, 64, 96, 256, 300, 513]
+# spp: the fewest that use lists and a full segment of 8 and of 16 lanes
+# (several lists a warp), the smallest whole-warp segment, tails of one sample,
+# one chunk, several chunks in a block, chunks that no block holds.
+SPP = [5, 8, 9, 16, 17, 31, 32, 33, 64, 96, 256, 300, 513]
 
 
 def _eye(n, kind):
@@ -94,7 +95,7 @@ def test_lists_change_no_bit(lib, small, kind, spp):
     lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     lib.loadGlTFscene(small["gltf"].encode())
     eh.gotoFirstCompoundEye(lib)
-    n = 701
+    n = 701 if spp > 16 else 2 ** 21 // (150 * spp) | 1
     P = 2 + 2 ** 21 // (n * spp)  # just past the fewest rays that use lists
     if P < 9:
         n, P = 2 ** 21 // (9 * spp) + 1, 9
@@ -102,6 +103,51 @@ def test_lists_change_no_bit(lib, small, kind, spp):
     assert with_lists[3] >= 400 * n * P and without[3] == 0  # the first did build lists
     for x, y in zip(with_lists[:3], without[:3]):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("segment", [8, 16])
+def test_lists_of_narrow_segments(lib, small, segment):
+    """Many samples in segments of 8 or 16 lanes: chunk partials of several
+    ommatidia a warp, with a last warp that is not full."""
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(small["gltf"].encode())
+    eh.gotoFirstCompoundEye(lib)
+    assert lib.crSetRenderLayout(128, segment) == 0
+    try:
+        with_lists, without = _both(lib, _eye(1401, "odd"), 50, _poses(small["boxes"], 31, 2))
+    finally:
+        lib.crSetRenderLayout(0, 32)
+    assert with_lists[3] > 400 * 1401 * 31
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("spp", [5, 8, 16, 20])
+def test_feature_rows_with_and_without_lists(lib, small, spp):
+    """Feature rows and 8-sample means of the denoiser."""
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    assert lib.crDenoiserInit(1) == 0
+    n = 3001
+    omm = _eye(n, "odd")
+    P = 2 ** 21 // (n * spp) + 2
+    p12 = scenes.open_poses(small["boxes"], P, np.random.default_rng(4))
+    got = []
+    for lists in (True, False):
+        lib.loadGlTFscene(small["gltf"].encode())
+        eh.gotoFirstCompoundEye(lib)
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(1)
+        x, base = np.zeros((P * n, 112), np.uint16), np.zeros((P * n, 3), np.float32)
+        if not lists:  # the statistics and rows of the first run are still held
+            assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + (40 << 20)) == 0
+        held = lib.crGetDeviceMemoryHeld()
+        try:
+            assert lib.crDenoiserFeatureRows(p12, P, spp, x, base) == 0, eh.lastError(lib)
+        finally:
+            lib.crSetDeviceMemoryCap(0)
+        assert (lib.crGetDeviceMemoryHeld() - held > 400 * P * n) == lists
+        got.append((x, base))
+    assert np.array_equal(got[0][0], got[1][0]) and np.array_equal(got[0][1], got[1][1], equal_nan=True)
 
 
 def test_lists_of_a_single_leaf_scene(lib, tmp_path):
