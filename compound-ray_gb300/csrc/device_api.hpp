@@ -283,17 +283,21 @@ cudaError_t inferDenoiser(const float* stats, const float4* omm, const int* nb, 
 // block waits on an mbarrier that nothing arrives on, for `polls` polls, then
 // sets kErrMmaTimeout in errFlag and returns.
 cudaError_t launchWaitProbe(uint32_t polls, uint32_t* errFlag, cudaStream_t stream);
-// Inputs of the tcgen05 prediction (mlp_tc.cu): per row of the P x N
-// statistics three float4 of derived values (derived: 3 N P float4), per
-// ommatidium its unit axis and acceptance angle (axes: N float4).
-cudaError_t deriveFeatureStats(const float* stats, const float4* omm, uint32_t N, uint32_t P, float4* derived,
-                               float4* axes, cudaStream_t stream);
+// Inputs of the tcgen05 prediction (mlp_tc.cu), in the eye's direction order
+// (`order`; null: index order): per row of the P x N statistics three float4
+// of derived values (derived: three planes of N P float4), per ommatidium its
+// unit axis and acceptance angle (axes: N float4).
+cudaError_t deriveFeatureStats(const float* stats, const float4* omm, uint32_t N, uint32_t P, const uint32_t* order,
+                               float4* derived, float4* axes, cudaStream_t stream);
+// The neighbour table (N x kNeighbours ommatidia) by position in that order:
+// nbSlots kNeighbours planes of N positions; slotOf: N words of scratch.
+cudaError_t slotNeighbours(const int* nb, const uint32_t* order, uint32_t N, uint32_t* slotOf, uint32_t* nbSlots,
+                           cudaStream_t stream);
 // The same prediction on the tcgen05 tensor cores (mlp_tc.cu) from
-// deriveFeatureStats' output: accumulators in TMEM, operands in shared
-// memory; errFlag receives kErrMmaTimeout if a bounded wait ran out.  order:
-// null, or the eye's direction order (rows of a tile are then neighbouring
-// ommatidia; results do not depend on it).
-cudaError_t inferDenoiserTc(const float4* derived, const float4* axes, const int* nb, uint32_t N, uint32_t P,
+// deriveFeatureStats' output and slotNeighbours' table for the same order:
+// accumulators in TMEM, operands in shared memory; errFlag receives
+// kErrMmaTimeout if a bounded wait ran out.
+cudaError_t inferDenoiserTc(const float4* derived, const float4* axes, const uint32_t* nbSlots, uint32_t N, uint32_t P,
                             const MlpWeights& w, float* out, uint32_t* errFlag, cudaStream_t stream,
                             bool residual = true, const uint32_t* order = nullptr);
 // Rows idx[offset .. offset + rows) of the training set, offset = *offset

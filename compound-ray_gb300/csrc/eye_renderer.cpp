@@ -1983,6 +1983,7 @@ struct DenoiseState {
   size_t cam = static_cast<size_t>(-1);
   uint64_t generation = ~0ull;
   DevBuf<int> nb;
+  DevBuf<uint32_t> nbSlots;  // the same by position in the direction order (tcgen05 inference)
   DevBuf<uint32_t> targetRng;  // XORWOW streams of the 1024-sample training targets
   uint32_t targetSpp = 0;
   bool targetReady = false;
@@ -2024,6 +2025,10 @@ EyeDev& denoiseEye(Renderer& r, DenoiseState& d) {
     d.nb.release();
     d.nb.ensure(std::max<size_t>(1, static_cast<size_t>(kNeighbours) * e.N));
     check(nearestOmmatidia(e.omm.ptr, e.N, d.nb.ptr, r.stream()), "neighbour search");
+    d.nbSlots.ensure((kNeighbours + 1) * std::max<size_t>(1, e.N));  // the table, then scratch
+    check(slotNeighbours(d.nb.ptr, e.order.ptr, e.N, d.nbSlots.ptr + static_cast<size_t>(kNeighbours) * e.N,
+                         d.nbSlots.ptr, r.stream()),
+          "neighbour table");
     d.targetReady = false;
     d.targetSpp = 0;
     d.adaptiveFrame = 0;
@@ -2198,10 +2203,10 @@ int crDenoiserRenderPosesDevice(const float* d_poses, size_t count, int featureS
           if (d.inferKernel == 1) {
             d.derived.ensure(static_cast<size_t>(3) * P * e.N);
             d.axes.ensure(std::max<size_t>(1, e.N));
-            check(deriveFeatureStats(st, e.omm.ptr, e.N, P, d.derived.ptr, d.axes.ptr, r.stream()), "feature statistics");
+            check(deriveFeatureStats(st, e.omm.ptr, e.N, P, e.order.ptr, d.derived.ptr, d.axes.ptr, r.stream()), "feature statistics");
           }
           check(d.inferKernel == 1
-                    ? inferDenoiserTc(d.derived.ptr, d.axes.ptr, d.nb.ptr, e.N, P, d.net.weights(),
+                    ? inferDenoiserTc(d.derived.ptr, d.axes.ptr, d.nbSlots.ptr, e.N, P, d.net.weights(),
                                       d_out + 3 * first * e.N, r.errWord(), r.stream(), true, e.order.ptr)
                     : inferDenoiser(st, e.omm.ptr, d.nb.ptr, e.N, P, d.net.weights(), d_out + 3 * first * e.N,
                                     r.stream()),
@@ -2566,12 +2571,12 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
           if (d.inferKernel == 1) {
             d.derived.ensure(3 * rows);
             d.axes.ensure(std::max<size_t>(1, e.N));
-            check(deriveFeatureStats(d.stats.ptr, e.omm.ptr, e.N, P, d.derived.ptr, d.axes.ptr, st),
+            check(deriveFeatureStats(d.stats.ptr, e.omm.ptr, e.N, P, e.order.ptr, d.derived.ptr, d.axes.ptr, st),
                   "feature statistics");
           }
           auto infer = [&](const MlpWeights& w, float* o, bool residual) {
             return d.inferKernel == 1
-                       ? inferDenoiserTc(d.derived.ptr, d.axes.ptr, d.nb.ptr, e.N, P, w, o, r.errWord(), st, residual,
+                       ? inferDenoiserTc(d.derived.ptr, d.axes.ptr, d.nbSlots.ptr, e.N, P, w, o, r.errWord(), st, residual,
                                          e.order.ptr)
                        : inferDenoiser(d.stats.ptr, e.omm.ptr, d.nb.ptr, e.N, P, w, o, st, residual);
           };

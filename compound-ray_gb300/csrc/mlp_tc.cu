@@ -3,30 +3,39 @@
 // Same function as inferKernel in mlp.cu (feature rows from the feature-render
 // statistics, 112 -> 128 -> 128 -> 128 -> 8 network with bf16 operands and
 // fp32 accumulation, bias + ReLU between layers, residual add), laid out for
-// sm_103a's MMA unit as a two-role pipeline in one persistent block of 768
+// sm_103a's MMA unit as a two-role pipeline in one persistent block of 1024
 // threads per SM:
 //   * all weights are staged once in shared memory as K-major UMMA operands
 //     (transposed to [out][in]) in the canonical no-swizzle layout: 8-row x
 //     16-byte core matrices, core matrices along K 128 bytes apart (leading
 //     byte offset) and 8-row groups K*16 bytes apart (stride byte offset);
 //   * feature warps 0-15 build the 112 features of each row of a 128-row
-//     tile (four threads per row: own block + neighbour 0 / neighbours 1-2 /
-//     3-4 / 5 + padding) from statistics derived once per row (deriveKernel:
-//     three float4) and unit axes (axesKernel), into one of two tile
-//     buffers, and signal it full on an mbarrier;
-//   * network warps 16-23 take the full buffer: one elected thread issues
-//     each layer's tcgen05.mma instructions (M = 128, N = 128, K = 16 each)
-//     into a 128-column TMEM accumulator and commits them to an mbarrier.
-//     Warps 16 + q and 20 + q read accumulator lanes 32 q .. +31, columns
-//     0-63 and 64-127, with tcgen05.ld, add the bias, apply ReLU, round to
-//     bf16 and write the next layer's operand into the same tile buffer (the
-//     MMAs that read it are done);
+//     tile from statistics derived once per row (deriveKernel: three float4)
+//     and unit axes (axesKernel), into one of three tile buffers, and signal
+//     it full on an mbarrier.  A warp holds one quarter of the features of 32
+//     rows, in whole 16-byte pieces (features 0-31, 32-63, 64-87, 88-111), so
+//     every store is a 16-byte row of a core matrix, without bank conflicts;
+//   * two groups of eight network warps (16-23 and 24-31) take the tiles in
+//     turn, each with a 128-column TMEM accumulator of its own: one elected
+//     thread of the group issues each layer's tcgen05.mma instructions (M =
+//     128, N = 128, K = 16 each) and commits them to the group's mbarrier.
+//     Warps q and 4 + q of a group read accumulator lanes 32 q .. +31,
+//     columns 0-63 and 64-127, with tcgen05.ld, add the bias, apply ReLU,
+//     round to bf16 and write the next layer's operand into the same tile
+//     buffer (the MMAs that read it are done);
 //     the last layer (N padded to 16) adds the residual base and writes the
 //     output, and its commit hands the buffer back to the feature warps.
-// So the feature warps gather tile i + 1 (and i + 2) while the network warps
-// run tile i.  Every mbarrier wait is bounded: on timeout the waiting side
-// records an error bit and stops; the other side then times out too, the
-// network warps wait (bounded) for their last commit, and the TMEM is freed.
+// A layer is a chain of waits (MMA, accumulator read, barrier) that leaves the
+// SM idle; with two tiles in flight one group's waits are the other's work,
+// and the third buffer lets the feature warps run ahead of both.  1.5 M rows
+// take 451 us with one group, two buffers, two-byte feature stores and a
+// 64-bit division a row, 358 us in this form, and 326 us with the statistics by
+// slot (deriveKernel); without any feature work 285 us: what is left is the
+// network side, whose operand reads, bias loads and activation stores share the
+// shared-memory pipe.
+// Every mbarrier wait is bounded: on timeout the waiting side records an error
+// bit and stops; the other side then times out too, the network warps wait
+// (bounded) for their last commit, and the TMEM is freed.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -41,9 +50,11 @@ namespace {
 
 constexpr int kTcRows = 128;
 constexpr int kFeatThreads = 512;  // feature warps 0-15: four threads per row
-constexpr int kNetThreads = 256;   // network warps 16-23: two per accumulator lane quarter
-constexpr int kTcThreads = kFeatThreads + kNetThreads;
-constexpr int kTmemCols = 128;
+constexpr int kNetThreads = 256;   // a network group's warps: two per accumulator lane quarter
+constexpr int kNetGroups = 2;
+constexpr int kTcThreads = kFeatThreads + kNetGroups * kNetThreads;
+constexpr int kTcBuffers = 3;
+constexpr int kTmemCols = 128 * kNetGroups;
 constexpr uint32_t kSpinLimit = 1u << 26;  // bounded waits (far longer than one layer's MMAs)
 
 // Byte offset of element (r, k) in a K-major no-swizzle operand with K
@@ -152,24 +163,41 @@ constexpr uint32_t kOffW1 = 0;
 constexpr uint32_t kOffW2 = kOffW1 + kW1Bytes;
 constexpr uint32_t kOffW3 = kOffW2 + kWBytes;
 constexpr uint32_t kOffW4 = kOffW3 + kWBytes;
-// Two tile buffers: features (K = 112 layout), then in place the hidden
-// activations of layers 1-3 (K = 128 layout).  Small enough that the rest of
-// the SM's 256 KB stays L1 cache for the feature gathers.
+// Tile buffers: features (K = 112 layout), then in place the hidden
+// activations of layers 1-3 (K = 128 layout).
 constexpr uint32_t kOffB0 = kOffW4 + kW4Bytes;
-constexpr uint32_t kOffB1 = kOffB0 + kActBytes;
-constexpr uint32_t kOffBias = kOffB1 + kActBytes;                   // 3 x 128 + 16 floats
-constexpr uint32_t kOffBar = kOffBias + (3 * kMlpHidden + 16) * 4;  // 5 mbarriers (8 B each) + TMEM address
-constexpr uint32_t kTcSmem = kOffBar + 48 + 128;                    // + alignment slack
+constexpr uint32_t kOffBias = kOffB0 + kTcBuffers * kActBytes;      // 3 x 128 + 16 floats
+constexpr uint32_t kBars = 2 * kTcBuffers + kNetGroups;             // full, empty, one per group's MMAs
+constexpr uint32_t kOffBar = kOffBias + (3 * kMlpHidden + 16) * 4;  // mbarriers (8 B each) + TMEM address
+constexpr uint32_t kTcSmem = kOffBar + 8 * kBars + 8 + 128;         // + alignment slack
 static_assert(kTcSmem <= 227 * 1024, "shared memory plan exceeds a block's limit");
 
-// Row (pose * N + ommatidium) processed at position x: poses in order, the
-// ommatidia of a pose in the eye's direction order, so that a tile's rows
-// are neighbouring ommatidia whose neighbour statistics overlap in L1.
-__device__ __forceinline__ uint64_t rowAt(uint64_t x, uint32_t N, const uint32_t* __restrict__ order) {
-  const uint64_t p = x / N;
-  const uint32_t j = static_cast<uint32_t>(x - p * N);
-  return p * N + (order ? __ldg(order + j) : j);
-}
+// Position of a thread's row: poses in order, the ommatidia of a pose in the
+// eye's direction order, so that a tile's rows are neighbouring ommatidia whose
+// neighbour statistics overlap in L1.  Steps from tile to tile without a
+// division.
+struct RowWalk {
+  uint64_t pos, stride;
+  uint32_t p, j, dp, dj, N;
+  __device__ __forceinline__ RowWalk(uint64_t first, uint64_t step, uint32_t n) : pos(first), stride(step), N(n) {
+    p = static_cast<uint32_t>(first / n);
+    j = static_cast<uint32_t>(first - static_cast<uint64_t>(p) * n);
+    dp = static_cast<uint32_t>(step / n);
+    dj = static_cast<uint32_t>(step - static_cast<uint64_t>(dp) * n);
+  }
+  __device__ __forceinline__ void next() {
+    pos += stride;
+    p += dp;
+    j += dj;
+    if (j >= N) {
+      j -= N;
+      ++p;
+    }
+  }
+  __device__ __forceinline__ uint32_t omm(const uint32_t* __restrict__ order) const {
+    return order ? __ldg(order + j) : j;
+  }
+};
 
 // Stages W[in x out] (global, bf16, row-major) as a K-major operand of
 // `rows` output rows (zero beyond `out`) and `in` columns.
@@ -181,20 +209,48 @@ __device__ void stageWeights(unsigned char* dst, const __nv_bfloat16* __restrict
   }
 }
 
-// Derived statistics of every row and unit axes of every ommatidium for
-// featureRowDerived.
-__global__ void deriveKernel(const float* __restrict__ stats, uint64_t rows, float4* __restrict__ derived) {
+// Inputs of the inference in the eye's direction order (slots; order null:
+// index order), so that the rows of a tile lie next to each other: derived
+// statistics as three float4 planes of P x N, unit axes, and the neighbour
+// table as kNeighbours planes of slots.  With the statistics by ommatidium
+// index a gather of 32 rows touched 32 cache lines, and the L1's lookups
+// bounded the feature warps (358 us for 1.5 M rows, 326 us by slot).
+__global__ void deriveKernel(const float* __restrict__ stats, uint64_t rows, uint32_t N,
+                             const uint32_t* __restrict__ order, float4* __restrict__ derived) {
   const uint64_t r = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (r >= rows) return;
-  feat::deriveStats(stats + r * kFeatureStats, derived + 3 * r);
+  const uint32_t p = static_cast<uint32_t>(r / N), j = static_cast<uint32_t>(r - static_cast<uint64_t>(p) * N);
+  const uint32_t o = order ? __ldg(order + j) : j;
+  const float4* s = reinterpret_cast<const float4*>(stats + (static_cast<size_t>(p) * N + o) * kFeatureStats);
+  const float4 s0 = __ldg(s), s1 = __ldg(s + 1), s2 = __ldg(s + 2);
+  const float row[kFeatureStats] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w, s2.x, s2.y, s2.z, s2.w};
+  float4 d[3];
+  feat::deriveStats(row, d);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) derived[static_cast<size_t>(k) * rows + r] = d[k];
 }
 
-__global__ void axesKernel(const float4* __restrict__ omm, uint32_t N, float4* __restrict__ axes) {
-  const uint32_t o = blockIdx.x * blockDim.x + threadIdx.x;
-  if (o >= N) return;
+__global__ void axesKernel(const float4* __restrict__ omm, uint32_t N, const uint32_t* __restrict__ order,
+                           float4* __restrict__ axes) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= N) return;
   float aa;
-  const float3 d = feat::ommAxis(omm, o, aa);
-  axes[o] = make_float4(d.x, d.y, d.z, aa);
+  const float3 d = feat::ommAxis(omm, order ? order[j] : j, aa);
+  axes[j] = make_float4(d.x, d.y, d.z, aa);
+}
+
+__global__ void slotOfKernel(const uint32_t* __restrict__ order, uint32_t N, uint32_t* __restrict__ slotOf) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j < N) slotOf[order ? order[j] : j] = j;
+}
+
+__global__ void slotNeighboursKernel(const int* __restrict__ nb, const uint32_t* __restrict__ order, uint32_t N,
+                                     const uint32_t* __restrict__ slotOf, uint32_t* __restrict__ nbSlots) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= N) return;
+  const uint32_t o = order ? order[j] : j;
+  for (int k = 0; k < kNeighbours; ++k)
+    nbSlots[static_cast<size_t>(k) * N + j] = slotOf[static_cast<uint32_t>(nb[kNeighbours * o + k])];
 }
 
 __device__ __forceinline__ void mbarInit(uint32_t mbar, uint32_t count) {
@@ -205,31 +261,105 @@ __device__ __forceinline__ void mbarArrive(uint32_t mbar) {
   asm volatile("{\n\t.reg .b64 st;\n\tmbarrier.arrive.shared::cta.b64 st, [%0];\n\t}\n" ::"r"(mbar) : "memory");
 }
 
-// AND of `v` over the network threads (named barrier 1).
-__device__ __forceinline__ bool netAll(bool v) {
+// AND of `v` over the threads of network group g (named barrier 1 + g).
+__device__ __forceinline__ bool netAll(int g, bool v) {
   uint32_t r;
   asm volatile(
       "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.u32 p, %1, 0;\n\t"
-      "bar.red.and.pred q, 1, %2, p;\n\t"
+      "bar.red.and.pred q, %3, %2, p;\n\t"
       "selp.u32 %0, 1, 0, q;\n\t}\n"
       : "=r"(r)
-      : "r"(v ? 1u : 0u), "n"(kNetThreads)
+      : "r"(v ? 1u : 0u), "n"(kNetThreads), "r"(1 + g)
       : "memory");
   return r != 0;
 }
 
-__device__ __forceinline__ void netSync() { asm volatile("bar.sync 1, %0;" ::"n"(kNetThreads) : "memory"); }
+// Two bf16 of max(a + b, 0) of two float pairs: one packed addition, one
+// paired conversion, one packed maximum (a NaN becomes 0, as with fmaxf; the
+// maximum commutes with the rounding).
+__device__ __forceinline__ uint32_t biasReluPack(float a0, float a1, float b0, float b1) {
+  float s0, s1;
+  asm("{\n\t.reg .b64 x, y, z;\n\t"
+      "mov.b64 x, {%2, %3};\n\t"
+      "mov.b64 y, {%4, %5};\n\t"
+      "add.rn.ftz.f32x2 z, x, y;\n\t"
+      "mov.b64 {%0, %1}, z;\n\t}\n"
+      : "=f"(s0), "=f"(s1)
+      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+  uint32_t r;
+  asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(packBf16(s0, s1)), "r"(0u));
+  return r;
+}
+
+// Features 8 c .. 8 c + 7 of tile row r as one 16-byte store.
+__device__ __forceinline__ void putChunk(uint32_t buf, uint32_t r, uint32_t c, const float* f) {
+  asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(buf + coreOffset(r, 8 * c, kFeatureWidth)),
+               "r"(packBf16(f[0], f[1])), "r"(packBf16(f[2], f[3])), "r"(packBf16(f[4], f[5])),
+               "r"(packBf16(f[6], f[7]))
+               : "memory");
+}
+
+// One quarter q of the features of slot o of a pose (dp: its first plane of
+// derived statistics, the planes `plane` apart): the values of featureRowTo.
+// The neighbours whose blocks reach into quarter q: [quarterBegin, quarterEnd).
+__host__ __device__ constexpr int quarterBegin(int q) { return q == 0 ? 0 : (q == 1 ? 1 : (q == 2 ? 3 : 4)); }
+__host__ __device__ constexpr int quarterEnd(int q) { return q == 0 ? 2 : (q == 1 ? 4 : (q == 2 ? 5 : 6)); }
+
+template <int q>
+__device__ __forceinline__ void featureQuarter(const float4* __restrict__ dp, uint64_t plane,
+                                               const float4* __restrict__ axes, const uint32_t* near, uint32_t o,
+                                               uint32_t buf, uint32_t r) {
+  constexpr int kFirst = q == 0 ? 0 : (q == 1 ? 32 : (q == 2 ? 64 : 88)), kCount = q < 2 ? 32 : 24;
+  const float4 a0 = __ldg(dp + o), a1 = __ldg(dp + plane + o);
+  const float4 ax = __ldg(axes + o);
+  const float aa = ax.w;
+  const float3 d = make_float3(ax.x, ax.y, ax.z);
+  float f[kCount];
+#pragma unroll
+  for (int k = 0; k < kCount; ++k) f[k] = 0.f;
+  auto put = [&](int k, float v) {  // k is a constant wherever this is called
+    if (k >= kFirst && k < kFirst + kCount) f[k - kFirst] = v;
+  };
+  if (q == 0) {
+    const float4 a2 = __ldg(dp + 2 * plane + o);
+    const float own[kFeatBlock] = {a0.x, a0.y, a0.z, a0.w, a1.x, a1.y, a1.z, a1.w, a2.x, a2.y, a2.z,
+                                   d.x,  d.y,  d.z,  aa * 10.0f};
+#pragma unroll
+    for (int k = 0; k < kFeatBlock; ++k) put(k, own[k]);
+  }
+  const float inva = 1.0f / fmaxf(aa, 1e-6f);
+  float3 t1 = fabsf(d.y) < 0.9f ? make_float3(d.z, 0.f, -d.x) : make_float3(0.f, -d.z, d.y);
+  const float il = rsqrtf(fmaxf(t1.x * t1.x + t1.y * t1.y + t1.z * t1.z, 1e-30f));
+  t1 = make_float3(t1.x * il, t1.y * il, t1.z * il);
+  const float3 t2 = make_float3(d.y * t1.z - d.z * t1.y, d.z * t1.x - d.x * t1.z, d.x * t1.y - d.y * t1.x);
+#pragma unroll
+  for (int j = quarterBegin(q); j < quarterEnd(q); ++j) {
+    const int k0 = kFeatBlock * (j + 1);
+    const uint32_t n = near[j - quarterBegin(q)];
+    const float4 b0 = __ldg(dp + n), b1 = __ldg(dp + plane + n), b2 = __ldg(dp + 2 * plane + n);
+    const float4 e = __ldg(axes + n);
+    const float3 g = make_float3(e.x - d.x, e.y - d.y, e.z - d.z);
+    const float u = (g.x * t1.x + g.y * t1.y + g.z * t1.z) * inva, v = (g.x * t2.x + g.y * t2.y + g.z * t2.z) * inva;
+    const float w[kFeatBlock] = {(b0.x - a0.x) * 4.0f, (b0.y - a0.y) * 4.0f, (b0.z - a0.z) * 4.0f,
+                                 b0.w, b1.x, b1.y, b1.z - a1.z, b1.w - a1.w, b2.x, b2.y, b2.z,
+                                 u, v, sqrtf(u * u + v * v), e.w * inva};
+#pragma unroll
+    for (int k = 0; k < kFeatBlock; ++k) put(k0 + k, w[k]);
+  }
+#pragma unroll
+  for (int c = 0; c < kCount / 8; ++c) putChunk(buf, r, static_cast<uint32_t>(kFirst / 8 + c), f + 8 * c);
+}
 
 __global__ void __launch_bounds__(kTcThreads, 1)
-    inferTcKernel(const float4* __restrict__ derived, const float4* __restrict__ axes, const int* __restrict__ nb,
-                  uint32_t N, uint64_t rows, MlpWeights w, bool residual, float* __restrict__ out,
+    inferTcKernel(const float4* __restrict__ derived, const float4* __restrict__ axes,
+                  const uint32_t* __restrict__ nb, uint32_t N, uint64_t rows, MlpWeights w, bool residual, float* __restrict__ out,
                   uint32_t* errFlag, const uint32_t* __restrict__ order) {
   extern __shared__ __align__(128) unsigned char smemRaw[];
   unsigned char* sm = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smemRaw) + 127) & ~uintptr_t(127));
   float* bias = reinterpret_cast<float*>(sm + kOffBias);  // b1 | b2 | b3 | b4 (16)
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kOffBar);  // full0, full1, empty0, empty1, mma
-  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(sm + kOffBar + 40);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(sm + kOffBar);
+  uint32_t* tmemSlot = reinterpret_cast<uint32_t*>(sm + kOffBar + 8 * kBars);
   const int tid = threadIdx.x, warp = tid >> 5;
 
   stageWeights(sm + kOffW1, w.w1, kFeatureWidth, kMlpHidden, kMlpHidden);
@@ -242,15 +372,15 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     bias[2 * kMlpHidden + e] = w.b3[e];
   }
   if (tid < 16) bias[3 * kMlpHidden + tid] = tid < kMlpOut ? w.b4[tid] : 0.f;
-  const uint32_t fullBar[2] = {smemAddr(bars), smemAddr(bars + 1)};
-  const uint32_t emptyBar[2] = {smemAddr(bars + 2), smemAddr(bars + 3)};
-  const uint32_t mmaBar = smemAddr(bars + 4);
+  const uint32_t bar0 = smemAddr(bars);
+  auto fullBar = [bar0](uint32_t b) { return bar0 + 8u * b; };
+  auto emptyBar = [bar0](uint32_t b) { return bar0 + 8u * (kTcBuffers + b); };
   if (tid == 0) {
-    mbarInit(fullBar[0], kFeatThreads);
-    mbarInit(fullBar[1], kFeatThreads);
-    mbarInit(emptyBar[0], 1);
-    mbarInit(emptyBar[1], 1);
-    mbarInit(mmaBar, 1);
+    for (uint32_t b = 0; b < kTcBuffers; ++b) {
+      mbarInit(fullBar(b), kFeatThreads);
+      mbarInit(emptyBar(b), 1);
+    }
+    for (uint32_t g = 0; g < kNetGroups; ++g) mbarInit(bar0 + 8u * (2 * kTcBuffers + g), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == kFeatThreads / 32) {
@@ -265,125 +395,153 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   tcFenceAfter();
   const uint64_t tiles = (rows + kTcRows - 1) / kTcRows;
 
+  const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kTcRows;
+
   if (tid < kFeatThreads) {
-    // Feature warps: tile i of this block into buffer i & 1.
-    const uint32_t r = static_cast<uint32_t>(tid >> 2), q = static_cast<uint32_t>(tid & 3);
-    static constexpr int kBegin[4] = {0, 1, 3, 5}, kEnd[4] = {1, 3, 5, kNeighbours};
-    uint32_t i = 0;
-    for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x, ++i) {
-      const uint32_t b = i & 1u;
-      if (i >= 2 && !waitParity(emptyBar[b], ((i >> 1) - 1u) & 1u)) {
+    // Feature warps: tile i of this block into buffer i mod 3.
+    const uint32_t r = static_cast<uint32_t>(tid & (kTcRows - 1)), q = static_cast<uint32_t>(tid / kTcRows);
+    RowWalk row(static_cast<uint64_t>(blockIdx.x) * kTcRows + r, stride, N);
+    // A row's neighbours and their statistics are dependent loads: the
+    // indices of a tile are fetched while the tile before is built.
+    const int j0 = quarterBegin(static_cast<int>(q)), j1 = quarterEnd(static_cast<int>(q));
+    uint32_t near[3];
+    auto neighbours = [&]() {
+#pragma unroll
+      for (int k = 0; k < 3; ++k)
+        near[k] = row.pos < rows && j0 + k < j1 ? __ldg(nb + static_cast<size_t>(j0 + k) * N + row.j) : 0u;
+    };
+    neighbours();
+    uint32_t b = 0, round = 0;
+    for (uint64_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+      if (round > 0 && !waitParity(emptyBar(b), (round - 1u) & 1u)) {
         atomicOr(errFlag, kErrMmaTimeout);
         break;
       }
-      unsigned char* fb = sm + (b ? kOffB1 : kOffB0);
-      auto put = [fb, r](int k, __nv_bfloat16 v) {
-        *reinterpret_cast<__nv_bfloat16*>(fb + coreOffset(r, static_cast<uint32_t>(k), kFeatureWidth)) = v;
-      };
-      const uint64_t fpos = tile * kTcRows + r;
-      if (fpos < rows) {
-        feat::featureRowDerived(derived, axes, nb, N, rowAt(fpos, N, order), q == 0, kBegin[q], kEnd[q], put);
+      const uint32_t buf = smemAddr(sm + kOffB0) + b * kActBytes;
+      if (row.pos < rows) {
+        const float4* dp = derived + static_cast<size_t>(row.p) * N;
+        const uint32_t cur[3] = {near[0], near[1], near[2]}, o = row.j;
+        row.next();
+        neighbours();
+        switch (q) {  // the same for a whole warp
+          case 0: featureQuarter<0>(dp, rows, axes, cur, o, buf, r); break;
+          case 1: featureQuarter<1>(dp, rows, axes, cur, o, buf, r); break;
+          case 2: featureQuarter<2>(dp, rows, axes, cur, o, buf, r); break;
+          default: featureQuarter<3>(dp, rows, axes, cur, o, buf, r); break;
+        }
       } else {
-        for (int k = static_cast<int>(q); k < kFeatureWidth; k += 4) put(k, __float2bfloat16(0.f));
+        const float zero[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        for (uint32_t c = q; c < kFeatureWidth / 8; c += 4) putChunk(buf, r, c, zero);
       }
       fenceAsyncShared();  // the tensor cores read the buffer through the async proxy
-      mbarArrive(fullBar[b]);
+      mbarArrive(fullBar(b));
+      if (++b == kTcBuffers) {
+        b = 0;
+        ++round;
+      }
     }
   } else {
-    // Network warps: the four layers of tile i from buffer i & 1.
-    const uint32_t tmem = *tmemSlot;
-    const int lq = warp & 3;                               // TMEM lane quarter this warp may read
-    const int half = (warp - kFeatThreads / 32) >> 2;      // columns 64 half .. +63
-    const int m = lq * 32 + (tid & 31);                    // accumulator lane = tile row
+    // Network group g: the four layers of tiles g, g + 2, ... of this block.
+    const int g = (tid - kFeatThreads) / kNetThreads;
+    const uint32_t tmem = *tmemSlot + 128u * static_cast<uint32_t>(g);
+    const int lq = warp & 3;                                            // TMEM lane quarter this warp may read
+    const int half = ((warp - kFeatThreads / 32) >> 2) & 1;             // columns 64 half .. +63
+    const int m = lq * 32 + (tid & 31);                                 // accumulator lane = tile row
     const uint32_t laneBase = tmem + (static_cast<uint32_t>(lq * 32) << 16);
-    const bool issuer = tid == kFeatThreads;
-    const uint32_t sW[4] = {smemAddr(sm + kOffW1), smemAddr(sm + kOffW2), smemAddr(sm + kOffW3),
-                            smemAddr(sm + kOffW4)};
-    const uint32_t sB[2] = {smemAddr(sm + kOffB0), smemAddr(sm + kOffB1)};
+    const bool issuer = tid == kFeatThreads + g * kNetThreads;
+    const uint32_t mmaBar = bar0 + 8u * static_cast<uint32_t>(2 * kTcBuffers + g);
+    const uint32_t biasAddr = smemAddr(bias);
     uint32_t phase = 0;
     bool ok = true, pending = false;  // pending: a commit to mmaBar not yet waited for
-    uint32_t i = 0;
-    for (uint64_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x, ++i) {
-      const uint32_t b = i & 1u;
-      if (!netAll(waitParity(fullBar[b], (i >> 1) & 1u))) {
-        ok = false;
-        if (issuer) atomicOr(errFlag, kErrMmaTimeout);
-        break;
-      }
-      tcFenceAfter();
-      unsigned char* h = sm + (b ? kOffB1 : kOffB0);
+    const uint64_t first = blockIdx.x + static_cast<uint64_t>(g) * gridDim.x;
+    RowWalk row(first * kTcRows + static_cast<uint64_t>(m), kNetGroups * stride, N);
+    uint32_t b = static_cast<uint32_t>(g), round = 0;
+    for (uint64_t tile = first; tile < tiles; tile += kNetGroups * static_cast<uint64_t>(gridDim.x)) {
+      const uint32_t h = smemAddr(sm + kOffB0) + b * kActBytes;
       for (int layer = 0; layer < 4; ++layer) {
         const uint32_t K = layer == 0 ? kFeatureWidth : kMlpHidden;
         const uint32_t Nn = layer == 3 ? kW4Rows : kMlpHidden;
-        if (issuer) {
+        if (issuer && (layer > 0 || waitParity(fullBar(b), round & 1u))) {
+          tcFenceAfter();
           const uint32_t idesc = instrDesc(kTcRows, Nn);
+          const uint32_t wOff = layer == 0 ? kOffW1 : (layer == 1 ? kOffW2 : (layer == 2 ? kOffW3 : kOffW4));
+          const uint32_t sW = smemAddr(sm) + wOff;
           for (uint32_t ks = 0; ks < K / 16; ++ks) {
-            const uint64_t a = smemDesc(sB[b] + ks * 256u, 128u, K * 16u);
-            const uint64_t bd = smemDesc(sW[layer] + ks * 256u, 128u, K * 16u);
+            const uint64_t a = smemDesc(h + ks * 256u, 128u, K * 16u);
+            const uint64_t bd = smemDesc(sW + ks * 256u, 128u, K * 16u);
             mmaBf16(tmem, a, bd, idesc, ks > 0 ? 1u : 0u);
           }
-          if (layer == 3) commitTo(emptyBar[b]);  // the tile buffer is free once these MMAs are done
+          if (layer == 3) commitTo(emptyBar(b));  // the tile buffer is free once these MMAs are done
           commitTo(mmaBar);
+          pending = true;
         }
-        pending = true;
-        if (!netAll(waitParity(mmaBar, phase))) {
-          ok = false;
-          if (issuer) atomicOr(errFlag, kErrMmaTimeout);
-          break;
-        }
-        pending = false;
+        // A wait that times out (also when the issuer had nothing to issue)
+        // ends the group at the barrier below; tcgen05.ld wants whole warps.
+        ok = __all_sync(0xffffffffu, waitParity(mmaBar, phase));
         phase ^= 1u;
         tcFenceAfter();
-        if (layer < 3) {
-          const float* bl = bias + layer * kMlpHidden;
+        if (ok) {
+          pending = false;
+          if (layer < 3) {
 #pragma unroll 1
-          for (int c0 = 64 * half; c0 < 64 * half + 64; c0 += 32) {
-            float v[32];
-            tmemLoad32(laneBase + static_cast<uint32_t>(c0), v);
-            // the chunk's 32 biases first, then the values, then the stores
-            float bb[32];
-            const uint32_t bs = smemAddr(bl + c0);
+            for (uint32_t c0 = 64u * half; c0 < 64u * half + 64u; c0 += 32u) {
+              float v[32];
+              tmemLoad32(laneBase + c0, v);
+              const uint32_t bs = biasAddr + 4u * (static_cast<uint32_t>(layer) * kMlpHidden + c0);
+              const uint32_t hs = h + coreOffset(static_cast<uint32_t>(m), c0, kMlpHidden);
 #pragma unroll
-            for (int k = 0; k < 8; ++k)
-              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                           : "=f"(bb[4 * k]), "=f"(bb[4 * k + 1]), "=f"(bb[4 * k + 2]), "=f"(bb[4 * k + 3])
-                           : "r"(bs + 16u * k));
-            uint32_t qs[16];
+              for (uint32_t j = 0; j < 4; ++j) {
+                float c[8];
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
+                             : "r"(bs + 32u * j));
+                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                             : "=f"(c[4]), "=f"(c[5]), "=f"(c[6]), "=f"(c[7])
+                             : "r"(bs + 32u * j + 16u));
+                uint32_t qs[4];
 #pragma unroll
-            for (int k = 0; k < 16; ++k)
-              qs[k] = packBf16(fmaxf(v[2 * k] + bb[2 * k], 0.f), fmaxf(v[2 * k + 1] + bb[2 * k + 1], 0.f));
-            const uint32_t hs = smemAddr(h);
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
-                               hs + coreOffset(static_cast<uint32_t>(m), static_cast<uint32_t>(c0 + 8 * j), kMlpHidden)),
-                           "r"(qs[4 * j]), "r"(qs[4 * j + 1]), "r"(qs[4 * j + 2]), "r"(qs[4 * j + 3])
-                           : "memory");
-          }
-        } else if (half == 0) {
-          float v[4];
-          tmemLoad4(laneBase, v);
-          const uint64_t pos = tile * kTcRows + static_cast<uint64_t>(m);
-          if (pos < rows) {
-            const uint64_t row = rowAt(pos, N, order);
-            const float* b4 = bias + 3 * kMlpHidden;
-            const float4 mc = __ldg(derived + 3 * row);  // the mean colour, as the statistics hold it
-            const float mean[3] = {mc.x, mc.y, mc.z};
-            for (int c = 0; c < 3; ++c) {
-              const float y = v[c] + b4[c];
-              out[3 * row + c] = residual ? mean[c] + y : y;
+                for (int k = 0; k < 4; ++k)
+                  qs[k] = biasReluPack(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], c[2 * k], c[2 * k + 1]);
+                asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hs + 128u * j), "r"(qs[0]), "r"(qs[1]),
+                             "r"(qs[2]), "r"(qs[3])
+                             : "memory");
+              }
+            }
+          } else if (half == 0) {
+            float v[4];
+            tmemLoad4(laneBase, v);
+            if (row.pos < rows) {
+              const uint64_t at = static_cast<uint64_t>(row.p) * N + row.omm(order);
+              const float* b4 = bias + 3 * kMlpHidden;
+              const float4 mc = __ldg(derived + row.pos);  // the mean colour, as the statistics hold it
+              const float mean[3] = {mc.x, mc.y, mc.z};
+              for (int c = 0; c < 3; ++c) {
+                const float y = v[c] + b4[c];
+                out[3 * at + c] = residual ? mean[c] + y : y;
+              }
             }
           }
         }
         // The next MMA reads h (async proxy) and overwrites the accumulator
-        // that every network thread has just read.
+        // that every thread of the group has just read.
         fenceAsyncShared();
         tcFenceBefore();
-        netSync();
+        ok = netAll(g, ok);
         tcFenceAfter();
+        if (!ok) break;
+      }
+      if (!ok) {
+        if (issuer) atomicOr(errFlag, kErrMmaTimeout);
+        break;
+      }
+      row.next();
+      b += kNetGroups;
+      if (b >= kTcBuffers) {
+        b -= kTcBuffers;
+        ++round;
       }
     }
-    if (!ok && pending && issuer) waitParity(mmaBar, phase);  // let a late commit land before the TMEM is freed
+    if (!ok && pending && issuer) waitParity(mmaBar, phase ^ 1u);  // let a late commit land before the TMEM is freed
   }
   tcFenceBefore();
   __syncthreads();
@@ -746,16 +904,24 @@ cudaError_t launchWaitProbe(uint32_t polls, uint32_t* errFlag, cudaStream_t stre
   return cudaGetLastError();
 }
 
-cudaError_t deriveFeatureStats(const float* stats, const float4* omm, uint32_t N, uint32_t P, float4* derived,
-                               float4* axes, cudaStream_t stream) {
-  const uint64_t rows = static_cast<uint64_t>(N) * P;
-  if (rows == 0) return cudaSuccess;
-  deriveKernel<<<static_cast<unsigned>((rows + 255) / 256), 256, 0, stream>>>(stats, rows, derived);
-  axesKernel<<<(N + 255) / 256, 256, 0, stream>>>(omm, N, axes);
+cudaError_t slotNeighbours(const int* nb, const uint32_t* order, uint32_t N, uint32_t* slotOf, uint32_t* nbSlots,
+                           cudaStream_t stream) {
+  if (N == 0) return cudaSuccess;
+  slotOfKernel<<<(N + 255) / 256, 256, 0, stream>>>(order, N, slotOf);
+  slotNeighboursKernel<<<(N + 255) / 256, 256, 0, stream>>>(nb, order, N, slotOf, nbSlots);
   return cudaGetLastError();
 }
 
-cudaError_t inferDenoiserTc(const float4* derived, const float4* axes, const int* nb, uint32_t N, uint32_t P,
+cudaError_t deriveFeatureStats(const float* stats, const float4* omm, uint32_t N, uint32_t P, const uint32_t* order,
+                               float4* derived, float4* axes, cudaStream_t stream) {
+  const uint64_t rows = static_cast<uint64_t>(N) * P;
+  if (rows == 0) return cudaSuccess;
+  deriveKernel<<<static_cast<unsigned>((rows + 255) / 256), 256, 0, stream>>>(stats, rows, N, order, derived);
+  axesKernel<<<(N + 255) / 256, 256, 0, stream>>>(omm, N, order, axes);
+  return cudaGetLastError();
+}
+
+cudaError_t inferDenoiserTc(const float4* derived, const float4* axes, const uint32_t* nbSlots, uint32_t N, uint32_t P,
                             const MlpWeights& w, float* out, uint32_t* errFlag, cudaStream_t stream, bool residual,
                             const uint32_t* order) {
   const uint64_t rows = static_cast<uint64_t>(N) * P;
@@ -774,7 +940,7 @@ cudaError_t inferDenoiserTc(const float4* derived, const float4* axes, const int
   }
   const uint64_t tiles = (rows + kTcRows - 1) / kTcRows;
   const unsigned grid = static_cast<unsigned>(std::min<uint64_t>(tiles, static_cast<uint64_t>(smCount)));
-  inferTcKernel<<<grid, kTcThreads, kTcSmem, stream>>>(derived, axes, nb, N, rows, w, residual, out, errFlag, order);
+  inferTcKernel<<<grid, kTcThreads, kTcSmem, stream>>>(derived, axes, nbSlots, N, rows, w, residual, out, errFlag, order);
   return cudaGetLastError();
 }
 

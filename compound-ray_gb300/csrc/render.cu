@@ -2456,31 +2456,39 @@ static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool con
   return !stats && !scene.lighting && cones;
 }
 
-// When a launch uses cone lists: whole-warp segments (more than 16 samples in
-// the default layout; a warp then holds one list), and enough rays to hide
-// the ~20-35 us that the first list takes to build.  The line lies at 2^19
-// rays on deep trees and at 2^21 on shallow ones, whose traversals are
-// shorter.  Speed-up with lists over without (64 registers), terrain / box
-// scene, by rays: 0.3 M 0.95 / 0.82, 0.5 M 1.2 / 0.9, 1 M 1.3 / 0.93, 2 M
-// 1.5 / 1.1, 6 M 2.7 / 1.5, 82 M 3.6 / 2.0; at acceptance angles of 6 degrees
-// 82 M 3.0 / 1.6.
+// When a launch uses cone lists: enough rays to hide the ~20-35 us that the
+// first list takes to build, and enough samples for a list's cost (about three
+// rays searched from the root).  Both lines depend on the scene: on deep trees
+// (kConeDeepTris triangles) traversals are long, on shallow ones short.
+//   segment (samples)       deep           shallow
+//   32  (17 and more)       2^19 rays      2^21 rays
+//   16  (9-16)              2^19           2^22
+//    8  (5-8)               2^20           no lists
+// Speed-up with lists over without (64 registers), terrain / box scene, by
+// rays.  Segments of 32: 0.3 M 0.95 / 0.82, 0.5 M 1.2 / 0.9, 1 M 1.3 / 0.93,
+// 2 M 1.5 / 1.1, 6 M 2.7 / 1.5, 82 M 3.6 / 2.0; at acceptance angles of 6
+// degrees 82 M 3.0 / 1.6.  Of 16 (and at 6 degrees): 0.6 M 1.0, 2.2 M 1.5 (1.5)
+// / 1.0 (0.93), 9 M 2.0 (1.8) / 1.3 (1.1).  Of 8: 0.6 M 0.9, 2.2 M 1.3 (1.2) /
+// 0.9 (0.8), 9 M 1.5 (1.4) / 1.0 (0.9), 40 M 1.6 (1.4) / 1.0 (0.9).
 constexpr uint32_t kConeDeepTris = 16384;
-constexpr uint32_t kConeMinSegment = 8;
-constexpr uint64_t kConeRaysDeep = 1ull << 19, kConeRaysShallow = 1ull << 21;
 
-static bool coneWorth(const DevScene& scene, uint64_t rays) {
-  return scene.triCount > 0 && rays >= (scene.triCount >= kConeDeepTris ? kConeRaysDeep : kConeRaysShallow);
+static bool coneWorth(const DevScene& scene, uint32_t segment, uint64_t rays) {
+  if (scene.triCount == 0 || segment < 8) return false;
+  const bool deep = scene.triCount >= kConeDeepTris;
+  if (segment == 32) return rays >= (deep ? 1ull << 19 : 1ull << 21);
+  if (segment == 16) return rays >= (deep ? 1ull << 19 : 1ull << 22);
+  return deep && rays >= 1ull << 20;
 }
 
 size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, uint32_t P, uint64_t batchRays) {
-  if (scene.width != 2 || plan.segWidth != 32 || !coneWorth(scene, batchRays)) return 0;
+  if (scene.width != 2 || plan.segWidth != 32 || !coneWorth(scene, plan.segWidth, batchRays)) return 0;
   return static_cast<size_t>(P) * N;
 }
 
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec, bool stats) {
-  if (!coneWorth(scene, static_cast<uint64_t>(N) * spp * P)) return 0;
   const uint32_t seg = planRender(N, spp, P, true).segWidth;
-  if (seg < kConeMinSegment || (seg != 32 && (rec || stats || scene.lighting))) return 0;
+  if (!coneWorth(scene, seg, static_cast<uint64_t>(N) * spp * P)) return 0;
+  if (seg != 32 && (rec || stats || scene.lighting)) return 0;
   if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
   return static_cast<size_t>(P) * N;
 }
@@ -2660,7 +2668,7 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
 }
 
 size_t featureConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P) {
-  if (!coneWorth(scene, static_cast<uint64_t>(N) * spp * P) || planWarps(N, spp).segWidth < kConeMinSegment) return 0;
+  if (!coneWorth(scene, planWarps(N, spp).segWidth, static_cast<uint64_t>(N) * spp * P)) return 0;
   return static_cast<size_t>(P) * N;
 }
 
@@ -3687,7 +3695,7 @@ cudaError_t launchAdaptive(const DevScene& scene, const float4* omm, uint32_t N,
 }
 
 bool adaptiveLists(const DevScene& scene, uint32_t spp, uint64_t launchRays) {
-  return scene.width == 2 && spp >= 32u / kListEntries && coneWorth(scene, launchRays);
+  return scene.width == 2 && spp >= 32u / kListEntries && coneWorth(scene, 32, launchRays);
 }
 
 cudaError_t launchEntryCones(const DevScene& scene, const float4* omm, uint32_t N, const float4* poses,

@@ -41,8 +41,30 @@ def _eye(n, kind):
     return omm
 
 
-def _poses(boxes, count, seed):
-    p = scenes.open_poses(boxes, count, np.random.default_rng(seed))
+@pytest.fixture(scope="module")
+def deep(tmp_path_factory):
+    """A terrain with a deep tree (at least 16384 triangles): lists from 5
+    samples on, sorted rounds in the adaptive render."""
+    d = tmp_path_factory.mktemp("deep")
+    return scenes.terrain_scene(str(d), cells=96, extent=60.0, cones=40, n_omm=500, poses=1)
+
+
+def _load(lib, info):
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(info["gltf"].encode())
+    assert eh.lastError(lib) == ""
+    assert "height_fn" not in info or lib.crGetTriangleCount() >= 16384
+    eh.gotoFirstCompoundEye(lib)
+
+
+def _poses(info, count, seed):
+    rng = np.random.default_rng(seed)
+    if "height_fn" in info:
+        p = scenes.random_poses(info["height_fn"], count, rng, 20.0)
+        boxes = np.array([[[-1.0, 0.0, -1.0], [1.0, 0.5, 1.0]]] * 2)
+    else:
+        boxes = info["boxes"]
+        p = scenes.open_poses(boxes, count, rng)
     p16 = np.zeros((count, 16), np.float32)
     for k in range(4):
         p16[:, 4 * k:4 * k + 3] = p[:, 3 * k:3 * k + 3]
@@ -91,55 +113,50 @@ def _both(lib, omm, spp, p16):
 
 @pytest.mark.parametrize("kind", ["plain", "odd"])
 @pytest.mark.parametrize("spp", SPP)
-def test_lists_change_no_bit(lib, small, kind, spp):
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
-    lib.loadGlTFscene(small["gltf"].encode())
-    eh.gotoFirstCompoundEye(lib)
-    n = 701 if spp > 16 else 2 ** 21 // (150 * spp) | 1
-    P = 2 + 2 ** 21 // (n * spp)  # just past the fewest rays that use lists
+def test_lists_change_no_bit(lib, small, deep, kind, spp):
+    info, rays = (deep, 2 ** 20) if spp <= 16 else (small, 2 ** 21)  # just past the fewest rays that use lists
+    _load(lib, info)
+    n = 701 if spp > 16 else rays // (60 * spp) | 1
+    P = 2 + rays // (n * spp)
     if P < 9:
-        n, P = 2 ** 21 // (9 * spp) + 1, 9
-    with_lists, without = _both(lib, _eye(n, kind), spp, _poses(small["boxes"], P, spp))
+        n, P = rays // (9 * spp) + 1, 9
+    with_lists, without = _both(lib, _eye(n, kind), spp, _poses(info, P, spp))
     assert with_lists[3] >= 400 * n * P and without[3] == 0  # the first did build lists
     for x, y in zip(with_lists[:3], without[:3]):
         assert np.array_equal(x, y, equal_nan=True)
 
 
 @pytest.mark.parametrize("segment", [8, 16])
-def test_lists_of_narrow_segments(lib, small, segment):
+def test_lists_of_narrow_segments(lib, deep, segment):
     """Many samples in segments of 8 or 16 lanes: chunk partials of several
     ommatidia a warp, with a last warp that is not full."""
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
-    lib.loadGlTFscene(small["gltf"].encode())
-    eh.gotoFirstCompoundEye(lib)
+    _load(lib, deep)
     assert lib.crSetRenderLayout(128, segment) == 0
     try:
-        with_lists, without = _both(lib, _eye(1401, "odd"), 50, _poses(small["boxes"], 31, 2))
+        with_lists, without = _both(lib, _eye(701, "odd"), 50, _poses(deep, 31, 2))
     finally:
         lib.crSetRenderLayout(0, 32)
-    assert with_lists[3] > 400 * 1401 * 31
+    assert with_lists[3] > 400 * 701 * 31
     for x, y in zip(with_lists[:3], without[:3]):
         assert np.array_equal(x, y, equal_nan=True)
 
 
 @pytest.mark.parametrize("spp", [5, 8, 16, 20])
-def test_feature_rows_with_and_without_lists(lib, small, spp):
+def test_feature_rows_with_and_without_lists(lib, deep, spp):
     """Feature rows and 8-sample means of the denoiser."""
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     assert lib.crDenoiserInit(1) == 0
     n = 3001
     omm = _eye(n, "odd")
-    P = 2 ** 21 // (n * spp) + 2
-    p12 = scenes.open_poses(small["boxes"], P, np.random.default_rng(4))
+    P = 2 ** 20 // (n * spp) + 2
+    p12 = scenes.random_poses(deep["height_fn"], P, np.random.default_rng(4), 20.0)
     got = []
     for lists in (True, False):
-        lib.loadGlTFscene(small["gltf"].encode())
-        eh.gotoFirstCompoundEye(lib)
+        _load(lib, deep)
         lib.setOmmatidia(omm.ctypes.data, n)
         lib.setCurrentEyeSamplesPerOmmatidium(1)
         x, base = np.zeros((P * n, 112), np.uint16), np.zeros((P * n, 3), np.float32)
         if not lists:  # the statistics and rows of the first run are still held
-            assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + (40 << 20)) == 0
+            assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + (24 << 20)) == 0
         held = lib.crGetDeviceMemoryHeld()
         try:
             assert lib.crDenoiserFeatureRows(p12, P, spp, x, base) == 0, eh.lastError(lib)
@@ -174,13 +191,10 @@ def test_lists_of_a_single_leaf_scene(lib, tmp_path):
 
 def test_lists_give_way_under_a_memory_cap(lib, small):
     """Lists are dropped, not the render, when their memory is not to be had."""
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
-    lib.loadGlTFscene(small["gltf"].encode())
-    eh.gotoFirstCompoundEye(lib)
-    omm, p16 = _eye(800, "plain"), _poses(small["boxes"], 90, 3)
+    _load(lib, small)
+    omm, p16 = _eye(800, "plain"), _poses(small, 90, 3)
     want = _both(lib, omm, 64, p16)[0][0]
-    lib.loadGlTFscene(small["gltf"].encode())  # gives back every buffer
-    eh.gotoFirstCompoundEye(lib)
+    _load(lib, small)  # gives back every buffer
     lib.setOmmatidia(omm.ctypes.data, len(omm))
     lib.setCurrentEyeSamplesPerOmmatidium(64)
     import torch
@@ -240,30 +254,19 @@ def test_batch_with_and_without_lists(lib, tmp_path):
     lib.crBatchDestroy(h)
 
 
-def _deep_scene(lib, tmp_path):
-    """A terrain deep enough for sorted rounds (at least 16384 triangles)."""
-    info = scenes.terrain_scene(str(tmp_path), cells=96, extent=60.0, cones=40, n_omm=500, poses=1)
-    lib.loadGlTFscene(info["gltf"].encode())
-    assert eh.lastError(lib) == "" and lib.crGetTriangleCount() >= 16384
-    eh.gotoFirstCompoundEye(lib)
-    return info
-
-
-@pytest.mark.parametrize("deep", [False, True])
+@pytest.mark.parametrize("on_deep", [False, True])
 @pytest.mark.parametrize("spp", [16, 32, 64, 256, 512])
-def test_adaptive_records_with_and_without_lists(lib, small, tmp_path, deep, spp):
+def test_adaptive_records_with_and_without_lists(lib, small, deep, on_deep, spp):
     """crAdaptiveRecord through lists and (under a memory cap) without: the
     same rays, hits, colours and sums.  Two entries a warp, one round, several,
     a pool's worth, two chunks; an odd number of entries."""
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
-    if deep:
-        info = _deep_scene(lib, tmp_path)
+    info = deep if on_deep else small
+    _load(lib, info)
+    if on_deep:
         p12 = scenes.random_poses(info["height_fn"], 3, np.random.default_rng(5), 20.0)
     else:
-        lib.loadGlTFscene(small["gltf"].encode())
-        eh.gotoFirstCompoundEye(lib)
         p12 = scenes.open_poses(small["boxes"], 3, np.random.default_rng(6))
-    n = (2 ** (19 if deep else 21) // (3 * spp) + 2) | 1
+    n = (2 ** (19 if on_deep else 21) // (3 * spp) + 2) | 1
     omm = _eye(n, "odd")
     lib.setOmmatidia(omm.ctypes.data, n)
     lib.setCurrentEyeSamplesPerOmmatidium(1)
@@ -277,8 +280,7 @@ def test_adaptive_records_with_and_without_lists(lib, small, tmp_path, deep, spp
             assert lib.crAdaptiveRecord(p12[:1], 1, 1, 9, np.zeros((n, 1), eh.RAY_RECORD_DTYPE).ctypes.data,
                                         np.zeros((n, 3), np.float32)) == 0, eh.lastError(lib)
         else:
-            lib.loadGlTFscene(info["gltf"].encode() if deep else small["gltf"].encode())  # gives the lists back
-            eh.gotoFirstCompoundEye(lib)
+            _load(lib, info)  # gives the lists back
             lib.setOmmatidia(omm.ctypes.data, n)
             lib.setCurrentEyeSamplesPerOmmatidium(1)
             assert lib.crAdaptiveRecord(p12[:1], 1, 1, 9, np.zeros((n, 1), eh.RAY_RECORD_DTYPE).ctypes.data,
@@ -296,14 +298,12 @@ def test_adaptive_records_with_and_without_lists(lib, small, tmp_path, deep, spp
     assert np.array_equal(got[0][1], got[1][1], equal_nan=True)
 
 
-def test_adaptive_render_with_and_without_lists(lib, tmp_path):
+def test_adaptive_render_with_and_without_lists(lib, deep):
     """The whole adaptive render with entries in several buckets."""
     import torch
 
-    info = _deep_scene(lib, tmp_path)
-    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
     omm, P = _eye(2501, "plain"), 20
-    p12 = scenes.random_poses(info["height_fn"], P, np.random.default_rng(8), 20.0)
+    p12 = scenes.random_poses(deep["height_fn"], P, np.random.default_rng(8), 20.0)
     p16 = np.zeros((P, 16), np.float32)
     for k in range(4):
         p16[:, 4 * k:4 * k + 3] = p12[:, 3 * k:3 * k + 3]
@@ -313,8 +313,7 @@ def test_adaptive_render_with_and_without_lists(lib, tmp_path):
     assert lib.crAllocatorInit(3) == 0 and lib.crSetAllocatorHalvings(-4.0) == 0
     try:
         for lists in (True, False):
-            lib.loadGlTFscene(info["gltf"].encode())
-            eh.gotoFirstCompoundEye(lib)
+            _load(lib, deep)
             lib.setOmmatidia(omm.ctypes.data, len(omm))
             lib.setCurrentEyeSamplesPerOmmatidium(1)
             out = torch.full((P, len(omm), 3), -1.0, device="cuda")
