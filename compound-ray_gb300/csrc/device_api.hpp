@@ -501,10 +501,12 @@ cudaError_t launchProject(const float* sums, uint32_t N, uchar4* frame, int w, i
                           cudaStream_t stream);
 // Candidates of the spherical projections binned by unit vector: a G^3 grid
 // over [-1, 1]^3, cell (cz * G + cy) * G + cx holding items[start[c] ..
-// start[c + 1]) (ommatidium indices >= 1, ascending).  G == 0: no candidate.
+// start[c + 1]) (ommatidium indices >= 1, ascending); vecs[k]: the vector of
+// items[k] and its length.  G == 0: no candidate.
 struct SphereGridView {
   const uint32_t* start = nullptr;  // G^3 + 1 offsets
   const uint32_t* items = nullptr;
+  const float4* vecs = nullptr;
   int G = 0;
 };
 // The four candidate sets: 0 positions, 1 directions, 2 directions of the
@@ -514,11 +516,14 @@ struct SphereGridSet {
 };
 
 // Spherical projections (kind: 0 positionwise, 1 orientationwise, 2 split
-// orientationwise, 3 orientationwise ids, 4 positionwise ids); lenScratch
-// holds 2 * N floats.  grids: the candidate grids (searched around each
-// pixel's point), or null for the exhaustive search in index order; both
-// give the same image.
-cudaError_t launchSpherical(const float4* omm, float* lenScratch, uint32_t N, const float* sums, uchar4* frame, int w,
+// orientationwise, 3 orientationwise ids, 4 positionwise ids); len: the
+// lengths of the ommatidia's N positions and N directions (launchLengths).
+// grids: the candidate grids (searched around each pixel's point), or null
+// for the exhaustive search in index order; both give the same image.
+cudaError_t launchLengths(const float4* omm, uint32_t N, float* len, cudaStream_t stream);
+cudaError_t launchGridVecs(const float4* omm, const float* len, uint32_t N, bool byPos, const uint32_t* items,
+                           uint32_t n, float4* vecs, cudaStream_t stream);
+cudaError_t launchSpherical(const float4* omm, const float* len, uint32_t N, const float* sums, uchar4* frame, int w,
                             int h, int kind, const SphereGridSet* grids, cudaStream_t stream);
 // raw_ommatidial_samples from a recorded frame (N x spp records).
 cudaError_t launchRawSamples(const RayRecord* rec, uint32_t N, uint32_t spp, uchar4* frame, int w, int h,

@@ -139,6 +139,7 @@ struct HostBuf {
 // One candidate grid of the spherical projections (SphereGridView).
 struct SphereGrid {
   DevBuf<uint32_t> start, items;
+  DevBuf<float4> vecs;
   int G = 0;
 };
 
@@ -149,7 +150,8 @@ struct EyeDev {
   DevBuf<float> sums;  // N x 3 of the last frame
   SphereGrid grids[4];  // spherical-projection candidates, built on first use
   bool gridsBuilt = false;
-  DevBuf<float> lens;  // 2 N: workspace of the spherical projections
+  DevBuf<float> lens;  // 2 N: lengths of positions and directions, for the spherical projections
+  bool lensBuilt = false;
   uint32_t N = 0, spp = 0;
   float maxRel = 0.f;  // largest |position - focal offset * unit axis| over the ommatidia
   bool configured = false;
@@ -158,9 +160,11 @@ struct EyeDev {
     for (SphereGrid& g : grids) {
       g.start.release();
       g.items.release();
+      g.vecs.release();
       g.G = 0;
     }
     gridsBuilt = false;
+    lensBuilt = false;
   }
   void release() {
     lens.release();
@@ -200,6 +204,7 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
     }
     g.start.release();
     g.items.release();
+    g.vecs.release();
     g.G = 0;
     if (idx.empty()) continue;
     const int G = std::max(1, std::min(128, static_cast<int>(std::lround(0.33 * std::sqrt(double(idx.size()))))));
@@ -217,8 +222,12 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
     for (size_t k = 0; k < idx.size(); ++k) items[fill[cellOf[k]]++] = idx[k];
     g.start.ensure(cells + 1);
     g.items.ensure(items.size());
+    g.vecs.ensure(items.size());
     check(cudaMemcpyAsync(g.start.ptr, start.data(), start.size() * 4, cudaMemcpyHostToDevice, st), "cudaMemcpy");
     check(cudaMemcpyAsync(g.items.ptr, items.data(), items.size() * 4, cudaMemcpyHostToDevice, st), "cudaMemcpy");
+    check(launchGridVecs(e.omm.ptr, e.lens.ptr, e.N, which == 0, g.items.ptr, static_cast<uint32_t>(items.size()),
+                         g.vecs.ptr, st),
+          "projection grid");
     check(cudaStreamSynchronize(st), "projection grid upload");
     g.G = G;
   }
@@ -732,16 +741,22 @@ struct Renderer {
     if (kind < 10) {
       check(launchProject(e.sums.ptr, e.N, frame.ptr, width, height, kind, stream()), "projection launch");
     } else if (kind < 20) {
+      if (!e.lensBuilt) {
+        e.lens.ensure(std::max<size_t>(1, 2 * static_cast<size_t>(e.N)));
+        check(launchLengths(e.omm.ptr, e.N, e.lens.ptr, stream()), "projection lengths");
+        check(cudaStreamSynchronize(stream()), "projection lengths");
+        e.lensBuilt = true;
+      }
       SphereGridSet set;
       if (projectionGrid) {
         if (!e.gridsBuilt) buildSphereGrids(e, omm, stream());
         for (int k = 0; k < 4; ++k) {
           set.g[k].start = e.grids[k].start.ptr;
           set.g[k].items = e.grids[k].items.ptr;
+          set.g[k].vecs = e.grids[k].vecs.ptr;
           set.g[k].G = e.grids[k].G;
         }
       }
-      e.lens.ensure(std::max<size_t>(1, 2 * static_cast<size_t>(e.N)));
       check(launchSpherical(e.omm.ptr, e.lens.ptr, e.N, e.sums.ptr, frame.ptr, width, height, kind - 10,
                             projectionGrid ? &set : nullptr, stream()),
             "projection launch");

@@ -2084,6 +2084,17 @@ __global__ void sphericalKernel(const float4* __restrict__ omm, const float* __r
 // the difference between a computed angle and the true one, so every
 // candidate left outside the box has a computed angle above the best.
 // A NaN angle never wins; a NaN angle of candidate 0 makes 0 the answer.
+//
+// The kernel waits for its loads and issues acosf; so a cell row is one range
+// of candidates, each is one 16-byte load (SphereGridView::vecs, in the order
+// of the items), and acosf is called only for a candidate whose cosine is
+// above the best one's less 4e-6.  The angle differs from another by at least
+// as much as its cosine does, and acosf is off by at most 2 ulp (0.5e-6 near
+// pi), so the others' computed angles are above the best; a NaN cosine is not
+// below and takes acosf.  The first box reaches half a cell: 1, 1/4 and 1/8
+// were 13 to 30 us slower.  20011 ommatidia on a 1023 x 511 image: 45 us; with
+// every candidate gathered by index and put through acosf, cell by cell from
+// a box of one cell, 101 us.
 __global__ void sphericalGridKernel(const float4* __restrict__ omm, const float* __restrict__ len, uint32_t N,
                                     SphereGridSet grids, const float* __restrict__ sums, uchar4* frame, int w, int h,
                                     int kind) {
@@ -2110,7 +2121,8 @@ __global__ void sphericalGridKernel(const float4* __restrict__ omm, const float*
     const float q[3] = {p.x * inv, p.y * inv, p.z * inv};
     auto cellOf = [&](float c) { return min(G - 1, max(0, static_cast<int>(floorf((c + 1.0f) / cell)))); };
     int vlo[3] = {1, 1, 1}, vhi[3] = {0, 0, 0};  // visited box (empty)
-    float r = cell;
+    float r = 0.5f * cell;
+    float floorCos = -2.0f;  // no candidate of a smaller cosine can win
     for (;;) {
       int lo[3], hi[3];
       for (int a = 0; a < 3; ++a) {
@@ -2118,20 +2130,28 @@ __global__ void sphericalGridKernel(const float4* __restrict__ omm, const float*
         hi[a] = cellOf(q[a] + r + 1e-5f);
       }
       for (int cz = lo[2]; cz <= hi[2]; ++cz)
-        for (int cy = lo[1]; cy <= hi[1]; ++cy)
-          for (int cx = lo[0]; cx <= hi[0]; ++cx) {
-            if (cx >= vlo[0] && cx <= vhi[0] && cy >= vlo[1] && cy <= vhi[1] && cz >= vlo[2] && cz <= vhi[2]) continue;
-            const uint32_t c = (static_cast<uint32_t>(cz) * G + cy) * G + cx;
-            const uint32_t e = __ldg(g->start + c + 1);
-            for (uint32_t k = __ldg(g->start + c); k < e; ++k) {
-              const uint32_t i = __ldg(g->items + k);
-              const float ang = sphericalAngle(omm, len, N, byPos, i, p, lp);
-              if (ang < best || (ang == best && i < bi)) {
-                best = ang;
-                bi = i;
-              }
+        for (int cy = lo[1]; cy <= hi[1]; ++cy) {
+          // A row of the visited box is searched again where the box grew
+          // along x (a candidate seen twice changes nothing).
+          if (lo[0] == vlo[0] && hi[0] == vhi[0] && cy >= vlo[1] && cy <= vhi[1] && cz >= vlo[2] && cz <= vhi[2])
+            continue;
+          const uint32_t row = (static_cast<uint32_t>(cz) * G + cy) * G;
+          const uint32_t e = __ldg(g->start + row + hi[0] + 1);
+          for (uint32_t k = __ldg(g->start + row + lo[0]); k < e; ++k) {
+            const float4 v = __ldg(g->vecs + k);
+            const float d = dot(mk(v.x, v.y, v.z), p), ll = v.w * lp;
+            if (d < floorCos * ll) continue;
+            const float c = d / ll;
+            const float ang = acosf(c);
+            if (ang > best || ang != ang) continue;
+            const uint32_t i = __ldg(g->items + k);
+            if (ang < best || i < bi) {
+              best = ang;
+              bi = i;
+              floorCos = c - 4e-6f;
             }
           }
+        }
       for (int a = 0; a < 3; ++a) {
         vlo[a] = lo[a];
         vhi[a] = hi[a];
@@ -2146,6 +2166,16 @@ __global__ void sphericalGridKernel(const float4* __restrict__ omm, const float*
     }
   }
   sphericalWrite(bi, kind, sums, frame, static_cast<size_t>(y) * w + x);
+}
+
+// SphereGridView::vecs of one grid; len: see sphericalAngle.
+__global__ void gridVecsKernel(const float4* __restrict__ omm, const float* __restrict__ len, uint32_t N, bool byPos,
+                               const uint32_t* __restrict__ items, uint32_t n, float4* vecs) {
+  const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
+  if (k >= n) return;
+  const uint32_t i = items[k];
+  const float4 a = omm[2 * i], b = omm[2 * i + 1];
+  vecs[k] = byPos ? make_float4(a.x, a.y, a.z, len[i]) : make_float4(a.w, b.x, b.y, len[N + i]);
 }
 
 __global__ void lengthsKernel(const float4* __restrict__ omm, uint32_t N, float* len) {
@@ -2770,16 +2800,28 @@ cudaError_t launchBatch(const DevScene& scene, const BatchTables& b, unsigned lo
   return cudaGetLastError();
 }
 
-cudaError_t launchSpherical(const float4* omm, float* lenScratch, uint32_t N, const float* sums, uchar4* frame, int w,
+cudaError_t launchLengths(const float4* omm, uint32_t N, float* len, cudaStream_t stream) {
+  if (N == 0) return cudaSuccess;
+  lengthsKernel<<<(N + 255) / 256, 256, 0, stream>>>(omm, N, len);
+  return cudaGetLastError();
+}
+
+cudaError_t launchGridVecs(const float4* omm, const float* len, uint32_t N, bool byPos, const uint32_t* items,
+                           uint32_t n, float4* vecs, cudaStream_t stream) {
+  if (n == 0) return cudaSuccess;
+  gridVecsKernel<<<(n + 255) / 256, 256, 0, stream>>>(omm, len, N, byPos, items, n, vecs);
+  return cudaGetLastError();
+}
+
+cudaError_t launchSpherical(const float4* omm, const float* len, uint32_t N, const float* sums, uchar4* frame, int w,
                             int h, int kind, const SphereGridSet* grids, cudaStream_t stream) {
   if (w <= 0 || h <= 0 || N == 0) return cudaSuccess;
   if (kind < 0 || kind > 4) return cudaErrorInvalidValue;
-  lengthsKernel<<<(N + 255) / 256, 256, 0, stream>>>(omm, N, lenScratch);
   dim3 grid((w + 127) / 128, h);
   if (grids)
-    sphericalGridKernel<<<grid, 128, 0, stream>>>(omm, lenScratch, N, *grids, sums, frame, w, h, kind);
+    sphericalGridKernel<<<grid, 128, 0, stream>>>(omm, len, N, *grids, sums, frame, w, h, kind);
   else
-    sphericalKernel<<<grid, 128, 0, stream>>>(omm, lenScratch, N, sums, frame, w, h, kind);
+    sphericalKernel<<<grid, 128, 0, stream>>>(omm, len, N, sums, frame, w, h, kind);
   return cudaGetLastError();
 }
 
