@@ -37,7 +37,7 @@ void Denoiser::release() {
                   wbf_, wbfT_, Xb_, static_cast<void*>(baseb_), static_cast<void*>(targetb_), static_cast<void*>(zs_), h_[0],
                   h_[1], h_[2], dz_[0], dz_[1], dz_[2], static_cast<void*>(y_), static_cast<void*>(dyf_), dyb_,
                   static_cast<void*>(lossSum_), static_cast<void*>(idx_), X_, static_cast<void*>(base_),
-                  static_cast<void*>(target_)})
+                  static_cast<void*>(target_), static_cast<void*>(part_), static_cast<void*>(carry_)})
     dfree(p);
   params_ = grads_ = m_ = v_ = nullptr;
   wbf_ = wbfT_ = Xb_ = nullptr;
@@ -47,6 +47,8 @@ void Denoiser::release() {
   idx_ = nullptr;
   X_ = nullptr;
   base_ = target_ = nullptr;
+  part_ = carry_ = nullptr;
+  partTiles_ = 0;
   cap_ = 0;
   rows_ = rowCap_ = 0;
   adamT_ = 0;
@@ -84,7 +86,7 @@ void Denoiser::ensureBatch(int rows) {
   if (rows <= cap_) return;
   for (void* p : {Xb_, static_cast<void*>(baseb_), static_cast<void*>(targetb_), static_cast<void*>(zs_), h_[0], h_[1],
                   h_[2], dz_[0], dz_[1], dz_[2], static_cast<void*>(y_), static_cast<void*>(dyf_), dyb_,
-                  static_cast<void*>(lossSum_), static_cast<void*>(idx_)})
+                  static_cast<void*>(idx_)})
     dfree(p);
   cap_ = rows;
   const size_t r = static_cast<size_t>(rows);
@@ -99,38 +101,69 @@ void Denoiser::ensureBatch(int rows) {
   y_ = dalloc<float>(r * kOut);
   dyf_ = dalloc<float>(r * kOut);
   dyb_ = dalloc<uint16_t>(r * kOut);
-  lossSum_ = dalloc<float>(1);
   idx_ = dalloc<uint32_t>(r);
 }
 
-void Denoiser::forward(const void* X, int rows, cudaStream_t s) {
-  // B operand of each layer: the tcgen05 GEMMs read the transposed weights
-  // (K contiguous), the mma.sync GEMMs the row-major ones.
-  const uint16_t* w = static_cast<const uint16_t*>(tc_ ? wbfT_ : wbf_);
-  auto ldw = [&](int kin, int nout) { return tc_ ? kin : nout; };
-  ck(gemm(1, rows, kHidden, kFeatureWidth, X, kFeatureWidth, false, w + offW1, ldw(kFeatureWidth, kHidden), tc_,
-          zs_, h_[0], kHidden, params_ + offB1, nullptr, s),
-     "layer 1");
-  ck(gemm(1, rows, kHidden, kHidden, h_[0], kHidden, false, w + offW2, ldw(kHidden, kHidden), tc_, zs_, h_[1],
-          kHidden, params_ + offB2, nullptr, s),
-     "layer 2");
-  ck(gemm(1, rows, kHidden, kHidden, h_[1], kHidden, false, w + offW3, ldw(kHidden, kHidden), tc_, zs_, h_[2],
-          kHidden, params_ + offB3, nullptr, s),
-     "layer 3");
-  ck(gemm(3, rows, kOut, kHidden, h_[2], kHidden, false, w + offW4, ldw(kHidden, kOut), tc_, y_, nullptr, kOut,
-          params_ + offB4, nullptr, s),
-     "layer 4");
+void Denoiser::ensureParts(int rows) {
+  const int tiles = std::min(kMaxTiles, (rows + kTileRows - 1) / kTileRows);
+  if (!carry_) carry_ = dalloc<float>(kParams);
+  if (tiles <= partTiles_) return;
+  dfree(part_);
+  part_ = nullptr;
+  partTiles_ = 0;
+  part_ = dalloc<float>(static_cast<size_t>(tiles) * kParams);
+  partTiles_ = tiles;
 }
 
-float Denoiser::forwardBackward(const void* X, const float* base, const float* target, int rows, bool wantLoss,
-                                cudaStream_t s) {
-  if (wantLoss) ck(cudaMemsetAsync(lossSum_, 0, 4, s), "memset");
-  step(X, base, target, rows, wantLoss ? lossSum_ : nullptr, s);
-  if (!wantLoss) return 0.f;
-  float e2 = 0.f;
-  ck(cudaMemcpyAsync(&e2, lossSum_, 4, cudaMemcpyDeviceToHost, s), "loss readback");
-  ck(cudaStreamSynchronize(s), "step");
-  return e2 / (3.0f * static_cast<float>(rows));
+void Denoiser::stepTc(const void* X, const float* base, const float* target, const uint32_t* order,
+                      const uint32_t* offset, int rows, float* lossAcc, const int* lossIndex, const AdamTarget* adam,
+                      cudaStream_t s) {
+  static_assert(kParams % 4 == 0 && offB1 % 4 == 0 && offW2 % 4 == 0 && offB2 % 4 == 0 && offW3 % 4 == 0 &&
+                    offB3 % 4 == 0 && offW4 % 4 == 0 && offB4 % 4 == 0,
+                "reduceStep takes the parameters in fours");
+  TrainTiles a{};
+  a.X = static_cast<const __nv_bfloat16*>(X);
+  a.base = base;
+  a.target = target;
+  a.order = order;
+  a.offset = offset;
+  a.rows = rows;
+  a.wT = static_cast<const __nv_bfloat16*>(wbfT_);
+  a.params = params_;
+  a.w = weightBlocks();
+  const size_t b[4] = {offB1, offB2, offB3, offB4};
+  for (int i = 0; i < 4; ++i) a.b[i] = static_cast<int>(b[i]);
+  a.part = part_;
+  a.stride = kParams;
+  a.lossSum = lossAcc;
+  a.lossIndex = lossIndex;
+  // A batch of more tiles than one launch takes carries its sums over.
+  const int tiles = (rows + kTileRows - 1) / kTileRows;
+  for (int first = 0; first < tiles; first += kMaxTiles) {
+    const int n = std::min(kMaxTiles, tiles - first);
+    const bool last = first + n == tiles;
+    a.firstTile = first;
+    ck(trainTiles(a, n, s), "training step");
+    ck(reduceStep(part_, n, static_cast<int>(kParams), a.w, first ? carry_ : nullptr, last ? nullptr : carry_,
+                  last && !adam ? grads_ : nullptr, last ? adam : nullptr, s),
+       "gradient sums");
+  }
+}
+
+void Denoiser::forward(const void* X, int rows, cudaStream_t s) {
+  const uint16_t* w = static_cast<const uint16_t*>(wbf_);
+  ck(gemmBf16(1, rows, kHidden, kFeatureWidth, X, kFeatureWidth, false, w + offW1, kHidden, false,
+          zs_, h_[0], kHidden, params_ + offB1, nullptr, s),
+     "layer 1");
+  ck(gemmBf16(1, rows, kHidden, kHidden, h_[0], kHidden, false, w + offW2, kHidden, false, zs_, h_[1],
+          kHidden, params_ + offB2, nullptr, s),
+     "layer 2");
+  ck(gemmBf16(1, rows, kHidden, kHidden, h_[1], kHidden, false, w + offW3, kHidden, false, zs_, h_[2],
+          kHidden, params_ + offB3, nullptr, s),
+     "layer 3");
+  ck(gemmBf16(3, rows, kOut, kHidden, h_[2], kHidden, false, w + offW4, kOut, false, y_, nullptr, kOut,
+          params_ + offB4, nullptr, s),
+     "layer 4");
 }
 
 // Forward, loss gradient and backward of one minibatch into grads_, with the
@@ -142,11 +175,11 @@ void Denoiser::step(const void* X, const float* base, const float* target, int r
   forward(X, rows, s);
   ck(mlpLoss(y_, kOut, base, target, rows, nullptr, dyf_, dyb_, lossAcc, s, lossIndex), "loss");
   // Output layer.
-  ck(gemm(0, kHidden, kOut, rows, h_[2], kHidden, true, dyb_, kOut, false, grads_ + offW4, nullptr, kOut, nullptr,
+  ck(gemmBf16(0, kHidden, kOut, rows, h_[2], kHidden, true, dyb_, kOut, false, grads_ + offW4, nullptr, kOut, nullptr,
               nullptr, s),
      "dW4");
   ck(colSumF32(dyf_, rows, kOut, kOut, grads_ + offB4, s), "db4");
-  ck(gemm(2, rows, kHidden, kOut, dyb_, kOut, false, w + offW4, kOut, true, nullptr, dz_[2], kHidden, nullptr, h_[2],
+  ck(gemmBf16(2, rows, kHidden, kOut, dyb_, kOut, false, w + offW4, kOut, true, nullptr, dz_[2], kHidden, nullptr, h_[2],
               s),
      "dZ3");
   // Hidden layers 3, 2, 1.
@@ -155,12 +188,12 @@ void Denoiser::step(const void* X, const float* base, const float* target, int r
   for (int l = 2; l >= 0; --l) {
     const void* in = l == 0 ? X : h_[l - 1];
     const int kin = l == 0 ? kFeatureWidth : kHidden;
-    ck(gemm(0, kin, kHidden, rows, in, kin, true, dz_[l], kHidden, false, grads_ + offW[l], nullptr, kHidden,
+    ck(gemmBf16(0, kin, kHidden, rows, in, kin, true, dz_[l], kHidden, false, grads_ + offW[l], nullptr, kHidden,
                 nullptr, nullptr, s),
        "dW");
     ck(colSumBf16(dz_[l], rows, kHidden, kHidden, grads_ + offB[l], s), "db");
     if (l > 0)
-      ck(gemm(2, rows, kHidden, kHidden, dz_[l], kHidden, false, w + offW[l], kHidden, true, nullptr, dz_[l - 1],
+      ck(gemmBf16(2, rows, kHidden, kHidden, dz_[l], kHidden, false, w + offW[l], kHidden, true, nullptr, dz_[l - 1],
                   kHidden, nullptr, h_[l - 1], s),
          "dZ");
   }
@@ -198,13 +231,16 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
   if (!ready()) throw std::runtime_error("denoiser not initialised");
   if (rows_ == 0) throw std::runtime_error("no training rows");
   if (steps <= 0) return;
+  if (batch == 0) throw std::runtime_error("empty batch");
   batch = static_cast<int>(std::min<size_t>(static_cast<size_t>(batch), rows_));
-  ensureBatch(batch);
+  if (tc) ensureParts(batch);
+  else ensureBatch(batch);
   // The shuffled order of an epoch, the step sizes and Adam's bias
   // corrections of every step, the per-step losses and the loop's position
   // (TrainState) live on the device.  The first step runs as plain launches
   // (it sets up what the kernels need), the next is captured as a CUDA graph
-  // and replayed for the rest; the host only reshuffles between epochs.
+  // and replayed for the rest; the host draws the next epoch's order while
+  // they run.
   std::mt19937 rng(seed);
   std::vector<uint32_t> perm(rows_);
   std::iota(perm.begin(), perm.end(), 0u);
@@ -219,7 +255,8 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
     sched[3 * st + 1] = 1.f / (1.f - powf(b1, t));
     sched[3 * st + 2] = 1.f / (1.f - powf(b2, t));
   }
-  uint32_t* permDev = dalloc<uint32_t>(rows_);
+  // Two orders: the next epoch's is drawn while this one's steps run.
+  uint32_t* permDev = dalloc<uint32_t>(2 * rows_);
   float* lossDev = dalloc<float>(static_cast<size_t>(steps));
   float* schedDev = dalloc<float>(sched.size());
   TrainState* state = dalloc<TrainState>(1);
@@ -233,14 +270,19 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
     dfree(schedDev);
     dfree(state);
   };
-  tc_ = tc;
   try {
     ck(cudaMemcpyAsync(permDev, perm.data(), rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
     ck(cudaMemcpyAsync(schedDev, sched.data(), sched.size() * 4, cudaMemcpyHostToDevice, s), "schedule");
     ck(cudaMemsetAsync(lossDev, 0, static_cast<size_t>(steps) * 4, s), "memset");
     ck(cudaMemsetAsync(state, 0, sizeof(TrainState), s), "memset");
     const WeightBlocks blocks = weightBlocks();
+    const AdamTarget adam{params_, m_, v_, static_cast<__nv_bfloat16*>(wbf_), static_cast<__nv_bfloat16*>(wbfT_),
+                          schedDev, state, static_cast<uint32_t>(batch), b1, b2, 1e-8f};
     auto oneStep = [&]() {
+      if (tc) {
+        stepTc(X_, base_, target_, permDev, &state->offset, batch, loss ? lossDev : nullptr, &state->step, &adam, s);
+        return;
+      }
       ck(gatherRows(X_, base_, target_, permDev, batch, Xb_, baseb_, targetb_, s, &state->offset), "gather");
       step(Xb_, baseb_, targetb_, batch, loss ? lossDev : nullptr, s, &state->step);
       ck(adamStep(params_, grads_, m_, v_, static_cast<int>(kParams), 0.f, b1, b2, 1e-8f, 1, wbf_, s, wbfT_, &blocks,
@@ -248,17 +290,8 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
          "adam");
       ck(advanceTrainState(state, static_cast<uint32_t>(batch), s), "advance");
     };
-    size_t cursor = 0;
+    size_t cursor = 0, half = 0;
     for (int st = 0; st < steps;) {
-      if (cursor + static_cast<size_t>(batch) > rows_) {
-        ck(cudaStreamSynchronize(s), "epoch");  // the previous order is no longer read
-        std::shuffle(perm.begin(), perm.end(), rng);
-        ck(cudaMemcpyAsync(permDev, perm.data(), rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
-        const TrainState at{st, 0u};
-        ck(cudaMemcpyAsync(state, &at, sizeof(at), cudaMemcpyHostToDevice, s), "state");
-        ck(cudaStreamSynchronize(s), "epoch");
-        cursor = 0;
-      }
       const int run = static_cast<int>(std::min<size_t>(static_cast<size_t>(steps - st),
                                                         (rows_ - cursor) / static_cast<size_t>(batch)));
       int done = 0;
@@ -282,20 +315,26 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
       for (; done < run; ++done) ck(cudaGraphLaunch(exec, s), "graph launch");
       st += run;
       cursor += static_cast<size_t>(run) * static_cast<size_t>(batch);
+      if (st < steps) {
+        half ^= 1u;
+        std::shuffle(perm.begin(), perm.end(), rng);
+        ck(cudaMemcpyAsync(permDev + half * rows_, perm.data(), rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
+        const TrainState at{st, static_cast<uint32_t>(half * rows_), 0u};
+        ck(cudaMemcpyAsync(state, &at, sizeof(at), cudaMemcpyHostToDevice, s), "state");
+        cursor = 0;
+      }
     }
     adamT_ += steps;
     if (loss) {
       ck(cudaMemcpyAsync(loss, lossDev, static_cast<size_t>(steps) * 4, cudaMemcpyDeviceToHost, s), "loss readback");
     }
     ck(cudaStreamSynchronize(s), "train");
-    tc_ = false;
     if (tc) {
       uint32_t flags = 0;
       ck(takeTcGemmError(&flags), "tcgen05 GEMM status");
       if (flags) throw std::runtime_error("a tcgen05 GEMM wait timed out during training");
     }
   } catch (...) {
-    tc_ = false;
     cleanup();
     throw;
   }
@@ -325,16 +364,19 @@ MlpWeights Denoiser::weights() const {
 float Denoiser::gradient(const void* X, const float* base, const float* target, int rows, float* gradsHost,
                          float* paramsHost, cudaStream_t s, bool tc) {
   if (!ready()) throw std::runtime_error("denoiser not initialised");
-  ensureBatch(rows);
-  tc_ = tc;
-  float l;
-  try {
-    l = forwardBackward(X, base, target, rows, true, s);
-  } catch (...) {
-    tc_ = false;
-    throw;
+  if (!lossSum_) lossSum_ = dalloc<float>(1);
+  ck(cudaMemsetAsync(lossSum_, 0, 4, s), "memset");
+  if (tc) {
+    ensureParts(rows);
+    stepTc(X, base, target, nullptr, nullptr, rows, lossSum_, nullptr, nullptr, s);
+  } else {
+    ensureBatch(rows);
+    step(X, base, target, rows, lossSum_, s);
   }
-  tc_ = false;
+  float e2 = 0.f;
+  ck(cudaMemcpyAsync(&e2, lossSum_, 4, cudaMemcpyDeviceToHost, s), "loss readback");
+  ck(cudaStreamSynchronize(s), "step");
+  const float l = e2 / (3.0f * static_cast<float>(rows));
   if (tc) {
     uint32_t flags = 0;
     ck(takeTcGemmError(&flags), "tcgen05 GEMM status");

@@ -48,8 +48,9 @@ class Denoiser {
   // `steps` Adam steps on minibatches of `batch` rows drawn by a seeded
   // shuffle of the training set; returns the mean squared error of each step
   // in `loss` (host, `steps` floats) if given.
-  // tc: the GEMMs run on the tcgen05 tensor cores (gemmBf16Tc), else on
-  // mma.sync (gemmBf16, the path the layer-by-layer prediction repeats).
+  // tc: the step runs on the tcgen05 tensor cores (trainTiles, reduceStep),
+  // else on mma.sync GEMMs (gemmBf16, the path the layer-by-layer prediction
+  // repeats).
   void train(int steps, int batch, float lr, uint32_t seed, float* loss, cudaStream_t s, bool tc = true);
 
   // Prediction for `rows` feature rows (device): out = base + net(X)[:, :3],
@@ -75,11 +76,16 @@ class Denoiser {
 
  private:
   void ensureBatch(int rows);
-  float forwardBackward(const void* X, const float* base, const float* target, int rows, bool wantLoss,
-                        cudaStream_t s);
   void step(const void* X, const float* base, const float* target, int rows, float* lossAcc, cudaStream_t s,
             const int* lossIndex = nullptr);
   void forward(const void* X, int rows, cudaStream_t s);
+  // The same on the tcgen05 tensor cores: gradients into grads_, or (adam)
+  // straight into a step.  order, offset: see TrainTiles.
+  void stepTc(const void* X, const float* base, const float* target, const uint32_t* order, const uint32_t* offset,
+              int rows, float* lossAcc, const int* lossIndex, const AdamTarget* adam, cudaStream_t s);
+  void ensureParts(int rows);
+  static constexpr int kTileRows = 128;
+  static constexpr int kMaxTiles = 512;  // of one launch: 95 MB of gradient sums
 
   float* params_ = nullptr;
   float* grads_ = nullptr;
@@ -94,12 +100,6 @@ class Denoiser {
                         {kHidden, kHidden, kHidden, kOut}};
   }
   int adamT_ = 0;
-  bool tc_ = false;  // GEMMs of the running train() on tcgen05
-  cudaError_t gemm(int mode, int M, int N, int K, const void* A, int lda, bool aTrans, const void* B, int ldb,
-                   bool bTrans, float* Cf, void* Hb, int ldc, const float* bias, const void* mask, cudaStream_t s) {
-    return tc_ ? gemmBf16Tc(mode, M, N, K, A, lda, aTrans, B, ldb, bTrans, Cf, Hb, ldc, bias, mask, s)
-               : gemmBf16(mode, M, N, K, A, lda, aTrans, B, ldb, bTrans, Cf, Hb, ldc, bias, mask, s);
-  }
   // batch work buffers
   int cap_ = 0;
   void* Xb_ = nullptr;
@@ -113,6 +113,10 @@ class Denoiser {
   void* dyb_ = nullptr;
   float* lossSum_ = nullptr;
   uint32_t* idx_ = nullptr;
+  // the tcgen05 step's gradient sums: one set per tile of a launch, and the carry between launches
+  float* part_ = nullptr;
+  float* carry_ = nullptr;
+  int partTiles_ = 0;
   // training set
   void* X_ = nullptr;
   float* base_ = nullptr;

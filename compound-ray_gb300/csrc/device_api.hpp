@@ -232,14 +232,6 @@ static_assert(kFeatBlock * (kNeighbours + 1) <= kFeatureWidth, "feature row too 
 cudaError_t gemmBf16(int mode, int M, int N, int K, const void* A, int lda, bool aTrans, const void* B, int ldb,
                      bool bTrans, float* Cf, void* Hb, int ldc, const float* bias, const void* mask,
                      cudaStream_t stream);
-// The same GEMMs on the tcgen05 tensor cores (mlp_tc.cu): 128 x 128 output
-// tiles, K in chunks of 64, accumulators in TMEM.  A timed-out wait is
-// recorded in a device word that takeTcGemmError reads and clears
-// (kErrMmaTimeout).
-cudaError_t gemmBf16Tc(int mode, int M, int N, int K, const void* A, int lda, bool aTrans, const void* B, int ldb,
-                       bool bTrans, float* Cf, void* Hb, int ldc, const float* bias, const void* mask,
-                       cudaStream_t stream);
-cudaError_t takeTcGemmError(uint32_t* flags);
 cudaError_t colSumBf16(const void* in, int M, int N, int ld, float* out, cudaStream_t stream);
 cudaError_t colSumF32(const float* in, int M, int N, int ld, float* out, cudaStream_t stream);
 // Position of a training loop on the device.  The kernels of one step read
@@ -247,6 +239,7 @@ cudaError_t colSumF32(const float* in, int M, int N, int ld, float* out, cudaStr
 struct TrainState {
   int step;         // index into the step-size schedule and the loss array
   uint32_t offset;  // first entry of this step's rows in the shuffled order
+  unsigned done;    // blocks of reduceStep that have finished
 };
 // lossIndex: null, or the device index added to lossSum.
 cudaError_t mlpLoss(const float* y, int ldy, const float* base, const float* target, int rows, float* pred, float* dyf,
@@ -254,8 +247,7 @@ cudaError_t mlpLoss(const float* y, int ldy, const float* base, const float* tar
 // state->step += 1, state->offset += rows.
 cudaError_t advanceTrainState(TrainState* state, uint32_t rows, cudaStream_t stream);
 // Row-major weight matrices inside a flat parameter vector.  Their
-// transposes (same offsets) are the K-contiguous operands of the tcgen05
-// forward GEMMs.
+// transposes (same offsets) are the operands of the tcgen05 training step.
 struct WeightBlocks {
   int count;
   int off[4], rows[4], cols[4];
@@ -267,6 +259,45 @@ struct WeightBlocks {
 cudaError_t adamStep(float* w, const float* g, float* m, float* v, int n, float lr, float b1, float b2, float eps,
                      int t, void* wb, cudaStream_t stream, void* wbT = nullptr, const WeightBlocks* blocks = nullptr,
                      const float* sched = nullptr, const int* stepIdx = nullptr);
+// Forward and backward pass of the tcgen05 training step (mlp_tc.cu): one
+// block per tile of 128 rows, tiles firstTile .. +tiles, the gradient sums of
+// the k-th of them at part + k stride.  There a weight matrix's gradient lies
+// at its offset in the parameters as float4 of four columns, [column / 4][row];
+// biases lie as in the parameters.  A timed-out wait is recorded in a device
+// word that takeTcGemmError reads and clears (kErrMmaTimeout).
+struct TrainTiles {
+  const __nv_bfloat16* X;   // feature rows (16-byte aligned)
+  const float* base;        // rows x 3
+  const float* target;      // rows x 3
+  const uint32_t* order;    // null, or row r of the step is X's row order[*offset + r]
+  const uint32_t* offset;   // null: 0
+  int rows, firstTile;
+  const __nv_bfloat16* wT;  // transposed weights at the offsets of `w`
+  const float* params;
+  WeightBlocks w;
+  int b[4];                 // offsets of the biases
+  float* part;
+  size_t stride;            // floats: the number of parameters, a multiple of 4
+  float* lossSum;           // null, or the squared error is added to lossSum[*lossIndex]
+  const int* lossIndex;     // null: 0
+};
+cudaError_t trainTiles(const TrainTiles& a, int tiles, cudaStream_t stream);
+cudaError_t takeTcGemmError(uint32_t* flags);
+// Gradients of n parameters from the tiles' sums (added in tile order to
+// `carry`, laid out like them; null: to zero).  Then one of: next (the sums,
+// for a later call's carry), g (the gradients, laid out like the parameters),
+// or Adam on w, m, v as in adamStep with its schedule at state->step, followed
+// by state->step += 1, state->offset += rows.
+struct AdamTarget {
+  float *w, *m, *v;
+  __nv_bfloat16 *wb, *wbT;
+  const float* sched;
+  TrainState* state;
+  uint32_t rows;
+  float b1, b2, eps;
+};
+cudaError_t reduceStep(const float* part, int tiles, int n, const WeightBlocks& blocks, const float* carry, float* next,
+                       float* g, const AdamTarget* adam, cudaStream_t stream);
 // wbT = bf16 transposes of `blocks` of the n fp32 parameters w.
 cudaError_t transposeWeightsBf16(const float* w, size_t n, void* wbT, const WeightBlocks& blocks, cudaStream_t stream);
 cudaError_t toBf16(const float* in, void* out, size_t n, cudaStream_t stream);

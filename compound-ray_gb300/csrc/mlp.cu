@@ -16,8 +16,8 @@
 //   knnKernel        six nearest ommatidia by axis direction;
 //   featureKernel    assembles the 112-wide bf16 feature rows.
 // These mma.sync GEMMs are the path the layer-by-layer prediction uses and
-// the training path of crSetDenoiserKernel(0); training runs on the tcgen05
-// GEMMs of mlp_tc.cu by default.
+// the training path of crSetDenoiserKernel(0); training runs on the fused
+// tcgen05 step of mlp_tc.cu by default.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -293,6 +293,13 @@ __device__ __forceinline__ float rsqrt_rn(float a) {
 //   m = b1 m + (1 - b1) g;  v = b2 v + (1 - b2) g g;
 //   w = w - lr (m c1) / (sqrt(v c2) + eps)
 // one correctly rounded float operation at a time, in this order.
+__device__ __forceinline__ float adamOne(float w, float gi, float& m, float& v, float lr, float b1, float b2, float eps,
+                                         float c1, float c2) {
+  m = radd(rmul(b1, m), rmul(rsub(1.f, b1), gi));
+  v = radd(rmul(b2, v), rmul(rmul(rsub(1.f, b2), gi), gi));
+  return rsub(w, rdiv(rmul(lr, rmul(m, c1)), radd(rsqrt_rn(rmul(v, c2)), eps)));
+}
+
 __global__ void adamKernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m,
                            float* __restrict__ v, int n, float lr, float b1, float b2, float eps, float c1, float c2,
                            __nv_bfloat16* __restrict__ wb, __nv_bfloat16* __restrict__ wbT, WeightBlocks blocks,
@@ -305,15 +312,79 @@ __global__ void adamKernel(float* __restrict__ w, const float* __restrict__ g, f
     c1 = e[1];
     c2 = e[2];
   }
-  const float gi = g[i];
-  const float mi = radd(rmul(b1, m[i]), rmul(rsub(1.f, b1), gi));
-  const float vi = radd(rmul(b2, v[i]), rmul(rmul(rsub(1.f, b2), gi), gi));
+  float mi = m[i], vi = v[i];
+  const float wi = adamOne(w[i], g[i], mi, vi, lr, b1, b2, eps, c1, c2);
   m[i] = mi;
   v[i] = vi;
-  const float wi = rsub(w[i], rdiv(rmul(lr, rmul(mi, c1)), radd(rsqrt_rn(rmul(vi, c2)), eps)));
   w[i] = wi;
   if (wb) wb[i] = __float2bfloat16(wi);
   if (wbT) putTransposed(i, wi, wbT, blocks);
+}
+
+// Sums of the tiles' gradients (see trainTileKernel), four parameters a
+// thread in the tiles' layout, and Adam on them: with the reductions, the
+// column sums and Adam as launches of their own a step was 10 launches
+// longer.  The sum runs over the tiles in order; 16 loads in flight a thread.
+__global__ void __launch_bounds__(64) reduceStepKernel(const float4* __restrict__ part, int tiles, int quads,
+                                                       WeightBlocks blocks, const float4* __restrict__ carry,
+                                                       float4* __restrict__ next, float* __restrict__ g, AdamTarget a) {
+  const int q = blockIdx.x * 64 + threadIdx.x;
+  if (q < quads) {
+    float4 s = carry ? carry[q] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 16
+    for (int k = 0; k < tiles; ++k) {
+      const float4 p = __ldg(part + static_cast<size_t>(k) * quads + q);
+      s.x += p.x;
+      s.y += p.y;
+      s.z += p.z;
+      s.w += p.w;
+    }
+    if (next) {
+      next[q] = s;
+    } else {
+      int i = 4 * q, t = 0, step = 0;  // parameter; place and stride of its transposes (stride 0: a bias)
+      for (int k = 0; k < blocks.count; ++k) {
+        const int j = i - blocks.off[k];
+        if (j < 0 || j >= blocks.rows[k] * blocks.cols[k]) continue;
+        const int c = j / 4 / blocks.rows[k], r = j / 4 - c * blocks.rows[k];
+        i = blocks.off[k] + r * blocks.cols[k] + 4 * c;
+        t = blocks.off[k] + 4 * c * blocks.rows[k] + r;
+        step = blocks.rows[k];
+        break;
+      }
+      if (g) {
+        *reinterpret_cast<float4*>(g + i) = s;
+      } else {
+        const float* e = a.sched + 3 * static_cast<size_t>(a.state->step);
+        const float lr = e[0], c1 = e[1], c2 = e[2];
+        float4 m = *reinterpret_cast<float4*>(a.m + i), v = *reinterpret_cast<float4*>(a.v + i);
+        float4 w = *reinterpret_cast<float4*>(a.w + i);
+        w.x = adamOne(w.x, s.x, m.x, v.x, lr, a.b1, a.b2, a.eps, c1, c2);
+        w.y = adamOne(w.y, s.y, m.y, v.y, lr, a.b1, a.b2, a.eps, c1, c2);
+        w.z = adamOne(w.z, s.z, m.z, v.z, lr, a.b1, a.b2, a.eps, c1, c2);
+        w.w = adamOne(w.w, s.w, m.w, v.w, lr, a.b1, a.b2, a.eps, c1, c2);
+        *reinterpret_cast<float4*>(a.m + i) = m;
+        *reinterpret_cast<float4*>(a.v + i) = v;
+        *reinterpret_cast<float4*>(a.w + i) = w;
+        const __nv_bfloat16 b[4] = {__float2bfloat16(w.x), __float2bfloat16(w.y), __float2bfloat16(w.z),
+                                    __float2bfloat16(w.w)};
+        *reinterpret_cast<uint2*>(a.wb + i) = make_uint2(pack2(b[0], b[1]), pack2(b[2], b[3]));
+        if (step)
+          for (int k = 0; k < 4; ++k) a.wbT[t + k * step] = b[k];
+      }
+    }
+  }
+  if (next || g) return;
+  // The last block moves the state on: every other has read it.
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    if (atomicAdd(&a.state->done, 1u) == gridDim.x - 1) {
+      a.state->done = 0u;
+      a.state->step += 1;
+      a.state->offset += a.rows;
+    }
+  }
 }
 
 __global__ void transposeWeightsKernel(const float* __restrict__ w, int n, __nv_bfloat16* __restrict__ wbT,
@@ -596,6 +667,17 @@ cudaError_t adamStep(float* w, const float* g, float* m, float* v, int n, float 
                                                    static_cast<__nv_bfloat16*>(wb), static_cast<__nv_bfloat16*>(wbT),
                                                    wbT && blocks ? *blocks : none, sched && stepIdx ? sched : nullptr,
                                                    stepIdx);
+  return cudaGetLastError();
+}
+
+cudaError_t reduceStep(const float* part, int tiles, int n, const WeightBlocks& blocks, const float* carry, float* next,
+                       float* g, const AdamTarget* adam, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  if (n % 4 || (!next && !g && !adam)) return cudaErrorInvalidValue;
+  const int quads = n / 4;
+  reduceStepKernel<<<(quads + 63) / 64, 64, 0, stream>>>(
+      reinterpret_cast<const float4*>(part), tiles, quads, blocks, reinterpret_cast<const float4*>(carry),
+      reinterpret_cast<float4*>(next), g, adam ? *adam : AdamTarget{});
   return cudaGetLastError();
 }
 

@@ -567,328 +567,368 @@ __global__ void waitProbeKernel(uint32_t polls, uint32_t* errFlag) {
 }
 
 // ---------------------------------------------------------------------------
-// Training GEMMs on the tcgen05 tensor cores: C[M x N] = sum_k a(m, k) b(n, k)
-// with the operand conventions of gemmBf16 (mlp.cu):
-//   a(m, k) = aTrans ? A[k * lda + m] : A[m * lda + k],
-//   b(n, k) = bTrans ? B[n * ldb + k] : B[k * ldb + n],
-// and its epilogues (0 fp32 store, 1 bias + ReLU to bf16 and the fp32
-// pre-activation, 2 ReLU-derivative mask to bf16, 3 bias to fp32).
-// One 256-thread block per 128 x 128 output tile (N padded to a multiple of
-// 16 for the MMA), K in chunks of 64 staged by the threads into shared
-// memory in the canonical K-major no-swizzle layout, 16 bytes per load; one
-// thread issues the chunk's four tcgen05.mma (K 16 each) into the TMEM
-// accumulator and commits them; warps w and w + 4 read accumulator lanes
-// 32 w .. +31, columns 0-63 and 64-127.  grid.z > 1 splits
-// K into slices that write partial tiles (ldc = N) for a reduction in slice
-// order.  Waits are bounded; a timeout sets g_tcGemmErr.
+// One training step's forward and backward pass for a tile of 128 rows, in
+// one block: the rows are gathered, the four layers, the loss gradient, the
+// input gradients and the tile's share of every weight and bias gradient are
+// computed without leaving the SM, and only that share is written
+// (kParams floats a tile; reduceStep sums the tiles in order).
+//
+// Every operand stays in shared memory in the canonical no-swizzle layout of
+// 8 x 8 core matrices (coreOffset), and each is used twice.  A tile image
+// [row][feature] is the K-major A operand of the next layer (K = features)
+// and, read with the transpose bit, the MN-major operand of the weight
+// gradient (K = rows, so core matrices along MN are 128 bytes apart and those
+// along K a row group apart); a weight image [out][in] is the K-major B operand of the
+// forward pass and the MN-major one of the input gradient.  So nothing is
+// transposed and no second copy of the weights is read.  dz of layer l
+// overwrites that layer's activations once the weight gradient that reads
+// them is done; the ReLU masks stay in registers (a thread reads the same
+// accumulator row and columns in both directions).
+//
+// 16 warps: warp w reads accumulator lanes 32 (w % 4) .. +31, columns
+// 32 (w / 4) .. +31; one thread issues.  TMEM columns: 0-127 the forward and
+// input-gradient accumulator, 128-143 dW4 and later 128-255 dW1, 256-383
+// dW3, 384-511 dW2.  While the MMAs of a layer run, the warps write out the
+// previous weight gradient and sum the bias gradient.
+//
+// A step is a chain of 8 dependent MMA groups, so its time is their latency
+// and not their work: as 23 launches (one GEMM per layer and direction, with
+// the activations in memory between them and split-K reductions) 8192 rows
+// took 190 us a step; in this form 28 us with the reduction and Adam.
+// The rows' sums are formed in the same order as there.  Waits are bounded; a
+// timeout sets g_tcGemmErr.
 // ---------------------------------------------------------------------------
-constexpr int kGemmTile = 128;
-constexpr int kGemmChunk = 64;
-constexpr uint32_t kGemmStage = kGemmTile * kGemmChunk * 2;  // bytes per operand stage
-// Dynamic shared memory per block, sized so that at most four blocks share
-// an SM: their four 128-column accumulators fill its 512 TMEM columns, and
-// no block ever waits in tcgen05.alloc.
-constexpr uint32_t kGemmSmem = 56 * 1024;
-static_assert(2 * kGemmStage + 128 <= kGemmSmem, "staging exceeds the block's shared memory");
-constexpr uint32_t kGemmMaskOff = 8 * 32 * 33 * 4;  // after the eight warps' fp32 epilogue tiles
-constexpr int kGemmMaskLd = 40;                     // bf16 per mask row: 80 bytes, 16-byte aligned rows
-static_assert(kGemmMaskOff % 16 == 0, "mask tiles must start 16-byte aligned");
-static_assert(kGemmMaskOff + 8 * 32 * kGemmMaskLd * 2 + 128 <= kGemmSmem,
-              "epilogue tiles exceed the block's shared memory");
+constexpr int kStepThreads = 512;
+constexpr uint32_t kStepXGroup = kFeatureWidth * 16u;  // bytes of 8 feature rows
+constexpr uint32_t kStepGroup = kMlpHidden * 16u;      // bytes of 8 rows of a 128-wide image
+constexpr uint32_t kOffStepX = 0;
+constexpr uint32_t kOffStepH = kOffStepX + kTcRows * kFeatureWidth * 2;  // three layers' activations, then dz
+constexpr uint32_t kOffStepW2 = kOffStepH + 3 * kActBytes;
+constexpr uint32_t kOffStepW3 = kOffStepW2 + kWBytes;
+constexpr uint32_t kOffStepW4 = kOffStepW3 + kWBytes;
+constexpr uint32_t kOffStepW1 = kOffStepW4 + kW4Bytes;
+constexpr uint32_t kOffStepDy = kOffStepW1 + kW1Bytes;               // 128 x 16 bf16, the upper 8 columns zero
+constexpr uint32_t kOffStepBias = kOffStepDy + kTcRows * 16 * 2;     // 3 x 128 + 8 floats; later 3 x 128 of dy in fp32
+constexpr uint32_t kStepSmem = kOffStepBias + (3 * kMlpHidden + 8) * 4 + 128;  // + alignment slack
+static_assert(kStepSmem + 64 <= 227 * 1024, "shared memory plan exceeds a block's limit");
+static_assert(kTcRows == kMlpHidden, "the weight gradients' M is a tile image's width");
+constexpr uint32_t kStepTmemCols = 512;
 __device__ uint32_t g_tcGemmErr;
 
-constexpr int kGemmThreads = 256;  // eight warps: two per accumulator lane quarter
+// instrDesc with MN-major operands.
+constexpr uint32_t kAMnMajor = 1u << 15, kBMnMajor = 1u << 16;
 
-// Stages rows [0, rowsValid) x chunk columns of an operand whose element
-// (r, c) is at P[(row0 + r) * ld + k0 + c] (K contiguous: 8 elements per
-// 16-byte load) or, when `kMajorInMemory` is false, at
-// P[(k0 + c) * ld + row0 + r] (rows contiguous: 8 rows per 16-byte load,
-// scattered to their core-matrix rows); zero outside rowsValid and kEnd.
-__device__ __forceinline__ void stageOperand(unsigned char* dst, const __nv_bfloat16* __restrict__ P, int ld,
-                                             bool kMajorInMemory, int row0, int rowsValid, int rowsPadded, int k0,
-                                             int kEnd, int tid) {
-  const bool vec = (reinterpret_cast<uintptr_t>(P) & 15) == 0 && (ld & 7) == 0;
-  if (kMajorInMemory) {
-    // groups of 8 consecutive k of one row
-    for (int e = tid; e < rowsPadded * (kGemmChunk / 8); e += kGemmThreads) {
-      const int r = e / (kGemmChunk / 8), c = (e % (kGemmChunk / 8)) * 8;
-      const int k = k0 + c;
-      uint4 v = make_uint4(0u, 0u, 0u, 0u);
-      if (r < rowsValid) {
-        const __nv_bfloat16* src = P + static_cast<size_t>(row0 + r) * ld + k;
-        if (vec && k + 8 <= kEnd) {
-          v = *reinterpret_cast<const uint4*>(src);
-        } else {
-          uint16_t t[8];
-          for (int j = 0; j < 8; ++j) t[j] = k + j < kEnd ? __bfloat16_as_ushort(src[j]) : 0;
-          v = make_uint4(t[0] | (uint32_t(t[1]) << 16), t[2] | (uint32_t(t[3]) << 16), t[4] | (uint32_t(t[5]) << 16),
-                         t[6] | (uint32_t(t[7]) << 16));
-        }
-      }
-      *reinterpret_cast<uint4*>(dst + coreOffset(static_cast<uint32_t>(r), static_cast<uint32_t>(c), kGemmChunk)) = v;
-    }
-  } else {
-    // 8 x 8 blocks (8 rows x 8 k), one per group of eight lanes: lane l8
-    // loads the block's 8 rows at k = 8 kg + l8 (16 bytes, rows contiguous in
-    // memory), the group transposes the block in three exchange rounds, and
-    // lane l8 stores row l8's 8 k as one 16-byte row of a core matrix, so the
-    // eight lanes of a store phase fill 128 contiguous bytes.
-    const int lane = tid & 31, q = lane >> 3, l8 = lane & 7;
-    const int groups = rowsPadded / 8, nBlocks = groups * (kGemmChunk / 8);  // nBlocks: a multiple of 4
-    for (int base = (tid >> 5) * 4; base < nBlocks; base += kGemmThreads / 8) {
-      const int b = base + q;  // < nBlocks for every lane: the warp runs each round whole
-      const int g = b % groups, kg = b / groups;
-      const int r = g * 8, k = k0 + kg * 8 + l8;
-      uint32_t w0 = 0u, w1 = 0u, w2 = 0u, w3 = 0u;
-      if (k < kEnd) {
-        const __nv_bfloat16* src = P + static_cast<size_t>(k) * ld + row0 + r;
-        if (vec && r + 8 <= rowsValid) {
-          const uint4 v = *reinterpret_cast<const uint4*>(src);
-          w0 = v.x; w1 = v.y; w2 = v.z; w3 = v.w;
-        } else {
-          uint32_t t[8];
-          for (int j = 0; j < 8; ++j) t[j] = r + j < rowsValid ? __bfloat16_as_ushort(src[j]) : 0u;
-          w0 = t[0] | (t[1] << 16); w1 = t[2] | (t[3] << 16); w2 = t[4] | (t[5] << 16); w3 = t[6] | (t[7] << 16);
-        }
-      }
-      // Round 1, lanes l8 ^ 4: elements 4-7 of the low lanes for 0-3 of the high ones.
-      {
-        const bool hi = l8 & 4;
-        const uint32_t r0 = __shfl_xor_sync(0xffffffffu, hi ? w0 : w2, 4);
-        const uint32_t r1 = __shfl_xor_sync(0xffffffffu, hi ? w1 : w3, 4);
-        if (hi) { w0 = r0; w1 = r1; } else { w2 = r0; w3 = r1; }
-      }
-      // Round 2, lanes l8 ^ 2: element pairs {2,3}, {6,7} against {0,1}, {4,5}.
-      {
-        const bool hi = l8 & 2;
-        const uint32_t r0 = __shfl_xor_sync(0xffffffffu, hi ? w0 : w1, 2);
-        const uint32_t r1 = __shfl_xor_sync(0xffffffffu, hi ? w2 : w3, 2);
-        if (hi) { w0 = r0; w2 = r1; } else { w1 = r0; w3 = r1; }
-      }
-      // Round 3, lanes l8 ^ 1: odd elements of the even lane for even
-      // elements of the odd lane, two per exchanged word.
-      {
-        const bool hi = l8 & 1;
-        const uint32_t s0 = hi ? __byte_perm(w0, w1, 0x5410) : __byte_perm(w0, w1, 0x7632);
-        const uint32_t s1 = hi ? __byte_perm(w2, w3, 0x5410) : __byte_perm(w2, w3, 0x7632);
-        const uint32_t r0 = __shfl_xor_sync(0xffffffffu, s0, 1);
-        const uint32_t r1 = __shfl_xor_sync(0xffffffffu, s1, 1);
-        if (hi) {
-          w0 = __byte_perm(r0, w0, 0x7610); w1 = __byte_perm(r0, w1, 0x7632);
-          w2 = __byte_perm(r1, w2, 0x7610); w3 = __byte_perm(r1, w3, 0x7632);
-        } else {
-          w0 = __byte_perm(w0, r0, 0x5410); w1 = __byte_perm(w1, r0, 0x7610);
-          w2 = __byte_perm(w2, r1, 0x5410); w3 = __byte_perm(w3, r1, 0x7610);
-        }
-      }
-      *reinterpret_cast<uint4*>(dst + coreOffset(static_cast<uint32_t>(r + l8), static_cast<uint32_t>(kg * 8),
-                                                 kGemmChunk)) = make_uint4(w0, w1, w2, w3);
-    }
+// 16 bytes to shared memory, zeros unless `valid`.
+__device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(valid ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void copyCommit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int kPending>
+__device__ __forceinline__ void copyWait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(kPending) : "memory");
+}
+
+// The image of `rows` rows (the first `valid` from `src`, row-major with
+// `in` columns, the others zero): core matrices in order, so piece e of 16
+// bytes lies at 16 e.
+__device__ __forceinline__ void copyImage(uint32_t dst, const __nv_bfloat16* __restrict__ src, int in, int rows,
+                                          int valid) {
+  for (int e = threadIdx.x; e < rows * in / 8; e += kStepThreads) {
+    const int g = (e >> 3) / (in / 8), c = (e >> 3) - g * (in / 8), n = g * 8 + (e & 7);
+    copy16(dst + 16u * static_cast<uint32_t>(e), src + static_cast<size_t>(n < valid ? n : 0) * in + 8 * c, n < valid);
   }
 }
 
-template <int kMode>
-__global__ void __launch_bounds__(kGemmThreads, 1)
-    gemmTcKernel(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda, bool aTrans,
-                 const __nv_bfloat16* __restrict__ B, int ldb, bool bTrans, float* __restrict__ Cf,
-                 __nv_bfloat16* __restrict__ Hb, int ldc, const float* __restrict__ bias,
-                 const __nv_bfloat16* __restrict__ mask, int kSlice) {
-  extern __shared__ __align__(128) unsigned char gemmSmem[];
-  unsigned char* stage =
-      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(gemmSmem) + 127) & ~uintptr_t(127));
+__global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a) {
+  extern __shared__ __align__(128) unsigned char stepSmem[];
+  unsigned char* sm =
+      reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(stepSmem) + 127) & ~uintptr_t(127));
   __shared__ uint64_t bar;
   __shared__ uint32_t tmemSlot;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * kGemmTile, n0 = blockIdx.x * kGemmTile;
-  const int Mt = min(kGemmTile, M - m0);
-  const int Nt = min(kGemmTile, N - n0);
-  const uint32_t Nn = static_cast<uint32_t>((Nt + 15) & ~15);  // MMA N: a multiple of 16
-  const int kBeg = kSlice ? static_cast<int>(blockIdx.z) * kSlice : 0;
-  const int kEnd = kSlice ? min(K, kBeg + kSlice) : K;
-  if (kSlice) Cf += static_cast<size_t>(blockIdx.z) * M * N;
-  unsigned char* sA = stage;
-  unsigned char* sB = stage + kGemmStage;
+  const int lq = warp & 3, cq = warp >> 2;
+  const int m = lq * 32 + lane;                           // accumulator lane: tile row, or row of a weight gradient
+  const uint32_t c0 = 32u * static_cast<uint32_t>(cq);    // first of this thread's 32 columns
+  const int row0 = (a.firstTile + static_cast<int>(blockIdx.x)) * kTcRows;
+  const bool valid = row0 + m < a.rows;
+  float* part = a.part + static_cast<size_t>(blockIdx.x) * a.stride;
+  const uint32_t base = smemAddr(sm);
   const uint32_t mbar = smemAddr(&bar);
   if (tid == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(mbar) : "memory");
+    mbarInit(mbar, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smemAddr(&tmemSlot)),
-                 "r"(kTmemCols)
+                 "r"(kStepTmemCols)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  tcFenceBefore();
-  __syncthreads();
-  tcFenceAfter();
-  const uint32_t tmem = tmemSlot;
-  uint32_t phase = 0;
-  bool ok = true, pending = false;
-  for (int k0 = kBeg; k0 < kEnd && ok; k0 += kGemmChunk) {
-    // a(m, k): K contiguous unless aTrans; b(n, k): K contiguous when bTrans.
-    stageOperand(sA, A, lda, !aTrans, m0, Mt, kGemmTile, k0, kEnd, tid);
-    stageOperand(sB, B, ldb, bTrans, n0, Nt, static_cast<int>(Nn), k0, kEnd, tid);
+  // Copies in the order of use: rows and W1, W2, W3 with W4.
+  const uint32_t* order = a.order ? a.order + (a.offset ? *a.offset : 0u) : nullptr;
+  for (int e = tid; e < kTcRows * kFeatureWidth / 8; e += kStepThreads) {
+    const int g = (e >> 3) / (kFeatureWidth / 8), c = (e >> 3) - g * (kFeatureWidth / 8), r = row0 + g * 8 + (e & 7);
+    const bool in = r < a.rows;
+    const size_t src = in ? (order ? __ldg(order + r) : static_cast<uint32_t>(r)) : 0u;
+    copy16(base + kOffStepX + 16u * static_cast<uint32_t>(e), a.X + src * kFeatureWidth + 8 * c, in);
+  }
+  copyImage(base + kOffStepW1, a.wT + a.w.off[0], kFeatureWidth, kMlpHidden, kMlpHidden);
+  copyCommit();
+  copyImage(base + kOffStepW2, a.wT + a.w.off[1], kMlpHidden, kMlpHidden, kMlpHidden);
+  copyCommit();
+  copyImage(base + kOffStepW3, a.wT + a.w.off[2], kMlpHidden, kMlpHidden, kMlpHidden);
+  copyImage(base + kOffStepW4, a.wT + a.w.off[3], kMlpHidden, static_cast<int>(kW4Rows), kMlpOut);
+  copyCommit();
+  float* bias = reinterpret_cast<float*>(sm + kOffStepBias);
+  if (tid < 3 * kMlpHidden) bias[tid] = a.params[a.b[tid / kMlpHidden] + tid % kMlpHidden];
+  else if (tid < 3 * kMlpHidden + kMlpOut) bias[tid] = a.params[a.b[3] + tid - 3 * kMlpHidden];
+  float own[3] = {0.f, 0.f, 0.f}, want[3] = {0.f, 0.f, 0.f};
+  if (cq == 0 && valid) {
+    const size_t src = order ? __ldg(order + row0 + m) : static_cast<uint32_t>(row0 + m);
+    for (int c = 0; c < 3; ++c) {
+      own[c] = a.base[3 * src + c];
+      want[c] = a.target[3 * src + c];
+    }
+  }
+  bool ok = true;
+  uint32_t phase = 0, commits = 0;
+  uint32_t tmem = 0;
+  // Everything written to shared memory before this is an operand after it,
+  // and every accumulator read before it may be overwritten.
+  auto meet = [&]() {
     fenceAsyncShared();
     tcFenceBefore();
-    __syncthreads();
+    ok = __syncthreads_and(ok);
     tcFenceAfter();
-    if (tid == 0) {
-      const uint32_t idesc = instrDesc(kGemmTile, Nn);
-      for (uint32_t ks = 0; ks < kGemmChunk / 16; ++ks) {
-        const uint64_t a = smemDesc(smemAddr(sA) + ks * 256u, 128u, kGemmChunk * 16u);
-        const uint64_t b = smemDesc(smemAddr(sB) + ks * 256u, 128u, kGemmChunk * 16u);
-        mmaBf16(tmem, a, b, idesc, (k0 > kBeg || ks > 0) ? 1u : 0u);
-      }
-      commitTo(mbar);
-    }
-    pending = true;
-    if (!__syncthreads_and(waitParity(mbar, phase))) {
-      ok = false;
-      if (tid == 0) atomicOr(&g_tcGemmErr, kErrMmaTimeout);
-      break;
-    }
-    pending = false;
+  };
+  auto commit = [&]() {
+    commitTo(mbar);
+    ++commits;
+  };
+  auto await = [&]() {
+    if (ok) ok = __all_sync(0xffffffffu, waitParity(mbar, phase));
     phase ^= 1u;
     tcFenceAfter();
-  }
-  if (ok) {
-    // Each warp turns its 32 rows x 32 columns through shared memory (the
-    // staging area is free once the MMAs are done), so that a store writes
-    // 32 consecutive columns of one row.
-    const int lq = warp & 3, half = warp >> 2;  // lane quarter, and columns 64 half .. +63
-    const uint32_t laneBase = tmem + (static_cast<uint32_t>(lq * 32) << 16);
-    const bool empty = kEnd <= kBeg;  // no chunk ran: the accumulator holds nothing
-    float* t = reinterpret_cast<float*>(stage) + warp * (32 * 33);
-    // kMode 2: the warp's 32 x 32 block of the mask, read in 16-byte pieces
-    // while the accumulators load, then turned through shared memory too.
-    __nv_bfloat16* mt = reinterpret_cast<__nv_bfloat16*>(stage + kGemmMaskOff) + warp * (32 * kGemmMaskLd);
-    const bool maskVec = kMode == 2 && (reinterpret_cast<uintptr_t>(mask) & 15) == 0 && (ldc & 7) == 0;
-    for (int c0 = 64 * half; c0 < min(Nt, 64 * half + 64); c0 += 32) {
-      uint4 mq[4];
-      if (kMode == 2) {
+  };
+  const uint32_t laneBits = static_cast<uint32_t>(lq * 32) << 16;
+  uint32_t mask[3];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const int m = m0 + lq * 32 + (lane >> 2) + 8 * i, cc = c0 + (lane & 3) * 8;
-          mq[i] = make_uint4(0u, 0u, 0u, 0u);
-          if (m < M) {
-            const __nv_bfloat16* src = mask + static_cast<size_t>(m) * ldc + n0 + cc;
-            if (maskVec && cc + 8 <= Nt) {
-              mq[i] = __ldg(reinterpret_cast<const uint4*>(src));
-            } else {
-              uint16_t e[8];
-              for (int j = 0; j < 8; ++j) e[j] = cc + j < Nt ? __bfloat16_as_ushort(src[j]) : 0;
-              mq[i] = make_uint4(e[0] | (uint32_t(e[1]) << 16), e[2] | (uint32_t(e[3]) << 16),
-                                 e[4] | (uint32_t(e[5]) << 16), e[6] | (uint32_t(e[7]) << 16));
-            }
-          }
-        }
-      }
+  for (int l = 0; l < 3; ++l) {
+    if (l == 0) copyWait<2>();
+    else if (l == 1) copyWait<1>();
+    else copyWait<0>();
+    meet();
+    if (l == 0) tmem = tmemSlot;
+    const uint32_t in = base + (l == 0 ? kOffStepX : kOffStepH + static_cast<uint32_t>(l - 1) * kActBytes);
+    const uint32_t out = base + kOffStepH + static_cast<uint32_t>(l) * kActBytes;
+    if (ok && tid == 0) {
+      const uint32_t w = base + (l == 0 ? kOffStepW1 : (l == 1 ? kOffStepW2 : kOffStepW3));
+      const uint32_t group = l == 0 ? kStepXGroup : kStepGroup;
+      for (uint32_t ks = 0; ks < (l == 0 ? kFeatureWidth : kMlpHidden) / 16; ++ks)
+        mmaBf16(tmem, smemDesc(in + ks * 256u, 128u, group), smemDesc(w + ks * 256u, 128u, group),
+                instrDesc(kTcRows, kMlpHidden), ks > 0 ? 1u : 0u);
+      commit();
+    }
+    await();
+    mask[l] = 0u;
+    if (ok) {
       float v[32];
-      if (!empty) tmemLoad32(laneBase + static_cast<uint32_t>(c0), v);
-      else
-        for (int j = 0; j < 32; ++j) v[j] = 0.f;
+      tmemLoad32(tmem + laneBits + c0, v);
+      const float* bl = bias + l * kMlpHidden + c0;
 #pragma unroll
-      for (int j = 0; j < 32; ++j) t[lane * 33 + j] = v[j];  // row `lane`, column j
-      if (kMode == 2) {
+      for (uint32_t j = 0; j < 4; ++j) {
+        uint32_t q[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          *reinterpret_cast<uint4*>(mt + ((lane >> 2) + 8 * i) * kGemmMaskLd + (lane & 3) * 8) = mq[i];
-      }
-      __syncwarp();
-      const int n = n0 + c0 + lane;
-      const bool colOk = c0 + lane < Nt;
-      const float bn = (kMode == 1 || kMode == 3) && colOk ? bias[n] : 0.f;
-#pragma unroll
-      for (int r = 0; r < 32; ++r) {
-        const int m = m0 + lq * 32 + r;
-        if (m >= M || !colOk) continue;
-        const size_t o = static_cast<size_t>(m) * ldc + n;
-        const float acc = t[r * 33 + lane];
-        if (kMode == 0) {
-          Cf[o] = acc;
-        } else if (kMode == 1) {
-          const float z = acc + bn;
-          Cf[o] = z;
-          Hb[o] = __float2bfloat16(fmaxf(z, 0.f));
-        } else if (kMode == 2) {
-          Hb[o] = __float2bfloat16(__bfloat162float(mt[r * kGemmMaskLd + lane]) > 0.f ? acc : 0.f);
-        } else {
-          Cf[o] = acc + bn;
+        for (int k = 0; k < 4; ++k) {
+          const int i = 8 * j + 2 * k;
+          const uint32_t h = packBf16(fmaxf(v[i] + bl[i], 0.f), fmaxf(v[i + 1] + bl[i + 1], 0.f));
+          q[k] = valid ? h : 0u;
+          if (q[k] & 0x7fffu) mask[l] |= 1u << i;
+          if (q[k] & 0x7fff0000u) mask[l] |= 2u << i;
         }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                         out + coreOffset(static_cast<uint32_t>(m), c0 + 8 * j, kMlpHidden)),
+                     "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3])
+                     : "memory");
       }
-      __syncwarp();
     }
   }
-  if (!ok && pending && tid == 0) waitParity(mbar, phase);  // let a late commit land before the TMEM is freed
+  // Output layer and the gradient of the mean squared error.
+  meet();
+  const uint32_t h3 = base + kOffStepH + 2 * kActBytes, dy = base + kOffStepDy;
+  if (ok && tid == 0) {
+    for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)
+      mmaBf16(tmem, smemDesc(h3 + ks * 256u, 128u, kStepGroup), smemDesc(base + kOffStepW4 + ks * 256u, 128u, kStepGroup),
+              instrDesc(kTcRows, kW4Rows), ks > 0 ? 1u : 0u);
+    commit();
+  }
+  await();
+  float* dyf = bias;  // [3][128], over the hidden layers' biases, which nothing reads any more
+  if (ok && cq == 0) {
+    float v[4];
+    tmemLoad4(tmem + laneBits, v);
+    const float scale = 2.0f / (3.0f * static_cast<float>(a.rows));
+    float e2 = 0.f, g[3];
+    for (int c = 0; c < 3; ++c) {
+      const float y = v[c] + bias[3 * kMlpHidden + c];
+      const float d = own[c] + y - want[c];
+      if (valid) e2 += d * d;
+      g[c] = valid ? scale * d : 0.f;
+      dyf[c * kTcRows + m] = g[c];
+    }
+    const uint32_t at = dy + coreOffset(static_cast<uint32_t>(m), 0, 16);
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %3};" ::"r"(at), "r"(packBf16(g[0], g[1])),
+                 "r"(packBf16(g[2], 0.f)), "r"(0u)
+                 : "memory");
+    asm volatile("st.shared.v4.b32 [%0], {%1, %1, %1, %1};" ::"r"(at + 128u), "r"(0u) : "memory");
+    if (a.lossSum) {
+      for (int s = 16; s >= 1; s >>= 1) e2 += __shfl_xor_sync(0xffffffffu, e2, s);
+      if (lane == 0) atomicAdd(a.lossSum + (a.lossIndex ? *a.lossIndex : 0), e2);
+    }
+  }
+  meet();
+  if (ok && tid == 0) {
+    for (uint32_t ks = 0; ks < kTcRows / 16; ++ks)  // dW4 = h3^T dy
+      mmaBf16(tmem + 128u, smemDesc(h3 + ks * 2 * kStepGroup, kStepGroup, 128u), smemDesc(dy + ks * 512u, 256u, 128u),
+              instrDesc(kMlpHidden, kW4Rows) | kAMnMajor | kBMnMajor, ks > 0 ? 1u : 0u);
+    // dZ3 = dy W4^T, K = 16
+    mmaBf16(tmem, smemDesc(dy, 128u, 256u), smemDesc(base + kOffStepW4, kStepGroup, 128u),
+            instrDesc(kTcRows, kMlpHidden) | kBMnMajor, 0u);
+    commit();
+  }
+  if (ok && warp == 0) {
+    // db4, in colSum's order: lane 8 c + w sums rows w, w + 16, .. and w + 8,
+    // w + 24, .., then the eight sums in order.
+    const int c = lane >> 3, w = lane & 7;
+    float s0 = 0.f, s1 = 0.f;
+    if (c < 3)
+      for (int r = w; r < kTcRows; r += 16) {
+        s0 += dyf[c * kTcRows + r];
+        s1 += dyf[c * kTcRows + r + 8];
+      }
+    const float s = s0 + s1;
+    float t = 0.f;
+    for (int k = 0; k < 8; ++k) t += __shfl_sync(0xffffffffu, s, (lane & 24) + k);
+    t = __shfl_sync(0xffffffffu, t, (lane & 3) * 8);
+    if (lane < kMlpOut) part[a.b[3] + lane] = lane < 3 ? t : 0.f;
+  }
+  // Columns c0 .. +31 of a weight gradient's row m, from TMEM column `at`:
+  // float4 of four columns by row, so that a warp writes 512 bytes in a row.
+  auto drain = [&](uint32_t at, int w, int in) {
+    float v[32];
+    tmemLoad32(tmem + at + laneBits + c0, v);
+    if (m < in) {
+      float4* dst = reinterpret_cast<float4*>(part + w) + static_cast<size_t>(c0 / 4) * in + m;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dst[static_cast<size_t>(j) * in] = make_float4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+    }
+  };
+#pragma unroll
+  for (int l = 2; l >= 0; --l) {
+    const uint32_t dz = base + kOffStepH + static_cast<uint32_t>(l) * kActBytes;
+    await();
+    if (ok) {
+      float v[32];
+      tmemLoad32(tmem + laneBits + c0, v);
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j) {
+        uint32_t q[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const int i = 8 * j + 2 * k;
+          q[k] = packBf16(mask[l] & (1u << i) ? v[i] : 0.f, mask[l] & (2u << i) ? v[i + 1] : 0.f);
+        }
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(
+                         dz + coreOffset(static_cast<uint32_t>(m), c0 + 8 * j, kMlpHidden)),
+                     "r"(q[0]), "r"(q[1]), "r"(q[2]), "r"(q[3])
+                     : "memory");
+      }
+    }
+    meet();
+    if (ok && tid == 0) {
+      const uint32_t in = base + (l == 0 ? kOffStepX : kOffStepH + static_cast<uint32_t>(l - 1) * kActBytes);
+      const uint32_t group = l == 0 ? kStepXGroup : kStepGroup;
+      const uint32_t acc = tmem + (l == 2 ? 256u : (l == 1 ? 384u : 128u));
+      // dW = in^T dz.  For l = 0 accumulator rows 112-127 hold nothing: the
+      // 16 columns past a feature row are the next row group's first.
+      if (l > 0) {
+        const uint32_t w = base + (l == 1 ? kOffStepW2 : kOffStepW3);
+        for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)  // dZ of the layer before: dz W^T
+          mmaBf16(tmem, smemDesc(dz + ks * 256u, 128u, kStepGroup), smemDesc(w + ks * 2 * kStepGroup, kStepGroup, 128u),
+                  instrDesc(kTcRows, kMlpHidden) | kBMnMajor, ks > 0 ? 1u : 0u);
+      }
+      for (uint32_t ks = 0; ks < kTcRows / 16; ++ks)
+        mmaBf16(acc, smemDesc(in + ks * 2 * group, group, 128u), smemDesc(dz + ks * 2 * kStepGroup, kStepGroup, 128u),
+                instrDesc(kMlpHidden, kMlpHidden) | kAMnMajor | kBMnMajor, ks > 0 ? 1u : 0u);
+      commit();
+    }
+    if (ok) {
+      if (warp < 8) {
+        // Bias gradient, in colSum's order: lane = 16 cg + 8 odd + w of warp
+        // k sums rows w + 8 i, i odd or even, of the 8 columns of core column
+        // 2 k + cg; then s0 + s1, and a column's eight sums in order.
+        const int w = lane & 7, odd = (lane >> 3) & 1, cg = 2 * warp + (lane >> 4);
+        float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const uint4 q = *reinterpret_cast<const uint4*>(sm + (dz - base) + (2 * i + odd) * kStepGroup + cg * 128 + w * 16);
+          const uint32_t x[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            s[2 * k] += __uint_as_float(x[k] << 16);
+            s[2 * k + 1] += __uint_as_float(x[k] & 0xffff0000u);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s[k] += __shfl_xor_sync(0xffffffffu, s[k], 8);
+        float mine = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          float t = 0.f;
+#pragma unroll
+          for (int r = 0; r < 8; ++r) t += __shfl_sync(0xffffffffu, s[k], (lane & 24) + r);
+          if (w == k) mine = t;
+        }
+        if (!odd) part[a.b[l] + cg * 8 + w] = mine;
+      }
+      if (l == 2) {
+        if (cq == 0) {
+          for (uint32_t k = 0; k < kMlpOut / 4; ++k) {
+            float v[4];
+            tmemLoad4(tmem + 128u + laneBits + 4 * k, v);
+            reinterpret_cast<float4*>(part + a.w.off[3])[k * kMlpHidden + m] = make_float4(v[0], v[1], v[2], v[3]);
+          }
+        }
+      } else if (l == 1) {
+        drain(256u, a.w.off[2], kMlpHidden);
+      } else {
+        drain(384u, a.w.off[1], kMlpHidden);
+      }
+    }
+  }
+  await();
+  if (ok) drain(128u, a.w.off[0], kFeatureWidth);
+  if (!ok && lane == 0) atomicOr(&g_tcGemmErr, kErrMmaTimeout);
+  if (!ok && tid == 0 && commits > 0) waitParity(mbar, (commits - 1) & 1u);  // let a late commit land before the TMEM is freed
   tcFenceBefore();
   __syncthreads();
   tcFenceAfter();
   if (warp == 0)
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmemSlot), "r"(kStepTmemCols) : "memory");
 }
-
-__global__ void tcSplitReduceKernel(const float* __restrict__ part, int slices, int M, int N, float* __restrict__ C,
-                                    int ldc) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= M * N) return;
-  const int m = i / N, n = i % N;
-  float s = 0.f;
-  for (int k = 0; k < slices; ++k) s += part[static_cast<size_t>(k) * M * N + i];
-  C[static_cast<size_t>(m) * ldc + n] = s;
-}
-
-float* g_tcSplit = nullptr;
-size_t g_tcSplitFloats = 0;
 
 }  // namespace
 
-cudaError_t gemmBf16Tc(int mode, int M, int N, int K, const void* A, int lda, bool aTrans, const void* B, int ldb,
-                       bool bTrans, float* Cf, void* Hb, int ldc, const float* bias, const void* mask,
-                       cudaStream_t stream) {
-  if (M <= 0 || N <= 0) return cudaSuccess;
-  if (mode < 0 || mode > 3) return cudaErrorInvalidValue;
-  const unsigned gx = static_cast<unsigned>((N + kGemmTile - 1) / kGemmTile);
-  const unsigned gy = static_cast<unsigned>((M + kGemmTile - 1) / kGemmTile);
-  auto a = static_cast<const __nv_bfloat16*>(A);
-  auto b = static_cast<const __nv_bfloat16*>(B);
-  auto h = static_cast<__nv_bfloat16*>(Hb);
-  auto mk = static_cast<const __nv_bfloat16*>(mask);
-  // Weight gradients: a long K over the minibatch and one or two output
-  // tiles; K is split into slices of 128 summed afterwards in slice order.
+cudaError_t trainTiles(const TrainTiles& a, int tiles, cudaStream_t stream) {
+  if (tiles <= 0) return cudaSuccess;
   static bool attrSet = false;
   if (!attrSet) {
-    const void* fns[4] = {reinterpret_cast<const void*>(gemmTcKernel<0>), reinterpret_cast<const void*>(gemmTcKernel<1>),
-                          reinterpret_cast<const void*>(gemmTcKernel<2>), reinterpret_cast<const void*>(gemmTcKernel<3>)};
-    for (const void* f : fns) {
-      const cudaError_t e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kGemmSmem);
-      if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = cudaFuncSetAttribute(trainTileKernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                               static_cast<int>(kStepSmem));
+    if (e != cudaSuccess) return e;
     attrSet = true;
   }
-  if (mode == 0 && K >= 1024 && gx * gy < 64) {
-    const int slice = 128, slices = (K + slice - 1) / slice;
-    const size_t need = static_cast<size_t>(slices) * M * N;
-    if (need > g_tcSplitFloats) {
-      if (g_tcSplit) cudaFree(g_tcSplit);
-      g_tcSplit = nullptr;
-      g_tcSplitFloats = 0;
-      const cudaError_t e = cudaMalloc(&g_tcSplit, need * sizeof(float));
-      if (e != cudaSuccess) return e;
-      g_tcSplitFloats = need;
-    }
-    gemmTcKernel<0><<<dim3(gx, gy, slices), kGemmThreads, kGemmSmem, stream>>>(M, N, K, a, lda, aTrans, b, ldb, bTrans,
-                                                                       g_tcSplit, nullptr, N, nullptr, nullptr, slice);
-    tcSplitReduceKernel<<<(M * N + 255) / 256, 256, 0, stream>>>(g_tcSplit, slices, M, N, Cf, ldc);
-    return cudaGetLastError();
-  }
-  const dim3 grid(gx, gy);
-  switch (mode) {
-    case 0: gemmTcKernel<0><<<grid, kGemmThreads, kGemmSmem, stream>>>(M, N, K, a, lda, aTrans, b, ldb, bTrans, Cf, h, ldc, bias, mk, 0); break;
-    case 1: gemmTcKernel<1><<<grid, kGemmThreads, kGemmSmem, stream>>>(M, N, K, a, lda, aTrans, b, ldb, bTrans, Cf, h, ldc, bias, mk, 0); break;
-    case 2: gemmTcKernel<2><<<grid, kGemmThreads, kGemmSmem, stream>>>(M, N, K, a, lda, aTrans, b, ldb, bTrans, Cf, h, ldc, bias, mk, 0); break;
-    default: gemmTcKernel<3><<<grid, kGemmThreads, kGemmSmem, stream>>>(M, N, K, a, lda, aTrans, b, ldb, bTrans, Cf, h, ldc, bias, mk, 0); break;
-  }
+  trainTileKernel<<<static_cast<unsigned>(tiles), kStepThreads, kStepSmem, stream>>>(a);
   return cudaGetLastError();
 }
 
