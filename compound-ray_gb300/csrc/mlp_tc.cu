@@ -85,12 +85,29 @@ __device__ __forceinline__ uint32_t smemAddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ void mmaBf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+// One lane of a converged warp.  MMAs are issued by a whole warp with this as
+// their predicate: behind a branch on the thread's index the compiler has to
+// move every descriptor to a uniform register in a loop over the lanes, and a
+// 128 x 128 x 16 MMA took 118 clocks to issue; like this it takes the 64 that
+// the MMA itself needs.
+__device__ __forceinline__ uint32_t electLane() {
+  uint32_t e;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(e));
+  return e;
+}
+
+__device__ __forceinline__ void mmaBf16(uint32_t elected, uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc,
+                                        uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
-      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(tmem),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected));
 }
 
 __device__ __forceinline__ void commitTo(uint32_t mbar) {
@@ -449,6 +466,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int m = lq * 32 + (tid & 31);                                 // accumulator lane = tile row
     const uint32_t laneBase = tmem + (static_cast<uint32_t>(lq * 32) << 16);
     const bool issuer = tid == kFeatThreads + g * kNetThreads;
+    const bool issuing = __shfl_sync(0xffffffffu, warp, 0) == (kFeatThreads + g * kNetThreads) / 32;  // the issuer's warp
     const uint32_t mmaBar = bar0 + 8u * static_cast<uint32_t>(2 * kTcBuffers + g);
     const uint32_t biasAddr = smemAddr(bias);
     uint32_t phase = 0;
@@ -461,18 +479,20 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       for (int layer = 0; layer < 4; ++layer) {
         const uint32_t K = layer == 0 ? kFeatureWidth : kMlpHidden;
         const uint32_t Nn = layer == 3 ? kW4Rows : kMlpHidden;
-        if (issuer && (layer > 0 || waitParity(fullBar(b), round & 1u))) {
+        if (issuing && (layer > 0 || __all_sync(0xffffffffu, waitParity(fullBar(b), round & 1u)))) {
           tcFenceAfter();
+          const uint32_t elected = electLane();
           const uint32_t idesc = instrDesc(kTcRows, Nn);
           const uint32_t wOff = layer == 0 ? kOffW1 : (layer == 1 ? kOffW2 : (layer == 2 ? kOffW3 : kOffW4));
           const uint32_t sW = smemAddr(sm) + wOff;
-          for (uint32_t ks = 0; ks < K / 16; ++ks) {
-            const uint64_t a = smemDesc(h + ks * 256u, 128u, K * 16u);
-            const uint64_t bd = smemDesc(sW + ks * 256u, 128u, K * 16u);
-            mmaBf16(tmem, a, bd, idesc, ks > 0 ? 1u : 0u);
+          const uint64_t a = smemDesc(h, 128u, K * 16u), bd = smemDesc(sW, 128u, K * 16u);
+#pragma unroll
+          for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)  // 16 in the descriptors' address: 256 bytes
+            if (ks < K / 16) mmaBf16(elected, tmem, a + 16u * ks, bd + 16u * ks, idesc, ks > 0 ? 1u : 0u);
+          if (elected) {
+            if (layer == 3) commitTo(emptyBar(b));  // the tile buffer is free once these MMAs are done
+            commitTo(mmaBar);
           }
-          if (layer == 3) commitTo(emptyBar(b));  // the tile buffer is free once these MMAs are done
-          commitTo(mmaBar);
           pending = true;
         }
         // A wait that times out (also when the issuer had nothing to issue)
@@ -701,8 +721,9 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
     ok = __syncthreads_and(ok);
     tcFenceAfter();
   };
-  auto commit = [&]() {
-    commitTo(mbar);
+  const bool issuing = __shfl_sync(0xffffffffu, warp, 0) == 0;
+  auto commit = [&](uint32_t elected) {
+    if (elected) commitTo(mbar);
     ++commits;
   };
   auto await = [&]() {
@@ -721,13 +742,15 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
     if (l == 0) tmem = tmemSlot;
     const uint32_t in = base + (l == 0 ? kOffStepX : kOffStepH + static_cast<uint32_t>(l - 1) * kActBytes);
     const uint32_t out = base + kOffStepH + static_cast<uint32_t>(l) * kActBytes;
-    if (ok && tid == 0) {
+    if (ok && issuing) {
+      const uint32_t elected = electLane();
       const uint32_t w = base + (l == 0 ? kOffStepW1 : (l == 1 ? kOffStepW2 : kOffStepW3));
       const uint32_t group = l == 0 ? kStepXGroup : kStepGroup;
+#pragma unroll
       for (uint32_t ks = 0; ks < (l == 0 ? kFeatureWidth : kMlpHidden) / 16; ++ks)
-        mmaBf16(tmem, smemDesc(in + ks * 256u, 128u, group), smemDesc(w + ks * 256u, 128u, group),
+        mmaBf16(elected, tmem, smemDesc(in + ks * 256u, 128u, group), smemDesc(w + ks * 256u, 128u, group),
                 instrDesc(kTcRows, kMlpHidden), ks > 0 ? 1u : 0u);
-      commit();
+      commit(elected);
     }
     await();
     mask[l] = 0u;
@@ -756,11 +779,13 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
   // Output layer and the gradient of the mean squared error.
   meet();
   const uint32_t h3 = base + kOffStepH + 2 * kActBytes, dy = base + kOffStepDy;
-  if (ok && tid == 0) {
+  if (ok && issuing) {
+    const uint32_t elected = electLane();
+#pragma unroll
     for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)
-      mmaBf16(tmem, smemDesc(h3 + ks * 256u, 128u, kStepGroup), smemDesc(base + kOffStepW4 + ks * 256u, 128u, kStepGroup),
+      mmaBf16(elected, tmem, smemDesc(h3 + ks * 256u, 128u, kStepGroup), smemDesc(base + kOffStepW4 + ks * 256u, 128u, kStepGroup),
               instrDesc(kTcRows, kW4Rows), ks > 0 ? 1u : 0u);
-    commit();
+    commit(elected);
   }
   await();
   float* dyf = bias;  // [3][128], over the hidden layers' biases, which nothing reads any more
@@ -787,14 +812,16 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
     }
   }
   meet();
-  if (ok && tid == 0) {
+  if (ok && issuing) {
+    const uint32_t elected = electLane();
+#pragma unroll
     for (uint32_t ks = 0; ks < kTcRows / 16; ++ks)  // dW4 = h3^T dy
-      mmaBf16(tmem + 128u, smemDesc(h3 + ks * 2 * kStepGroup, kStepGroup, 128u), smemDesc(dy + ks * 512u, 256u, 128u),
+      mmaBf16(elected, tmem + 128u, smemDesc(h3 + ks * 2 * kStepGroup, kStepGroup, 128u), smemDesc(dy + ks * 512u, 256u, 128u),
               instrDesc(kMlpHidden, kW4Rows) | kAMnMajor | kBMnMajor, ks > 0 ? 1u : 0u);
     // dZ3 = dy W4^T, K = 16
-    mmaBf16(tmem, smemDesc(dy, 128u, 256u), smemDesc(base + kOffStepW4, kStepGroup, 128u),
+    mmaBf16(elected, tmem, smemDesc(dy, 128u, 256u), smemDesc(base + kOffStepW4, kStepGroup, 128u),
             instrDesc(kTcRows, kMlpHidden) | kBMnMajor, 0u);
-    commit();
+    commit(elected);
   }
   if (ok && warp == 0) {
     // db4, in colSum's order: lane 8 c + w sums rows w, w + 16, .. and w + 8,
@@ -845,7 +872,8 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
       }
     }
     meet();
-    if (ok && tid == 0) {
+    if (ok && issuing) {
+      const uint32_t elected = electLane();
       const uint32_t in = base + (l == 0 ? kOffStepX : kOffStepH + static_cast<uint32_t>(l - 1) * kActBytes);
       const uint32_t group = l == 0 ? kStepXGroup : kStepGroup;
       const uint32_t acc = tmem + (l == 2 ? 256u : (l == 1 ? 384u : 128u));
@@ -853,14 +881,16 @@ __global__ void __launch_bounds__(kStepThreads, 1) trainTileKernel(TrainTiles a)
       // 16 columns past a feature row are the next row group's first.
       if (l > 0) {
         const uint32_t w = base + (l == 1 ? kOffStepW2 : kOffStepW3);
+#pragma unroll
         for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)  // dZ of the layer before: dz W^T
-          mmaBf16(tmem, smemDesc(dz + ks * 256u, 128u, kStepGroup), smemDesc(w + ks * 2 * kStepGroup, kStepGroup, 128u),
+          mmaBf16(elected, tmem, smemDesc(dz + ks * 256u, 128u, kStepGroup), smemDesc(w + ks * 2 * kStepGroup, kStepGroup, 128u),
                   instrDesc(kTcRows, kMlpHidden) | kBMnMajor, ks > 0 ? 1u : 0u);
       }
+#pragma unroll
       for (uint32_t ks = 0; ks < kTcRows / 16; ++ks)
-        mmaBf16(acc, smemDesc(in + ks * 2 * group, group, 128u), smemDesc(dz + ks * 2 * kStepGroup, kStepGroup, 128u),
+        mmaBf16(elected, acc, smemDesc(in + ks * 2 * group, group, 128u), smemDesc(dz + ks * 2 * kStepGroup, kStepGroup, 128u),
                 instrDesc(kMlpHidden, kMlpHidden) | kAMnMajor | kBMnMajor, ks > 0 ? 1u : 0u);
-      commit();
+      commit(elected);
     }
     if (ok) {
       if (warp < 8) {
