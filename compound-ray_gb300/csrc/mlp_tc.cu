@@ -11,28 +11,32 @@
 //     byte offset) and 8-row groups K*16 bytes apart (stride byte offset);
 //   * feature warps 0-15 build the 112 features of each row of a 128-row
 //     tile from statistics derived once per row (deriveKernel: three float4)
-//     and unit axes (axesKernel), into one of three tile buffers, and signal
+//     and unit axes (axesKernel), into one of four tile buffers, and signal
 //     it full on an mbarrier.  A warp holds one quarter of the features of 32
 //     rows, in whole 16-byte pieces (features 0-31, 32-63, 64-87, 88-111), so
 //     every store is a 16-byte row of a core matrix, without bank conflicts;
-//   * two groups of eight network warps (16-23 and 24-31) take the tiles in
-//     turn, each with a 128-column TMEM accumulator of its own: one elected
-//     thread of the group issues each layer's tcgen05.mma instructions (M =
-//     128, N = 128, K = 16 each) and commits them to the group's mbarrier.
-//     Warps q and 4 + q of a group read accumulator lanes 32 q .. +31,
-//     columns 0-63 and 64-127, with tcgen05.ld, add the bias, apply ReLU,
-//     round to bf16 and write the next layer's operand into the same tile
-//     buffer (the MMAs that read it are done);
-//     the last layer (N padded to 16) adds the residual base and writes the
-//     output, and its commit hands the buffer back to the feature warps.
+//   * four groups of four network warps (16-19, .. 28-31) take the tiles in
+//     turn, each with a 128-column TMEM accumulator of its own: one warp of
+//     the group issues each layer's tcgen05.mma instructions (M = 128,
+//     N = 128, K = 16 each) and commits them to the group's mbarrier.  The
+//     hidden layers compute outputs by rows (A the weights, B the tile), so a
+//     thread of warp q reads one output's accumulators for all 128 rows
+//     (tcgen05.ld, lane 32 q ..), adds the bias that it holds in a register,
+//     applies ReLU, rounds to bf16 and writes 16-byte pieces of eight rows
+//     into the same tile buffer (the MMAs that read it are done): the next
+//     layer's MN-major operand.  The last layer (N padded to 16) has the rows
+//     as M again, adds the residual base and writes the output, and its commit
+//     hands the buffer back to the feature warps.
 // A layer is a chain of waits (MMA, accumulator read, barrier) that leaves the
-// SM idle; with two tiles in flight one group's waits are the other's work,
-// and the third buffer lets the feature warps run ahead of both.  1.5 M rows
-// take 451 us with one group, two buffers, two-byte feature stores and a
-// 64-bit division a row, 358 us in this form, and 326 us with the statistics by
-// slot (deriveKernel); without any feature work 285 us: what is left is the
-// network side, whose operand reads, bias loads and activation stores share the
-// shared-memory pipe.
+// SM idle; with four tiles in flight one group's waits are the others' work.
+// 1.5 M rows took 451 us with one group, two buffers, two-byte feature stores
+// and a 64-bit division a row; 358 with two groups of eight warps and three
+// buffers; 326 with the statistics by slot (deriveKernel); 265 with MMAs
+// issued by a converged warp (electLane); 240 with four groups; 218 in this
+// form (rows by outputs read the biases from shared memory, whose pipe the
+// MMAs' operands fill).  Without feature work it is 58 us less, without the
+// hidden layers' epilogue 47, without both 85: the MMAs alone are 80 us at
+// their rate.
 // Every mbarrier wait is bounded: on timeout the waiting side records an error
 // bit and stops; the other side then times out too, the network warps wait
 // (bounded) for their last commit, and the TMEM is freed.
@@ -50,10 +54,11 @@ namespace {
 
 constexpr int kTcRows = 128;
 constexpr int kFeatThreads = 512;  // feature warps 0-15: four threads per row
-constexpr int kNetThreads = 256;   // a network group's warps: two per accumulator lane quarter
-constexpr int kNetGroups = 2;
+constexpr int kNetThreads = 128;   // a network group's warps: one per accumulator lane quarter
+constexpr uint32_t kNetShares = kNetThreads / 128;
+constexpr int kNetGroups = 4;
 constexpr int kTcThreads = kFeatThreads + kNetGroups * kNetThreads;
-constexpr int kTcBuffers = 3;
+constexpr int kTcBuffers = 4;
 constexpr int kTmemCols = 128 * kNetGroups;
 constexpr uint32_t kSpinLimit = 1u << 26;  // bounded waits (far longer than one layer's MMAs)
 
@@ -80,6 +85,9 @@ __device__ __forceinline__ uint64_t smemDesc(uint32_t saddr, uint32_t lbo, uint3
 __host__ __device__ constexpr uint32_t instrDesc(uint32_t M, uint32_t N) {
   return (1u << 4) | (1u << 7) | (1u << 10) | ((N >> 3) << 17) | ((M >> 4) << 24);
 }
+
+// The same with an MN-major operand.
+constexpr uint32_t kAMnMajor = 1u << 15, kBMnMajor = 1u << 16;
 
 __device__ __forceinline__ uint32_t smemAddr(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -292,18 +300,18 @@ __device__ __forceinline__ bool netAll(int g, bool v) {
   return r != 0;
 }
 
-// Two bf16 of max(a + b, 0) of two float pairs: one packed addition, one
-// paired conversion, one packed maximum (a NaN becomes 0, as with fmaxf; the
-// maximum commutes with the rounding).
-__device__ __forceinline__ uint32_t biasReluPack(float a0, float a1, float b0, float b1) {
+// Two bf16 of max(a + b, 0): one packed addition, one paired conversion, one
+// packed maximum (a NaN becomes 0, as with fmaxf; the maximum commutes with
+// the rounding).
+__device__ __forceinline__ uint32_t biasReluPack(float a0, float a1, float b) {
   float s0, s1;
   asm("{\n\t.reg .b64 x, y, z;\n\t"
       "mov.b64 x, {%2, %3};\n\t"
-      "mov.b64 y, {%4, %5};\n\t"
+      "mov.b64 y, {%4, %4};\n\t"
       "add.rn.ftz.f32x2 z, x, y;\n\t"
       "mov.b64 {%0, %1}, z;\n\t}\n"
       : "=f"(s0), "=f"(s1)
-      : "f"(a0), "f"(a1), "f"(b0), "f"(b1));
+      : "f"(a0), "f"(a1), "f"(b));
   uint32_t r;
   asm("max.bf16x2 %0, %1, %2;" : "=r"(r) : "r"(packBf16(s0, s1)), "r"(0u));
   return r;
@@ -462,13 +470,13 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     const int g = (tid - kFeatThreads) / kNetThreads;
     const uint32_t tmem = *tmemSlot + 128u * static_cast<uint32_t>(g);
     const int lq = warp & 3;                                            // TMEM lane quarter this warp may read
-    const int half = ((warp - kFeatThreads / 32) >> 2) & 1;             // columns 64 half .. +63
+    const uint32_t share = static_cast<uint32_t>((warp - kFeatThreads / 32) >> 2) % kNetShares;
+    const uint32_t cBeg = share * (kMlpHidden / kNetShares), cEnd = cBeg + kMlpHidden / kNetShares;  // its columns
     const int m = lq * 32 + (tid & 31);                                 // accumulator lane = tile row
     const uint32_t laneBase = tmem + (static_cast<uint32_t>(lq * 32) << 16);
     const bool issuer = tid == kFeatThreads + g * kNetThreads;
     const bool issuing = __shfl_sync(0xffffffffu, warp, 0) == (kFeatThreads + g * kNetThreads) / 32;  // the issuer's warp
     const uint32_t mmaBar = bar0 + 8u * static_cast<uint32_t>(2 * kTcBuffers + g);
-    const uint32_t biasAddr = smemAddr(bias);
     uint32_t phase = 0;
     bool ok = true, pending = false;  // pending: a commit to mmaBar not yet waited for
     const uint64_t first = blockIdx.x + static_cast<uint64_t>(g) * gridDim.x;
@@ -478,17 +486,21 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       const uint32_t h = smemAddr(sm + kOffB0) + b * kActBytes;
       for (int layer = 0; layer < 4; ++layer) {
         const uint32_t K = layer == 0 ? kFeatureWidth : kMlpHidden;
-        const uint32_t Nn = layer == 3 ? kW4Rows : kMlpHidden;
         if (issuing && (layer > 0 || __all_sync(0xffffffffu, waitParity(fullBar(b), round & 1u)))) {
           tcFenceAfter();
           const uint32_t elected = electLane();
-          const uint32_t idesc = instrDesc(kTcRows, Nn);
+          const uint32_t idesc = layer == 3 ? instrDesc(kTcRows, kW4Rows) | kAMnMajor
+                                            : instrDesc(kMlpHidden, kTcRows) | (layer > 0 ? kBMnMajor : 0u);
           const uint32_t wOff = layer == 0 ? kOffW1 : (layer == 1 ? kOffW2 : (layer == 2 ? kOffW3 : kOffW4));
           const uint32_t sW = smemAddr(sm) + wOff;
-          const uint64_t a = smemDesc(h, 128u, K * 16u), bd = smemDesc(sW, 128u, K * 16u);
+          const uint64_t x = layer == 0 ? smemDesc(h, 128u, K * 16u) : smemDesc(h, kMlpHidden * 16u, 128u);
+          const uint64_t w = smemDesc(sW, 128u, K * 16u);
+          const uint32_t xStep = layer == 0 ? 16u : 2u * kMlpHidden;  // 16 bytes of address: 16 features on
 #pragma unroll
-          for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)  // 16 in the descriptors' address: 256 bytes
-            if (ks < K / 16) mmaBf16(elected, tmem, a + 16u * ks, bd + 16u * ks, idesc, ks > 0 ? 1u : 0u);
+          for (uint32_t ks = 0; ks < kMlpHidden / 16; ++ks)
+            if (ks < K / 16)
+              mmaBf16(elected, tmem, layer == 3 ? x + ks * xStep : w + 16u * ks, layer == 3 ? w + 16u * ks : x + ks * xStep,
+                      idesc, ks > 0 ? 1u : 0u);
           if (elected) {
             if (layer == 3) commitTo(emptyBar(b));  // the tile buffer is free once these MMAs are done
             commitTo(mmaBar);
@@ -503,31 +515,24 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         if (ok) {
           pending = false;
           if (layer < 3) {
-#pragma unroll 1
-            for (uint32_t c0 = 64u * half; c0 < 64u * half + 64u; c0 += 32u) {
+            const float own = bias[layer * kMlpHidden + m];
+#pragma unroll
+            for (uint32_t c0 = cBeg; c0 < cEnd; c0 += 32u) {
               float v[32];
               tmemLoad32(laneBase + c0, v);
-              const uint32_t bs = biasAddr + 4u * (static_cast<uint32_t>(layer) * kMlpHidden + c0);
               const uint32_t hs = h + coreOffset(static_cast<uint32_t>(m), c0, kMlpHidden);
 #pragma unroll
               for (uint32_t j = 0; j < 4; ++j) {
-                float c[8];
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(c[0]), "=f"(c[1]), "=f"(c[2]), "=f"(c[3])
-                             : "r"(bs + 32u * j));
-                asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                             : "=f"(c[4]), "=f"(c[5]), "=f"(c[6]), "=f"(c[7])
-                             : "r"(bs + 32u * j + 16u));
                 uint32_t qs[4];
 #pragma unroll
                 for (int k = 0; k < 4; ++k)
-                  qs[k] = biasReluPack(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], c[2 * k], c[2 * k + 1]);
+                  qs[k] = biasReluPack(v[8 * j + 2 * k], v[8 * j + 2 * k + 1], own);
                 asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(hs + 128u * j), "r"(qs[0]), "r"(qs[1]),
                              "r"(qs[2]), "r"(qs[3])
                              : "memory");
               }
             }
-          } else if (half == 0) {
+          } else if (share == 0) {
             float v[4];
             tmemLoad4(laneBase, v);
             if (row.pos < rows) {
@@ -634,9 +639,6 @@ static_assert(kStepSmem + 64 <= 227 * 1024, "shared memory plan exceeds a block'
 static_assert(kTcRows == kMlpHidden, "the weight gradients' M is a tile image's width");
 constexpr uint32_t kStepTmemCols = 512;
 __device__ uint32_t g_tcGemmErr;
-
-// instrDesc with MN-major operands.
-constexpr uint32_t kAMnMajor = 1u << 15, kBMnMajor = 1u << 16;
 
 // 16 bytes to shared memory, zeros unless `valid`.
 __device__ __forceinline__ void copy16(uint32_t dst, const void* src, bool valid) {
