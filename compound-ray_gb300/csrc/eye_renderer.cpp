@@ -235,6 +235,12 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
 }
 
 constexpr uint32_t kMaxPosesPerLaunch = 256;
+// Small eyes take more poses a launch, up to this many while the launch's rays
+// stay within kSmallLaunchRays (256 MB of pre-drawn numbers): every launch
+// ends on blocks that run alone (1000 poses x 1000 ommatidia x 32 samples of
+// the box scene: 1.25 ms as four launches, 1.07 as two, 0.97 as one).
+constexpr uint32_t kMaxSmallPosesPerLaunch = 1024;
+constexpr uint64_t kSmallLaunchRays = uint64_t(1) << 25;
 constexpr size_t kConeListBytes = size_t(1) << 30;  // cone lists of one launch at most
 constexpr size_t kBatchConeBytes = size_t(4) << 30;  // cone lists of one batch at most
 constexpr size_t kTuneSlots = 20;
@@ -643,7 +649,7 @@ struct Renderer {
   void renderDevicePoses(EyeDev& e, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                          unsigned long long* stats = nullptr) {
     ensureRng(e);
-    const size_t perLaunch = posesPerLaunch(e.N);
+    const size_t perLaunch = launchPoses(e, count, rec != nullptr, stats != nullptr);
     for (size_t first = 0; first < count; first += perLaunch) {
       const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
       DevEye de = devEye(e);
@@ -673,6 +679,30 @@ struct Renderer {
     return std::max<size_t>(1, kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N)));
   }
   static size_t posesPerLaunch(uint32_t N) { return std::min<size_t>(kMaxPosesPerLaunch, conePoses(N)); }
+
+  // The same for a render of `count` poses, more for small eyes when the
+  // memory for it is to be had; not while the stream is being captured (it
+  // may be the first render of so many poses, and would allocate).
+  size_t launchPoses(const EyeDev& e, size_t count, bool rec, bool stats) {
+    const size_t usual = posesPerLaunch(e.N);
+    const uint64_t rays = std::max<uint64_t>(1, static_cast<uint64_t>(e.N) * e.spp);
+    const size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, conePoses(e.N), count});
+    if (most <= usual) return usual;
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
+    if (st != cudaStreamCaptureStatusNone) return usual;
+    const uint32_t P = static_cast<uint32_t>(most);
+    const size_t drawn = rec || stats ? 0 : renderDrawBytes(e.N, e.spp, P) / sizeof(float2);
+    const size_t sums = std::max(renderScratchFloats(dev, e.N, e.spp, P, rec, stats, false, false),
+                                 renderScratchFloats(dev, e.N, e.spp, P, rec, stats, false, true));
+    if ((!drawn || draws.tryEnsure(drawn)) && (!sums || scratch.tryEnsure(sums)) &&
+        (!(cutFactor > 0.f) || cuts.tryEnsure(static_cast<size_t>(P) * kCutStride)))
+      return most;
+    draws.release();
+    scratch.release();
+    cuts.release();
+    return usual;
+  }
 
   // Sets de.cones to a buffer of `lists` cone lists when there are any to
   // build and the memory is to be had; not while the stream is being captured

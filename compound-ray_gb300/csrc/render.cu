@@ -2656,9 +2656,12 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     // With cone lists a task is short: twice the tasks, for a smaller last wave
-    // (1000 poses x 1000 ommatidia x 32 samples of the box scene: 1.28 ms
-    // against 1.37 at the same number, and 1.32 at four times).
-    plan = splitPoses(plan, P, eye.cones ? 2 * kFillWarps : kFillWarps);
+    // (256 poses x 1000 ommatidia x 32 samples of the box scene: 0.32 ms
+    // against 0.34 at the same number, and 0.33 at four times).  A launch of
+    // more than 256 poses keeps the ranges that 256 have (here 8 poses; 1000
+    // poses: 0.97 ms, with ranges of 16 0.98, of 4 1.00).
+    const uint64_t warps = eye.cones ? 2 * kFillWarps : kFillWarps;
+    plan = splitPoses(plan, P, warps * std::max(256u, P) / 256);
   }
   if (eye.cones) {
     const cudaError_t e = launchCones(scene, eye, poses, P, stream);

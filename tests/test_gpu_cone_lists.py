@@ -330,3 +330,32 @@ def test_adaptive_render_with_and_without_lists(lib, deep):
         lib.crSetAllocatorHalvings(0.0)
     assert len(np.unique(res[0][1])) >= 2 and (res[0][1] != 255).mean() > 0.5
     assert np.array_equal(res[0][1], res[1][1]) and np.array_equal(res[0][0], res[1][0])
+
+
+@pytest.mark.parametrize("n,spp,P", [(3, 5, 1025), (40, 32, 700), (701, 8, 513), (33, 513, 257)])
+def test_long_launches_of_small_eyes(lib, small, n, spp, P):
+    """More than 256 poses in one launch, and in launches of 256 when the
+    memory for one is not to be had."""
+    _load(lib, small)
+    poses = _poses(small, P, n)
+    long, usual = _both(lib, _eye(n, "plain"), spp, poses)
+    for x, y in zip(long[:3], usual[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
+    _load(lib, small)
+    omm = _eye(n, "plain")
+    import torch
+
+    d_poses = torch.from_numpy(poses).cuda()
+    for cap in (False, True):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        _render(lib, lib.crRenderPosesDevice, d_poses, 255, n)  # the buffers of a usual launch
+        if cap:
+            assert lib.crSetDeviceMemoryCap(lib.crGetDeviceMemoryHeld() + 8 * 10 * n * spp + 4096) == 0
+        try:
+            got = _render(lib, lib.crRenderPosesDevice, d_poses, P, n)
+        finally:
+            lib.crSetDeviceMemoryCap(0)
+        if not cap:
+            want = got
+    assert np.array_equal(got, want, equal_nan=True)
