@@ -1011,19 +1011,6 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const float4* __res
   out[0] = make_float4(__uint_as_float(count), c.o.x, c.o.y, c.o.z);
 }
 
-// Cone lists of P poses of an eye, list (p, o) at cones + (p * N + o) *
-// kConeStride; threads in the eye's direction order.
-__global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses,
-                                                           uint32_t P) {
-  __shared__ uint2 work[kConeEntries * kConeThreads];
-  const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
-  if (i >= static_cast<uint64_t>(P) * eye.N) return;
-  const uint32_t p = static_cast<uint32_t>(i / eye.N), slot = static_cast<uint32_t>(i - static_cast<uint64_t>(p) * eye.N);
-  const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
-  coneList(sc, eye.omm, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
-           eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
-}
-
 // Copies a warp's list into shared memory asynchronously, one float4 a lane:
 // the list of pose p + 1 arrives while pose p is traced.
 static_assert(kConeStride <= 32, "one float4 of a list for each lane");
@@ -1400,9 +1387,8 @@ __global__ void rngInitKernel(DevEye eye, uint32_t* errFlag) {
 // stream, in the order the render kernel would draw them (one normal, then
 // one uniform per frame), into draws[(p * N + o) * spp + s]; the states
 // advance by P frames, exactly as a render of the P poses would leave them.
-__global__ void drawsKernel(DevEye eye, uint32_t P) {
+__device__ __forceinline__ void drawStream(const DevEye& eye, uint32_t P, size_t idx) {
   const size_t total = static_cast<size_t>(eye.N) * eye.spp;
-  const size_t idx = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (idx >= total) return;
   curandState st;
   loadState(eye.rng, total, idx, st);
@@ -1415,8 +1401,8 @@ __global__ void drawsKernel(DevEye eye, uint32_t P) {
   };
   // Pairs of frames: one Box-Muller transform gives both normals, and drawing
   // the pair without the branch on the cached one lets its arithmetic overlap
-  // the generator's serial chain, which is what bounds this kernel (a thread
-  // per stream).
+  // the generator's serial chain, which is what bounds this (a thread per
+  // stream).
   uint32_t p = 0;
   if (P > 0 && st.boxmuller_flag != 0) {
     one();
@@ -1432,6 +1418,30 @@ __global__ void drawsKernel(DevEye eye, uint32_t P) {
   }
   if (p < P) one();
   storeState(eye.rng, total, idx, st);
+}
+
+__global__ void drawsKernel(DevEye eye, uint32_t P) {
+  drawStream(eye, P, static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x);
+}
+
+// Cone lists of P poses of an eye, list (p, o) at cones + (p * N + o) *
+// kConeStride; threads in the eye's direction order.  The first drawBlocks
+// blocks are drawsKernel's work instead: a few long chains that leave most of
+// the GPU idle when they run alone (1000 poses x 1000 ommatidia x 32 samples:
+// 0.97 ms as a launch of their own, 0.94 here).
+__global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses,
+                                                           uint32_t P, uint32_t drawBlocks) {
+  __shared__ uint2 work[kConeEntries * kConeThreads];
+  if (blockIdx.x < drawBlocks) {
+    drawStream(eye, P, static_cast<size_t>(blockIdx.x) * kConeThreads + threadIdx.x);
+    return;
+  }
+  const uint64_t i = static_cast<uint64_t>(blockIdx.x - drawBlocks) * kConeThreads + threadIdx.x;
+  if (i >= static_cast<uint64_t>(P) * eye.N) return;
+  const uint32_t p = static_cast<uint32_t>(i / eye.N), slot = static_cast<uint32_t>(i - static_cast<uint64_t>(p) * eye.N);
+  const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
+  coneList(sc, eye.omm, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+           eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
 // SplitMix64's output function (Steele, Lea and Flood, "Fast splittable
@@ -2632,11 +2642,16 @@ cudaError_t runRenderWidth(const DevScene& scene, const DevEye& eye, const float
 }
 }  // namespace
 
-static cudaError_t launchCones(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
+// draw: pre-draws the launch's random numbers too.
+static cudaError_t launchCones(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P, bool draw,
                                cudaStream_t stream) {
-  const uint64_t lists = static_cast<uint64_t>(P) * eye.N, blocks = (lists + kConeThreads - 1) / kConeThreads;
+  const uint64_t lists = static_cast<uint64_t>(P) * eye.N;
+  const uint64_t streams = draw ? static_cast<uint64_t>(eye.N) * eye.spp : 0;
+  const uint64_t drawBlocks = (streams + kConeThreads - 1) / kConeThreads;
+  const uint64_t blocks = drawBlocks + (lists + kConeThreads - 1) / kConeThreads;
   if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
-  coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P);
+  coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P,
+                                                                        static_cast<uint32_t>(drawBlocks));
   return cudaGetLastError();
 }
 
@@ -2651,10 +2666,12 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
   if (plan.chunks > 1 && !plan.inBlock && scratch == nullptr) return cudaErrorInvalidValue;
   if (eye.draws) {
     if (plan.inBlock) return cudaErrorInvalidValue;  // planRender keeps splittable launches out of shared memory
-    const size_t total = static_cast<size_t>(eye.N) * eye.spp;
-    drawsKernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(eye, P);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
+    if (!eye.cones) {  // else launchCones draws
+      const size_t total = static_cast<size_t>(eye.N) * eye.spp;
+      drawsKernel<<<static_cast<unsigned>((total + 255) / 256), 256, 0, stream>>>(eye, P);
+      const cudaError_t e = cudaGetLastError();
+      if (e != cudaSuccess) return e;
+    }
     // With cone lists a task is short: twice the tasks, for a smaller last wave
     // (256 poses x 1000 ommatidia x 32 samples of the box scene: 0.32 ms
     // against 0.34 at the same number, and 0.33 at four times).  A launch of
@@ -2664,7 +2681,7 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     plan = splitPoses(plan, P, warps * std::max(256u, P) / 256);
   }
   if (eye.cones) {
-    const cudaError_t e = launchCones(scene, eye, poses, P, stream);
+    const cudaError_t e = launchCones(scene, eye, poses, P, eye.draws != nullptr, stream);
     if (e != cudaSuccess) return e;
   } else if (eye.cuts && (scene.width == 2 || rec || scene.lighting)) {  // the wide BVH searches without a cut
     if (!(eye.cutRadius > 0.f)) return cudaErrorInvalidValue;
@@ -2716,7 +2733,7 @@ cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float
   plan = splitPoses(plan, P, 4 * kFillWarps);
   if (eye.cones) {
     if (featureConeLists(scene, eye.N, eye.spp, P) == 0) return cudaErrorInvalidValue;
-    const cudaError_t e = launchCones(scene, eye, poses, P, stream);
+    const cudaError_t e = launchCones(scene, eye, poses, P, false, stream);
     if (e != cudaSuccess) return e;
     return runRender<3, kConeRegs>(scene, eye, poses, P, plan, stats, nullptr, errFlag, nullptr, nullptr, stream);
   }
