@@ -3404,6 +3404,9 @@ __global__ void labelKernel(const float* __restrict__ outs, int k, uint64_t rows
 __global__ void allocateKernel(const float* __restrict__ pred, uint64_t rows, uint32_t featureSpp,
                                uint8_t* __restrict__ level, unsigned long long* __restrict__ counts, float halvings,
                                float exponent, const float* __restrict__ stats, float costExponent) {
+  __shared__ unsigned int cnt[kAdaptiveBuckets];
+  if (threadIdx.x < kAdaptiveBuckets) cnt[threadIdx.x] = 0u;
+  __syncthreads();
   const uint64_t e = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   int bucket = -1;  // counted bucket of this row (-1: none)
   if (e < rows) {
@@ -3430,10 +3433,16 @@ __global__ void allocateKernel(const float* __restrict__ pred, uint64_t rows, ui
     level[e] = lv;
     if (lv != kNoRender) bucket = lv & 0x7f;
   }
-  // One atomic per bucket and warp (blockDim is a multiple of 32).
+  // One shared atomic per bucket and warp (blockDim is a multiple of 32), one
+  // global per bucket and block: the nine counters are every block's, and with
+  // one global atomic per warp they bound the kernel (1 M entries: 22.7 us,
+  // here 8.5).
   const unsigned peers = __match_any_sync(0xffffffffu, bucket);
   if (bucket >= 0 && (threadIdx.x & 31u) == static_cast<unsigned>(__ffs(peers) - 1))
-    atomicAdd(counts + bucket, static_cast<unsigned long long>(__popc(peers)));
+    atomicAdd(&cnt[bucket], static_cast<unsigned int>(__popc(peers)));
+  __syncthreads();
+  if (threadIdx.x < kAdaptiveBuckets && cnt[threadIdx.x] != 0u)
+    atomicAdd(counts + threadIdx.x, static_cast<unsigned long long>(cnt[threadIdx.x]));
 }
 
 // Ordered bucket lists in three steps, so that every bucket lists its
@@ -3468,22 +3477,30 @@ __global__ void __launch_bounds__(kScatterTile) bucketCountKernel(const uint8_t*
 
 // One warp per bucket: tileCounts[t][k] becomes the first slot of tile t's
 // bucket-k entries (bucket k starting at bucketBase[k]); the warp scans 32
-// tiles per step with shuffles.
+// times kScanTiles tiles per step, kScanTiles loads in flight a lane (a step
+// is a load's latency: 977 tiles took 16 us at one tile a lane, here 11).
+constexpr int kScanTiles = 8;
+
 __global__ void bucketScanKernel(unsigned long long* __restrict__ tileCounts, uint64_t tiles,
                                  const unsigned long long* __restrict__ bucketBase) {
   const int k = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (k >= static_cast<int>(kAdaptiveBuckets)) return;  // whole warps
   unsigned long long run = bucketBase[k];
-  for (uint64_t t0 = 0; t0 < tiles; t0 += 32) {
-    const uint64_t t = t0 + lane;
-    const unsigned long long c = t < tiles ? tileCounts[t * kAdaptiveBuckets + k] : 0ull;
-    unsigned long long inc = c;  // inclusive prefix over the warp's 32 tiles
-    for (int d = 1; d < 32; d <<= 1) {
-      const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, d);
-      if (lane >= d) inc += o;
+  for (uint64_t t0 = lane; t0 < tiles + lane; t0 += 32 * kScanTiles) {
+    unsigned long long c[kScanTiles];
+#pragma unroll
+    for (int j = 0; j < kScanTiles; ++j)
+      c[j] = t0 + 32 * j < tiles ? tileCounts[(t0 + 32 * j) * kAdaptiveBuckets + k] : 0ull;
+#pragma unroll
+    for (int j = 0; j < kScanTiles; ++j) {
+      unsigned long long inc = c[j];  // inclusive prefix over the warp's 32 tiles
+      for (int d = 1; d < 32; d <<= 1) {
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= d) inc += o;
+      }
+      if (t0 + 32 * j < tiles) tileCounts[(t0 + 32 * j) * kAdaptiveBuckets + k] = run + inc - c[j];
+      run += __shfl_sync(0xffffffffu, inc, 31);
     }
-    if (t < tiles) tileCounts[t * kAdaptiveBuckets + k] = run + inc - c;
-    run += __shfl_sync(0xffffffffu, inc, 31);
   }
 }
 
@@ -3786,7 +3803,7 @@ cudaError_t launchAllocate(const float* pred, uint64_t rows, uint32_t featureSpp
                            const float* stats, float costExponent) {
   if (rows == 0) return cudaSuccess;
   if (costExponent != 0.0f && !stats) return cudaErrorInvalidValue;
-  allocateKernel<<<static_cast<unsigned>((rows + 255) / 256), 256, 0, stream>>>(
+  allocateKernel<<<static_cast<unsigned>((rows + 1023) / 1024), 1024, 0, stream>>>(
       pred, rows, featureSpp, level, counts, halvings, exponent, stats, costExponent);
   return cudaGetLastError();
 }
