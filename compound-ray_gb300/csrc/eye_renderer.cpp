@@ -681,13 +681,15 @@ struct Renderer {
   static size_t posesPerLaunch(uint32_t N) { return std::min<size_t>(kMaxPosesPerLaunch, conePoses(N)); }
 
   // The same for a render of `count` poses, more for small eyes when the
-  // memory for it is to be had; not while the stream is being captured (it
-  // may be the first render of so many poses, and would allocate).
+  // memory for it is to be had; not under a memory cap (the larger buffers
+  // stay, and a later render may need that room) and not while the stream is
+  // being captured (it may be the first render of so many poses, and would
+  // allocate).
   size_t launchPoses(const EyeDev& e, size_t count, bool rec, bool stats) {
     const size_t usual = posesPerLaunch(e.N);
     const uint64_t rays = std::max<uint64_t>(1, static_cast<uint64_t>(e.N) * e.spp);
     const size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, conePoses(e.N), count});
-    if (most <= usual) return usual;
+    if (most <= usual || devCap()) return usual;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
     if (st != cudaStreamCaptureStatusNone) return usual;
