@@ -811,7 +811,9 @@ __device__ __forceinline__ v3 rayOrigin(v3 p, v3 x, v3 y, v3 z, v3 rel) {
 // frame or axis that is orthonormal to 1e-3 (others get no list:
 // kConeFromRoot); boxes and edge planes are widened by a few float ulps of
 // (extent + |origin|); distances of entries are stored shortened by 0.5%,
-// which covers |direction| != 1.
+// which covers |direction| != 1.  The cone is the half ahead of its apex, so a
+// negative focal offset, whose rays also hit what lies between the ommatidium
+// and their origin (t in [offset, 0)), gets no list either.
 // ---------------------------------------------------------------------------
 constexpr float kConeSigmas = 3.75f;
 constexpr float kConeMaxAngle = 0.5f;  // wider cones are searched from the root
@@ -915,7 +917,7 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const float4* __res
   const bool ok = fabsf(dot(ax, ax) - 1.0f) <= tol && fabsf(dot(x, x) - 1.0f) <= tol &&
                   fabsf(dot(y, y) - 1.0f) <= tol && fabsf(dot(z, z) - 1.0f) <= tol && fabsf(dot(x, y)) <= tol &&
                   fabsf(dot(x, z)) <= tol && fabsf(dot(y, z)) <= tol && theta <= kConeMaxAngle &&
-                  fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z) < 1e15f && fabsf(fpo) < 1e15f;
+                  fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z) < 1e15f && fpo >= 0.0f && fpo < 1e15f;
   if (!ok) {  // also for NaNs
     out[0] = make_float4(__uint_as_float(kConeFromRoot), c.o.x, c.o.y, c.o.z);
     return;

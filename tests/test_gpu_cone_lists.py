@@ -359,3 +359,22 @@ def test_long_launches_of_small_eyes(lib, small, n, spp, P):
         if not cap:
             want = got
     assert np.array_equal(got, want, equal_nan=True)
+
+
+@pytest.mark.parametrize("on_deep,spp", [(False, 32), (False, 100), (True, 8), (True, 33)])
+def test_negative_focal_offsets(lib, small, deep, on_deep, spp):
+    """Rays of a negative focal offset start ahead of the ommatidium and hit
+    what lies between (the ground and boxes here), in every kind of launch."""
+    info = deep if on_deep else small
+    _load(lib, info)
+    n, rays = 801, 2 ** 20 if on_deep else 2 ** 21
+    P = max(9, rays // (n * spp) + 2)
+    omm = _eye(n, "plain")
+    omm[::10, 7] = -np.linspace(0.3, 3.0, len(omm[::10]), dtype=np.float32)
+    poses = _poses(info, P, spp)
+    with_lists, without = _both(lib, omm, spp, poses)
+    assert with_lists[3] >= 400 * n * P
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
+    omm[::10, 7] = 0.0  # the offsets do decide what is seen
+    assert not np.array_equal(_both(lib, omm, spp, poses)[1][0][:, ::10], without[0][:, ::10], equal_nan=True)
