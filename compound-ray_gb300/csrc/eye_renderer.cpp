@@ -361,6 +361,7 @@ struct Renderer {
     poses.release();
     scratch.release();
     draws.release();
+    cuts.release();
     cones.release();
     batchOut.release();
     err.release();
@@ -649,6 +650,7 @@ struct Renderer {
   void renderDevicePoses(EyeDev& e, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                          unsigned long long* stats = nullptr) {
     ensureRng(e);
+    uint32_t* errFlag = errWord();  // before the lists: an allocation may give them back
     const size_t perLaunch = launchPoses(e, count, rec != nullptr, stats != nullptr);
     for (size_t first = 0; first < count; first += perLaunch) {
       const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
@@ -656,7 +658,7 @@ struct Renderer {
       withDraws(de, P, !rec && !stats);
       withCuts(de, P, e.maxRel);
       float* s = withCones(de, P, scratch, rec != nullptr, stats != nullptr);
-      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * e.N, s, errWord(), rec, stream(), stats),
+      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * e.N, s, errFlag, rec, stream(), stats),
             "render launch");
     }
   }
@@ -732,7 +734,8 @@ struct Renderer {
 
   // Cone lists of `count` entries for adaptive launches of `rays` rays at `spp`
   // (or more) samples each; null when those do not use them or the memory is
-  // not to be had.
+  // not to be had.  Every other buffer of the launch is allocated before: an
+  // allocation may give the lists back.
   const float4* entryCones(const EyeDev& e, const float4* dposes, const uint32_t* entries, uint64_t count, uint32_t spp,
                            uint64_t rays) {
     if (!count || !adaptiveLists(dev, spp, rays) || count * kConeStride * sizeof(float4) > kConeListBytes ||
@@ -2164,13 +2167,14 @@ void denoiseFeatures(Renderer& r, DenoiseState& d, EyeDev& e, const float4* dpos
   r.withCuts(fe, static_cast<uint32_t>(count), e.maxRel);
   // One launch for all poses, or, with cone lists, one for each kConeListBytes
   // of them.
+  uint32_t* err = r.errWord();  // before the lists: an allocation may give them back
   const size_t perLaunch =
       !cost && featureConeLists(r.dev, e.N, featSpp, static_cast<uint32_t>(count)) ? r.conePoses(e.N) : count;
   for (size_t first = 0; first < count; first += perLaunch) {
     const uint32_t P = static_cast<uint32_t>(std::min(perLaunch, count - first));
     r.takeCones(fe, cost ? 0 : featureConeLists(r.dev, e.N, featSpp, P));
-    check(launchFeatures(r.dev, fe, dposes + 4 * first, P, d.stats.ptr + first * e.N * kFeatureStats, r.errWord(),
-                         r.stream(), false),
+    check(launchFeatures(r.dev, fe, dposes + 4 * first, P, d.stats.ptr + first * e.N * kFeatureStats, err, r.stream(),
+                         false),
           "feature render");
     fe.frame0 += P;
   }
@@ -2236,12 +2240,13 @@ int crDenoiserAddTrainingPoses(const float* poses12, size_t count, int featureSp
         denoiseFeatures(r, d, e, d.poses.ptr, count, static_cast<uint32_t>(featureSpp));
         DevEye te = streamsFor(r, e, d.targetRng, d.targetSpp, d.targetReady, static_cast<uint32_t>(targetSpp));
         d.out.ensure(std::max<size_t>(1, count * e.N * 3));
+        uint32_t* err = r.errWord();
         const size_t perLaunch = Renderer::posesPerLaunch(e.N);
         for (size_t first = 0; first < count; first += perLaunch) {
           const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
           float* scr = r.withCones(te, P, d.scratch, false, false);
-          check(launchRender(r.dev, te, d.poses.ptr + 4 * first, P, d.out.ptr + 3 * first * e.N, scr, r.errWord(),
-                             nullptr, r.stream()),
+          check(launchRender(r.dev, te, d.poses.ptr + 4 * first, P, d.out.ptr + 3 * first * e.N, scr, err, nullptr,
+                             r.stream()),
                 "target render");
         }
         d.net.addRows(d.X.ptr, d.base.ptr, d.out.ptr, count * e.N, r.stream());
@@ -2513,21 +2518,23 @@ int crAllocatorAddTrainingPoses(const float* poses12, size_t count, int featureS
         check(cudaMemsetAsync(d.labels.ptr, 0, rows * 2, st), "cudaMemset");
         d.labelOuts.ensure(static_cast<size_t>(seeds) * rows * 3);
         d.partials.ensure(std::max<size_t>(1, adaptivePartialFloats(rows, 1024)));
-        const float4* cones = nullptr;  // the same entries in every launch: their lists are built once
+        DevEye ce;
+        r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
+        uint32_t* err = r.errWord();
+        // The same entries in every launch: their lists are built once.  No
+        // allocation follows that could take their memory.
+        const float4* cones = nullptr;
         for (uint32_t c = 4; c <= 1024; c *= 2) {
           const uint32_t* ent = d.entries.ptr;
           float* part = d.partials.ptr;
           if (!cones) cones = r.entryCones(e, d.poses.ptr, ent, rows, c, rows * c);
           const AdaptiveLaunch L = planAdaptive(&ent, &rows, &c, &part, 1, cones ? &cones : nullptr);
-          DevEye ce;
-          r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
           if (ce.cuts)
             check(launchCuts(r.dev, d.poses.ptr, static_cast<uint32_t>(count), ce.cutRadius, ce.maxRel, ce.cuts, st),
                   "cuts");
           for (int k = 0; k < seeds; ++k)
             check(launchAdaptive(r.dev, e.omm.ptr, e.N, d.poses.ptr, L, 0x5eed0000ull + static_cast<uint64_t>(k),
-                                 d.labelOuts.ptr + static_cast<size_t>(k) * rows * 3, r.errWord(), nullptr, st,
-                                 ce.cuts),
+                                 d.labelOuts.ptr + static_cast<size_t>(k) * rows * 3, err, nullptr, st, ce.cuts),
                   "label render");
           check(launchLabels(d.labelOuts.ptr, seeds, rows, c, threshold, d.labels.ptr, st), "labels");
         }
@@ -2707,7 +2714,10 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
               firstList = k;
               listRays += cnt[k] * (4ull << k);
             }
-            const float4* cones = nullptr;
+            DevEye ce;
+            r.withCuts(ce, P, e.maxRel);
+            uint32_t* err = r.errWord();
+            const float4* cones = nullptr;  // last: no allocation follows that could take their memory
             if (firstList < kAdaptiveBuckets)
               cones = r.entryCones(e, poses + 4 * first, d.entries.ptr + off[firstList], total - off[firstList],
                                    4u << firstList, listRays);
@@ -2721,19 +2731,16 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
               cone[k] = k >= firstList ? cones + (off[k] - off[firstList]) * kConeStride : nullptr;
             }
             const AdaptiveLaunch L = planAdaptive(ent, n, spp, part, firstList);
-            DevEye ce;
-            if (L.totalPools) {
-              r.withCuts(ce, P, e.maxRel);
-              if (ce.cuts) check(launchCuts(r.dev, poses + 4 * first, P, ce.cutRadius, ce.maxRel, ce.cuts, st), "cuts");
-            }
+            if (L.totalPools && ce.cuts)
+              check(launchCuts(r.dev, poses + 4 * first, P, ce.cutRadius, ce.maxRel, ce.cuts, st), "cuts");
             check(launchAdaptive(r.dev, e.omm.ptr, e.N, poses + 4 * first, L, 0xada90000ull + d.adaptiveFrame,
-                                 d.sums.ptr, r.errWord(), nullptr, st, ce.cuts),
+                                 d.sums.ptr, err, nullptr, st, ce.cuts),
                   "adaptive render");
             if (cones) {
               const uint32_t f = firstList;
               const AdaptiveLaunch LL = planAdaptive(ent + f, n + f, spp + f, part + f, kAdaptiveBuckets - f, cone + f);
               check(launchAdaptive(r.dev, e.omm.ptr, e.N, poses + 4 * first, LL, 0xada90000ull + d.adaptiveFrame,
-                                   d.sums.ptr, r.errWord(), nullptr, st),
+                                   d.sums.ptr, err, nullptr, st),
                     "adaptive render");
             }
           }
@@ -2845,14 +2852,15 @@ int crAdaptiveRecord(const float* poses12, size_t count, int spp, unsigned long 
         const uint32_t* ep = ent.ptr;
         float* pp = part.ptr;
         const uint32_t c = static_cast<uint32_t>(spp);
-        const float4* cones = r.entryCones(e, d.poses.ptr, ep, rows, c, rows * c);
-        const AdaptiveLaunch L = planAdaptive(&ep, &rows, &c, &pp, 1, cones ? &cones : nullptr);
         DevEye ce;
         r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
+        uint32_t* err = r.errWord();
+        const float4* cones = r.entryCones(e, d.poses.ptr, ep, rows, c, rows * c);  // last, as above
+        const AdaptiveLaunch L = planAdaptive(&ep, &rows, &c, &pp, 1, cones ? &cones : nullptr);
         if (ce.cuts)
           check(launchCuts(r.dev, d.poses.ptr, static_cast<uint32_t>(count), ce.cutRadius, ce.maxRel, ce.cuts, st),
                 "cuts");
-        check(launchAdaptive(r.dev, e.omm.ptr, e.N, d.poses.ptr, L, seed, s.ptr, r.errWord(), rec.ptr, st, ce.cuts),
+        check(launchAdaptive(r.dev, e.omm.ptr, e.N, d.poses.ptr, L, seed, s.ptr, err, rec.ptr, st, ce.cuts),
               "adaptive render");
         check(cudaMemcpyAsync(records, rec.ptr, rows * spp * sizeof(RayRecord), cudaMemcpyDeviceToHost, st),
               "cudaMemcpy");

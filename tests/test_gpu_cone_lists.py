@@ -378,3 +378,38 @@ def test_negative_focal_offsets(lib, small, deep, on_deep, spp):
         assert np.array_equal(x, y, equal_nan=True)
     omm[::10, 7] = 0.0  # the offsets do decide what is seen
     assert not np.array_equal(_both(lib, omm, spp, poses)[1][0][:, ::10], without[0][:, ::10], equal_nan=True)
+
+
+@pytest.mark.parametrize("slack", [0, 40000, 90000])
+def test_record_with_cuts_under_a_cap_that_fits_the_lists(lib, small, slack):
+    """crAdaptiveRecord with a cut radius and a memory cap that has room for
+    the lists, but (up to 69,360 bytes more) not for the lists and the cuts:
+    the cuts come first, and the lists are left out."""
+    P, spp = 256, 32
+    p12 = np.ascontiguousarray(scenes.open_poses(small["boxes"], P, np.random.default_rng(6)), np.float32)
+    n = 2 ** 21 // (P * spp) + 3
+    rows = P * n
+    assert lib.crSetCutRadius(1.0 / 32) == 0
+    got = []
+    try:
+        for cap in (False, True):
+            _load(lib, small)
+            omm = _eye(n, "plain")
+            lib.setOmmatidia(omm.ctypes.data, n)
+            lib.setCurrentEyeSamplesPerOmmatidium(1)
+            assert lib.crAdaptiveRecord(p12[:1], 1, 1, 9, np.zeros((n, 1), eh.RAY_RECORD_DTYPE).ctypes.data,
+                                        np.zeros((n, 3), np.float32)) == 0, eh.lastError(lib)
+            rec, sums = np.zeros((rows, spp), eh.RAY_RECORD_DTYPE), np.zeros((rows, 3), np.float32)
+            held = lib.crGetDeviceMemoryHeld()
+            if cap:  # entries, sums, records, poses (perhaps held already); the lists
+                need = rows * (4 + 12 + 64 * spp) + 4 + 64 * (P - 1)
+                lib.crSetDeviceMemoryCap(held + need + rows * 31 * 16 + slack)
+            try:
+                assert lib.crAdaptiveRecord(p12, P, spp, 9, rec.ctypes.data, sums) == 0, eh.lastError(lib)
+            finally:
+                lib.crSetDeviceMemoryCap(0)
+            assert (lib.crGetDeviceMemoryHeld() - held >= rows * (64 * spp + 400)) == (not cap or slack > 272 * (P - 1))
+            got.append((rec, sums))
+    finally:
+        lib.crSetCutRadius(0.0)
+    assert got[0][0].tobytes() == got[1][0].tobytes() and np.array_equal(got[0][1], got[1][1])
