@@ -1044,6 +1044,14 @@ __device__ __forceinline__ int coneRef(const float4* list, uint32_t k) { return 
 // (24 uneven eyes 5.0 ms, the adaptive terrain render 2.19 ms; with one loop
 // whose step is a node or a leaf 5.16 and 2.42 ms, with the lanes held
 // together by votes 5.3 and 2.38 ms).
+//
+// The stack needs no guard beside the search from the root's: when coneList
+// adds an entry of tree depth d that has children, at most d nodes wait on its
+// own stack (a sibling of each ancestor), and no more entries than those
+// follow (either the list is full with them, or its steps are used up and they
+// are added as they are).  So the entries that wait here under the path of a
+// subtree at depth d are no more than the d that a search from the root may
+// have put there; under a leaf nothing is pushed.
 constexpr int kStackEntry = 0x40000000;  // stack values from here on are kStackEntry + entry
 
 template <bool kCount>

@@ -413,3 +413,61 @@ def test_record_with_cuts_under_a_cap_that_fits_the_lists(lib, small, slack):
     finally:
         lib.crSetCutRadius(0.0)
     assert got[0][0].tobytes() == got[1][0].tobytes() and np.array_equal(got[0][1], got[1][1])
+
+
+@pytest.fixture(scope="module")
+def chain(tmp_path_factory):
+    """A scene whose linear BVH is nearly as deep as the traversal stack:
+    every facet's Morton code shares one bit less with the origin's."""
+    rng = np.random.default_rng(3)
+    c = [rng.uniform(0, 2.0 ** -22, 3) for _ in range(8)]
+    r = [2.0 ** -21] * 8
+    for k in range(57):
+        e = np.zeros(3)
+        e[k % 3] = 1.2 * 2.0 ** -(1 + k // 3)
+        c.append(e)
+        r.append(0.4 * 2.0 ** -(1 + k // 3))
+    for e in np.eye(3):  # the corners of the unit cube
+        c.append(e)
+        r.append(0.2)
+    tri = np.array([[-1, -1, 0], [1, -1, 0], [0, 1, 0]]) + np.zeros(3)
+    v = np.concatenate([x + s * tri for x, s in zip(c, r)])
+    d = tmp_path_factory.mktemp("chain")
+    g = scenes.GltfBuilder()
+    g.mesh("chain", v.astype(np.float32), np.arange(len(v)).reshape(-1, 3), colours=rng.uniform(0, 1, (len(v), 4)))
+    a = scenes.fibonacci_sphere(10)
+    scenes.write_eye(str(d / "e.eye"), a * 0.001, a, 0.05, 0.0)
+    g.compound_camera("eye", "e.eye")
+    return {"gltf": g.write(str(d / "chain.gltf"))}
+
+
+@pytest.mark.parametrize("spp", [32, 100])
+def test_lists_of_a_tree_as_deep_as_the_stack(lib, chain, spp):
+    """A list's entries wait on the stack of a subtree's search, which needs no
+    more of it than a search from the root."""
+    n = 701
+    P = max(12, 2 ** 21 // (n * spp) + 2)
+    omm = _eye(n, "plain")
+    rng = np.random.default_rng(5)
+    axis = np.ones(3) / math.sqrt(3.0)
+    omm[:600, 3:6] = axis  # most look along the diagonal, some exactly
+    omm[200:600, 3:6] += rng.normal(0, 0.05, (400, 3))
+    omm[200:600, 3:6] /= np.linalg.norm(omm[200:600, 3:6], axis=1)[:, None]
+    omm[:, 0:3] = 0.0
+    omm[100:300, 6] = 0.0
+    p = np.zeros((P, 16), np.float32)
+    p[:, 0:3] = -axis * 10.0 ** rng.uniform(-7, 0, (P, 1)) + rng.normal(0, 1, (P, 3)) * 10.0 ** rng.uniform(-9, -2, (P, 1))
+    p[::3, 0:3] = -axis * 10.0 ** rng.uniform(-7, 0, (len(p[::3]), 1))
+    p[:, 4] = p[:, 9] = p[:, 14] = 1.0
+    assert lib.crSetBvhBuilder(1) == 0
+    try:
+        _load(lib, chain)
+        with_lists, without = _both(lib, omm, spp, p)
+    finally:
+        lib.crSetBvhBuilder(0)
+    depth = ctypes.c_uint32()
+    lib.crGetBvhStats(None, None, ctypes.byref(depth))
+    assert 54 <= depth.value <= 62
+    assert with_lists[3] >= 400 * n * P and len(np.unique(without[0][0])) > 3
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y)
