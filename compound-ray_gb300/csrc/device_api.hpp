@@ -143,8 +143,9 @@ struct WarpPlan {
 // The default plan: 32-sample segments (whole ommatidia when spp < 32).
 WarpPlan planWarps(uint32_t N, uint32_t spp);
 // Layout of the plain render kernel, process-wide (the autotuner sets it):
-// block size in threads (0 = 128, or for few poses the smallest of 128, 256,
-// 512 that holds all chunk warps of an ommatidium) and samples per warp segment
+// block size in threads (0 = the smallest of 128, 256, 512 that holds all
+// chunk warps of an ommatidium, else 128; long launches through cone lists:
+// 128) and samples per warp segment
 // (0 = 32, or 8 / 16: segments of 8 or 16 samples, several ommatidia per
 // warp; a smaller segment changes the order in which samples are summed,
 // so results change within float rounding).  Results never depend on the

@@ -697,8 +697,7 @@ struct Renderer {
     if (st != cudaStreamCaptureStatusNone) return usual;
     const uint32_t P = static_cast<uint32_t>(most);
     const size_t drawn = rec || stats ? 0 : renderDrawBytes(e.N, e.spp, P) / sizeof(float2);
-    const size_t sums = std::max(renderScratchFloats(dev, e.N, e.spp, P, rec, stats, false, false),
-                                 renderScratchFloats(dev, e.N, e.spp, P, rec, stats, false, true));
+    const size_t sums = renderScratchFloats(dev, e.N, e.spp, P, rec, stats);
     if ((!drawn || draws.tryEnsure(drawn)) && (!sums || scratch.tryEnsure(sums)) &&
         (!(cutFactor > 0.f) || cuts.tryEnsure(static_cast<size_t>(P) * kCutStride)))
       return most;
@@ -708,28 +707,33 @@ struct Renderer {
     return usual;
   }
 
-  // Sets de.cones to a buffer of `lists` cone lists when there are any to
-  // build and the memory is to be had; not while the stream is being captured
-  // (the buffer may be given back before the captured graph runs).
-  void takeCones(DevEye& de, size_t lists) {
+  // Sets de.cones to a buffer of `lists` cone lists, followed by `floats`
+  // floats (returned), when there are any to build and the memory is to be
+  // had; not while the stream is being captured (the buffer may be given back
+  // before the captured graph runs).
+  float* takeCones(DevEye& de, size_t lists, size_t floats = 0) {
     de.cones = nullptr;
-    if (!lists || lists * kConeStride * sizeof(float4) > kConeListBytes) return;
+    const size_t n = lists * kConeStride;
+    if (!lists || n * sizeof(float4) > kConeListBytes) return nullptr;
     cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
     check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
-    if (st == cudaStreamCaptureStatusNone && cones.tryEnsure(lists * kConeStride)) de.cones = cones.ptr;
+    if (st != cudaStreamCaptureStatusNone || !cones.tryEnsure(n + (floats + 3) / 4)) return nullptr;
+    de.cones = cones.ptr;
+    return reinterpret_cast<float*>(cones.ptr + n);
   }
 
-  // Cone lists for a P-pose launch that uses them, when the memory for them
-  // is to be had, and the launch's scratch (returned; null when it needs
-  // none).
+  // The scratch of a P-pose launch (returned; null when it needs none), and
+  // cone lists for it when it uses them and their memory is to be had.  The
+  // scratch of a launch without lists is allocated either way, so that a
+  // render that is captured after this one, or finds no room for lists, needs
+  // no more memory; what only the lists' layout needs lies behind the lists.
   float* withCones(DevEye& de, uint32_t P, DevBuf<float>& scr, bool rec, bool stats) {
-    takeCones(de, conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec, stats));
-    for (;;) {
-      const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, de.cones != nullptr);
-      if (need) scr.ensure(need);
-      if (!de.cones || cones.ptr) return need ? scr.ptr : nullptr;
-      de.cones = nullptr;  // the scratch took their memory
-    }
+    const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, false);
+    if (need) scr.ensure(need);
+    const size_t lists = conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec, stats);
+    const size_t more = lists && !need ? renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, true) : 0;
+    float* behind = takeCones(de, lists, more);
+    return more && de.cones ? behind : (need ? scr.ptr : nullptr);
   }
 
   // Cone lists of `count` entries for adaptive launches of `rays` rays at `spp`

@@ -2430,8 +2430,10 @@ constexpr size_t kChunkSmemMax = 96 * 1024;  // shared memory for in-block chunk
 // The plain render's plan under the process-wide layout: the segment width,
 // then the block size, and whether the chunk partials of P poses are summed
 // in shared memory (possible when a block holds whole ommatidium groups and
-// their partials fit kChunkSmemMax).
-WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, bool inBlockAllowed = true) {
+// their partials fit kChunkSmemMax; through cone lists, for whole-warp
+// segments).
+WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, bool inBlockAllowed = true,
+                    bool cones = false) {
   WarpPlan p = planWarps(N, spp);
   if (g_samplesPerWarp && g_samplesPerWarp < p.segWidth) {
     p.segWidth = g_samplesPerWarp;
@@ -2441,12 +2443,13 @@ WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, boo
   }
   uint32_t bw = g_blockThreads / 32;
   if (bw == 0) {
-    // The automatic layout sums chunks in the block only where that saves the
-    // second launch (few poses): on long launches the block's barriers cost
-    // more than the partials' round trip (256 terrain poses: 7.3 ms with
-    // 256-thread blocks and sums in the block, 6.9 ms with 128 and scratch).
+    // Through cone lists the automatic layout sums chunks in the block only
+    // where that saves the second launch (few poses): on long launches the
+    // block's barriers cost more than the partials' round trip (256 terrain
+    // poses: 7.3 ms with 256-thread blocks and sums in the block, 6.9 ms with
+    // 128 and scratch).
     bw = 4;
-    if (p.chunks > 1 && P <= kInBlockPoses && !forceScratch && inBlockAllowed)
+    if (p.chunks > 1 && (!cones || P <= kInBlockPoses) && !forceScratch && inBlockAllowed)
       for (uint32_t c : {4u, 8u, 16u})
         if (p.chunks <= c && c % p.chunks == 0) {
           bw = c;
@@ -2457,7 +2460,7 @@ WarpPlan planRender(uint32_t N, uint32_t spp, uint32_t P, bool forceScratch, boo
   // A small eye's launch may spread its poses over more warps (pre-drawn
   // random numbers, splitPoses): that plan keeps the chunk partials in scratch.
   const bool maySplit = P >= 2 && p.tasks < kFillWarps / 2;
-  if (p.chunks > 1 && p.segWidth == 32 && !forceScratch && inBlockAllowed && !maySplit && bw % p.chunks == 0) {
+  if (p.chunks > 1 && (!cones || p.segWidth == 32) && !forceScratch && inBlockAllowed && !maySplit && bw % p.chunks == 0) {
     const uint32_t G = bw / p.chunks;
     const size_t bytes = static_cast<size_t>(G) * p.ommPerWarp * kInBlockPoses * p.chunks * 3 * sizeof(float);
     if (bytes <= kChunkSmemMax) {
@@ -2499,10 +2502,10 @@ WarpPlan planBatch(uint32_t N, uint32_t spp) {
 
 uint32_t batchBlockThreads() { return g_blockThreads ? g_blockThreads : 128u; }
 
-// In-block chunk sums are built for the plain and recording renders through
-// cone lists only.
-static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats, bool cones) {
-  return !stats && !scene.lighting && cones;
+// In-block chunk sums are built for the plain and recording renders on the
+// two-wide BVH only, with and without cone lists.
+static bool inBlockAllowed(const DevScene& scene, bool rec, bool stats) {
+  return !stats && !scene.lighting && (scene.width == 2 || rec);
 }
 
 // When a launch uses cone lists: enough rays to hide the ~20-35 us that the
@@ -2544,7 +2547,7 @@ size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t
 
 size_t renderScratchFloats(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec, bool stats,
                            bool forceScratch, bool cones) {
-  const WarpPlan p = planRender(N, spp, P, forceScratch, inBlockAllowed(scene, rec, stats, cones));
+  const WarpPlan p = planRender(N, spp, P, forceScratch, inBlockAllowed(scene, rec, stats), cones);
   if (p.chunks == 1 || p.inBlock) return 0;
   return static_cast<size_t>(P) * N * p.chunks * 3;
 }
@@ -2589,20 +2592,24 @@ cudaError_t runRenderKernel(const DevScene& scene, const DevEye& eye, const floa
 }
 
 // The instance for the two-wide BVH: through the cone lists when the eye has
-// them (with in-block chunk sums where the plan says so; planRender offers
-// those only to plain and recording renders), else without.
+// them, else without; with in-block chunk sums where the plan says so
+// (planRender offers those only to plain and recording renders).
 template <int kMode, int kRegs>
 cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                       const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                       unsigned long long* stats, cudaStream_t stream) {
   constexpr bool kHasCone = kMode == 0 || kMode == 3 ? kRegs == kConeRegs : true;
-  constexpr bool kHasInBlock = kHasCone && (kMode == 0 || kMode == 1);
+  constexpr bool kHasInBlock = kMode == 0 || kMode == 1;
   constexpr bool kMayDraw = kHasCone && (kMode == 0 || kMode == 4);  // only plain renders pre-draw
   constexpr bool kSegments = kHasCone && (kMode == 0 || kMode == 3);  // several lists a warp
-  if (plan.inBlock && (!kHasInBlock || !eye.cones || plan.segWidth != 32)) return cudaErrorInvalidValue;
-  if (!eye.cones)
+  if (plan.inBlock && (!kHasInBlock || (eye.cones && plan.segWidth != 32))) return cudaErrorInvalidValue;
+  if (!eye.cones) {
+    if (plan.inBlock)
+      return runRenderKernel<kMode, kRegs, 2, kHasInBlock, 0>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
+                                                              stats, stream);
     return runRenderKernel<kMode, kRegs, 2, false, 0>(scene, eye, poses, P, plan, out, scratch, errFlag, rec, stats,
                                                       stream);
+  }
   if constexpr (kHasCone) {
     if (plan.inBlock)
       return runRenderKernel<kMode, kRegs, 2, kHasInBlock, 1>(scene, eye, poses, P, plan, out, scratch, errFlag, rec,
@@ -2671,7 +2678,7 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
   if (eye.cones && renderConeLists(scene, eye.N, eye.spp, P, rec != nullptr, stats != nullptr) == 0)
     return cudaErrorInvalidValue;
   WarpPlan plan = planRender(eye.N, eye.spp, P, forceScratch,
-                             inBlockAllowed(scene, rec != nullptr, stats != nullptr, eye.cones != nullptr));
+                             inBlockAllowed(scene, rec != nullptr, stats != nullptr), eye.cones != nullptr);
   if (plan.chunks > 1 && !plan.inBlock && scratch == nullptr) return cudaErrorInvalidValue;
   if (eye.draws) {
     if (plan.inBlock) return cudaErrorInvalidValue;  // planRender keeps splittable launches out of shared memory

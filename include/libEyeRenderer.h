@@ -182,9 +182,10 @@ int crAutotune(const float* d_poses, size_t count, int* bestVariant, float* msPe
  * radius was 0). */
 int crGetAutotuneTimes(float* ms, size_t n);
 /* No counterpart in the reference.  Layout of the render kernel: block size
- * in threads (0 = 128, or, for up to 16 poses through cone lists, the smallest
- * of 128 / 256 / 512 holding all 32-sample chunk warps of an ommatidium, whose
- * chunk sums then stay in shared memory) and samples per warp segment (8, 16 or 32; below 32 a warp
+ * in threads (0 = the smallest of 128 / 256 / 512 holding all 32-sample chunk
+ * warps of an ommatidium, whose chunk sums then stay in shared memory; else
+ * 128, as in launches of more than 16 poses through cone lists) and samples
+ * per warp segment (8, 16 or 32; below 32 a warp
  * holds several ommatidia, and the samples are summed in another order:
  * results change within float rounding).  The block size changes no result.
  * Also used by batches created afterwards.  0 on success. */

@@ -471,3 +471,78 @@ def test_lists_of_a_tree_as_deep_as_the_stack(lib, chain, spp):
     assert with_lists[3] >= 400 * n * P and len(np.unique(without[0][0])) > 3
     for x, y in zip(with_lists[:3], without[:3]):
         assert np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n,spp,P,lists", [(2000, 256, 4, False), (101, 64, 1, False), (6000, 128, 2, False),
+                                           (700, 512, 17, True), (900, 64, 300, True), (1100, 100, 40, True)])
+def test_no_more_memory_than_without_lists(lib, small, n, spp, P, lists):
+    """Chunk sums stay in the block with and without lists, or need no more
+    scratch than without: under a cap of what the launch without lists holds,
+    every call is accepted, before and after one with lists."""
+    import torch
+
+    _load(lib, small)
+    omm, p16 = _eye(n, "plain"), _poses(small, max(P, 9), P)[:P]
+    d_poses = torch.from_numpy(p16).cuda()
+    got = []
+    for capped in (True, False, True):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        _render(lib, lib.crRenderPosesDevice, d_poses, 1, n)
+        held = lib.crGetDeviceMemoryHeld()
+        if capped and not got:  # 8 bytes a ray where the poses are spread over the warps, for 256 poses at most
+            chunks = (spp + 31) // 32
+            split = P > 1 and n * chunks < 8192
+            room = min(P, 256) * n * (8 * spp + 12 * chunks) if split else 0
+            assert lists or split or room == 0
+            lib.crSetDeviceMemoryCap(held + room)
+        elif capped:
+            lib.crSetDeviceMemoryCap(held)
+        try:
+            got.append(_render(lib, lib.crRenderPosesDevice, d_poses, P, n))
+        finally:
+            lib.crSetDeviceMemoryCap(0)
+        if got[1:] and not capped:
+            assert (lib.crGetDeviceMemoryHeld() - held > 400 * min(P, 256) * n) == lists
+    for g in got[1:]:
+        assert np.array_equal(g, got[0], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,spp,P", [(6000, 256, 1), (6000, 400, 1), (700, 512, 17), (900, 64, 300), (40, 32, 700)])
+def test_capture_after_one_render(lib, small, deep, n, spp, P):
+    """A render captured into a graph after the same render once outside: the
+    capture allocates nothing, and its replay gives the next frames."""
+    import torch
+
+    info = deep if P == 1 else small  # a single frame with lists
+    _load(lib, info)
+    omm, p16 = _eye(n, "plain"), _poses(info, max(P, 9), P)[:P]
+    d_poses = torch.from_numpy(p16).cuda()
+    out = torch.zeros((P, n, 3), device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    res = []
+    for captured in (False, True):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        assert lib.crSetStream(st.cuda_stream) == 0
+        try:
+            render = lambda: lib.crRenderPosesDevice(d_poses.data_ptr(), P, out.data_ptr())
+            assert render() == 0
+            held = lib.crGetDeviceMemoryHeld()
+            if captured:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=st):
+                    rc = render()
+                assert rc == 0, eh.lastError(lib)
+                assert lib.crGetDeviceMemoryHeld() == held
+                for _ in range(2):
+                    with torch.cuda.stream(st):
+                        g.replay()
+            else:
+                assert render() == 0 and render() == 0
+            assert lib.crSynchronize() == 0
+        finally:
+            lib.crSetStream(None)
+        res.append(out.cpu().numpy())
+    assert np.array_equal(res[0], res[1], equal_nan=True)
