@@ -53,8 +53,8 @@ size_t& devCap() {
   return cap;
 }
 
-// Gives back the buffers that only make renders faster (Renderer::cones);
-// true when there was one.  An allocation that fails tries again after it.
+// Gives back the memory that only makes renders faster (Renderer::extra);
+// true when there was some.  An allocation that fails tries again after it.
 bool releaseOptional();
 
 template <typename T>
@@ -322,7 +322,11 @@ struct Renderer {
   DevBuf<float> scratch;
   DevBuf<float2> draws;  // pre-drawn random numbers of small-eye launches
   DevBuf<float4> cuts;   // per-pose near-field cuts
-  DevBuf<float4> cones;   // cone lists of a launch
+  // What only makes a launch faster: cone lists, and the buffers of launches
+  // of more than kMaxPosesPerLaunch poses.  Given back when an allocation
+  // would fail without (releaseOptional), so the buffers above are allocated
+  // first, and never used by a launch that the caller captures.
+  DevBuf<float4> extra;
   bool conesOff = false; // crAutotune times variants and cut radii without cone lists
   float cutFactor = 0.f; // cut radius as a fraction of the scene extent (0: off)
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
@@ -362,7 +366,7 @@ struct Renderer {
     scratch.release();
     draws.release();
     cuts.release();
-    cones.release();
+    extra.release();
     batchOut.release();
     err.release();
     dev = DevScene{};
@@ -650,18 +654,96 @@ struct Renderer {
   void renderDevicePoses(EyeDev& e, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                          unsigned long long* stats = nullptr) {
     ensureRng(e);
-    uint32_t* errFlag = errWord();  // before the lists: an allocation may give them back
-    const size_t perLaunch = launchPoses(e, count, rec != nullptr, stats != nullptr);
+    renderLaunches(devEye(e), d_poses, count, d_out, rec, stats, scratch, true, e.maxRel);
+  }
+
+  // The launches of a render.  plain: with pre-drawn numbers and near-field
+  // cuts where they apply, and launches of more than kMaxPosesPerLaunch poses
+  // for small eyes.  Everything that a launch of up to kMaxPosesPerLaunch
+  // poses without lists needs is allocated first, in buffers that stay: a
+  // render captured after this one, or one that finds no room for more, needs
+  // no other.
+  void renderLaunches(DevEye de, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
+                      unsigned long long* stats, DevBuf<float>& scr, bool plain, float maxRel) {
+    if (!count) return;
+    uint32_t* errFlag = errWord();
+    const uint32_t usual = static_cast<uint32_t>(
+        std::min<size_t>({kMaxPosesPerLaunch, std::max<size_t>(1, conePoses(de.N)), count}));
+    withDraws(de, usual, plain && !rec && !stats);
+    if (plain) withCuts(de, usual, maxRel);
+    const DevEye kept = de;
+    const size_t need = renderScratchFloats(dev, de.N, de.spp, usual, rec, stats);
+    if (need) scr.ensure(need);
+    // More poses a launch for small eyes, fewer where a usual launch's lists
+    // would not fit kConeListBytes; usual launches when the memory is not to
+    // be had.  No long launches under a memory cap, whose room is for others.
+    size_t perLaunch = usual;
+    float4* x = nullptr;
+    if (!capturing()) {
+      const size_t fit = conePoses(de.N), rays = std::max<size_t>(1, static_cast<size_t>(de.N) * de.spp);
+      size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, count});
+      if (coneLists(de, std::min(most, fit), rec, stats)) most = std::min(most, fit);
+      if (plain && !devCap() && most > usual) {
+        const size_t n = extraFor(de, most, rec, stats, plain).total;
+        if (!n || (x = takeExtra(n))) perLaunch = most;
+      }
+      const size_t some = std::min<size_t>(usual, fit);
+      if (perLaunch == usual && coneLists(de, some, rec, stats) &&
+          (x = takeExtra(extraFor(de, some, rec, stats, plain).total)))
+        perLaunch = some;
+    }
     for (size_t first = 0; first < count; first += perLaunch) {
       const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
-      DevEye de = devEye(e);
-      withDraws(de, P, !rec && !stats);
-      withCuts(de, P, e.maxRel);
-      float* s = withCones(de, P, scratch, rec != nullptr, stats != nullptr);
-      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * e.N, s, errFlag, rec, stream(), stats),
+      float* s = renderScratchFloats(dev, de.N, de.spp, P, rec, stats) ? scr.ptr : nullptr;
+      de = kept;
+      if (!renderDrawBytes(de.N, de.spp, P)) de.draws = nullptr;
+      if (x) {
+        const Extra l = extraFor(de, P, rec, stats, plain);
+        if (l.cones) de.cones = x;
+        if (l.sums) s = reinterpret_cast<float*>(x + l.cones);
+        if (l.draws) de.draws = reinterpret_cast<float2*>(x + l.cones + l.sums);
+        if (l.cuts) de.cuts = x + l.cones + l.sums + l.draws;
+      }
+      check(launchRender(dev, de, d_poses + 4 * first, P, d_out + 3 * first * de.N, s, errFlag, rec, stream(), stats),
             "render launch");
     }
   }
+
+  // What a launch of P poses takes from `extra`, in float4, one after another:
+  // its lists, the chunk partials that the usual scratch has no room for, and
+  // the pre-drawn numbers and cuts of more than kMaxPosesPerLaunch poses.
+  struct Extra {
+    size_t cones = 0, sums = 0, draws = 0, cuts = 0, total = 0;
+  };
+  Extra extraFor(const DevEye& de, size_t poses, bool rec, bool stats, bool plain) const {
+    const uint32_t P = static_cast<uint32_t>(poses);
+    const bool more = P > kMaxPosesPerLaunch;
+    Extra x;
+    x.cones = coneLists(de, poses, rec, stats) * kConeStride;
+    const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats);
+    if (more || (x.cones && !need))
+      x.sums = (renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, x.cones != 0) + 3) / 4;
+    if (more && plain && !rec && !stats) x.draws = (renderDrawBytes(de.N, de.spp, P) + 15) / 16;
+    if (more && de.cuts) x.cuts = poses * kCutStride;
+    x.total = x.cones + x.sums + x.draws + x.cuts;
+    return x;
+  }
+
+  // Lists that a launch of P poses uses, as far as they fit kConeListBytes.
+  size_t coneLists(const DevEye& de, size_t P, bool rec, bool stats) const {
+    if (conesOff || P == 0 || P > conePoses(de.N)) return 0;
+    return renderConeLists(dev, de.N, de.spp, static_cast<uint32_t>(P), rec, stats);
+  }
+  // Poses of an eye whose lists fit kConeListBytes.
+  static size_t conePoses(uint32_t N) { return kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N)); }
+
+  bool capturing() {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
+    return st != cudaStreamCaptureStatusNone;
+  }
+  // `extra` with room for n float4, or null; not while capturing().
+  float4* takeExtra(size_t n) { return extra.tryEnsure(n) ? extra.ptr : nullptr; }
 
   // Near-field cuts for a P-pose launch when a cut radius is set and the
   // traversal stack has room for the cut entries above the deepest leaf.
@@ -675,67 +757,6 @@ struct Renderer {
     de.maxRel = maxRel;
   }
 
-  // Poses of one launch: at most kMaxPosesPerLaunch, and fewer for large eyes
-  // so that a launch's cone lists stay within kConeListBytes.
-  static size_t conePoses(uint32_t N) {
-    return std::max<size_t>(1, kConeListBytes / (sizeof(float4) * kConeStride * std::max<size_t>(1, N)));
-  }
-  static size_t posesPerLaunch(uint32_t N) { return std::min<size_t>(kMaxPosesPerLaunch, conePoses(N)); }
-
-  // The same for a render of `count` poses, more for small eyes when the
-  // memory for it is to be had; not under a memory cap (the larger buffers
-  // stay, and a later render may need that room) and not while the stream is
-  // being captured (it may be the first render of so many poses, and would
-  // allocate).
-  size_t launchPoses(const EyeDev& e, size_t count, bool rec, bool stats) {
-    const size_t usual = posesPerLaunch(e.N);
-    const uint64_t rays = std::max<uint64_t>(1, static_cast<uint64_t>(e.N) * e.spp);
-    const size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, conePoses(e.N), count});
-    if (most <= usual || devCap()) return usual;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
-    if (st != cudaStreamCaptureStatusNone) return usual;
-    const uint32_t P = static_cast<uint32_t>(most);
-    const size_t drawn = rec || stats ? 0 : renderDrawBytes(e.N, e.spp, P) / sizeof(float2);
-    const size_t sums = renderScratchFloats(dev, e.N, e.spp, P, rec, stats);
-    if ((!drawn || draws.tryEnsure(drawn)) && (!sums || scratch.tryEnsure(sums)) &&
-        (!(cutFactor > 0.f) || cuts.tryEnsure(static_cast<size_t>(P) * kCutStride)))
-      return most;
-    draws.release();
-    scratch.release();
-    cuts.release();
-    return usual;
-  }
-
-  // Sets de.cones to a buffer of `lists` cone lists, followed by `floats`
-  // floats (returned), when there are any to build and the memory is to be
-  // had; not while the stream is being captured (the buffer may be given back
-  // before the captured graph runs).
-  float* takeCones(DevEye& de, size_t lists, size_t floats = 0) {
-    de.cones = nullptr;
-    const size_t n = lists * kConeStride;
-    if (!lists || n * sizeof(float4) > kConeListBytes) return nullptr;
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
-    if (st != cudaStreamCaptureStatusNone || !cones.tryEnsure(n + (floats + 3) / 4)) return nullptr;
-    de.cones = cones.ptr;
-    return reinterpret_cast<float*>(cones.ptr + n);
-  }
-
-  // The scratch of a P-pose launch (returned; null when it needs none), and
-  // cone lists for it when it uses them and their memory is to be had.  The
-  // scratch of a launch without lists is allocated either way, so that a
-  // render that is captured after this one, or finds no room for lists, needs
-  // no more memory; what only the lists' layout needs lies behind the lists.
-  float* withCones(DevEye& de, uint32_t P, DevBuf<float>& scr, bool rec, bool stats) {
-    const size_t need = renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, false);
-    if (need) scr.ensure(need);
-    const size_t lists = conesOff ? 0 : renderConeLists(dev, de.N, de.spp, P, rec, stats);
-    const size_t more = lists && !need ? renderScratchFloats(dev, de.N, de.spp, P, rec, stats, false, true) : 0;
-    float* behind = takeCones(de, lists, more);
-    return more && de.cones ? behind : (need ? scr.ptr : nullptr);
-  }
-
   // Cone lists of `count` entries for adaptive launches of `rays` rays at `spp`
   // (or more) samples each; null when those do not use them or the memory is
   // not to be had.  Every other buffer of the launch is allocated before: an
@@ -743,10 +764,11 @@ struct Renderer {
   const float4* entryCones(const EyeDev& e, const float4* dposes, const uint32_t* entries, uint64_t count, uint32_t spp,
                            uint64_t rays) {
     if (!count || !adaptiveLists(dev, spp, rays) || count * kConeStride * sizeof(float4) > kConeListBytes ||
-        !cones.tryEnsure(count * kConeStride))
+        capturing())
       return nullptr;
-    check(launchEntryCones(dev, e.omm.ptr, e.N, dposes, entries, count, cones.ptr, stream()), "cone lists");
-    return cones.ptr;
+    float4* cones = takeExtra(count * kConeStride);
+    if (cones) check(launchEntryCones(dev, e.omm.ptr, e.N, dposes, entries, count, cones, stream()), "cone lists");
+    return cones;
   }
 
   // Gives a P-pose launch of a small eye a buffer for its pre-drawn random
@@ -811,8 +833,8 @@ Renderer& R() {
 }
 
 bool releaseOptional() {
-  const bool had = R().cones.ptr != nullptr;
-  R().cones.release();
+  const bool had = R().extra.ptr != nullptr;
+  R().extra.release();
   return had;
 }
 
@@ -2172,11 +2194,14 @@ void denoiseFeatures(Renderer& r, DenoiseState& d, EyeDev& e, const float4* dpos
   // One launch for all poses, or, with cone lists, one for each kConeListBytes
   // of them.
   uint32_t* err = r.errWord();  // before the lists: an allocation may give them back
-  const size_t perLaunch =
-      !cost && featureConeLists(r.dev, e.N, featSpp, static_cast<uint32_t>(count)) ? r.conePoses(e.N) : count;
+  size_t perLaunch = count;
+  const size_t some = std::min<size_t>(count, Renderer::conePoses(e.N));
+  const size_t lists = cost || !some ? 0 : featureConeLists(r.dev, e.N, featSpp, static_cast<uint32_t>(some));
+  float4* cones = lists && !r.capturing() ? r.takeExtra(lists * kConeStride) : nullptr;
+  if (cones) perLaunch = some;
   for (size_t first = 0; first < count; first += perLaunch) {
     const uint32_t P = static_cast<uint32_t>(std::min(perLaunch, count - first));
-    r.takeCones(fe, cost ? 0 : featureConeLists(r.dev, e.N, featSpp, P));
+    fe.cones = cones && featureConeLists(r.dev, e.N, featSpp, P) ? cones : nullptr;
     check(launchFeatures(r.dev, fe, dposes + 4 * first, P, d.stats.ptr + first * e.N * kFeatureStats, err, r.stream(),
                          false),
           "feature render");
@@ -2242,17 +2267,9 @@ int crDenoiserAddTrainingPoses(const float* poses12, size_t count, int featureSp
         EyeDev& e = denoiseEye(r, d);
         uploadPoses12(d.poses, poses12, count, r.stream());
         denoiseFeatures(r, d, e, d.poses.ptr, count, static_cast<uint32_t>(featureSpp));
-        DevEye te = streamsFor(r, e, d.targetRng, d.targetSpp, d.targetReady, static_cast<uint32_t>(targetSpp));
+        const DevEye te = streamsFor(r, e, d.targetRng, d.targetSpp, d.targetReady, static_cast<uint32_t>(targetSpp));
         d.out.ensure(std::max<size_t>(1, count * e.N * 3));
-        uint32_t* err = r.errWord();
-        const size_t perLaunch = Renderer::posesPerLaunch(e.N);
-        for (size_t first = 0; first < count; first += perLaunch) {
-          const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
-          float* scr = r.withCones(te, P, d.scratch, false, false);
-          check(launchRender(r.dev, te, d.poses.ptr + 4 * first, P, d.out.ptr + 3 * first * e.N, scr, err, nullptr,
-                             r.stream()),
-                "target render");
-        }
+        r.renderLaunches(te, d.poses.ptr, count, d.out.ptr, nullptr, nullptr, d.scratch, false, 0.f);
         d.net.addRows(d.X.ptr, d.base.ptr, d.out.ptr, count * e.N, r.stream());
         r.checkErrWord();
         return 0;

@@ -546,3 +546,61 @@ def test_capture_after_one_render(lib, small, deep, n, spp, P):
             lib.crSetStream(None)
         res.append(out.cpu().numpy())
     assert np.array_equal(res[0], res[1], equal_nan=True)
+
+
+def test_captured_render_survives_longer_ones(lib, small):
+    """A captured render of 256 poses keeps its buffers when renders of more
+    poses follow outside the capture, with room for their own and without."""
+    import torch
+
+    _load(lib, small)
+    n, spp, P = 901, 32, 256
+    omm, p16 = _eye(n, "plain"), _poses(small, 1024, 3)
+    d_poses = torch.from_numpy(p16).cuda()
+    out = torch.zeros((1024, n, 3), device="cuda")
+    other = torch.zeros((1024, n, 3), device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    res = []
+    assert lib.crSetCutRadius(1.0 / 32) == 0 and lib.crSetStream(st.cuda_stream) == 0
+    try:
+        for captured in (False, True):
+            lib.setOmmatidia(omm.ctypes.data, n)
+            lib.setCurrentEyeSamplesPerOmmatidium(spp)
+            render = lambda count, o: lib.crRenderPosesDevice(d_poses.data_ptr(), count, o.data_ptr())
+            assert render(P, out) == 0
+            if captured:
+                g = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(g, stream=st):
+                    rc = render(P, out)
+                assert rc == 0, eh.lastError(lib)
+            for cap in (0, 1):
+                lib.crSetDeviceMemoryCap(cap and lib.crGetDeviceMemoryHeld())
+                try:
+                    assert render(1024, other) == 0, eh.lastError(lib)
+                finally:
+                    lib.crSetDeviceMemoryCap(0)
+                assert render(1024, other) == 0 and lib.crSynchronize() == 0
+                if captured:
+                    with torch.cuda.stream(st):
+                        g.replay()
+                else:
+                    assert render(P, out) == 0
+                assert lib.crSynchronize() == 0
+                res.append((out.cpu().numpy(), other.cpu().numpy()))
+    finally:
+        lib.crSetStream(None)
+        lib.crSetCutRadius(0.0)
+    for a, b in zip(res[:2], res[2:]):
+        assert np.array_equal(a[0], b[0], equal_nan=True) and np.array_equal(a[1], b[1], equal_nan=True)
+
+
+@pytest.mark.parametrize("n,spp,P", [(3, 64, 257), (701, 9, 513), (2900, 8, 769), (40, 33, 1025)])
+def test_tails_of_long_launches(lib, small, deep, n, spp, P):
+    """A last launch of one pose after long ones, which sums in the block and
+    draws for itself."""
+    info = deep if spp < 17 else small
+    _load(lib, info)
+    long, usual = _both(lib, _eye(n, "plain"), spp, _poses(info, P, n))
+    for x, y in zip(long[:3], usual[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
