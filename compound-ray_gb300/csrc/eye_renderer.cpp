@@ -667,8 +667,7 @@ struct Renderer {
                       unsigned long long* stats, DevBuf<float>& scr, bool plain, float maxRel) {
     if (!count) return;
     uint32_t* errFlag = errWord();
-    const uint32_t usual = static_cast<uint32_t>(
-        std::min<size_t>({kMaxPosesPerLaunch, std::max<size_t>(1, conePoses(de.N)), count}));
+    const uint32_t usual = static_cast<uint32_t>(std::min<size_t>(kMaxPosesPerLaunch, count));
     withDraws(de, usual, plain && !rec && !stats);
     if (plain) withCuts(de, usual, maxRel);
     const DevEye kept = de;

@@ -604,3 +604,32 @@ def test_tails_of_long_launches(lib, small, deep, n, spp, P):
     long, usual = _both(lib, _eye(n, "plain"), spp, _poses(info, P, n))
     for x, y in zip(long[:3], usual[:3]):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+def test_poses_of_a_launch_without_lists(lib, small):
+    """Renders that build no lists take 256 poses a launch, however many
+    ommatidia the eye has (the launches of a captured render are counted)."""
+    import torch
+
+    _load(lib, small)
+    n, spp, P = 100000, 4, 256
+    omm = _eye(n, "plain")
+    d_poses = torch.from_numpy(_poses(small, P, 1)).cuda()
+    out = torch.zeros((P, n, 3), device="cuda")
+    st = torch.cuda.Stream()
+    cu = ctypes.CDLL("libcuda.so.1")
+    s, graph, nodes = ctypes.c_void_p(st.cuda_stream), ctypes.c_void_p(), ctypes.c_size_t()
+    torch.cuda.synchronize()
+    lib.setOmmatidia(omm.ctypes.data, n)
+    lib.setCurrentEyeSamplesPerOmmatidium(spp)
+    assert lib.crSetStream(st.cuda_stream) == 0
+    try:
+        assert lib.crRenderPosesDevice(d_poses.data_ptr(), 1, out.data_ptr()) == 0 and lib.crSynchronize() == 0
+        assert cu.cuStreamBeginCapture_v2(s, 1) == 0  # thread-local mode
+        rc = lib.crRenderPosesDevice(d_poses.data_ptr(), P, out.data_ptr())
+        assert cu.cuStreamEndCapture(s, ctypes.byref(graph)) == 0 and rc == 0
+    finally:
+        lib.crSetStream(None)
+    assert cu.cuGraphGetNodes(graph, None, ctypes.byref(nodes)) == 0
+    cu.cuGraphDestroy(graph)
+    assert nodes.value == 1
