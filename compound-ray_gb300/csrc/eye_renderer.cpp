@@ -325,8 +325,11 @@ struct Renderer {
   // What only makes a launch faster: cone lists, and the buffers of launches
   // of more than kMaxPosesPerLaunch poses.  Given back when an allocation
   // would fail without (releaseOptional), so the buffers above are allocated
-  // first, and never used by a launch that the caller captures.
+  // first, and never used by a launch that the caller captures.  Calls on
+  // different streams share it: each waits for the last one's event.
   DevBuf<float4> extra;
+  cudaEvent_t extraUsed = nullptr;
+  bool extraTaken = false;  // since the last event
   bool conesOff = false; // crAutotune times variants and cut radii without cone lists
   float cutFactor = 0.f; // cut radius as a fraction of the scene extent (0: off)
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
@@ -367,6 +370,8 @@ struct Renderer {
     draws.release();
     cuts.release();
     extra.release();
+    if (extraUsed) cudaEventDestroy(extraUsed);
+    extraUsed = nullptr;
     batchOut.release();
     err.release();
     dev = DevScene{};
@@ -666,6 +671,7 @@ struct Renderer {
   void renderLaunches(DevEye de, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                       unsigned long long* stats, DevBuf<float>& scr, bool plain, float maxRel) {
     if (!count) return;
+    const ExtraUse use{*this};
     uint32_t* errFlag = errWord();
     const uint32_t usual = static_cast<uint32_t>(std::min<size_t>(kMaxPosesPerLaunch, count));
     withDraws(de, usual, plain && !rec && !stats);
@@ -741,8 +747,23 @@ struct Renderer {
     check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
     return st != cudaStreamCaptureStatusNone;
   }
-  // `extra` with room for n float4, or null; not while capturing().
-  float4* takeExtra(size_t n) { return extra.tryEnsure(n) ? extra.ptr : nullptr; }
+  // `extra` with room for n float4, or null; not while capturing().  For
+  // launches on the current stream, issued while an ExtraUse lives.
+  float4* takeExtra(size_t n) {
+    if (!extra.tryEnsure(n)) return nullptr;
+    if (extraUsed) check(cudaStreamWaitEvent(stream(), extraUsed, 0), "cudaStreamWaitEvent");
+    else check(cudaEventCreateWithFlags(&extraUsed, cudaEventDisableTiming), "cudaEventCreate");
+    extraTaken = true;
+    return extra.ptr;
+  }
+  // Marks the end of a call's launches that may use `extra`.
+  struct ExtraUse {
+    Renderer& r;
+    ~ExtraUse() {
+      if (r.extraTaken) cudaEventRecord(r.extraUsed, r.userStream ? r.userStream : r.ownStream);
+      r.extraTaken = false;
+    }
+  };
 
   // Near-field cuts for a P-pose launch when a cut radius is set and the
   // traversal stack has room for the cut entries above the deepest leaf.
@@ -759,7 +780,7 @@ struct Renderer {
   // Cone lists of `count` entries for adaptive launches of `rays` rays at `spp`
   // (or more) samples each; null when those do not use them or the memory is
   // not to be had.  Every other buffer of the launch is allocated before: an
-  // allocation may give the lists back.
+  // allocation may give the lists back.  The caller holds an ExtraUse.
   const float4* entryCones(const EyeDev& e, const float4* dposes, const uint32_t* entries, uint64_t count, uint32_t spp,
                            uint64_t rays) {
     if (!count || !adaptiveLists(dev, spp, rays) || count * kConeStride * sizeof(float4) > kConeListBytes ||
@@ -2192,6 +2213,7 @@ void denoiseFeatures(Renderer& r, DenoiseState& d, EyeDev& e, const float4* dpos
   r.withCuts(fe, static_cast<uint32_t>(count), e.maxRel);
   // One launch for all poses, or, with cone lists, one for each kConeListBytes
   // of them.
+  const Renderer::ExtraUse use{r};
   uint32_t* err = r.errWord();  // before the lists: an allocation may give them back
   size_t perLaunch = count;
   const size_t some = std::min<size_t>(count, Renderer::conePoses(e.N));
@@ -2543,6 +2565,7 @@ int crAllocatorAddTrainingPoses(const float* poses12, size_t count, int featureS
         uint32_t* err = r.errWord();
         // The same entries in every launch: their lists are built once.  No
         // allocation follows that could take their memory.
+        const Renderer::ExtraUse use{r};
         const float4* cones = nullptr;
         for (uint32_t c = 4; c <= 1024; c *= 2) {
           const uint32_t* ent = d.entries.ptr;
@@ -2737,6 +2760,7 @@ int crAdaptiveRenderPosesDevice(const float* d_poses, size_t count, int featureS
             DevEye ce;
             r.withCuts(ce, P, e.maxRel);
             uint32_t* err = r.errWord();
+            const Renderer::ExtraUse use{r};
             const float4* cones = nullptr;  // last: no allocation follows that could take their memory
             if (firstList < kAdaptiveBuckets)
               cones = r.entryCones(e, poses + 4 * first, d.entries.ptr + off[firstList], total - off[firstList],
@@ -2875,6 +2899,7 @@ int crAdaptiveRecord(const float* poses12, size_t count, int spp, unsigned long 
         DevEye ce;
         r.withCuts(ce, static_cast<uint32_t>(count), e.maxRel);
         uint32_t* err = r.errWord();
+        const Renderer::ExtraUse use{r};
         const float4* cones = r.entryCones(e, d.poses.ptr, ep, rows, c, rows * c);  // last, as above
         const AdaptiveLaunch L = planAdaptive(&ep, &rows, &c, &pp, 1, cones ? &cones : nullptr);
         if (ce.cuts)

@@ -420,7 +420,13 @@ int crSetBvhBuilder(int kind);
 int crGetBvhBuilder(void);
 
 /* Makes the library launch on `stream` (a cudaStream_t; null = the library's
- * own stream).  Returns 0 on success. */
+ * own stream).  Returns 0 on success.
+ * Calls on different streams: the memory that long renders share for their
+ * cone lists is handed on by the library, so such a render waits for the one
+ * before it.  Everything else that two calls share is the caller's to order:
+ * an eye's random streams, the pre-drawn numbers of small eyes, the scratch of
+ * eyes whose chunk sums do not fit a block, the near-field cuts, and the
+ * buffers of the learned forms. */
 int crSetStream(void* stream);
 
 /* Blocks until the library stream is idle; returns 0 or -1 on a CUDA error. */

@@ -633,3 +633,45 @@ def test_poses_of_a_launch_without_lists(lib, small):
     assert cu.cuGraphGetNodes(graph, None, ctypes.byref(nodes)) == 0
     cu.cuGraphDestroy(graph)
     assert nodes.value == 1
+
+
+def test_long_renders_on_two_streams(lib, tmp_path):
+    """Renders of two eyes issued back to back on two streams share the memory
+    of their lists; each gives the frames that it gives alone."""
+    import torch
+
+    P, spp, rounds = 9, 128, 6
+    info = scenes.batch_scene(str(tmp_path), n_eyes=2, poses_per_eye=P, n_min=2600, n_max=3400)
+    lib.loadGlTFscene(info["gltf"].encode())
+    cams = [info["first_batch_camera"], info["first_batch_camera"] + 1]
+    p12 = info["poses"].reshape(-1, 12)
+    p16 = np.zeros((len(p12), 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = p12[:, 3 * k:3 * k + 3]
+    d_poses = torch.from_numpy(p16).cuda()
+    assert all(4 * n >= 8192 and n * spp * P >= 2 ** 21 for n in info["n"])  # no pre-drawn numbers; lists
+    streams = [torch.cuda.Stream(), torch.cuda.Stream()]
+    res = []
+    try:
+        for apart in (True, False):
+            out = [torch.full((rounds, P, n, 3), -1.0, device="cuda") for n in info["n"]]
+            for c in cams:
+                lib.gotoCamera(c)
+                for k in (1, spp):  # a change of the sample count restarts the streams
+                    lib.setCurrentEyeSamplesPerOmmatidium(k)
+                    assert lib.crRenderPosesDevice(d_poses.data_ptr(), 1, out[cams.index(c)].data_ptr()) == 0
+                    assert lib.crSynchronize() == 0
+            torch.cuda.synchronize()
+            for k in range(rounds):
+                for i, c in enumerate(cams):
+                    lib.gotoCamera(c)
+                    lib.crSetStream(streams[i].cuda_stream)
+                    assert lib.crRenderPosesDevice(d_poses[i * P:].data_ptr(), P, out[i][k].data_ptr()) == 0
+                    if apart:
+                        assert lib.crSynchronize() == 0
+            torch.cuda.synchronize()
+            res.append([o.cpu().numpy() for o in out])
+    finally:
+        lib.crSetStream(None)
+    for a, b in zip(*res):
+        assert (a >= 0).all() and np.array_equal(a, b)
