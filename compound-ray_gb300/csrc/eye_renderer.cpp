@@ -53,8 +53,9 @@ size_t& devCap() {
   return cap;
 }
 
-// Gives back the memory that only makes renders faster (Renderer::extra);
-// true when there was some.  An allocation that fails tries again after it.
+// Gives back memory that only makes renders faster (Renderer::extra, then the
+// batches' lists, one batch at a time); true when there was some.  An
+// allocation that fails tries again after it.
 bool releaseOptional();
 
 template <typename T>
@@ -90,11 +91,13 @@ struct DevBuf {
     release();
     if (n == 0) return;
     const size_t bytes = n * sizeof(T);
-    if (devCap() && devHeld() + bytes > devCap() && !(releaseOptional() && devHeld() + bytes <= devCap()))
+    while (devCap() && devHeld() + bytes > devCap() && releaseOptional()) {
+    }
+    if (devCap() && devHeld() + bytes > devCap())
       throw std::runtime_error("device memory cap reached: " + std::to_string(devHeld()) + " bytes held, " +
                                std::to_string(bytes) + " more requested, cap " + std::to_string(devCap()));
     cudaError_t e = cudaMalloc(reinterpret_cast<void**>(&ptr), bytes);
-    if (e != cudaSuccess && releaseOptional()) {
+    while (e != cudaSuccess && releaseOptional()) {
       cudaGetLastError();
       e = cudaMalloc(reinterpret_cast<void**>(&ptr), bytes);
     }
@@ -852,12 +855,6 @@ Renderer& R() {
   return r;
 }
 
-bool releaseOptional() {
-  const bool had = R().extra.ptr != nullptr;
-  R().extra.release();
-  return had;
-}
-
 // A batch of eyes recorded as one CUDA graph (see crBatchCreate).
 struct Batch {
   std::vector<int> cams;
@@ -868,7 +865,9 @@ struct Batch {
   DevBuf<unsigned long long> ctrl;
   DevBuf<float> scratch;
   DevBuf<float4> cuts;  // per eye P x kCutStride, when the near-field cut is on
-  DevBuf<float4> cones;  // cone lists of the eyes that use them
+  std::vector<BatchEye> eyes;  // the table's contents
+  std::vector<size_t> lists;   // cone lists of each eye that uses them
+  DevBuf<float4> cones;        // those lists; given back when other buffers need the memory
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   BatchTables tables;
@@ -880,6 +879,8 @@ struct Batch {
     if (graph) cudaGraphDestroy(graph);
     exec = nullptr;
     graph = nullptr;
+    eyes.clear();
+    lists.clear();
     table.release();
     bases.release();
     ctrl.release();
@@ -894,9 +895,75 @@ std::map<int, Batch>& batches() {
   return b;
 }
 
+bool releaseOptional() {
+  if (R().extra.ptr) {
+    R().extra.release();
+    return true;
+  }
+  for (auto& kv : batches())
+    if (kv.second.cones.ptr) {  // recorded again without them when next launched
+      kv.second.cones.release();
+      return true;
+    }
+  return false;
+}
+
 void releaseBatches() {
   for (auto& kv : batches()) kv.second.release();
   batches().clear();
+}
+
+// Fills a batch's device tables, with cone lists in `cones` when that is
+// allocated, and records its graph: reset the counters, build the lists, the
+// persistent launches, the chunk sums.
+void recordBatch(Renderer& r, Batch& b) {
+  const size_t n = b.eyes.size();
+  uint32_t* err = r.errWord();
+  std::vector<unsigned long long> bases(4 * n);  // lists' tasks, other tasks, cells, lists
+  BatchTables bt;
+  for (size_t i = 0; i < n; ++i) {
+    BatchEye& be = b.eyes[i];
+    be.eye.cones = b.cones.ptr && b.lists[i] ? b.cones.ptr + bt.lists * kConeStride : nullptr;
+    bases[i] = bt.tasksLists;
+    bases[n + i] = bt.tasksOther;
+    bases[2 * n + i] = bt.cells;
+    bases[3 * n + i] = bt.lists;
+    if (!be.eye.N) continue;
+    if (be.eye.cones) bt.lists += b.lists[i];
+    (be.eye.cones ? bt.tasksLists : bt.tasksOther) += be.plan.tasks;
+    if (be.plan.chunks > 1) bt.cells += static_cast<unsigned long long>(b.P) * be.eye.N;
+  }
+  bt.eyes = b.table.ptr;
+  bt.taskBaseLists = b.bases.ptr;
+  bt.taskBaseOther = b.bases.ptr + n;
+  bt.cellBase = b.bases.ptr + 2 * n;
+  bt.coneBase = b.bases.ptr + 3 * n;
+  bt.nEyes = static_cast<uint32_t>(n);
+  cudaStream_t st = r.stream();
+  check(cudaMemcpyAsync(b.table.ptr, b.eyes.data(), n * sizeof(BatchEye), cudaMemcpyHostToDevice, st), "cudaMemcpy");
+  check(cudaMemcpyAsync(b.bases.ptr, bases.data(), bases.size() * sizeof(unsigned long long), cudaMemcpyHostToDevice, st),
+        "cudaMemcpy");
+  check(cudaStreamSynchronize(st), "batch set-up");
+  int dev = 0, sms = 0;
+  check(cudaGetDevice(&dev), "cudaGetDevice");
+  check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
+  const int blocksLists = bt.tasksLists ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, true)) : 0;
+  const int blocksOther = bt.tasksOther ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, false)) : 0;
+  check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
+  cudaError_t ce = cudaMemsetAsync(b.ctrl.ptr, 0, (3 + n) * sizeof(unsigned long long), st);
+  if (ce == cudaSuccess) ce = cudaMemsetAsync(b.ctrl.ptr + 1, 0xff, sizeof(unsigned long long), st);
+  if (ce == cudaSuccess)
+    ce = launchBatch(r.dev, bt, b.ctrl.ptr, err, b.variant, blocksLists, blocksOther, b.cutPoses, st);
+  cudaGraph_t g = nullptr;
+  const cudaError_t ee = cudaStreamEndCapture(st, &g);
+  check(ce, "batch capture");
+  check(ee, "cudaStreamEndCapture");
+  if (b.exec) cudaGraphExecDestroy(b.exec);
+  if (b.graph) cudaGraphDestroy(b.graph);
+  b.exec = nullptr;
+  b.graph = g;
+  check(cudaGraphInstantiate(&b.exec, b.graph, 0), "cudaGraphInstantiate");
+  b.tables = bt;
 }
 
 thread_local std::string g_lastError;
@@ -1566,10 +1633,16 @@ int crBatchCreate(const int* cams, size_t nCams, size_t posesPerCam, const float
         if (!cams || nCams == 0 || posesPerCam == 0 || !d_poses || !d_out)
           throw std::runtime_error("empty batch or null pointer");
         Batch b;
+        struct Release {  // whatever fails below
+          Batch* b;
+          ~Release() {
+            if (b) b->release();
+          }
+        } guard{&b};
         b.cams.assign(cams, cams + nCams);
         b.P = posesPerCam;
-        std::vector<BatchEye> table(nCams);
-        std::vector<unsigned long long> bases(4 * nCams);  // lists' tasks, other tasks, cells, lists
+        std::vector<BatchEye>& table = b.eyes;
+        table.resize(nCams);
         size_t outOff = 0, scratchFloats = 0;
         // The near-field cut radius in force now is recorded into the graph.
         r.ensureUploaded();
@@ -1614,65 +1687,31 @@ int crBatchCreate(const int* cams, size_t nCams, size_t posesPerCam, const float
         b.table.ensure(nCams);
         b.bases.ensure(4 * nCams);
         b.ctrl.ensure(3 + nCams);
-        // Cone lists of the eyes that use them, as far as kBatchConeBytes goes
-        // and when that memory is to be had.
-        BatchTables& bt = b.tables;
+        r.errWord();
+        b.variant = renderVariant();
+        // Cone lists of the eyes that use them, as far as kBatchConeBytes and a
+        // quarter of the free memory go (they stay as long as the batch, so
+        // other allocators must find room beside them).
         uint64_t batchRays = 0;
         for (const BatchEye& be : table) batchRays += static_cast<uint64_t>(be.eye.N) * be.eye.spp * be.P;
-        std::vector<size_t> lists(nCams, 0);
+        size_t freeBytes = 0, totalBytes = 0;
+        check(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
+        const size_t most = std::min(kBatchConeBytes, freeBytes / 4) / (kConeStride * sizeof(float4));
+        b.lists.assign(nCams, 0);
+        size_t lists = 0;
         for (size_t i = 0; i < nCams; ++i) {
           const size_t n = batchConeLists(r.dev, table[i].plan, table[i].eye.N, table[i].P, batchRays);
-          bases[3 * nCams + i] = bt.lists;
-          if ((bt.lists + n) * kConeStride * sizeof(float4) > kBatchConeBytes) continue;
-          lists[i] = n;
-          bt.lists += n;
+          if (lists + n > most) continue;
+          b.lists[i] = n;
+          lists += n;
         }
-        if (bt.lists && !b.cones.tryEnsure(bt.lists * kConeStride)) bt.lists = 0;
-        for (size_t i = 0; i < nCams; ++i) {
-          BatchEye& be = table[i];
-          if (bt.lists && lists[i]) be.eye.cones = b.cones.ptr + bases[3 * nCams + i] * kConeStride;
-          bases[i] = bt.tasksLists;
-          bases[nCams + i] = bt.tasksOther;
-          bases[2 * nCams + i] = bt.cells;
-          if (!be.eye.N) continue;
-          (be.eye.cones ? bt.tasksLists : bt.tasksOther) += be.plan.tasks;
-          if (be.plan.chunks > 1) bt.cells += static_cast<unsigned long long>(posesPerCam) * be.eye.N;
-        }
-        cudaStream_t st = r.stream();
-        check(cudaMemcpyAsync(b.table.ptr, table.data(), nCams * sizeof(BatchEye), cudaMemcpyHostToDevice, st), "cudaMemcpy");
-        check(cudaMemcpyAsync(b.bases.ptr, bases.data(), bases.size() * sizeof(unsigned long long),
-                              cudaMemcpyHostToDevice, st),
-              "cudaMemcpy");
-        bt.eyes = b.table.ptr;
-        bt.taskBaseLists = b.bases.ptr;
-        bt.taskBaseOther = b.bases.ptr + nCams;
-        bt.cellBase = b.bases.ptr + 2 * nCams;
-        bt.coneBase = b.bases.ptr + 3 * nCams;
-        bt.nEyes = static_cast<uint32_t>(nCams);
-        uint32_t* err = r.errWord();
-        check(cudaStreamSynchronize(st), "batch set-up");
-        int dev = 0, sms = 0;
-        check(cudaGetDevice(&dev), "cudaGetDevice");
-        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "cudaDeviceGetAttribute");
-        b.variant = renderVariant();
-        const int blocksLists = bt.tasksLists ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, true)) : 0;
-        const int blocksOther = bt.tasksOther ? sms * std::max(1, batchBlocksPerSM(b.variant, r.dev.width, false)) : 0;
-        // Record: reset the counters, the persistent launches, the chunk sums.
-        check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-        cudaError_t ce = cudaMemsetAsync(b.ctrl.ptr, 0, (3 + nCams) * sizeof(unsigned long long), st);
-        if (ce == cudaSuccess) ce = cudaMemsetAsync(b.ctrl.ptr + 1, 0xff, sizeof(unsigned long long), st);
-        if (ce == cudaSuccess)
-          ce = launchBatch(r.dev, bt, b.ctrl.ptr, err, b.variant, blocksLists, blocksOther, b.cutPoses, st);
-        cudaGraph_t g = nullptr;
-        const cudaError_t ee = cudaStreamEndCapture(st, &g);
-        check(ce, "batch capture");
-        check(ee, "cudaStreamEndCapture");
-        b.graph = g;
-        check(cudaGraphInstantiate(&b.exec, b.graph, 0), "cudaGraphInstantiate");
+        if (lists) b.cones.tryEnsure(lists * kConeStride);
+        recordBatch(r, b);
         b.generation = r.generation;
         int id = 1;
         while (batches().count(id)) ++id;
         batches()[id] = std::move(b);
+        guard.b = nullptr;
         return id;
       },
       -1);
@@ -1687,6 +1726,7 @@ int crBatchLaunch(int handle) {
         if (it == batches().end()) throw std::runtime_error("unknown batch handle");
         if (it->second.generation != R().generation)
           throw std::runtime_error("batch invalidated by a change of scene or eye configuration; recreate it");
+        if (it->second.tables.lists && !it->second.cones.ptr) recordBatch(R(), it->second);
         check(cudaGraphLaunch(it->second.exec, R().stream()), "cudaGraphLaunch");
         return 0;
       },

@@ -675,3 +675,51 @@ def test_long_renders_on_two_streams(lib, tmp_path):
         lib.crSetStream(None)
     for a, b in zip(*res):
         assert (a >= 0).all() and np.array_equal(a, b)
+
+
+def test_batch_gives_its_lists_back(lib, tmp_path):
+    """Under a memory cap that a batch's lists fill, a later render takes what
+    it needs from them, and the batch goes on without."""
+    import torch
+
+    P, spp = 5, [33, 256, 100]
+    info = scenes.batch_scene(str(tmp_path), n_eyes=len(spp), poses_per_eye=P, n_min=1500, n_max=3000)
+    cams = np.arange(info["first_batch_camera"], info["first_batch_camera"] + len(spp), dtype=np.int32)
+    p12 = info["poses"].reshape(-1, 12)
+    p16 = np.zeros((len(p12), 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = p12[:, 3 * k:3 * k + 3]
+    d_poses = torch.from_numpy(p16).cuda()
+    n0 = info["n"][0]
+    lists = 31 * 16 * P * sum(info["n"])
+    res = []
+    for cap in (False, True):
+        lib.loadGlTFscene(info["gltf"].encode())  # gives back every buffer
+        for i, c in enumerate(cams):
+            lib.gotoCamera(int(c))
+            for k in (1, spp[i]):  # a change of the sample count restarts the streams
+                lib.setCurrentEyeSamplesPerOmmatidium(k)
+                _render(lib, lib.crRenderPosesDevice, d_poses[i * P:], 1, info["n"][i])
+        lib.gotoCamera(int(cams[0]))
+        out = torch.full((3 * P * sum(info["n"]),), -1.0, device="cuda")
+        torch.cuda.synchronize()
+        held = lib.crGetDeviceMemoryHeld()
+        h = lib.crBatchCreate(cams, len(cams), P, d_poses.data_ptr(), out.data_ptr())
+        assert h > 0, eh.lastError(lib)
+        batch = lib.crGetDeviceMemoryHeld()
+        assert batch - held >= lists
+        frames = []
+        try:
+            for k in range(2):
+                assert lib.crBatchLaunch(h) == 0 and lib.crSynchronize() == 0, eh.lastError(lib)
+                frames.append(out.cpu().numpy())
+                if cap:
+                    lib.crSetDeviceMemoryCap(batch + 4096)
+                frames.append(_render(lib, lib.crRenderPosesDevice, d_poses, 6 + k, n0))
+        finally:
+            lib.crSetDeviceMemoryCap(0)
+        assert (lib.crGetDeviceMemoryHeld() < batch) == cap
+        lib.crBatchDestroy(h)
+        res.append(frames)
+    for a, b in zip(*res):
+        assert (a >= 0).all() and np.array_equal(a, b)
