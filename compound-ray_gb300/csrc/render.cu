@@ -2242,8 +2242,9 @@ __device__ __forceinline__ uint32_t lastAtMost(const T* base, uint32_t n, uint64
 // Persistent kernel over the warp tasks of every eye of a batch: each warp
 // takes the next task from a global counter until none are left.  Task t
 // belongs to the last eye whose taskBase <= t; the eyes' tasks are laid out
-// one eye after another.  ctrl[1] = earliest start
-// (ns), ctrl[2 + e] = completion time of eye e's last task (ns).
+// one eye after another.  ctrl[1] = earliest start (ns; the kernels that build
+// lists and cuts stamp it too), ctrl[2 + e] = completion time of eye e's last
+// task (ns).
 // kCone: the kernel of the eyes that have cone lists (taskBase then counts
 // theirs alone, and the other kernel's the others').
 template <int kRegs, int kWidth = 2, int kCone = 0>
@@ -2274,7 +2275,9 @@ __global__ void __maxnreg__(kRegs) batchKernel(DevScene sc, const BatchEye* __re
 // Near-field cuts of every eye of a batch: group i of eight lanes builds the
 // cut of pose i % P of eye i / P (each eye has P poses) when that eye has a
 // cut buffer.
-__global__ void batchCutKernel(DevScene sc, const BatchEye* __restrict__ eyes, uint32_t nEyes, uint32_t P) {
+__global__ void batchCutKernel(DevScene sc, const BatchEye* __restrict__ eyes, uint32_t nEyes, uint32_t P,
+                               unsigned long long* ctrl) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&ctrl[1], globalTimerNs());
   const uint64_t i = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / kCutEntries;
   const bool in = i < static_cast<uint64_t>(nEyes) * P;
   const uint32_t e = in ? static_cast<uint32_t>(i / P) : 0u, p = in ? static_cast<uint32_t>(i % P) : 0u;
@@ -2288,8 +2291,9 @@ __global__ void batchCutKernel(DevScene sc, const BatchEye* __restrict__ eyes, u
 // order.
 __global__ void __launch_bounds__(kConeThreads)
     batchConeKernel(DevScene sc, const BatchEye* __restrict__ eyes, const unsigned long long* __restrict__ coneBase,
-                    uint32_t nEyes, unsigned long long totalLists) {
+                    uint32_t nEyes, unsigned long long totalLists, unsigned long long* ctrl) {
   __shared__ uint2 work[kConeEntries * kConeThreads];
+  if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&ctrl[1], globalTimerNs());
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
   if (i >= totalLists) return;
   const uint32_t e = lastAtMost(coneBase, nEyes, i);
@@ -2812,13 +2816,14 @@ cudaError_t launchBatch(const DevScene& scene, const BatchTables& b, unsigned lo
     const uint64_t blocks = (b.lists + kConeThreads - 1) / kConeThreads;
     if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
     batchConeKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, b.eyes, b.coneBase, nEyes,
-                                                                                b.lists);
+                                                                                b.lists, ctrl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
   if (cutPoses && b.tasksOther) {
     const uint64_t n = static_cast<uint64_t>(nEyes) * cutPoses;
-    batchCutKernel<<<static_cast<unsigned>((n * kCutEntries + 63) / 64), 64, 0, stream>>>(scene, b.eyes, nEyes, cutPoses);
+    batchCutKernel<<<static_cast<unsigned>((n * kCutEntries + 63) / 64), 64, 0, stream>>>(scene, b.eyes, nEyes, cutPoses,
+                                                                                               ctrl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }

@@ -723,3 +723,39 @@ def test_batch_gives_its_lists_back(lib, tmp_path):
         res.append(frames)
     for a, b in zip(*res):
         assert (a >= 0).all() and np.array_equal(a, b)
+
+
+def test_batch_latencies_count_the_lists(lib, tmp_path):
+    """crBatchLatencies counts from the start of the launch, the building of
+    lists (over 0.1 ms of this batch) included."""
+    import torch
+
+    P = 50
+    info = scenes.batch_scene(str(tmp_path), n_eyes=1, poses_per_eye=P, n_min=30000, n_max=30000)
+    lib.loadGlTFscene(info["gltf"].encode())
+    cams = np.array([info["first_batch_camera"]], np.int32)
+    p16 = np.zeros((P, 16), np.float32)
+    for k in range(4):
+        p16[:, 4 * k:4 * k + 3] = info["poses"].reshape(-1, 12)[:, 3 * k:3 * k + 3]
+    d_poses, out = torch.from_numpy(p16).cuda(), torch.zeros((P, 30000, 3), device="cuda")
+    st = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    lib.gotoCamera(int(cams[0]))
+    lib.setCurrentEyeSamplesPerOmmatidium(17)
+    assert lib.crSetStream(st.cuda_stream) == 0
+    try:
+        h = lib.crBatchCreate(cams, 1, P, d_poses.data_ptr(), out.data_ptr())
+        assert h > 0, eh.lastError(lib)
+        lat, total, apart = np.zeros(1, np.float32), ctypes.c_float(0.0), []
+        for _ in range(5):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record(st)
+            assert lib.crBatchLaunch(h) == 0
+            b.record(st)
+            assert lib.crSynchronize() == 0
+            assert lib.crBatchLatencies(h, lat, ctypes.byref(total)) == 0 and lat[0] == total.value
+            apart.append(a.elapsed_time(b) - total.value)  # the counters' reset before, the launch itself
+        lib.crBatchDestroy(h)
+    finally:
+        lib.crSetStream(None)
+    assert -0.01 < min(apart) < 0.06, apart
