@@ -1054,10 +1054,9 @@ __device__ __forceinline__ int coneRef(const float4* list, uint32_t k) { return 
 // have put there; under a leaf nothing is pushed.
 constexpr int kStackEntry = 0x40000000;  // stack values from here on are kStackEntry + entry
 
-template <bool kCount>
 __device__ __forceinline__ void searchEntries(const DevScene& sc, v3 org, v3 dir, float tmin,
                                               const float4* __restrict__ list, uint32_t later, Hit& h,
-                                              uint32_t* errFlag, uint32_t& nodeVisits, uint32_t& triTests) {
+                                              uint32_t* errFlag) {
   const Ray r = setupRay(org, dir, sc.extent);
   int stack[kStackSize];
   int sp = 0, node = 0;
@@ -1078,7 +1077,6 @@ __device__ __forceinline__ void searchEntries(const DevScene& sc, v3 org, v3 dir
   }
   while (more) {
     while (more && node >= 0) {
-      if (kCount) ++nodeVisits;
       const float4* n = sc.nodes + 4 * node;
       const float4 n0 = __ldg(n + 0);
       const float4 n1 = __ldg(n + 1);
@@ -1105,7 +1103,6 @@ __device__ __forceinline__ void searchEntries(const DevScene& sc, v3 org, v3 dir
     if (!more) break;
     const uint32_t code = ~static_cast<uint32_t>(node);
     const uint32_t first = code >> 3, count = (code & 7u) + 1u;
-    if (kCount) triTests += count;
     for (uint32_t k = 0; k < count; ++k) {
       const float4* t = sc.tris + 3 * (first + k);
       testTriangle(r, __ldg(t), __ldg(t + 1), __ldg(t + 2), first + k, tmin, h);
@@ -1123,10 +1120,9 @@ __device__ __forceinline__ void searchEntries(const DevScene& sc, v3 org, v3 dir
 // lanes at a time, 10.9 ms instead of 6.5 for 256 terrain poses).  A test
 // reads three rows in the ray's axis order, without selects or subtractions.
 // Entries that are subtrees come last, when most of them begin beyond the hit.
-template <bool kCount>
 __device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __restrict__ list, uint32_t listed,
                                           uint32_t entries, v3 org, v3 dir, float tmin, float nd, Hit& h,
-                                          uint32_t* errFlag, uint32_t& nodeVisits, uint32_t& triTests) {
+                                          uint32_t* errFlag) {
   h.t = 1e16f;
   h.id = 0xffffffffu;
   h.pos = 0;
@@ -1141,7 +1137,6 @@ __device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __re
       const int node = __float_as_int(rows[1].w);
       if (node < 0 && (~node & 7) == 0) {
         if (rows[0].w <= h.t) {
-          if (kCount) ++triTests;
           const float4 x = rows[ray.kx], y = rows[ray.ky], z = rows[ray.kz];
           testRelative(ray, x.x, y.x, z.x, x.y, y.y, z.y, x.z, y.z, z.z, __float_as_uint(rows[2].w),
                        ~static_cast<uint32_t>(node) >> 3, tmin, h);
@@ -1152,7 +1147,7 @@ __device__ __forceinline__ void traceCone(const DevScene& sc, const float4* __re
     }
     __syncwarp();
   }
-  if (later) searchEntries<kCount>(sc, org, dir, tmin, list, later, h, errFlag, nodeVisits, triTests);
+  if (later) searchEntries(sc, org, dir, tmin, list, later, h, errFlag);
   __syncwarp();
 }
 
@@ -1789,7 +1784,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         const uint32_t listed = kCone == 1 || slot < eye.N ? __float_as_uint(head.x) : 0u;
         uint32_t entries = listed == kConeFromRoot ? 0u : listed;
         if (kCone == 2) entries = __reduce_max_sync(0xffffffffu, entries);
-        traceCone<kCount>(sc, list, listed, entries, org, dir, fpo, nd, h, errFlag, nodeVisits, triTests);
+        traceCone(sc, list, listed, entries, org, dir, fpo, nd, h, errFlag);
       } else {
         org = rayOrigin(mk(P0.x, P0.y, P0.z), mk(X.x, X.y, X.z), mk(Y.x, Y.y, Y.z), mk(Z.x, Z.y, Z.z), relPos);
       }
@@ -2544,7 +2539,7 @@ size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, u
 size_t renderConeLists(const DevScene& scene, uint32_t N, uint32_t spp, uint32_t P, bool rec, bool stats) {
   const uint32_t seg = planRender(N, spp, P, true).segWidth;
   if (!coneWorth(scene, seg, static_cast<uint64_t>(N) * spp * P)) return 0;
-  if (seg != 32 && (rec || stats || scene.lighting)) return 0;
+  if (stats || (seg != 32 && (rec || scene.lighting))) return 0;  // counting renders count the tree's search
   if (scene.width != 2 && !rec && !scene.lighting) return 0;  // the wide BVH is searched from its root
   return static_cast<size_t>(P) * N;
 }
@@ -2602,7 +2597,7 @@ template <int kMode, int kRegs>
 cudaError_t runRender(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P,
                       const WarpPlan& plan, float* out, float* scratch, uint32_t* errFlag, RayRecord* rec,
                       unsigned long long* stats, cudaStream_t stream) {
-  constexpr bool kHasCone = kMode == 0 || kMode == 3 ? kRegs == kConeRegs : true;
+  constexpr bool kHasCone = kMode == 0 || kMode == 3 ? kRegs == kConeRegs : kMode != 2;
   constexpr bool kHasInBlock = kMode == 0 || kMode == 1;
   constexpr bool kMayDraw = kHasCone && (kMode == 0 || kMode == 4);  // only plain renders pre-draw
   constexpr bool kSegments = kHasCone && (kMode == 0 || kMode == 3);  // several lists a warp
@@ -3315,8 +3310,7 @@ __global__ void __maxnreg__(kConeRegs)
         const v3 rel = rotatePoint(splayed, d.y * CR_PI_F, axis);
         const v3 dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
         Hit h;
-        uint32_t nv = 0, tt = 0;
-        traceCone<false>(sc, list, listed, entries, org, dir, fpo, valid ? d.x : 0.0f, h, errFlag, nv, tt);
+        traceCone(sc, list, listed, entries, org, dir, fpo, valid ? d.x : 0.0f, h, errFlag);
         v3 c;
         float b1 = 0.f, b2 = 0.f;
         if (h.id != 0xffffffffu) {

@@ -759,3 +759,28 @@ def test_batch_latencies_count_the_lists(lib, tmp_path):
     finally:
         lib.crSetStream(None)
     assert -0.01 < min(apart) < 0.06, apart
+
+
+def test_measured_traversal_of_long_renders(lib, deep):
+    """crMeasureTraversal counts the search of the tree however many rays the
+    render has: the mean of its poses' own counts."""
+    import torch
+
+    _load(lib, deep)
+    n, spp, P = 1001, 32, 32
+    omm = _eye(n, "plain")
+    d_poses = torch.from_numpy(_poses(deep, P, 2)[9:]).cuda()
+    P -= 9
+    assert n * spp * P >= 2 ** 19
+    torch.cuda.synchronize()
+    counts = []
+    for per in (P, 1):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        a = np.zeros(2)
+        for k in range(0, P, per):
+            nv, tt = ctypes.c_double(), ctypes.c_double()
+            assert lib.crMeasureTraversal(d_poses[k:].data_ptr(), per, ctypes.byref(nv), ctypes.byref(tt)) == 0
+            a += np.array([nv.value, tt.value]) * per / P
+        counts.append(a)
+    assert np.allclose(counts[0], counts[1], rtol=1e-12) and counts[0][0] > 5
