@@ -333,6 +333,7 @@ struct Renderer {
   DevBuf<float4> extra;
   cudaEvent_t extraUsed = nullptr;
   bool extraTaken = false;  // since the last event
+  unsigned long long extraStream = 0;  // of the last use (cudaStreamGetId)
   bool conesOff = false; // crAutotune times variants and cut radii without cone lists
   float cutFactor = 0.f; // cut radius as a fraction of the scene extent (0: off)
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
@@ -754,8 +755,11 @@ struct Renderer {
   // launches on the current stream, issued while an ExtraUse lives.
   float4* takeExtra(size_t n) {
     if (!extra.tryEnsure(n)) return nullptr;
-    if (extraUsed) check(cudaStreamWaitEvent(stream(), extraUsed, 0), "cudaStreamWaitEvent");
-    else check(cudaEventCreateWithFlags(&extraUsed, cudaEventDisableTiming), "cudaEventCreate");
+    unsigned long long id = 0;  // unlike the handle, never that of an earlier stream
+    check(cudaStreamGetId(stream(), &id), "cudaStreamGetId");
+    if (!extraUsed) check(cudaEventCreateWithFlags(&extraUsed, cudaEventDisableTiming), "cudaEventCreate");
+    else if (id != extraStream) check(cudaStreamWaitEvent(stream(), extraUsed, 0), "cudaStreamWaitEvent");
+    extraStream = id;
     extraTaken = true;
     return extra.ptr;
   }
