@@ -33,6 +33,11 @@ constexpr uint32_t kVersion = 1;
 }  // namespace
 
 void Denoiser::release() {
+  releaseNetwork();
+  releaseOrders();
+}
+
+void Denoiser::releaseNetwork() {
   for (void* p : {static_cast<void*>(params_), static_cast<void*>(grads_), static_cast<void*>(m_), static_cast<void*>(v_),
                   wbf_, wbfT_, Xb_, static_cast<void*>(baseb_), static_cast<void*>(targetb_), static_cast<void*>(zs_), h_[0],
                   h_[1], h_[2], dz_[0], dz_[1], dz_[2], static_cast<void*>(y_), static_cast<void*>(dyf_), dyb_,
@@ -55,7 +60,7 @@ void Denoiser::release() {
 }
 
 void Denoiser::init(uint32_t seed, cudaStream_t s) {
-  release();
+  releaseNetwork();
   params_ = dalloc<float>(kParams);
   grads_ = dalloc<float>(kParams);
   m_ = dalloc<float>(kParams);
@@ -113,6 +118,25 @@ void Denoiser::ensureParts(int rows) {
   partTiles_ = 0;
   part_ = dalloc<float>(static_cast<size_t>(tiles) * kParams);
   partTiles_ = tiles;
+}
+
+void Denoiser::ensureOrders() {
+  const size_t bytes = 2 * (rows_ * 4 + sizeof(TrainState));
+  if (bytes <= orderBytes_) return;
+  releaseOrders();
+  ordersPinned_ = cudaHostAlloc(&orders_, bytes, cudaHostAllocDefault) == cudaSuccess;
+  if (!ordersPinned_) {
+    cudaGetLastError();
+    orders_ = ::operator new(bytes);
+  }
+  orderBytes_ = bytes;
+}
+
+void Denoiser::releaseOrders() {
+  if (orders_ && ordersPinned_) cudaFreeHost(orders_);
+  if (orders_ && !ordersPinned_) ::operator delete(orders_);
+  orders_ = nullptr;
+  orderBytes_ = 0;
 }
 
 void Denoiser::stepTc(const void* X, const float* base, const float* target, const uint32_t* order,
@@ -241,10 +265,12 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
   // (it sets up what the kernels need), the next is captured as a CUDA graph
   // and replayed for the rest; the host draws the next epoch's order while
   // they run.
+  ensureOrders();
+  TrainState* at = static_cast<TrainState*>(orders_);  // of the two orders that follow
+  uint32_t* perm = reinterpret_cast<uint32_t*>(at + 2);
   std::mt19937 rng(seed);
-  std::vector<uint32_t> perm(rows_);
-  std::iota(perm.begin(), perm.end(), 0u);
-  std::shuffle(perm.begin(), perm.end(), rng);
+  std::iota(perm, perm + rows_, 0u);
+  std::shuffle(perm, perm + rows_, rng);
   std::vector<float> sched(3 * static_cast<size_t>(steps));
   const float b1 = 0.9f, b2 = 0.999f;
   for (int st = 0; st < steps; ++st) {
@@ -255,7 +281,11 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
     sched[3 * st + 1] = 1.f / (1.f - powf(b1, t));
     sched[3 * st + 2] = 1.f / (1.f - powf(b2, t));
   }
-  // Two orders: the next epoch's is drawn while this one's steps run.
+  // Two orders, on the host and on the device: the next epoch's is drawn while
+  // this one's steps run.  The host's are page-locked, so a queued copy reads
+  // them when its turn comes, and a half is only written again after its
+  // event (after the whole stream where page-locked memory is not to be had).
+  cudaEvent_t uploaded[2] = {nullptr, nullptr};
   uint32_t* permDev = dalloc<uint32_t>(2 * rows_);
   float* lossDev = dalloc<float>(static_cast<size_t>(steps));
   float* schedDev = dalloc<float>(sched.size());
@@ -265,13 +295,17 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
   auto cleanup = [&]() {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
+    for (cudaEvent_t e : uploaded)
+      if (e) cudaEventDestroy(e);
     dfree(permDev);
     dfree(lossDev);
     dfree(schedDev);
     dfree(state);
   };
   try {
-    ck(cudaMemcpyAsync(permDev, perm.data(), rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
+    for (cudaEvent_t& e : uploaded) ck(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+    ck(cudaMemcpyAsync(permDev, perm, rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
+    ck(cudaEventRecord(uploaded[0], s), "event");
     ck(cudaMemcpyAsync(schedDev, sched.data(), sched.size() * 4, cudaMemcpyHostToDevice, s), "schedule");
     ck(cudaMemsetAsync(lossDev, 0, static_cast<size_t>(steps) * 4, s), "memset");
     ck(cudaMemsetAsync(state, 0, sizeof(TrainState), s), "memset");
@@ -316,11 +350,16 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
       st += run;
       cursor += static_cast<size_t>(run) * static_cast<size_t>(batch);
       if (st < steps) {
+        const uint32_t* last = perm + half * rows_;
         half ^= 1u;
-        std::shuffle(perm.begin(), perm.end(), rng);
-        ck(cudaMemcpyAsync(permDev + half * rows_, perm.data(), rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
-        const TrainState at{st, static_cast<uint32_t>(half * rows_), 0u};
-        ck(cudaMemcpyAsync(state, &at, sizeof(at), cudaMemcpyHostToDevice, s), "state");
+        ck(ordersPinned_ ? cudaEventSynchronize(uploaded[half]) : cudaStreamSynchronize(s), "epoch");
+        uint32_t* next = perm + half * rows_;
+        std::copy(last, last + rows_, next);
+        std::shuffle(next, next + rows_, rng);
+        at[half] = TrainState{st, static_cast<uint32_t>(half * rows_), 0u};
+        ck(cudaMemcpyAsync(permDev + half * rows_, next, rows_ * 4, cudaMemcpyHostToDevice, s), "perm");
+        ck(cudaMemcpyAsync(state, at + half, sizeof(TrainState), cudaMemcpyHostToDevice, s), "state");
+        ck(cudaEventRecord(uploaded[half], s), "event");
         cursor = 0;
       }
     }
@@ -335,6 +374,7 @@ void Denoiser::train(int steps, int batch, float lr, uint32_t seed, float* loss,
       if (flags) throw std::runtime_error("a tcgen05 GEMM wait timed out during training");
     }
   } catch (...) {
+    cudaStreamSynchronize(s);  // copies that still read the orders
     cleanup();
     throw;
   }

@@ -84,6 +84,9 @@ class Denoiser {
   void stepTc(const void* X, const float* base, const float* target, const uint32_t* order, const uint32_t* offset,
               int rows, float* lossAcc, const int* lossIndex, const AdamTarget* adam, cudaStream_t s);
   void ensureParts(int rows);
+  void releaseNetwork();
+  void ensureOrders();
+  void releaseOrders();
   static constexpr int kTileRows = 128;
   static constexpr int kMaxTiles = 512;  // of one launch: 95 MB of gradient sums
 
@@ -117,6 +120,10 @@ class Denoiser {
   float* part_ = nullptr;
   float* carry_ = nullptr;
   int partTiles_ = 0;
+  // train()'s two shuffled orders on the host, behind their TrainStates; page-locked where possible
+  void* orders_ = nullptr;
+  size_t orderBytes_ = 0;
+  bool ordersPinned_ = false;
   // training set
   void* X_ = nullptr;
   float* base_ = nullptr;
