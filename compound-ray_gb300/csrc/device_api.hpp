@@ -381,6 +381,7 @@ struct BatchTables {
   const unsigned long long* cellBase = nullptr;
   const unsigned long long* coneBase = nullptr;
   unsigned long long tasksLists = 0, tasksOther = 0, cells = 0, lists = 0;
+  unsigned long long rays = 0;  // of the whole batch
   uint32_t nEyes = 0;
 };
 // The cone lists, the persistent launch over the warp tasks of the eyes that

@@ -932,6 +932,7 @@ void recordBatch(Renderer& r, Batch& b) {
     bases[n + i] = bt.tasksOther;
     bases[2 * n + i] = bt.cells;
     bases[3 * n + i] = bt.lists;
+    bt.rays += static_cast<unsigned long long>(be.eye.N) * be.eye.spp * be.P;
     if (!be.eye.N) continue;
     if (be.eye.cones) bt.lists += b.lists[i];
     (be.eye.cones ? bt.tasksLists : bt.tasksOther) += be.plan.tasks;

@@ -816,7 +816,6 @@ __device__ __forceinline__ v3 rayOrigin(v3 p, v3 x, v3 y, v3 z, v3 rel) {
 // and their origin (t in [offset, 0)), gets no list either.
 // ---------------------------------------------------------------------------
 constexpr float kConeSigmas = 3.75f;
-constexpr float kConeMaxAngle = 0.5f;  // wider cones are searched from the root
 constexpr int kConeSteps = 64;         // node visits of one list at most
 constexpr uint32_t kConeFromRoot = 0xffffffffu;
 constexpr int kConeThreads = 128;
@@ -897,6 +896,8 @@ __device__ __forceinline__ bool coneTriangle(const Cone& c, float4 v0, float4 v1
 //       (the subtraction each ray would make).  w: the entry distance, the
 //       ref (as in the BVH, a leaf as one entry for each of its triangles that
 //       the cone meets while there is room), the triangle's id.
+// maxAngle: wider cones (half-angles in rad) are searched from the root
+// (coneMaxAngle).
 // work: the thread's column of a [kConeEntries][kConeThreads] array, holding
 // the entries found (from the front) and the traversal stack (from the back).
 //
@@ -904,7 +905,7 @@ __device__ __forceinline__ bool coneTriangle(const Cone& c, float4 v0, float4 v1
 // 32 neighbouring ommatidia share a warp, whose lanes walk nearly the same
 // nodes, instead of the lanes of a warp sharing a list.
 __device__ __forceinline__ void coneList(const DevScene& sc, const float4* __restrict__ omm, uint32_t o,
-                                         const float4* __restrict__ pose, uint2* __restrict__ work,
+                                         const float4* __restrict__ pose, float maxAngle, uint2* __restrict__ work,
                                          float4* __restrict__ out) {
   const float4 P0 = __ldg(pose), X = __ldg(pose + 1), Y = __ldg(pose + 2), Z = __ldg(pose + 3);
   const float4 r0 = __ldg(omm + 2 * o), r1 = __ldg(omm + 2 * o + 1);
@@ -916,7 +917,7 @@ __device__ __forceinline__ void coneList(const DevScene& sc, const float4* __res
   const float tol = 1e-3f;
   const bool ok = fabsf(dot(ax, ax) - 1.0f) <= tol && fabsf(dot(x, x) - 1.0f) <= tol &&
                   fabsf(dot(y, y) - 1.0f) <= tol && fabsf(dot(z, z) - 1.0f) <= tol && fabsf(dot(x, y)) <= tol &&
-                  fabsf(dot(x, z)) <= tol && fabsf(dot(y, z)) <= tol && theta <= kConeMaxAngle &&
+                  fabsf(dot(x, z)) <= tol && fabsf(dot(y, z)) <= tol && theta <= maxAngle &&
                   fabsf(c.o.x) + fabsf(c.o.y) + fabsf(c.o.z) < 1e15f && fpo >= 0.0f && fpo < 1e15f;
   if (!ok) {  // also for NaNs
     out[0] = make_float4(__uint_as_float(kConeFromRoot), c.o.x, c.o.y, c.o.z);
@@ -1433,7 +1434,7 @@ __global__ void drawsKernel(DevEye eye, uint32_t P) {
 // the GPU idle when they run alone (1000 poses x 1000 ommatidia x 32 samples:
 // 0.97 ms as a launch of their own, 0.94 here).
 __global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye eye, const float4* __restrict__ poses,
-                                                           uint32_t P, uint32_t drawBlocks) {
+                                                           uint32_t P, float maxAngle, uint32_t drawBlocks) {
   __shared__ uint2 work[kConeEntries * kConeThreads];
   if (blockIdx.x < drawBlocks) {
     drawStream(eye, P, static_cast<size_t>(blockIdx.x) * kConeThreads + threadIdx.x);
@@ -1443,7 +1444,7 @@ __global__ void __launch_bounds__(kConeThreads) coneKernel(DevScene sc, DevEye e
   if (i >= static_cast<uint64_t>(P) * eye.N) return;
   const uint32_t p = static_cast<uint32_t>(i / eye.N), slot = static_cast<uint32_t>(i - static_cast<uint64_t>(p) * eye.N);
   const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
-  coneList(sc, eye.omm, o, poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+  coneList(sc, eye.omm, o, poses + 4 * static_cast<size_t>(p), maxAngle, work + threadIdx.x,
            eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
@@ -2286,7 +2287,7 @@ __global__ void batchCutKernel(DevScene sc, const BatchEye* __restrict__ eyes, u
 // order.
 __global__ void __launch_bounds__(kConeThreads)
     batchConeKernel(DevScene sc, const BatchEye* __restrict__ eyes, const unsigned long long* __restrict__ coneBase,
-                    uint32_t nEyes, unsigned long long totalLists, unsigned long long* ctrl) {
+                    uint32_t nEyes, unsigned long long totalLists, float maxAngle, unsigned long long* ctrl) {
   __shared__ uint2 work[kConeEntries * kConeThreads];
   if (blockIdx.x == 0 && threadIdx.x == 0) atomicMin(&ctrl[1], globalTimerNs());
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
@@ -2296,7 +2297,7 @@ __global__ void __launch_bounds__(kConeThreads)
   const uint64_t local = i - coneBase[e];
   const uint32_t p = static_cast<uint32_t>(local / eye.N), slot = static_cast<uint32_t>(local % eye.N);
   const uint32_t o = eye.order ? __ldg(eye.order + slot) : slot;
-  coneList(sc, eye.omm, o, eyes[e].poses + 4 * static_cast<size_t>(p), work + threadIdx.x,
+  coneList(sc, eye.omm, o, eyes[e].poses + 4 * static_cast<size_t>(p), maxAngle, work + threadIdx.x,
            eye.cones + (static_cast<size_t>(p) * eye.N + o) * kConeStride);
 }
 
@@ -2531,6 +2532,27 @@ static bool coneWorth(const DevScene& scene, uint32_t segment, uint64_t rays) {
   return deep && rays >= 1ull << 20;
 }
 
+// Half-angle (3.75 standard deviations) of the widest cone that gets a list; the
+// rays of wider ones search from the root.  A wide cone meets more than a list
+// holds: building it costs the most and saves the least, and short launches
+// wait for it.  0.25, 0.35, 0.4 and 0.5 rad are acceptance angles of 8.9, 12.4,
+// 14.2 and 17.8 degrees.  Speed-up over the renders without lists (tuned cut)
+// of acceptance angles 9.5 / 13 / 17.6, with lists and from the root:
+//   terrain, 6000 x 32, 0.6 M rays   1.11 0.94 0.85, 1.10 1.11 1.16  (no cut)
+//            6000 x 256, 1.5 M       1.50 1.27 1.18, 1.01 1.13 1.24
+//            6000 x 256, 98 M        2.23 1.69 1.44, 0.95 1.16 1.33
+//            6000 x 16, 0.6 M        1.11 0.98 0.85, 1.06 1.08 1.11  (12 samples, no cut)
+//            6000 x 8, 12 M          1.39 1.12 0.96, 1.09 1.12 1.15  (no cut)
+//   box      6000 x 32, 2.3 M        1.07 1.00 0.93, 1.14 1.13 1.14
+//            6000 x 256, 15 M        1.28 1.11 0.98, 0.97 0.99 0.99
+//            6000 x 16, 24 M         1.07 0.95 0.86, 1.00 1.00 1.01
+constexpr float kConeEntryAngle = 0.25f;  // of adaptive entries: lists 1.34 1.26 1.21, from the root 1.40 1.34 1.31
+static float coneMaxAngle(const DevScene& scene, uint32_t segment, uint64_t rays) {
+  const bool deep = scene.triCount >= kConeDeepTris, full = segment == 32;
+  if (rays >= 1ull << 22 && (full || deep)) return full ? 0.5f : 0.35f;
+  return deep && full && rays >= 1ull << 20 ? 0.4f : 0.25f;
+}
+
 size_t batchConeLists(const DevScene& scene, const WarpPlan& plan, uint32_t N, uint32_t P, uint64_t batchRays) {
   if (scene.width != 2 || plan.segWidth != 32 || !coneWorth(scene, plan.segWidth, batchRays)) return 0;
   return static_cast<size_t>(P) * N;
@@ -2659,14 +2681,15 @@ cudaError_t runRenderWidth(const DevScene& scene, const DevEye& eye, const float
 
 // draw: pre-draws the launch's random numbers too.
 static cudaError_t launchCones(const DevScene& scene, const DevEye& eye, const float4* poses, uint32_t P, bool draw,
-                               cudaStream_t stream) {
+                               uint32_t segment, cudaStream_t stream) {
   const uint64_t lists = static_cast<uint64_t>(P) * eye.N;
+  const float maxAngle = coneMaxAngle(scene, segment, lists * eye.spp);
   const uint64_t streams = draw ? static_cast<uint64_t>(eye.N) * eye.spp : 0;
   const uint64_t drawBlocks = (streams + kConeThreads - 1) / kConeThreads;
   const uint64_t blocks = drawBlocks + (lists + kConeThreads - 1) / kConeThreads;
   if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
   coneKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, eye, poses, P,
-                                                                        static_cast<uint32_t>(drawBlocks));
+                                                                        maxAngle, static_cast<uint32_t>(drawBlocks));
   return cudaGetLastError();
 }
 
@@ -2696,7 +2719,7 @@ cudaError_t launchRender(const DevScene& scene, const DevEye& eye, const float4*
     plan = splitPoses(plan, P, warps * std::max(256u, P) / 256);
   }
   if (eye.cones) {
-    const cudaError_t e = launchCones(scene, eye, poses, P, eye.draws != nullptr, stream);
+    const cudaError_t e = launchCones(scene, eye, poses, P, eye.draws != nullptr, plan.segWidth, stream);
     if (e != cudaSuccess) return e;
   } else if (eye.cuts && (scene.width == 2 || rec || scene.lighting)) {  // the wide BVH searches without a cut
     if (!(eye.cutRadius > 0.f)) return cudaErrorInvalidValue;
@@ -2753,7 +2776,7 @@ cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float
   plan = splitPoses(plan, P, (deep ? 8 : 4) * kFillWarps);
   if (eye.cones) {
     if (featureConeLists(scene, eye.N, eye.spp, P) == 0) return cudaErrorInvalidValue;
-    const cudaError_t e = launchCones(scene, eye, poses, P, false, stream);
+    const cudaError_t e = launchCones(scene, eye, poses, P, false, plan.segWidth, stream);
     if (e != cudaSuccess) return e;
     return runRender<3, kConeRegs>(scene, eye, poses, P, plan, stats, nullptr, errFlag, nullptr, nullptr, stream);
   }
@@ -2811,7 +2834,8 @@ cudaError_t launchBatch(const DevScene& scene, const BatchTables& b, unsigned lo
     const uint64_t blocks = (b.lists + kConeThreads - 1) / kConeThreads;
     if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
     batchConeKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, b.eyes, b.coneBase, nEyes,
-                                                                                b.lists, ctrl);
+                                                                                b.lists, coneMaxAngle(scene, 32, b.rays),
+                                                                                ctrl);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
@@ -3182,12 +3206,13 @@ __global__ void __launch_bounds__(128, kMinBlocks)
 // Cone lists of a bucket's entries, list i at B.cones + i * kConeStride.
 __global__ void __launch_bounds__(kConeThreads)
     entryConeKernel(DevScene sc, const float4* __restrict__ omm, uint32_t N, const float4* __restrict__ poses,
-                    const uint32_t* __restrict__ entries, uint64_t count, float4* __restrict__ cones) {
+                    const uint32_t* __restrict__ entries, uint64_t count, float maxAngle,
+                    float4* __restrict__ cones) {
   __shared__ uint2 work[kConeEntries * kConeThreads];
   const uint64_t i = static_cast<uint64_t>(blockIdx.x) * kConeThreads + threadIdx.x;
   if (i >= count) return;
   const uint32_t e = entries[i], p = e / N;
-  coneList(sc, omm, e - p * N, poses + 4 * static_cast<size_t>(p), work + threadIdx.x, cones + i * kConeStride);
+  coneList(sc, omm, e - p * N, poses + 4 * static_cast<size_t>(p), maxAngle, work + threadIdx.x, cones + i * kConeStride);
 }
 
 // The adaptive render through cone lists (entries of at least 16 samples, see
@@ -3803,7 +3828,7 @@ cudaError_t launchEntryCones(const DevScene& scene, const float4* omm, uint32_t 
   const uint64_t blocks = (count + kConeThreads - 1) / kConeThreads;
   if (blocks > 0x7fffffffULL) return cudaErrorInvalidConfiguration;
   entryConeKernel<<<static_cast<unsigned>(blocks), kConeThreads, 0, stream>>>(scene, omm, N, poses, entries, count,
-                                                                             cones);
+                                                                             kConeEntryAngle, cones);
   return cudaGetLastError();
 }
 

@@ -784,3 +784,21 @@ def test_measured_traversal_of_long_renders(lib, deep):
             a += np.array([nv.value, tt.value]) * per / P
         counts.append(a)
     assert np.allclose(counts[0], counts[1], rtol=1e-12) and counts[0][0] > 5
+
+
+# rays around each line of coneMaxAngle, for every segment width and depth of tree
+@pytest.mark.parametrize("on_deep,n,spp,P", [(True, 1301, 32, 13), (True, 1301, 32, 50), (True, 1301, 32, 110),
+                                             (True, 1301, 16, 30), (True, 1301, 16, 250), (True, 1301, 8, 200),
+                                             (True, 1301, 8, 410), (False, 1301, 32, 55), (False, 1301, 32, 110),
+                                             (False, 1301, 16, 210)])
+def test_wide_cones(lib, small, deep, on_deep, n, spp, P):
+    """Acceptance angles of 6 to 20 degrees: some get lists, some do not,
+    depending on the launch."""
+    info = deep if on_deep else small
+    _load(lib, info)
+    omm = _eye(n, "plain")
+    omm[:, 6] = np.radians(np.random.default_rng(n).uniform(6.0, 20.0, n))
+    with_lists, without = _both(lib, omm, spp, _poses(info, P, n))
+    assert with_lists[3] >= 400 * n * min(P, 256)
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
