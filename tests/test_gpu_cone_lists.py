@@ -802,3 +802,79 @@ def test_wide_cones(lib, small, deep, on_deep, n, spp, P):
     assert with_lists[3] >= 400 * n * min(P, 256)
     for x, y in zip(with_lists[:3], without[:3]):
         assert np.array_equal(x, y, equal_nan=True)
+
+
+def test_batch_of_odd_eyes(lib, tmp_path):
+    """Odd eyes and poses in a batch with lists, against each eye's render
+    without."""
+    import torch
+
+    P, spp = 9, [33, 128]
+    info = scenes.batch_scene(str(tmp_path), n_eyes=2, poses_per_eye=P, n_min=2000, n_max=2000)
+    lib.setOmmatidia.argtypes = [ctypes.c_void_p, ctypes.c_size_t]
+    lib.loadGlTFscene(info["gltf"].encode())
+    cams = np.arange(info["first_batch_camera"], info["first_batch_camera"] + 2, dtype=np.int32)
+    boxes = scenes.small_scene(str(tmp_path / "b"))["boxes"]
+    d_poses = torch.from_numpy(np.concatenate([_poses({"boxes": boxes}, P, k) for k in (1, 2)])).cuda()
+    omm = _eye(2000, "odd")
+    out = torch.full((2, P, 2000, 3), -1.0, device="cuda")
+    want = []
+    for batch in (False, True):
+        for i, c in enumerate(cams):
+            lib.gotoCamera(int(c))
+            lib.setOmmatidia(omm.ctypes.data, 2000)
+            lib.setCurrentEyeSamplesPerOmmatidium(spp[i])
+            _render(lib, lib.crRenderPosesDevice, d_poses[i * P:], 1, 2000)
+            if not batch:
+                want.append(_render(lib, lib.crRenderPosesDeviceNoAlloc, d_poses[i * P:], P, 2000))
+    h = lib.crBatchCreate(cams, 2, P, d_poses.data_ptr(), out.data_ptr())
+    assert h > 0 and lib.crBatchLaunch(h) == 0 and lib.crSynchronize() == 0, eh.lastError(lib)
+    lib.crBatchDestroy(h)
+    for i in range(2):
+        assert np.array_equal(out[i].cpu().numpy(), want[i], equal_nan=True)
+
+
+@pytest.mark.parametrize("spp", [17, 64])
+def test_lit_renders_through_lists(lib, small, spp):
+    _load(lib, small)
+    n = 701
+    P = max(9, 2 ** 21 // (n * spp) + 2)
+    assert lib.crSetLighting(1) == 0
+    try:
+        with_lists, without = _both(lib, _eye(n, "odd"), spp, _poses(small, P, spp))
+    finally:
+        lib.crSetLighting(0)
+    assert with_lists[3] >= 400 * n * P
+    for x, y in zip(with_lists[:3], without[:3]):
+        assert np.array_equal(x, y, equal_nan=True)
+
+
+@pytest.mark.parametrize("pose", [0, 1, 2, 3, 4, 5, 7])
+def test_recorded_frames_through_lists(lib, small, deep, pose):
+    """A recorded frame of an odd eye at odd poses: the colours of the same
+    frame without lists, and records that add up to them."""
+    import torch
+
+    info = deep if pose % 2 else small
+    _load(lib, info)
+    n, spp = (6001, 350) if info is small else (3001, 200)
+    omm, p = _eye(n, "odd"), _poses(info, 9, 4)[pose]
+    d_pose = torch.from_numpy(p.reshape(1, 16)).cuda()
+    got = []
+    for record in (True, False):
+        lib.setOmmatidia(omm.ctypes.data, n)
+        lib.setCurrentEyeSamplesPerOmmatidium(spp)
+        _render(lib, lib.crRenderPosesDevice, d_pose, 1, n)
+        if record:
+            lib.setCameraPosition(*[float(v) for v in p[0:3]])
+            lib.setCameraLocalSpace(*[float(v) for k in (4, 8, 12) for v in p[k:k + 3]])
+            rec, col = np.zeros((n, spp), eh.RAY_RECORD_DTYPE), np.zeros((n, 3), np.float32)
+            assert lib.crRenderFrameRecorded(rec.ctypes.data) == 0, eh.lastError(lib)
+            assert lib.getOmmatidialColoursF32(col) == 0
+            got.append(col)
+        else:
+            got.append(_render(lib, lib.crRenderPosesDeviceNoAlloc, d_pose, 1, n)[0])
+    assert np.array_equal(got[0], got[1], equal_nan=True)
+    total = rec["rgb"].sum(1, dtype=np.float64) / spp
+    ok = np.isfinite(got[0])
+    assert np.allclose(total[ok], got[0][ok], rtol=1e-4, atol=1e-6)
