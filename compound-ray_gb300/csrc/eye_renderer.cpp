@@ -53,9 +53,10 @@ size_t& devCap() {
   return cap;
 }
 
-// Gives back memory that only makes renders faster (Renderer::extra, then the
-// batches' lists, one batch at a time); true when there was some.  An
-// allocation that fails tries again after it.
+// Gives back memory that only makes renders faster (Renderer::extra, the
+// batches' lists, one batch at a time, then what the spherical projections
+// keep); true when there was some.  An allocation that fails tries again after
+// it.
 bool releaseOptional();
 
 template <typename T>
@@ -169,13 +170,16 @@ struct EyeDev {
     gridsBuilt = false;
     lensBuilt = false;
   }
-  void release() {
+  void releaseProjection() {
     lens.release();
+    releaseGrids();
+  }
+  void release() {
     omm.release();
     order.release();
     rng.release();
     sums.release();
-    releaseGrids();
+    releaseProjection();
     N = spp = 0;
     configured = false;
     haveSums = false;
@@ -188,9 +192,11 @@ struct EyeDev {
 // Index 0 is left out (it is every pixel's starting candidate), and so are
 // vectors of zero or non-finite length (their angle is NaN and never wins).
 // Unit vectors in double pick the cell; G ~ sqrt(n) / 3 puts about two
-// candidates in a cell that the sphere crosses.
-void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_t st) {
+// candidates in a cell that the sphere crosses.  False, and no grids, when there
+// is no memory for the candidates' vectors.
+bool buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_t st) {
   const size_t N = omm.size();
+  size_t count[4] = {0, 0, 0, 0};
   for (int which = 0; which < 4; ++which) {
     SphereGrid& g = e.grids[which];
     std::vector<uint32_t> idx;
@@ -225,16 +231,27 @@ void buildSphereGrids(EyeDev& e, const std::vector<Ommatidium>& omm, cudaStream_
     for (size_t k = 0; k < idx.size(); ++k) items[fill[cellOf[k]]++] = idx[k];
     g.start.ensure(cells + 1);
     g.items.ensure(items.size());
-    g.vecs.ensure(items.size());
     check(cudaMemcpyAsync(g.start.ptr, start.data(), start.size() * 4, cudaMemcpyHostToDevice, st), "cudaMemcpy");
     check(cudaMemcpyAsync(g.items.ptr, items.data(), items.size() * 4, cudaMemcpyHostToDevice, st), "cudaMemcpy");
-    check(launchGridVecs(e.omm.ptr, e.lens.ptr, e.N, which == 0, g.items.ptr, static_cast<uint32_t>(items.size()),
-                         g.vecs.ptr, st),
-          "projection grid");
     check(cudaStreamSynchronize(st), "projection grid upload");
     g.G = G;
+    count[which] = items.size();
+  }
+  for (int which = 0; which < 4; ++which) {
+    SphereGrid& g = e.grids[which];
+    if (!count[which]) continue;
+    while (!g.vecs.tryEnsure(count[which]))
+      if (!releaseOptional()) {
+        e.releaseGrids();
+        e.lensBuilt = true;
+        return false;
+      }
+    check(launchGridVecs(e.omm.ptr, e.lens.ptr, e.N, which == 0, g.items.ptr, static_cast<uint32_t>(count[which]),
+                         g.vecs.ptr, st),
+          "projection grid");
   }
   e.gridsBuilt = true;
+  return true;
 }
 
 constexpr uint32_t kMaxPosesPerLaunch = 256;
@@ -339,6 +356,7 @@ struct Renderer {
   // Timings of the last crAutotune (ms): variants 0-2, block 128/256/512,
   // samples per warp 8/16/32, cut radius 0, 1/256 .. 1/16 of the extent.
   std::vector<float> tuneTimes;
+  bool projecting = false;  // project() is using an eye's lengths and grids
   bool projectionGrid = true;  // spherical projections search candidate grids (false: every candidate)
   DevBuf<float> batchOut;
   DevBuf<uint32_t> err;
@@ -825,6 +843,11 @@ struct Renderer {
 
   void project(EyeDev& e, const std::vector<Ommatidium>& omm, const std::string& shader, const RayRecord* rec) {
     ensureFrame();
+    struct Projecting {
+      bool& on;
+      ~Projecting() { on = false; }
+    } guard{projecting};
+    projecting = true;
     const int kind = projectionKind(shader);
     if (kind < 10) {
       check(launchProject(e.sums.ptr, e.N, frame.ptr, width, height, kind, stream()), "projection launch");
@@ -836,8 +859,8 @@ struct Renderer {
         e.lensBuilt = true;
       }
       SphereGridSet set;
-      if (projectionGrid) {
-        if (!e.gridsBuilt) buildSphereGrids(e, omm, stream());
+      const bool grid = projectionGrid && (e.gridsBuilt || buildSphereGrids(e, omm, stream()));
+      if (grid) {
         for (int k = 0; k < 4; ++k) {
           set.g[k].start = e.grids[k].start.ptr;
           set.g[k].items = e.grids[k].items.ptr;
@@ -846,7 +869,7 @@ struct Renderer {
         }
       }
       check(launchSpherical(e.omm.ptr, e.lens.ptr, e.N, e.sums.ptr, frame.ptr, width, height, kind - 10,
-                            projectionGrid ? &set : nullptr, stream()),
+                            grid ? &set : nullptr, stream()),
             "projection launch");
     } else {
       check(launchRawSamples(rec, e.N, e.spp, frame.ptr, width, height, stream()), "projection launch");
@@ -909,7 +932,13 @@ bool releaseOptional() {
       kv.second.cones.release();
       return true;
     }
-  return false;
+  bool had = false;
+  if (!R().projecting)
+    for (EyeDev& e : R().eyes) {
+      had = had || e.lens.ptr;
+      e.releaseProjection();
+    }
+  return had;
 }
 
 void releaseBatches() {
