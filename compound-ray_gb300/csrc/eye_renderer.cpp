@@ -769,9 +769,16 @@ struct Renderer {
     check(cudaStreamIsCapturing(stream(), &st), "cudaStreamIsCapturing");
     return st != cudaStreamCaptureStatusNone;
   }
-  // `extra` with room for n float4, or null; not while capturing().  For
-  // launches on the current stream, issued while an ExtraUse lives.
+  // `extra` with room for n float4 (at most a quarter of the free memory: it
+  // stays, and other allocators must find room beside it), or null; not while
+  // capturing().  For launches on the current stream, issued while an ExtraUse
+  // lives.
   float4* takeExtra(size_t n) {
+    if (n > extra.count) {
+      size_t freeBytes = 0, totalBytes = 0;
+      check(cudaMemGetInfo(&freeBytes, &totalBytes), "cudaMemGetInfo");
+      if (n > (freeBytes / sizeof(float4) + extra.count) / 4) return nullptr;
+    }
     if (!extra.tryEnsure(n)) return nullptr;
     unsigned long long id = 0;  // unlike the handle, never that of an earlier stream
     check(cudaStreamGetId(stream(), &id), "cudaStreamGetId");
