@@ -55,10 +55,9 @@ namespace {
 constexpr int kTcRows = 128;
 constexpr int kFeatThreads = 512;  // feature warps 0-15: four threads per row
 constexpr int kNetThreads = 128;   // a network group's warps: one per accumulator lane quarter
-constexpr uint32_t kNetShares = kNetThreads / 128;
 constexpr int kNetGroups = 4;
 constexpr int kTcThreads = kFeatThreads + kNetGroups * kNetThreads;
-constexpr int kTcBuffers = 4;
+constexpr int kTcBuffers = kNetGroups;  // tile buffers: group g works in buffer g
 constexpr int kTmemCols = 128 * kNetGroups;
 constexpr uint32_t kSpinLimit = 1u << 26;  // bounded waits (far longer than one layer's MMAs)
 
@@ -423,7 +422,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
   const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kTcRows;
 
   if (tid < kFeatThreads) {
-    // Feature warps: tile i of this block into buffer i mod 3.
+    // Feature warps: tile i of this block into buffer i mod kTcBuffers.
     const uint32_t r = static_cast<uint32_t>(tid & (kTcRows - 1)), q = static_cast<uint32_t>(tid / kTcRows);
     RowWalk row(static_cast<uint64_t>(blockIdx.x) * kTcRows + r, stride, N);
     // A row's neighbours and their statistics are dependent loads: the
@@ -466,13 +465,12 @@ __global__ void __launch_bounds__(kTcThreads, 1)
       }
     }
   } else {
-    // Network group g: the four layers of tiles g, g + 2, ... of this block.
+    // Network group g: the four layers of tiles g, g + kNetGroups, ... of this
+    // block, in buffer g.
     const int g = (tid - kFeatThreads) / kNetThreads;
     const uint32_t tmem = *tmemSlot + 128u * static_cast<uint32_t>(g);
     const int lq = warp & 3;                                            // TMEM lane quarter this warp may read
-    const uint32_t share = static_cast<uint32_t>((warp - kFeatThreads / 32) >> 2) % kNetShares;
-    const uint32_t cBeg = share * (kMlpHidden / kNetShares), cEnd = cBeg + kMlpHidden / kNetShares;  // its columns
-    const int m = lq * 32 + (tid & 31);                                 // accumulator lane = tile row
+    const int m = lq * 32 + (tid & 31);                                 // accumulator lane: an output, last layer a tile row
     const uint32_t laneBase = tmem + (static_cast<uint32_t>(lq * 32) << 16);
     const bool issuer = tid == kFeatThreads + g * kNetThreads;
     const bool issuing = __shfl_sync(0xffffffffu, warp, 0) == (kFeatThreads + g * kNetThreads) / 32;  // the issuer's warp
@@ -481,9 +479,9 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     bool ok = true, pending = false;  // pending: a commit to mmaBar not yet waited for
     const uint64_t first = blockIdx.x + static_cast<uint64_t>(g) * gridDim.x;
     RowWalk row(first * kTcRows + static_cast<uint64_t>(m), kNetGroups * stride, N);
-    uint32_t b = static_cast<uint32_t>(g), round = 0;
-    for (uint64_t tile = first; tile < tiles; tile += kNetGroups * static_cast<uint64_t>(gridDim.x)) {
-      const uint32_t h = smemAddr(sm + kOffB0) + b * kActBytes;
+    const uint32_t b = static_cast<uint32_t>(g), h = smemAddr(sm + kOffB0) + b * kActBytes;
+    uint32_t round = 0;
+    for (uint64_t tile = first; tile < tiles; tile += kNetGroups * static_cast<uint64_t>(gridDim.x), ++round) {
       for (int layer = 0; layer < 4; ++layer) {
         const uint32_t K = layer == 0 ? kFeatureWidth : kMlpHidden;
         if (issuing && (layer > 0 || __all_sync(0xffffffffu, waitParity(fullBar(b), round & 1u)))) {
@@ -517,7 +515,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
           if (layer < 3) {
             const float own = bias[layer * kMlpHidden + m];
 #pragma unroll
-            for (uint32_t c0 = cBeg; c0 < cEnd; c0 += 32u) {
+            for (uint32_t c0 = 0; c0 < kTcRows; c0 += 32u) {
               float v[32];
               tmemLoad32(laneBase + c0, v);
               const uint32_t hs = h + coreOffset(static_cast<uint32_t>(m), c0, kMlpHidden);
@@ -532,7 +530,7 @@ __global__ void __launch_bounds__(kTcThreads, 1)
                              : "memory");
               }
             }
-          } else if (share == 0) {
+          } else {
             float v[4];
             tmemLoad4(laneBase, v);
             if (row.pos < rows) {
@@ -560,11 +558,6 @@ __global__ void __launch_bounds__(kTcThreads, 1)
         break;
       }
       row.next();
-      b += kNetGroups;
-      if (b >= kTcBuffers) {
-        b -= kTcBuffers;
-        ++round;
-      }
     }
     if (!ok && pending && issuer) waitParity(mmaBar, phase ^ 1u);  // let a late commit land before the TMEM is freed
   }
