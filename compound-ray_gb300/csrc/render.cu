@@ -794,6 +794,19 @@ __device__ __forceinline__ v3 rayOrigin(v3 p, v3 x, v3 y, v3 z, v3 rel) {
   return p + x * rel.x + y * rel.y + z * rel.z;
 }
 
+// generateOffsetRay's perpendicular axis (shaders.cu:655-657), including its
+// test on the component sum.
+__device__ __forceinline__ v3 splayAxis(v3 axis) {
+  const v3 perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
+  return (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
+}
+// A sample's direction in the world: the axis splayed about `perp`, turned
+// about the axis, in the pose's frame.
+__device__ __forceinline__ v3 rayDirection(v3 axis, v3 perp, float splay, float turn, float4 X, float4 Y, float4 Z) {
+  const v3 rel = rotatePoint(rotatePoint(axis, splay, perp), turn, axis);
+  return mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
+}
+
 // ---------------------------------------------------------------------------
 // Cone lists.  All samples of one ommatidium at one pose share their origin
 // and leave within a few standard deviations of its axis, so what they can
@@ -1347,6 +1360,36 @@ __device__ __forceinline__ v3 shadeMiss(int miss, v3 dirIn) {
   return c;
 }
 
+// Unlit colour of a ray's hit or miss, with the hit's barycentrics (0 for a
+// miss).
+__device__ __forceinline__ v3 shadeRay(const DevScene& sc, const Hit& h, v3 dir, float& b1, float& b2) {
+  b1 = b2 = 0.f;
+  if (h.id == 0xffffffffu) return shadeMiss(sc.miss, dir);
+  b1 = xdiv(h.V, h.det);
+  b2 = xdiv(h.W, h.det);
+  return shadeHit(sc, h.pos, b1, b2);
+}
+
+__device__ __forceinline__ void putRecord(RayRecord& R, float nd, float ud, v3 org, v3 dir, const Hit& h, float b1,
+                                          float b2, v3 c) {
+  R.normalDraw = nd;
+  R.uniformDraw = ud;
+  R.ox = org.x;
+  R.oy = org.y;
+  R.oz = org.z;
+  R.dx = dir.x;
+  R.dy = dir.y;
+  R.dz = dir.z;
+  R.t = h.id != 0xffffffffu ? h.t : -1.0f;
+  R.b1 = b1;
+  R.b2 = b2;
+  R.hitId = h.id != 0xffffffffu ? static_cast<int32_t>(h.id) : -1;
+  R.r = c.x;
+  R.g = c.y;
+  R.b = c.z;
+  R.pad = 0.f;
+}
+
 // ---------------------------------------------------------------------------
 // Generator state transfer (structure of arrays, see DevEye).
 // ---------------------------------------------------------------------------
@@ -1667,10 +1710,7 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
     const v3 pos = mk(a.x, a.y, a.z);
     fpo = b.w;
     sd = b.z / FWHM_SD_RATIO;
-    // generateOffsetRay's perpendicular axis (shaders.cu:655-657), including
-    // its test on the component sum.
-    perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
-    perp = (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
+    perp = splayAxis(axis);
     relPos = relativeOrigin(pos, axis, fpo);
   }
   const float invSpp = 1.0f / static_cast<float>(eye.spp);
@@ -1819,25 +1859,8 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
       } else {
         c = shadeMiss(sc.miss, dir);
       }
-      if (kRecord && valid) {
-        RayRecord& R = rec[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s];
-        R.normalDraw = nd;
-        R.uniformDraw = ud;
-        R.ox = org.x;
-        R.oy = org.y;
-        R.oz = org.z;
-        R.dx = dir.x;
-        R.dy = dir.y;
-        R.dz = dir.z;
-        R.t = h.id != 0xffffffffu ? h.t : -1.0f;
-        R.b1 = b1;
-        R.b2 = b2;
-        R.hitId = h.id != 0xffffffffu ? static_cast<int32_t>(h.id) : -1;
-        R.r = c.x;
-        R.g = c.y;
-        R.b = c.z;
-        R.pad = 0.f;
-      }
+      if (kRecord && valid)
+        putRecord(rec[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s], nd, ud, org, dir, h, b1, b2, c);
       if (!kCone || valid) col = c * invSpp;
       if (kFeat && (!kCone || valid)) {
         fCost = static_cast<float>(nodeVisits + triTests - steps0) * invSpp;
@@ -1878,53 +1901,53 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         flushChunkSums(part, plan, eye, out, pg0, p + 1 - pg0);
       }
     } else {
-    for (uint32_t m = segWidth >> 1; m >= 1u; m >>= 1) {
-      col.x += __shfl_xor_sync(0xffffffffu, col.x, static_cast<int>(m));
-      col.y += __shfl_xor_sync(0xffffffffu, col.y, static_cast<int>(m));
-      col.z += __shfl_xor_sync(0xffffffffu, col.z, static_cast<int>(m));
-      if (kFeat) {
-        f2x += __shfl_xor_sync(0xffffffffu, f2x, static_cast<int>(m));
-        f2y += __shfl_xor_sync(0xffffffffu, f2y, static_cast<int>(m));
-        f2z += __shfl_xor_sync(0xffffffffu, f2z, static_cast<int>(m));
-        fHit += __shfl_xor_sync(0xffffffffu, fHit, static_cast<int>(m));
-        fT += __shfl_xor_sync(0xffffffffu, fT, static_cast<int>(m));
-        fnx += __shfl_xor_sync(0xffffffffu, fnx, static_cast<int>(m));
-        fny += __shfl_xor_sync(0xffffffffu, fny, static_cast<int>(m));
-        fnz += __shfl_xor_sync(0xffffffffu, fnz, static_cast<int>(m));
-        fCost += __shfl_xor_sync(0xffffffffu, fCost, static_cast<int>(m));
+      for (uint32_t m = segWidth >> 1; m >= 1u; m >>= 1) {
+        col.x += __shfl_xor_sync(0xffffffffu, col.x, static_cast<int>(m));
+        col.y += __shfl_xor_sync(0xffffffffu, col.y, static_cast<int>(m));
+        col.z += __shfl_xor_sync(0xffffffffu, col.z, static_cast<int>(m));
+        if (kFeat) {
+          f2x += __shfl_xor_sync(0xffffffffu, f2x, static_cast<int>(m));
+          f2y += __shfl_xor_sync(0xffffffffu, f2y, static_cast<int>(m));
+          f2z += __shfl_xor_sync(0xffffffffu, f2z, static_cast<int>(m));
+          fHit += __shfl_xor_sync(0xffffffffu, fHit, static_cast<int>(m));
+          fT += __shfl_xor_sync(0xffffffffu, fT, static_cast<int>(m));
+          fnx += __shfl_xor_sync(0xffffffffu, fnx, static_cast<int>(m));
+          fny += __shfl_xor_sync(0xffffffffu, fny, static_cast<int>(m));
+          fnz += __shfl_xor_sync(0xffffffffu, fnz, static_cast<int>(m));
+          fCost += __shfl_xor_sync(0xffffffffu, fCost, static_cast<int>(m));
+        }
       }
-    }
-    if (kFeat) {
+      if (kFeat) {
+        if (segLane == 0u && o < eye.N) {
+          float* dst = out + (static_cast<size_t>(p) * eye.N + o) * kFeatureStats;
+          dst[0] = col.x;
+          dst[1] = col.y;
+          dst[2] = col.z;
+          dst[3] = f2x;
+          dst[4] = f2y;
+          dst[5] = f2z;
+          dst[6] = fHit;
+          dst[7] = fT;
+          dst[8] = fnx;
+          dst[9] = fny;
+          dst[10] = fnz;
+          dst[kCostStat] = fCost;
+        }
+        continue;
+      }
       if (segLane == 0u && o < eye.N) {
-        float* dst = out + (static_cast<size_t>(p) * eye.N + o) * kFeatureStats;
+        float* dst = dst0 + (part ? (p - p0) % kInBlockPoses : p) * dstStride;
         dst[0] = col.x;
         dst[1] = col.y;
         dst[2] = col.z;
-        dst[3] = f2x;
-        dst[4] = f2y;
-        dst[5] = f2z;
-        dst[6] = fHit;
-        dst[7] = fT;
-        dst[8] = fnx;
-        dst[9] = fny;
-        dst[10] = fnz;
-        dst[kCostStat] = fCost;
       }
-      continue;
-    }
-    if (segLane == 0u && o < eye.N) {
-      float* dst = dst0 + (part ? (p - p0) % kInBlockPoses : p) * dstStride;
-      dst[0] = col.x;
-      dst[1] = col.y;
-      dst[2] = col.z;
-    }
-    // In-block sums: after each group of kInBlockPoses poses (and the last),
-    // the block sums the group's partials (every warp of the block runs the
-    // same poses, so all of them reach these barriers).
-    if (part && ((p - p0 + 1) % kInBlockPoses == 0 || p + 1 == p1)) {
-      const uint32_t pg0 = p0 + (p - p0) / kInBlockPoses * kInBlockPoses;
-      flushChunkSums(part, plan, eye, out, pg0, p + 1 - pg0);
-    }
+      // In-block sums: after each group of kInBlockPoses poses (and the last),
+      // the block sums the group's partials (every warp of the block runs the
+      // same poses, so all of them reach these barriers).
+      if (part && ((p - p0 + 1) % kInBlockPoses == 0 || p + 1 == p1)) {
+        const uint32_t pg0 = p0 + (p - p0) / kInBlockPoses * kInBlockPoses;
+        flushChunkSums(part, plan, eye, out, pg0, p + 1 - pg0);
+      }
     }
   }
   if (!kFeat && valid && !draws) {
@@ -1953,12 +1976,10 @@ __global__ void __maxnreg__(kRegs) renderKernel(DevScene sc, DevEye eye, const f
   const uint32_t lane = threadIdx.x & 31u;
   const uint64_t task = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
   if (task >= plan.tasks) return;  // whole warps exit together (never with inBlock: whole blocks)
+  float* part = nullptr;
+  if (kInBlock) part = reinterpret_cast<float*>(renderSmem + (kCone ? (blockDim.x >> 5) * coneWarpFloat4(1) : 0));
   renderTask<kMode, kWidth, kCone, kDraws>(sc, eye, poses, P, plan, task, out, scratch, errFlag, rec, nodeVisits,
-                                           triTests,
-                                   kInBlock ? reinterpret_cast<float*>(
-                                                  renderSmem + (kCone ? (blockDim.x >> 5) * coneWarpFloat4(1) : 0))
-                                            : nullptr,
-                                   renderSmem);
+                                           triTests, part, renderSmem);
   if (kCount) {
     unsigned long long nv = nodeVisits, tt = triTests;
     for (int m = 16; m >= 1; m >>= 1) {
@@ -2968,6 +2989,29 @@ constexpr uint32_t kAdaptiveWarps = 4;  // warps per 128-thread block
 
 __device__ __forceinline__ uint32_t lanesBelow(uint32_t lane) { return (1u << lane) - 1u; }
 
+// Bitonic sort by one warp of each task's (key, position) pairs, ascending:
+// tasks of 32 * 2^lspl slots, nSlots in all.
+__device__ __forceinline__ void sortSlots(uint32_t* key, uint32_t* idx, uint32_t lspl, uint32_t nSlots, uint32_t lane) {
+  const uint32_t n = 32u << lspl, lhalf = 4 + lspl;  // n / 2 = 2^lhalf compare-exchanges per task
+  for (uint32_t size = 2; size <= n; size <<= 1)
+    for (uint32_t ls = __ffs(size) - 2, stride = size >> 1; stride > 0; stride >>= 1, --ls) {
+      for (uint32_t m = lane; m < nSlots / 2; m += 32u) {
+        const uint32_t seg = (m >> lhalf) << (lhalf + 1), mm = m & ((1u << lhalf) - 1u);
+        const uint32_t lo = seg + (((mm >> ls) << ls) << 1) + (mm & (stride - 1u)), hi = lo + stride;
+        const bool up = ((lo - seg) & size) == 0u;
+        const uint32_t ka = key[lo], kb = key[hi];
+        if ((ka > kb) == up) {
+          key[lo] = kb;
+          key[hi] = ka;
+          const uint32_t t2 = idx[lo];
+          idx[lo] = idx[hi];
+          idx[hi] = t2;
+        }
+      }
+      __syncwarp();
+    }
+}
+
 template <int kWidth, int kMinBlocks = 5>
 __global__ void __launch_bounds__(128, kMinBlocks)
     adaptiveKernel(DevScene sc, const float4* __restrict__ omm, uint32_t N, const float4* __restrict__ poses,
@@ -3039,26 +3083,7 @@ __global__ void __launch_bounds__(128, kMinBlocks)
     }
   }
   __syncwarp();
-  if (sorted) {  // bitonic sort of each task's (key, position) pairs, ascending
-    const uint32_t n = 32u * spl, lhalf = 4 + lspl;  // n / 2 = 2^lhalf compare-exchanges per task
-    for (uint32_t size = 2; size <= n; size <<= 1)
-      for (uint32_t ls = __ffs(size) - 2, stride = size >> 1; stride > 0; stride >>= 1, --ls) {
-        for (uint32_t m = lane; m < nSlots / 2; m += 32u) {
-          const uint32_t seg = (m >> lhalf) << (lhalf + 1), mm = m & ((1u << lhalf) - 1u);
-          const uint32_t lo = seg + (((mm >> ls) << ls) << 1) + (mm & (stride - 1u)), hi = lo + stride;
-          const bool up = ((lo - seg) & size) == 0u;
-          const uint32_t ka = key[lo], kb = key[hi];
-          if ((ka > kb) == up) {
-            key[lo] = kb;
-            key[hi] = ka;
-            const uint32_t t2 = idx[lo];
-            idx[lo] = idx[hi];
-            idx[hi] = t2;
-          }
-        }
-        __syncwarp();
-      }
-  }
+  if (sorted) sortSlots(key, idx, lspl, nSlots, lane);
 
   // 2. Trace with refill.
   int stack[kWidth == 2 ? kStackSize : kWideStackSize];
@@ -3077,38 +3102,14 @@ __global__ void __launch_bounds__(128, kMinBlocks)
   for (;;) {
     // Shade the rays that finished in the last burst.
     if (slot >= 0 && !live) {
-      v3 c;
-      float b1 = 0.f, b2 = 0.f;
-      if (h.id != 0xffffffffu) {
-        b1 = xdiv(h.V, h.det);
-        b2 = xdiv(h.W, h.det);
-        c = shadeHit(sc, h.pos, b1, b2);
-      } else {
-        c = shadeMiss(sc.miss, dir);
-      }
+      float b1, b2;
+      const v3 c = shadeRay(sc, h, dir, b1, b2);
       const uint32_t j = static_cast<uint32_t>(slot);
       colR[j] = c.x;
       colG[j] = c.y;
       colB[j] = c.z;
-      if (rec) {
-        RayRecord& R = rec[static_cast<size_t>(slotEntry(j)) * spp + slotSample(j, slotK(j))];
-        R.normalDraw = nd;
-        R.uniformDraw = ud;
-        R.ox = org.x;
-        R.oy = org.y;
-        R.oz = org.z;
-        R.dx = dir.x;
-        R.dy = dir.y;
-        R.dz = dir.z;
-        R.t = h.id != 0xffffffffu ? h.t : -1.0f;
-        R.b1 = b1;
-        R.b2 = b2;
-        R.hitId = h.id != 0xffffffffu ? static_cast<int32_t>(h.id) : -1;
-        R.r = c.x;
-        R.g = c.y;
-        R.b = c.z;
-        R.pad = 0.f;
-      }
+      if (rec)
+        putRecord(rec[static_cast<size_t>(slotEntry(j)) * spp + slotSample(j, slotK(j))], nd, ud, org, dir, h, b1, b2, c);
       slot = -1;
     }
     // Refill once enough lanes are idle (or all are).
@@ -3130,16 +3131,12 @@ __global__ void __launch_bounds__(128, kMinBlocks)
             const v3 axis = mk(a.w, b.x, b.y);
             fpo = b.w;
             const float sd = b.z / FWHM_SD_RATIO;
-            v3 perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
-            perp = (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
-            const v3 relPos = mk(a.x, a.y, a.z) - normalize(axis) * fpo;
+            const v3 perp = splayAxis(axis);
+            const v3 relPos = relativeOrigin(mk(a.x, a.y, a.z), axis, fpo);
             const float4* pp = poses + 4 * p;
             const float4 P0 = __ldg(pp), X = __ldg(pp + 1), Y = __ldg(pp + 2), Z = __ldg(pp + 3);
-            org = mk(P0.x, P0.y, P0.z) + mk(X.x, X.y, X.z) * relPos.x + mk(Y.x, Y.y, Y.z) * relPos.y +
-                  mk(Z.x, Z.y, Z.z) * relPos.z;
-            const v3 splayed = rotatePoint(axis, nd * sd, perp);
-            const v3 rel = rotatePoint(splayed, ud * CR_PI_F, axis);
-            dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
+            org = rayOrigin(mk(P0.x, P0.y, P0.z), mk(X.x, X.y, X.z), mk(Y.x, Y.y, Y.z), mk(Z.x, Z.y, Z.z), relPos);
+            dir = rayDirection(axis, perp, nd * sd, ud * CR_PI_F, X, Y, Z);
             ray = setupRay(org, dir, sc.extent);
             dlen = sqrtf(dot(dir, dir));
             if (kWidth == 2) {
@@ -3266,7 +3263,7 @@ __global__ void __maxnreg__(kConeRegs)
   };
   fetch(0);
 
-  if (sorted) {  // as adaptiveKernel: draws and keys of every slot, then a bitonic sort of each task's
+  if (sorted) {  // as adaptiveKernel: draws and keys of every slot, sorted task by task
     const uint32_t nSlots = nTasks * spl * 32u;
     for (uint32_t j = lane; j < nSlots; j += 32u) {
       const uint32_t q = (j >> 5) >> lspl, k = j & ((32u << lspl) - 1u);
@@ -3280,24 +3277,7 @@ __global__ void __maxnreg__(kConeRegs)
       idx[j] = k;
     }
     __syncwarp();
-    const uint32_t n = 32u * spl, lhalf = 4 + lspl;
-    for (uint32_t size = 2; size <= n; size <<= 1)
-      for (uint32_t ls = __ffs(size) - 2, stride = size >> 1; stride > 0; stride >>= 1, --ls) {
-        for (uint32_t m = lane; m < nSlots / 2; m += 32u) {
-          const uint32_t seg = (m >> lhalf) << (lhalf + 1), mm = m & ((1u << lhalf) - 1u);
-          const uint32_t lo = seg + (((mm >> ls) << ls) << 1) + (mm & (stride - 1u)), hi = lo + stride;
-          const bool up = ((lo - seg) & size) == 0u;
-          const uint32_t ka = key[lo], kb = key[hi];
-          if ((ka > kb) == up) {
-            key[lo] = kb;
-            key[hi] = ka;
-            const uint32_t t2 = idx[lo];
-            idx[lo] = idx[hi];
-            idx[hi] = t2;
-          }
-        }
-        __syncwarp();
-      }
+    sortSlots(key, idx, lspl, nSlots, lane);
   }
 
   for (uint32_t q = 0; q < nTasks; ++q) {
@@ -3322,8 +3302,7 @@ __global__ void __maxnreg__(kConeRegs)
       const float4 a = __ldg(omm + 2 * o), b = __ldg(omm + 2 * o + 1);
       const v3 axis = mk(a.w, b.x, b.y);
       const float fpo = b.w, sd = b.z / FWHM_SD_RATIO;
-      v3 perp = cross(mk(0.0f, 1.0f, 0.0f), axis);
-      perp = (perp.x + perp.y + perp.z == 0.0f) ? mk(0.0f, 0.0f, 1.0f) : normalize(perp);
+      const v3 perp = splayAxis(axis);
       const float4* pp = poses + 4 * static_cast<size_t>(p);
       for (uint32_t r = 0; r < spl; ++r) {
         const uint32_t seg = q << (5 + lspl), j = seg + (r << 5) + lane;
@@ -3331,39 +3310,12 @@ __global__ void __maxnreg__(kConeRegs)
         const uint32_t sample = (chunk << (5 + lspl)) + k;
         const float2 d = sorted ? draw[seg + k] : netDraw(seed, e, sample);
         const float4 X = __ldg(pp + 1), Y = __ldg(pp + 2), Z = __ldg(pp + 3);
-        const v3 splayed = rotatePoint(axis, d.x * sd, perp);
-        const v3 rel = rotatePoint(splayed, d.y * CR_PI_F, axis);
-        const v3 dir = mk(X.x, X.y, X.z) * rel.x + mk(Y.x, Y.y, Y.z) * rel.y + mk(Z.x, Z.y, Z.z) * rel.z;
+        const v3 dir = rayDirection(axis, perp, d.x * sd, d.y * CR_PI_F, X, Y, Z);
         Hit h;
         traceCone(sc, list, listed, entries, org, dir, fpo, valid ? d.x : 0.0f, h, errFlag);
-        v3 c;
-        float b1 = 0.f, b2 = 0.f;
-        if (h.id != 0xffffffffu) {
-          b1 = xdiv(h.V, h.det);
-          b2 = xdiv(h.W, h.det);
-          c = shadeHit(sc, h.pos, b1, b2);
-        } else {
-          c = shadeMiss(sc.miss, dir);
-        }
-        if (kRec && valid) {
-          RayRecord& R = rec[static_cast<size_t>(i) * spp + sample];
-          R.normalDraw = d.x;
-          R.uniformDraw = d.y;
-          R.ox = org.x;
-          R.oy = org.y;
-          R.oz = org.z;
-          R.dx = dir.x;
-          R.dy = dir.y;
-          R.dz = dir.z;
-          R.t = h.id != 0xffffffffu ? h.t : -1.0f;
-          R.b1 = b1;
-          R.b2 = b2;
-          R.hitId = h.id != 0xffffffffu ? static_cast<int32_t>(h.id) : -1;
-          R.r = c.x;
-          R.g = c.y;
-          R.b = c.z;
-          R.pad = 0.f;
-        }
+        float b1, b2;
+        const v3 c = shadeRay(sc, h, dir, b1, b2);
+        if (kRec && valid) putRecord(rec[static_cast<size_t>(i) * spp + sample], d.x, d.y, org, dir, h, b1, b2, c);
         if (valid) {
           col.x = fmaf(c.x, invSpp, col.x);
           col.y = fmaf(c.y, invSpp, col.y);
