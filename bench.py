@@ -363,6 +363,16 @@ def run_reference(args):
     print(json.dumps(line), flush=True)
 
 
+# The result line: short, so that a reader of the output's end has it whole.
+# Everything measured stands in the "details:" line before it.
+HEADLINE = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "config", "eye_frames_per_s", "e2e", "gpu_launches", "clocks")
+
+
+def headline(line):
+    return {k: line[k] for k in HEADLINE if k in line}
+
+
 def run_ours(args):
     import torch
 
@@ -578,8 +588,9 @@ def run_ours(args):
                             "peak_source": "32 MB L2-resident device copy, read + write bytes, best of 20, "
                                            "measured in this run"},
                      "demand_bytes_per_ray": per_ray,
-                     "demand_note": "node, triangle and shading bytes the traversal requests per ray; L1 serves "
-                                    "most of them, so they are not an L2 or DRAM figure",
+                     "demand_note": "node, triangle and shading bytes that a search of the tree from its root "
+                                    "requests per ray (fewer through cone lists); L1 serves most of them, so they "
+                                    "are not an L2 or DRAM figure",
                      "hbm_peak_gbs": hbm_peak, "hbm_peak_source": src,
                      "node_visits_per_ray": nodes.value, "tri_tests_per_ray": tris.value,
                      "hit_fraction": hit_frac, "launch_ms": statistics.mean(full), "rays_per_launch": rays_launch,
@@ -609,7 +620,8 @@ def run_ours(args):
         sm = scenes.small_scene(os.path.join(tempfile.gettempdir(), "cr_bench_small_%d" % scenes.SEED))
         c1 = cpu_baseline({"gltf": sm["gltf"], "poses": np.stack([sm["pose"]] * 256), "spp": sm["spp"]}, 2.0)
         line["cpu_baseline"]["small_scene_rays_per_s"] = c1["value"]
-    print(json.dumps(line), flush=True)
+    print("details: " + json.dumps(line))
+    print(json.dumps(headline(line)), flush=True)
     if world > 1:
         torch.distributed.destroy_process_group()
 

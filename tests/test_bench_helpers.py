@@ -49,3 +49,18 @@ def test_rmse_per_channel():
     a[..., 2] = -0.1
     r = bench.rmse_per_channel(a, ref)
     assert np.allclose(r, [0.3, 0.0, 0.1])
+
+
+def test_the_result_line_is_short():
+    """The last line holds the result and no more, whatever was measured."""
+    import json
+
+    keys = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling",
+            "vs_baseline", "dtype", "data", "e2e", "gpu_launches")
+    line = dict.fromkeys(keys, 1.0)
+    line["config"] = bench.bench_config({"n_omm": 6000, "spp": 256, "triangles": 588288}, 1024)
+    line["clocks"] = {"sm_mhz": 2070.0, "sm_max_mhz": 2070.0, "reasons": []}
+    line["learned_allocator"] = {"table": list(range(5000))}
+    short = bench.headline(line)
+    assert all(short[k] == line[k] for k in keys + ("config", "clocks"))
+    assert len(json.dumps(short)) < 1500
