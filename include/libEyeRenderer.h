@@ -156,7 +156,9 @@ int renderBatch(const int* cams, size_t nCams, size_t posesPerCam, const float* 
 
 /* Diagnostic: renders `count` device poses (layout of crRenderPosesDevice)
  * of the current eye and reports the mean BVH node visits and triangle tests
- * per ray.  Advances the random streams like a render.  0 on success. */
+ * per ray of a search of the tree (long renders go through cone lists instead,
+ * with the same results and fewer visits).  Advances the random streams like
+ * a render.  0 on success. */
 int crMeasureTraversal(const float* d_poses, size_t count, double* nodesPerRay, double* trisPerRay);
 
 /* Autotuner: times every variant of the render kernel on `count` device
@@ -230,7 +232,10 @@ int crGetProjectionSearch(void);
  * crSetDeviceMemoryCap: device bytes the library's buffers may hold in
  * total (0: no cap, the default); an allocation past it fails like an
  * out-of-memory cudaMalloc: the call returns its error sentinel and the
- * library stays usable.  crGetDeviceMemoryHeld: the bytes they hold now.
+ * library stays usable.  What only makes renders faster (cone lists, also
+ * those of batches, the buffers of launches of more than 256 poses, what the
+ * spherical projections keep) counts as held, but is given back before an
+ * allocation fails.  crGetDeviceMemoryHeld: the bytes they hold now.
  * crSelfTestBoundedWait: runs the tcgen05 kernels' bounded mbarrier wait on
  * a barrier that nothing arrives on, for `polls` polls; 1 when the wait ran
  * out and reported it through the error word (then cleared), 0 when it did
@@ -361,7 +366,9 @@ int crAdaptiveLastPass(float* prediction, float* cost, uint8_t* level, size_t ro
  * bursts of `steps` BVH steps; between bursts its idle lanes take new samples
  * once at least refillIdle (1..32) of its 32 lanes are idle (32 = whole
  * rounds of 32 rays, no refill).  Defaults 16 and 16.  Results do not depend
- * on it (each entry's samples are summed in a fixed order).  0 on success. */
+ * on it (each entry's samples are summed in a fixed order).  Entries of 16
+ * samples and more of a long render go through cone lists, in whole rounds:
+ * the schedule and the occupancy below are for the others.  0 on success. */
 int crSetAdaptiveSchedule(int refillIdle, int steps);
 int crGetAdaptiveSchedule(int* refillIdle, int* steps);
 /* No counterpart in the reference.  Occupancy of the adaptive render's kernel
