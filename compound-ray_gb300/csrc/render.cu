@@ -2788,12 +2788,15 @@ cudaError_t launchFeatures(const DevScene& scene, const DevEye& eye, const float
   if (plan.chunks != 1) return cudaErrorInvalidValue;  // feature renders use at most 32 samples
   if (!eye.netDraws) return cudaErrorInvalidValue;  // feature renders draw from shifted nets
   // Counter-based draws: spread the poses over enough warps for about a
-  // dozen waves, so that the last one costs little; twice that where rays
+  // dozen waves, so that the last one costs little; twice that where many rays
   // search a deep tree from its root, whose longest warps take several times
-  // the mean (16 poses of 30,000 ommatidia on the terrain: the adaptive render
-  // 2.04 ms against 2.09; on the box scene 1.204 against 1.195, and through
-  // lists 0.819 against 0.807, so not there).
-  const bool deep = !eye.cones && scene.triCount >= kConeDeepTris;
+  // the mean.  Adaptive renders of the terrain with hardly any rays but these,
+  // 8 samples, against the same without the second factor: 384,000 to 512,000
+  // entries 1.01-1.06x (30,000 ommatidia x 16 poses 839 -> 791 us), 20,000 to
+  // 128,000 entries 0.98-1.01x, so not there; on the box scene 0.99x, and
+  // through lists 0.985x.
+  const uint64_t rays = static_cast<uint64_t>(eye.N) * eye.spp * P;
+  const bool deep = !eye.cones && scene.triCount >= kConeDeepTris && rays >= 1ull << 21;
   plan = splitPoses(plan, P, (deep ? 8 : 4) * kFillWarps);
   if (eye.cones) {
     if (featureConeLists(scene, eye.N, eye.spp, P) == 0) return cudaErrorInvalidValue;
