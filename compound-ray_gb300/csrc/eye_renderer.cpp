@@ -706,18 +706,18 @@ struct Renderer {
     // be had.  No long launches under a memory cap, whose room is for others.
     size_t perLaunch = usual;
     float4* x = nullptr;
-    if (!capturing()) {
-      const size_t fit = conePoses(de.N), rays = std::max<size_t>(1, static_cast<size_t>(de.N) * de.spp);
-      size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, count});
-      if (coneLists(de, std::min(most, fit), rec, stats)) most = std::min(most, fit);
-      if (plain && !devCap() && most > usual) {
+    const size_t fit = conePoses(de.N), rays = std::max<size_t>(1, static_cast<size_t>(de.N) * de.spp);
+    size_t most = std::min<size_t>({kMaxSmallPosesPerLaunch, kSmallLaunchRays / rays, count});
+    if (coneLists(de, std::min(most, fit), rec, stats)) most = std::min(most, fit);
+    if (!plain || devCap()) most = 0;
+    const size_t some = std::min<size_t>(usual, fit);
+    const bool lists = coneLists(de, some, rec, stats) != 0;
+    if ((most > usual || lists) && !capturing()) {
+      if (most > usual) {
         const size_t n = extraFor(de, most, rec, stats, plain).total;
         if (!n || (x = takeExtra(n))) perLaunch = most;
       }
-      const size_t some = std::min<size_t>(usual, fit);
-      if (perLaunch == usual && coneLists(de, some, rec, stats) &&
-          (x = takeExtra(extraFor(de, some, rec, stats, plain).total)))
-        perLaunch = some;
+      if (perLaunch == usual && lists && (x = takeExtra(extraFor(de, some, rec, stats, plain).total))) perLaunch = some;
     }
     for (size_t first = 0; first < count; first += perLaunch) {
       const uint32_t P = static_cast<uint32_t>(std::min<size_t>(perLaunch, count - first));
