@@ -692,7 +692,7 @@ struct Renderer {
   // no other.
   void renderLaunches(DevEye de, const float4* d_poses, size_t count, float* d_out, RayRecord* rec,
                       unsigned long long* stats, DevBuf<float>& scr, bool plain, float maxRel) {
-    if (!count) return;
+    if (!count || !de.N) return;
     const ExtraUse use{*this};
     uint32_t* errFlag = errWord();
     const uint32_t usual = static_cast<uint32_t>(std::min<size_t>(kMaxPosesPerLaunch, count));

@@ -878,3 +878,18 @@ def test_recorded_frames_through_lists(lib, small, deep, pose):
     total = rec["rgb"].sum(1, dtype=np.float64) / spp
     ok = np.isfinite(got[0])
     assert np.allclose(total[ok], got[0][ok], rtol=1e-4, atol=1e-6)
+
+
+def test_renders_of_an_empty_eye(lib, small):
+    """No ommatidia: every render succeeds and writes nothing."""
+    import torch
+
+    _load(lib, small)
+    d_poses = torch.from_numpy(_poses(small, 300, 1)).cuda()
+    out = torch.full((300,), -1.0, device="cuda")
+    torch.cuda.synchronize()
+    lib.setOmmatidia(None, 0)
+    for P in (1, 4, 300):
+        assert lib.crRenderPosesDevice(d_poses.data_ptr(), P, out.data_ptr()) == 0, eh.lastError(lib)
+    assert lib.crSynchronize() == 0
+    assert (out.cpu().numpy() == -1.0).all()
