@@ -1363,11 +1363,17 @@ __device__ __forceinline__ v3 shadeMiss(int miss, v3 dirIn) {
 // Unlit colour of a ray's hit or miss, with the hit's barycentrics (0 for a
 // miss).
 __device__ __forceinline__ v3 shadeRay(const DevScene& sc, const Hit& h, v3 dir, float& b1, float& b2) {
-  b1 = b2 = 0.f;
-  if (h.id == 0xffffffffu) return shadeMiss(sc.miss, dir);
-  b1 = xdiv(h.V, h.det);
-  b2 = xdiv(h.W, h.det);
-  return shadeHit(sc, h.pos, b1, b2);
+  v3 c;
+  b1 = 0.f;
+  b2 = 0.f;
+  if (h.id != 0xffffffffu) {
+    b1 = xdiv(h.V, h.det);
+    b2 = xdiv(h.W, h.det);
+    c = shadeHit(sc, h.pos, b1, b2);
+  } else {
+    c = shadeMiss(sc.miss, dir);
+  }
+  return c;
 }
 
 __device__ __forceinline__ void putRecord(RayRecord& R, float nd, float ud, v3 org, v3 dir, const Hit& h, float b1,
@@ -1849,16 +1855,9 @@ __device__ __forceinline__ void renderTask(const DevScene& sc, const DevEye& eye
         else
           traceClosest<kCount>(sc, ray, fpo, 1e16f, h, errFlag, nodeVisits, triTests);
       }
-      v3 c;
-      float b1 = 0.f, b2 = 0.f;
-      if (h.id != 0xffffffffu) {
-        b1 = xdiv(h.V, h.det);
-        b2 = xdiv(h.W, h.det);
-        c = shadeHit(sc, h.pos, b1, b2);
-        if (kLit) c = shadeLit(sc, h, b1, b2, dir, c, errFlag);
-      } else {
-        c = shadeMiss(sc.miss, dir);
-      }
+      float b1, b2;
+      v3 c = shadeRay(sc, h, dir, b1, b2);
+      if (kLit && h.id != 0xffffffffu) c = shadeLit(sc, h, b1, b2, dir, c, errFlag);
       if (kRecord && valid)
         putRecord(rec[(static_cast<size_t>(p) * eye.N + o) * eye.spp + s], nd, ud, org, dir, h, b1, b2, c);
       if (!kCone || valid) col = c * invSpp;
